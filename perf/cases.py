@@ -430,6 +430,21 @@ def scalar(fn, x):
     return float(fn(torch.tensor([x], dtype=torch.float64))[0])
 
 
+def halves(a):
+    """a as a sum of two numbers of 26 bits each, so that products of halves are exact."""
+    c = a * 134217729.0
+    h = c - (c - a)
+    return h, a - h
+
+
+def turn(t, f):
+    """2 pi times the fraction of t f: the turns of a time shift of seconds, with no rounding of their whole part."""
+    a, b = halves(torch.full_like(f, t))
+    c, d = halves(f)
+    p = [a * c, a * d, b * c, b * d]
+    return 2 * PI * sum(x - torch.round(x) for x in reversed(p))
+
+
 def wave_d(p, f):
     """h+ and hx of IMRPhenomD, t_c and the phase at f_ref as the framework's defaults set them."""
     d = PhenomD(p)
@@ -438,7 +453,7 @@ def wave_d(p, f):
     y = (d.x3 - a5 * d.xr) / d.xd
     shift = M / d.eta * (d.a1fit + a2 / d.x3 ** 2 + a3 / d.x3 ** 0.25 + a4 / (d.xd * (1 + y * y)))
     x = M * f
-    ph = d.phase(x) - ((2 * PI * p["tc"] + shift) * (f - fref) + 2 * p["phiRef"] + scalar(d.phase, M * fref))
+    ph = d.phase(x) - (turn(p["tc"], f - fref) + shift * (f - fref) + 2 * p["phiRef"] + scalar(d.phase, M * fref))
     amp = torch.where(x > d.cut, 0.0, d.A0 * M ** (7 / 6) * x ** (-7.0 / 6) * d.amplitude(x))
     h = torch.polar(amp.abs(), -ph) * torch.sign(amp)
     c = np.cos(p["incl_angle"])
@@ -539,7 +554,7 @@ def wave_p(p, f):
         hp = hp + a + b
         hc = hc + 1j * (a - b)
     amp = torch.where(x > d.cut, 0.0, d.A0 * M ** (7 / 6) / (4 * np.sqrt(5 / (64 * PI))) * x ** (-7.0 / 6) * d.amplitude(x))
-    phase = d.phase(x) + 2 * ep - 2 * PI * p["tc"] * (f - p["f_ref"]) + 2 * ph + 2 * PI * t_corr * f
+    phase = d.phase(x) + 2 * ep - turn(p["tc"], f - p["f_ref"]) + 2 * ph + 2 * PI * t_corr * f
     h = torch.polar(torch.ones_like(f), -phase) * amp
     hp, hc = hp * h, hc * h
     cz, sz = np.cos(2 * zeta), np.sin(2 * zeta)
