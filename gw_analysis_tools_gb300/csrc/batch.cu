@@ -58,16 +58,27 @@ static int choose_occ(gwgpu_context *c, int mixed, const std::string &key) {
   return gwk::batch_default_occ(1);
 }
 
-static int persistent_grid(int device, int mixed, int ndet, int occ) {
-  static int cache[2][gwt::kMaxDet + 1][5] = {{{0}}};
-  int &g = cache[mixed ? 1 : 0][ndet][occ & 3];
+enum { kFormFp64 = 0, kFormMixed = 1, kFormAcc = 2 };  // FP64 bins, mixed, FP64 form on two-float bins
+
+static int persistent_grid(int device, int form, int ndet, int occ) {
+  static int cache[3][gwt::kMaxDet + 1][5] = {{{0}}};
+  int &g = cache[form][ndet][occ & 3];
   if (g) return g;
   cudaDeviceProp p;
   cudaGetDeviceProperties(&p, device);
-  int per_sm = gwk::batch_occupancy(mixed, ndet, occ);
+  int per_sm = form == kFormAcc ? gwk::batch_acc_occupancy(ndet) : gwk::batch_occupancy(form, ndet, occ);
   if (per_sm < 1) per_sm = 1;
   g = p.multiProcessorCount * per_sm;
   return g;
+}
+
+// Bins per item of the two-float form: about three items per resident block,
+// so that the last ones end together, in whole passes; at most 16 passes (a
+// thread's two-float sums keep their digits) and an item's fixed cost (staging
+// and reduction, about one pass) stays small.
+static int acc_tile(long long bins, int slots) {
+  const long long t = bins / (3LL * std::max(slots, 1)) / 256 * 256;
+  return (int)std::min(4096LL, std::max(256LL, t));
 }
 
 static char *align256(char *p) { return (char *)(((uintptr_t)p + 255) & ~(uintptr_t)255); }
@@ -161,21 +172,16 @@ int plan_batch(gwgpu_context *c, Lane &L, int n, const int *handles, int ndet, i
 }
 
 static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, const int *d_approx, int n,
-                           int ndet, double T_segment, int mixed, int occ, double *d_out, int *d_status,
+                           int ndet, double T_segment, int form, int occ, double *d_out, int *d_status,
                            int *status_out, void *reqs, double *partials, unsigned *cnt) {
   const Plan &pl = L.plan;
   const bool timing = c->timing && &L == &c->lane;
   if (timing) cudaEventRecord(c->t_ev[0], L.stream);
   cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (size_t)(n + 32 + gwk::kOrderBuckets), L.stream);
   if (e != cudaSuccess) return c->fail(e, "batch counters");
-  // mixed form: the prologue writes the work order (most live bins first)
-  const bool ordered = mixed && c->order_items && !c->prologue_serial;
-  // FP64 form: the cooperative prologue writes each IMRPhenomD request's
-  // coefficients on the grid after the Request records, for the bin
-  // kernel's table form (with the FP64 n^(-7/6) table)
-  gwt::WaveF64 *w64 = nullptr;
-  if (!mixed && !c->prologue_serial && c->tm76d && c->tm76d_n > 0)
-    w64 = (gwt::WaveF64 *)((char *)reqs + sizeof(gwt::Request) * (size_t)n);
+  // mixed and two-float forms: the prologue writes the work order
+  const bool ordered = form != kFormFp64 && c->order_items && !c->prologue_serial;
+  const int mixed = form == kFormMixed;
   gwk::OrderArgs ord;
   if (ordered) {
     ord.fill = (int *)(cnt + n + 32);
@@ -187,16 +193,18 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   }
   if (c->prologue_serial)
     e = gwk::launch_prologue_serial((const gwt::GenParams *)d_params, d_approx, n, pl.handles, ndet, T_segment, 1,
-                                    c->streams_dev, c->qnm_dev, mixed ? nullptr : (gwt::Request *)reqs,
-                                    mixed ? (gwt::MixedReq *)reqs : nullptr, mixed, d_status, L.stream);
+                                    c->streams_dev, c->qnm_dev, form == kFormFp64 ? (gwt::Request *)reqs : nullptr,
+                                    mixed ? (gwt::MixedReq *)reqs : nullptr,
+                                    form == kFormAcc ? (gwt::AccReq *)reqs : nullptr, mixed, d_status, L.stream);
   else
     e = gwk::launch_prologue((const gwt::GenParams *)d_params, d_approx, n, pl.handles, ndet, T_segment, 1,
-                             c->streams_dev, c->qnm_dev, mixed ? nullptr : (gwt::Request *)reqs,
-                             mixed ? (gwt::MixedReq *)reqs : nullptr, mixed, d_status, L.stream, ord, w64);
+                             c->streams_dev, c->qnm_dev, form == kFormFp64 ? (gwt::Request *)reqs : nullptr,
+                             mixed ? (gwt::MixedReq *)reqs : nullptr, mixed, d_status, L.stream, ord,
+                             form == kFormAcc ? (gwt::AccReq *)reqs : nullptr);
   if (e != cudaSuccess) return c->fail(e, "prologue launch");
   if (timing) cudaEventRecord(c->t_ev[1], L.stream);
   gwk::BatchArgs a;
-  a.req = mixed ? nullptr : (const gwt::Request *)reqs;
+  a.req = form == kFormFp64 ? (const gwt::Request *)reqs : nullptr;
   a.mreq = mixed ? (const gwt::MixedReq *)reqs : nullptr;
   a.handles = pl.handles;
   a.ndet = ndet;
@@ -215,12 +223,13 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   a.status = d_status;
   a.status_out = status_out ? status_out : d_status;
   a.tables = c->tables;
-  a.w64 = w64;
-  a.tm76d = w64 ? c->tm76d : nullptr;
-  a.tm76d_n = w64 ? c->tm76d_n : 0;
-  int grid = std::min(pl.nitems, persistent_grid(c->device, mixed, ndet, occ));
+  a.areq = form == kFormAcc ? (const gwt::AccReq *)reqs : nullptr;
+  a.acc = c->acc;
+  a.lut = c->acc_lut;
+  int grid = std::min(pl.nitems, persistent_grid(c->device, form, ndet, occ));
   if (grid < 1) grid = 1;
-  e = gwk::launch_batch(a, mixed, grid, occ, L.stream, c->pdl);
+  if (form == kFormAcc) e = gwk::launch_batch_acc(a, grid, L.stream, c->pdl);
+  else e = gwk::launch_batch(a, mixed, grid, occ, L.stream, c->pdl);
   if (&L == &c->lane) {
     c->last_shape[0] = pl.tile;
     c->last_shape[1] = occ;
@@ -251,12 +260,21 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
     L.shape.ndet = ndet;
     L.shape.epoch = c->streams_epoch;
     L.shape.mixed = mixed;
+    L.shape.acc = !mixed && c->acc_lut;
+    L.shape.bins = 0;
+    for (size_t i = 0; i < nh; i++) {
+      const gwgpu_context::Stream *s = c->get_stream(h_handles[i]);
+      L.shape.acc = L.shape.acc && s && s->dev.wd && s->dev.n0 + s->dev.N - 1 <= c->acc.nmax;
+      if (s && i % ndet == 0) L.shape.bins += s->dev.N;
+    }
   }
-  if (tile <= 0) tile = choose_tile(c, mixed, L.tk);
+  const int form = mixed ? kFormMixed : L.shape.acc ? kFormAcc : kFormFp64;
+  if (tile <= 0) {
+    tile = choose_tile(c, mixed, L.tk);
+    if (form == kFormAcc && c->tile_override <= 0 && !c->tuned.count(L.tk))
+      tile = acc_tile(L.shape.bins, persistent_grid(c->device, kFormAcc, ndet, 0));
+  }
   const int occ = choose_occ(c, mixed, L.tk);
-  // FP64 batches: the n^(-7/6) table of the table form, built before any
-  // capture (a failure leaves the frequency form)
-  if (!mixed && c->ensure_tm76d(c->tables.nmax) != GWGPU_OK) c->last_error.clear();
   bool replanned = false;
   if (!same || !L.plan.valid || L.plan.tile != tile) {
     int st = plan_batch(c, L, n, h_handles, ndet, tile);
@@ -267,7 +285,7 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
     L.plan.valid = true;
     replanned = true;
   }
-  size_t rq = mixed ? sizeof(gwt::MixedReq) : sizeof(gwt::Request) + sizeof(gwt::WaveF64);
+  size_t rq = mixed ? sizeof(gwt::MixedReq) : form == kFormAcc ? sizeof(gwt::AccReq) : sizeof(gwt::Request);
   size_t bytes = rq * n + 512 + sizeof(double) * (size_t)L.plan.nitems * gwk::kAcc + 256 +
                  sizeof(unsigned) * (size_t)(n + 32 + gwk::kOrderBuckets);
   void *old = L.work;
@@ -279,13 +297,13 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
   }
   char *p = (char *)L.work;
   void *reqs = p;
-  p = align256(p + rq * n);  // FP64: Request[n], then WaveF64[n] (below)
+  p = align256(p + rq * n);
   double *partials = (double *)p;
   p = align256(p + sizeof(double) * (size_t)L.plan.nitems * gwk::kAcc);
   unsigned *cnt = (unsigned *)p;
   auto sequence = [&]() {
     if (io) cudaMemcpyAsync(io->h2d_dst, io->h2d_src, io->h2d_bytes, cudaMemcpyHostToDevice, L.stream);
-    int r = launch_sequence(c, L, d_params, d_approx, n, ndet, T_segment, mixed, occ, d_out, d_status, status_out,
+    int r = launch_sequence(c, L, d_params, d_approx, n, ndet, T_segment, form, occ, d_out, d_status, status_out,
                             reqs, partials, cnt);
     if (!r && io) cudaMemcpyAsync(io->d2h_dst, io->d2h_src, io->d2h_bytes, cudaMemcpyDeviceToHost, L.stream);
     return r;
@@ -293,7 +311,7 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
   if (!use_graph || c->timing) return sequence();
   char gk[320];
   snprintf(gk, sizeof(gk), "%p|%p|%p|%p|%p|%d|%d|%.17g|%d|%p|%p|%zu|%p|%p|%zu", (const void *)d_params,
-           (const void *)d_approx, (const void *)d_out, (const void *)d_status, (const void *)status_out, mixed, occ,
+           (const void *)d_approx, (const void *)d_out, (const void *)d_status, (const void *)status_out, form, occ,
            T_segment, n,
            io ? io->h2d_src : nullptr, io ? io->h2d_dst : nullptr, io ? io->h2d_bytes : 0,
            io ? io->d2h_dst : nullptr, io ? (const void *)io->d2h_src : nullptr, io ? io->d2h_bytes : 0);

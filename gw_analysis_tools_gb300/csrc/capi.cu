@@ -171,6 +171,47 @@ int gwgpu_context::ensure_tm76d(int nmax) {
   return GWGPU_OK;
 }
 
+int gwgpu_context::ensure_acc(int nmax) {
+  int st = ensure_tables(nmax);
+  if (st) return st;
+  if (!acc_lut) {
+    std::vector<gwt::AccLut> h(1);
+    gwt::ff_fill_tables(h[0].turn, h[0].ex);
+    void *p;
+    if ((st = dalloc(&p, sizeof(gwt::AccLut), "sine table"))) return st;
+    cudaError_t e = cudaMemcpy(p, h.data(), sizeof(gwt::AccLut), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail(e, "sine table");
+    acc_lut = (gwt::AccLut *)p;
+  }
+  if (nmax <= acc.nmax) return GWGPU_OK;
+  const size_t n1 = (size_t)std::max(nmax, std::min(tables.nmax, std::max(2 * acc.nmax, 1 << 16))) + 1;
+  void *p;
+  if ((st = dalloc(&p, 80 * n1, "two-float tables"))) return st;
+  gwt::AccTables t;
+  gwt::ff4 *q = (gwt::ff4 *)p;
+  t.pw = q;
+  t.ph = q + n1;
+  t.pv = q + 2 * n1;
+  double *v = (double *)(q + 3 * n1);
+  const double *src[4] = {tables.t13, tables.tm53, tables.tln, tables.t34};
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < 4 && e == cudaSuccess; i++)
+    e = cudaMemcpyAsync(v + i * n1, src[i], 8 * n1, cudaMemcpyDeviceToDevice, stream);
+  t.t13 = v;
+  t.tm53 = v + n1;
+  t.tln = v + 2 * n1;
+  t.t34 = v + 3 * n1;
+  t.nmax = (int)n1 - 1;
+  if (e == cudaSuccess) e = gwk::launch_acc_tables(t, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) {
+    dfree(p);
+    return fail(e, "two-float tables");
+  }
+  acc = t;
+  return GWGPU_OK;
+}
+
 int gwgpu_context::sync_streams_table() {
   size_t bytes = sizeof(StreamDev) * std::max<size_t>(streams.size(), 1);
   if (streams_dev_cap < streams.size() || !streams_dev) {
@@ -292,6 +333,40 @@ void *gwgpu_context_stream(gwgpu_context *c) { return c ? (void *)c->stream : nu
 size_t gwgpu_context_bytes_in_use(gwgpu_context *c) { return c ? c->in_use : 0; }
 
 // ------------------------------------------------------------ data registry
+// The two-float pairs of a registered stream with finite weights on a uniform
+// grid (FP64 form, phenom_acc.h).  Without the memory for them the stream
+// keeps the FP64 bins.
+static void acc_stream(gwgpu_context *c, gwgpu_context::Stream &s, const double *freqs) {
+  StreamDev &d = s.dev;
+  if ((long long)d.n0 + d.N > gwt::kAccMaxN || c->ensure_acc(d.n0 + d.N) != GWGPU_OK) {
+    c->last_error.clear();
+    return;
+  }
+  // f_k = (n0 + k) dfq to the last bit when the product is exact (dfq with 24
+  // zero bits at its end) and equal; a grid that is not carries its distances
+  int ex;
+  const double mant = std::ldexp(std::frexp(d.dfq, &ex), 29);
+  bool exact = mant == std::floor(mant);
+  for (int k = 0; k < d.N && exact; k++) exact = (double)(d.n0 + k) * d.dfq == freqs[k];
+  void *p;
+  if (c->dalloc(&p, (exact ? 24 : 28) * (size_t)d.N, "two-float stream") != GWGPU_OK) {
+    c->last_error.clear();
+    return;
+  }
+  StreamDev t = d;
+  t.wd = (const gwt::ff4 *)p;
+  t.wf = (const gwt::ff *)(t.wd + d.N);
+  t.dev = exact ? nullptr : (const float *)(t.wf + d.N);
+  cudaError_t e = gwk::launch_acc_stream(t, !exact, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) {
+    c->dfree(p);
+    return;
+  }
+  d = t;
+  s.mem.push_back(p);
+}
+
 // One detector stream; weights (GAUSSLEG) or null (Simpson's rule).
 static int register_stream(gwgpu_context *c, const char *detector, const double *freqs, int N, const double *data,
                            const double *psd, const double *weights, int log10F, int *handle) {
@@ -316,6 +391,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     if (std::fabs(freqs[k] - (freqs[0] + k * d.df)) > 1e-9 * d.df * (1 + k)) uniform = false;
   double n0f = freqs[0] / d.df;
   d.n0 = (int)std::llround(n0f);
+  d.dfq = (freqs[N - 1] - freqs[0]) / (N - 1);
   d.uniform_int = uniform && d.n0 >= 1 && std::fabs(n0f - d.n0) < 1e-6 && (d.n0 + (double)N) < 1.5e9;
   // integration weights: Simpson's rule, (4 df/3) s_k (util.h:844-856), or the
   // GAUSSLEG branch, 4 w_k (times f_k ln 10 for log10F) (mcmc_gw.cpp:820-862);
@@ -327,8 +403,10 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     iw[k] = weights ? 4.0 * weights[k] * (log10F ? freqs[k] * std::log(10.) : 1.0) : c3 * sw;
   }
   double wmax = 0, dmax = 0;
+  bool finite = true;
   for (int k = 0; k < N; k++) {
     W[k] = iw[k] / psd[k];
+    finite = finite && std::isfinite(W[k] * data[2 * k]) && std::isfinite(W[k] * data[2 * k + 1]);
     if (std::isfinite(W[k])) wmax = std::max(wmax, std::fabs(W[k]));
     double m = std::fabs(W[k] * data[2 * k]) + std::fabs(W[k] * data[2 * k + 1]);
     if (std::isfinite(m)) dmax = std::max(dmax, m);
@@ -342,14 +420,14 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     wh[k] = (float)(W[k] / d.wscale);
   }
   int st;
-  void *pf, *pd, *pp, *pip, *pdh, *pwh, *piw = nullptr;
   std::vector<double> ip(N);  // the reciprocal PSD: the FP64 kernels multiply instead of dividing
   for (int k = 0; k < N; k++) ip[k] = 1.0 / psd[k];
-  if ((st = c->dalloc(&pf, 8 * (size_t)N, "freqs")) || (st = c->dalloc(&pd, 16 * (size_t)N, "data")) ||
-      (st = c->dalloc(&pp, 8 * (size_t)N, "psd")) || (st = c->dalloc(&pip, 8 * (size_t)N, "inverse psd")) ||
-      (st = c->dalloc(&pdh, 8 * (size_t)N, "dhat")) || (st = c->dalloc(&pwh, 4 * (size_t)N, "what")) ||
-      (weights && (st = c->dalloc(&piw, 8 * (size_t)N, "integration weights"))))
-    return st;
+  // one allocation for the stream's arrays, each on a 256-byte boundary
+  const size_t row = ((size_t)N + 31) / 32 * 32;
+  char *mem;
+  if ((st = c->dalloc((void **)&mem, row * (weights ? 60 : 52), "data stream"))) return st;
+  void *pd = mem, *pf = mem + 16 * row, *pp = mem + 24 * row, *pip = mem + 32 * row, *pdh = mem + 40 * row,
+       *pwh = mem + 48 * row, *piw = weights ? mem + 52 * row : nullptr;
   cudaMemcpyAsync(pip, ip.data(), 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
   if (piw) cudaMemcpyAsync(piw, iw.data(), 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(pf, freqs, 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
@@ -358,7 +436,10 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   cudaMemcpyAsync(pdh, dh.data(), 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(pwh, wh.data(), 4 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
   cudaError_t e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return c->fail(e, "data upload");
+  if (e != cudaSuccess) {
+    c->dfree(mem);
+    return c->fail(e, "data upload");
+  }
   d.freqs = (const double *)pf;
   d.data = (const double *)pd;
   d.psd = (const double *)pp;
@@ -367,8 +448,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   d.what = (const float *)pwh;
   d.iw = (const double *)piw;
   s.live = true;
-  s.mem = {pf, pd, pp, pip, pdh, pwh};
-  if (piw) s.mem.push_back(piw);
+  s.mem = {mem};
   s.host_freqs.assign(freqs, freqs + N);
   uint64_t hsh = 1469598103934665603ull;
   const unsigned char *pb = (const unsigned char *)psd;
@@ -388,6 +468,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   if (d.uniform_int) {
     st = c->ensure_tables(d.n0 + N);
     if (st) return st;
+    if (finite) acc_stream(c, s, freqs);
   }
   c->streams.push_back(s);
   *handle = (int)c->streams.size() - 1;
@@ -561,19 +642,7 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   if (st) return st;
   cudaError_t e = cudaHostGetDevicePointer((void **)&hd, h, 0);
   if (e != cudaSuccess) return c->fail(e, "plain result mapping");
-  // IMRPhenomD on uniform grids: the waveform from the request's coefficients
-  // on the grid and the power tables
-  gwk::PlainTab pt;
-  bool uni = ap == gwt::kPhenomD && !r.m.status && sd[0].n0 >= 1;
-  for (int d = 0; d < ndet; d++) uni = uni && sd[d].uniform_int;
-  if (uni && sd[0].n0 + sd[0].N - 1 <= c->tables.nmax && c->ensure_tm76d(sd[0].n0 + sd[0].N - 1) == GWGPU_OK &&
-      sd[0].n0 + sd[0].N - 1 <= c->tm76d_n) {
-    gwt::wave64_prologue(r, sd[0].df, pt.w);
-    pt.t = c->tables;
-    pt.tm76d = c->tm76d;
-    pt.use = 1;
-  }
-  e = gwk::launch_plain(r, sd, ndet, part, cnt, hd, nullptr, c->stream, &pt);
+  e = gwk::launch_plain_any(r, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream);
   if (e != cudaSuccess) return c->fail(e, "plain launch");
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return c->fail(e, "plain");

@@ -40,6 +40,11 @@ struct gwgpu_context {
   double *qnm_dev = nullptr;
   gwt::Tables tables{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
   std::vector<void *> table_mem;
+  // FP64 form on two-float bins: tables by n and the sine/exp tables.  Grown
+  // blocks stay allocated until the context goes (a launch captured by the
+  // caller may hold their addresses); each is at least twice the one before.
+  gwt::AccTables acc{};
+  gwt::AccLut *acc_lut = nullptr;
   double *tm76d = nullptr;  // FP64 n^(-7/6), built on first Fisher use
   int tm76d_n = 0;
   std::vector<Stream> streams;
@@ -77,6 +82,7 @@ struct gwgpu_context {
   int pinned(int slot, size_t bytes, void **out);
   int ensure_tables(int nmax);
   int ensure_tm76d(int nmax);
+  int ensure_acc(int nmax);
   int sync_streams_table();
   const Stream *get_stream(int handle) const;
   unsigned *counter(int i);

@@ -2,8 +2,8 @@
 //
 //   k_waveform / k_response   fourier_waveform / fourier_detector_response arrays (FP64)
 //   k_inner                   Log_Likelihood_internal on given arrays (FP64 Simpson)
-//   k_plain                   the drop-in: one request per launch, FP64, fused
-//                             waveform -> projection -> Simpson inner product
+//   k_plain                   one request per launch, FP64 bins from their frequency: grids
+//                             and streams that acc.cu's two-float bins do not take
 //   k_prologue                batched per-request FP64 prologue, one thread per request
 //   k_batch<fp64|mixed>       persistent fused bin kernel over (request, bin tile) items
 //
@@ -13,6 +13,7 @@
 #include <cstdint>
 #include <cstdio>
 
+#include "kernel_util.cuh"
 #include "kernels.h"
 
 namespace gwk {
@@ -23,12 +24,6 @@ struct PlainStreams {
 };
 
 __device__ __forceinline__ double2 to_d2(cd a) { return make_double2(a.re, a.im); }
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // Block-wide FP64 sums of NV values per thread; result valid in thread 0.
 // smem must hold 32 * NV doubles.
@@ -81,21 +76,6 @@ cudaError_t launch_response(const Request &r, int slot, int apply_shift, const d
   int block = 128, grid = (N + block - 1) / block;
   k_response<<<grid, block, 0, s>>>(r, slot, apply_shift, freqs, N, (double2 *)out);
   return cudaGetLastError();
-}
-
-// ------------------------------------------------ last-block finalisation
-// Returns true in every thread of the block that finished last.
-__device__ __forceinline__ bool arrive_last(unsigned *counter, unsigned expected) {
-  __shared__ bool s_last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    unsigned prev = atomicAdd(counter, 1u);
-    s_last = (prev == expected - 1);
-  }
-  __syncthreads();
-  if (s_last) __threadfence();
-  return s_last;
 }
 
 // ------------------------------------------------------ Simpson inner product
@@ -167,51 +147,6 @@ __device__ __forceinline__ void fp64_bin(const Request &r, const StreamDev *st, 
     v[2 * d + 1] += w * ((dd.x * x.re + dd.y * x.im) * iS);
   }
 }
-// The same with each detector's arrival-time rotation e^{i tau_d f} given
-// (rc, rs): the batched kernel builds it on uniform grids as the product of a
-// per-pass and a per-thread factor instead of one sincos per detector-bin.
-template <int NDET>
-__device__ __forceinline__ void fp64_acc_rot(const Request &r, const StreamDev *st, int k, int N, cd hp, cd hc,
-                                             const double *rc, const double *rs, double (&v)[2 * NDET]) {
-  const double ws = simpson_weight(k, N);
-#pragma unroll
-  for (int d = 0; d < NDET; d++) {
-    const cd y = response_bin(r.det[d], hp, hc, 0.0, false);  // the frequency enters through (rc, rs)
-    const cd x{y.re * rc[d] - y.im * rs[d], y.re * rs[d] + y.im * rc[d]};
-    double2 dd = ((const double2 *)st[d].data)[k];
-    const double iS = st[d].ipsd ? st[d].ipsd[k] : 1.0 / st[d].psd[k];
-    const double w = st[d].iw ? st[d].iw[k] : ws;
-    v[2 * d] += w * ((x.re * x.re + x.im * x.im) * iS);
-    v[2 * d + 1] += w * ((dd.x * x.re + dd.y * x.im) * iS);
-  }
-}
-template <int NDET>
-__device__ __forceinline__ void fp64_bin_rot(const Request &r, const StreamDev *st, int k, int N, const double *rc,
-                                             const double *rs, double (&v)[2 * NDET]) {
-  cd hp, hc;
-  wave_bin(r, st[0].freqs[k], hp, hc);
-  fp64_acc_rot<NDET>(r, st, k, N, hp, hc, rc, rs, v);
-}
-// IMRPhenomD at bin n = n0 + k of a uniform grid from the coefficients and
-// tables of PlainTab (d_bin's values to ~1e-12 relative).
-__device__ __forceinline__ void d_bin_tab(const Request &r, const gwt::WaveF64 &x, const gwt::Tables &tb,
-                                          const double *tm76d, int n, double f, cd &hp, cd &hc) {
-  if (n > x.n_cut) {
-    hp = cd{0., 0.};
-    hc = cd{0., 0.};
-    return;
-  }
-  const double t = __ldg(tb.t13 + n), rr = __ldg(tb.tm53 + n), lnn = __ldg(tb.tln + n), t34 = __ldg(tb.t34 + n),
-               m76 = __ldg(tm76d + n);
-  const double amp = x.A_scale * wave64_amp(x, n, t, m76);
-  const double phase = wave64_phase(x, n, t, rr, lnn, t34) - (x.tcl * (f - x.fref) + x.phic);
-  double sn, cs;
-  sincos(phase, &sn, &cs);
-  const cd h{amp * cs, -(amp * sn)};
-  const double ci = r.m.s.cos_incl, fac = r.m.s.fac_incl;
-  hc = cd{h.im * ci, -h.re * ci};
-  hp = cd{h.re * fac, h.im * fac};
-}
 template <int NDET>
 __device__ __forceinline__ double fp64_finalize(const double *s, const StreamDev *st) {
   double ll = 0;
@@ -224,57 +159,16 @@ __device__ __forceinline__ double fp64_finalize(const double *s, const StreamDev
 }
 
 // ------------------------------------------------------------------ plain
-// On uniform grids each block's arrival-time rotations come from a table:
-// thread t = 16 a + b of a block starting at bin k0 takes
-// e^{i tau (f_k0 + t df)} = e^{i tau f_k0} e^{i tau 16 a df} e^{i tau b df},
-// 25 sincos per detector and block (one per thread for the first 25 NDET
-// threads) instead of one per detector-bin.
-constexpr int kPlainRot = 1 + 8 + 16;
 template <int NDET>
 __global__ void __launch_bounds__(128) k_plain(const __grid_constant__ Request r, const __grid_constant__ PlainStreams ps,
-                                               const __grid_constant__ PlainTab pt, double *partials,
-                                               unsigned *counter, double *out, int *status) {
+                                               double *partials, unsigned *counter, double *out, int *status) {
   __shared__ double smem[32 * 2 * NDET];
-  __shared__ double2 s_rot[NDET * kPlainRot];
   const int N = ps.s[0].N;
   double v[2 * NDET];
 #pragma unroll
   for (int j = 0; j < 2 * NDET; j++) v[j] = 0.0;
-  bool uniform = blockDim.x == 128 && (long long)gridDim.x * 128 >= N;  // one bin per thread
-#pragma unroll
-  for (int d = 0; d < NDET; d++) uniform = uniform && ps.s[d].uniform_int;
-  if (uniform) {
-    const int k0 = blockIdx.x * 128;
-    for (int e = threadIdx.x; e < NDET * kPlainRot; e += blockDim.x) {
-      const int d = e / kPlainRot, j = e - d * kPlainRot;
-      const double tau = r.det[d].tau, df = ps.s[0].df;
-      const double arg = j == 0 ? tau * ps.s[0].freqs[min(k0, N - 1)]
-                                : tau * ((j <= 8 ? 16.0 * (j - 1) : (double)(j - 9)) * df);
-      double sn, cs;
-      sincos(arg, &sn, &cs);
-      s_rot[e] = make_double2(cs, sn);
-    }
-    __syncthreads();
-    const int k = k0 + threadIdx.x;
-    if (k < N) {
-      const int a = threadIdx.x >> 4, b = threadIdx.x & 15;
-      double rc[NDET], rs[NDET];
-#pragma unroll
-      for (int d = 0; d < NDET; d++) {
-        const double2 B = s_rot[d * kPlainRot], A = s_rot[d * kPlainRot + 1 + a], C = s_rot[d * kPlainRot + 9 + b];
-        const double xr = B.x * A.x - B.y * A.y, xi = B.x * A.y + B.y * A.x;
-        rc[d] = xr * C.x - xi * C.y;
-        rs[d] = xr * C.y + xi * C.x;
-      }
-      cd hp, hc;
-      if (pt.use) d_bin_tab(r, pt.w, pt.t, pt.tm76d, ps.s[0].n0 + k, ps.s[0].freqs[k], hp, hc);
-      else wave_bin(r, ps.s[0].freqs[k], hp, hc);
-      fp64_acc_rot<NDET>(r, ps.s, k, N, hp, hc, rc, rs, v);
-    }
-  } else {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x)
-      fp64_bin<NDET>(r, ps.s, k, N, v);
-  }
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x)
+    fp64_bin<NDET>(r, ps.s, k, N, v);
   block_sum<2 * NDET>(v, smem);
   if (threadIdx.x == 0)
 #pragma unroll
@@ -302,6 +196,7 @@ cudaError_t plain_preload() {
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain<2>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain<3>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain<4>);
+  if (e == cudaSuccess) e = plain_acc_preload();
   return e;
 }
 int plain_blocks(int N) {
@@ -309,17 +204,15 @@ int plain_blocks(int N) {
   return g < 1 ? 1 : g;
 }
 cudaError_t launch_plain(const Request &r, const StreamDev *streams, int ndet, double *partials, unsigned *counter,
-                         double *out, int *status, cudaStream_t s, const PlainTab *tab) {
+                         double *out, int *status, cudaStream_t s) {
   PlainStreams ps;
   for (int d = 0; d < ndet; d++) ps.s[d] = streams[d];
-  PlainTab pt;
-  if (tab) pt = *tab;
   int grid = plain_blocks(streams[0].N);
   switch (ndet) {
-    case 1: k_plain<1><<<grid, 128, 0, s>>>(r, ps, pt, partials, counter, out, status); break;
-    case 2: k_plain<2><<<grid, 128, 0, s>>>(r, ps, pt, partials, counter, out, status); break;
-    case 3: k_plain<3><<<grid, 128, 0, s>>>(r, ps, pt, partials, counter, out, status); break;
-    case 4: k_plain<4><<<grid, 128, 0, s>>>(r, ps, pt, partials, counter, out, status); break;
+    case 1: k_plain<1><<<grid, 128, 0, s>>>(r, ps, partials, counter, out, status); break;
+    case 2: k_plain<2><<<grid, 128, 0, s>>>(r, ps, partials, counter, out, status); break;
+    case 3: k_plain<3><<<grid, 128, 0, s>>>(r, ps, partials, counter, out, status); break;
+    case 4: k_plain<4><<<grid, 128, 0, s>>>(r, ps, partials, counter, out, status); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -329,7 +222,7 @@ cudaError_t launch_plain(const Request &r, const StreamDev *streams, int ndet, d
 __global__ void k_prologue(const GenParams *__restrict__ params, const int *__restrict__ approx, int n,
                            const int *__restrict__ handles, int ndet, double T_segment, int tc_from_segment,
                            const StreamDev *__restrict__ streams, const double *__restrict__ qnm, Request *req,
-                           MixedReq *mreq, int want_mixed, int *status) {
+                           MixedReq *mreq, AccReq *areq, int want_mixed, int *status) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   GenParams p = params[i];
@@ -350,7 +243,7 @@ __global__ void k_prologue(const GenParams *__restrict__ params, const int *__re
     request_prologue(r, p, ap, dets, ndet, qnm);
     if (r.m.status) st = 4;
     if (req) req[i] = r;
-    if (want_mixed) {
+    if (want_mixed || areq) {
       if (!s0.uniform_int) st = st ? st : 1;
       double ds[kMaxDet], ws[kMaxDet];
       unsigned long long wk[kMaxDet];
@@ -359,14 +252,17 @@ __global__ void k_prologue(const GenParams *__restrict__ params, const int *__re
         ws[d] = streams[handles[i * ndet + d]].wscale;
         wk[d] = streams[handles[i * ndet + d]].wkey;
       }
-      mixed_prologue(r, s0.df, mreq[i], ds, ws);
-      mixed_fold_shared_weights(mreq[i], wk, ndet);
+      if (areq) acc_prologue(r, s0.dfq, areq[i], ds, ws);
+      else mixed_prologue(r, s0.df, mreq[i], ds, ws);
+      mixed_fold_shared_weights(areq ? areq[i].m : mreq[i], wk, ndet);
     }
   } else {
     st = 4;
-    if (want_mixed) mreq[i] = MixedReq{};
+    if (areq) areq[i].m = MixedReq{};
+    else if (want_mixed) mreq[i] = MixedReq{};
   }
-  if (st && want_mixed) mreq[i].status = st;
+  if (st && areq) areq[i].m.status = st;
+  else if (st && want_mixed) mreq[i].status = st;
   if (st && req) req[i].m.status = st;
   status[i] = st;
 }
@@ -396,14 +292,6 @@ __global__ void k_prologue(const GenParams *__restrict__ params, const int *__re
 //   S6  W0 Pv2: detector phases and factors; outputs;  W1-W3 the bin kernel's work order
 // (per-warp clock stamps of each stage guided the split: IMRPhenomD, warm,
 // before this split S3 20.2k / S5 22.2k / S6 13.0k cycles on the longest warp)
-// Programmatic dependent launch: a kernel launched with the programmatic
-// stream-serialisation attribute may start while the one before it on the
-// stream still runs; grid_dep_wait() returns once that kernel has completed
-// and its memory is visible, and grid_dep_trigger() lets the next kernel start
-// launching.  Without the attribute both are no-ops.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // Longest-processing-time-first order for the persistent mixed kernel: an
 // item's work is its live 256-bin passes (bins below the request's cut
 // f <= 0.2/M, where the model is non-zero; beyond it a pass costs nothing), and
@@ -455,7 +343,8 @@ struct CoopSmem {
 // 0 stores the results, warps 1-3 call tail(warp, lane, act, i, kcut) with
 // kcut the end of request i's live bins (0 when it will not be evaluated);
 // tail is warp-collective.
-template <class Sync, class Tail>
+// ACC: the FP64 form's constants (areq) instead of the mixed form's (mreq).
+template <bool ACC, class Sync, class Tail>
 __device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int warp, int lane,
                                                    const GenParams *__restrict__ params,
                                                    const int *__restrict__ approx, int n,
@@ -463,8 +352,12 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int w
                                                    int tc_from_segment, const StreamDev *__restrict__ streams,
                                                    const double *__restrict__ qnm, Request *req, MixedReq *mreq,
                                                    int want_mixed, int *status, Sync sync, Tail tail,
-                                                   gwt::WaveF64 *w64 = nullptr) {
+                                                   AccReq *areq = nullptr) {
   Request *s_r = sm.r;
+  auto mx = [&](int j) -> MixedReq & {
+    if constexpr (ACC) return areq[j].m;
+    else return mreq[j];
+  };
   GenParams *s_p = sm.p;
   AmpConn *s_ac = sm.ac;
   PhaseConnParts *s_pc = sm.pc;
@@ -496,7 +389,7 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int w
     s_p[lane] = q;
     s_st[lane] = st;
     s_bad[lane] = bad;
-    s_df[lane] = s0.df;
+    s_df[lane] = ACC ? s0.dfq : s0.df;
     s_uni[lane] = s0.uniform_int;
     r.approximant = ap;
     r.ndet = ndet;
@@ -611,20 +504,23 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int w
   if (run) {
     if (warp == 3 && pv2) r.p.t_corr = r.m.s.shift_time ? pv2_shift_solve(r.m, s_shift[lane]) : 0.0;
     if (want_mixed) {
-      MixedReq &x = mreq[i];
+      MixedReq &x = mx(i);
       const double df = s_df[lane];
       if (warp == 0) mixed_amp_coeffs(r, df, x);
       if (warp == 1) mixed_phase_coeffs(r, df, x);
+      if constexpr (ACC) {
+        if (warp == 0) acc_amp_coeffs(r, df, areq[i]);
+        if (warp == 1) acc_phase_coeffs(r, df, areq[i]);
+      }
       if (warp == 2) {
         mixed_regions(r, df, x);  // sets x.A_scale
         if (pv2) mixed_pv2_coeffs(r, df, x);
         else mixed_det_factors_a(r, x, x.A_scale, s_ds[lane], s_ws[lane]);
       }
-      if (warp == 3 && !pv2) mixed_det_phase(r, df, x);
-    } else if (w64 && warp == 0 && !pv2 && s_uni[lane]) {
-      // FP64 batches, IMRPhenomD on a uniform grid: the waveform's
-      // coefficients on the grid for the bin kernel's table form
-      wave64_prologue(r, s_df[lane], w64[i]);
+      if (warp == 3 && !pv2) {
+        if constexpr (ACC) acc_det_phase(r, df, areq[i]);
+        else mixed_det_phase(r, df, x);
+      }
     }
   }
   sync();
@@ -637,16 +533,22 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int w
       if (want_mixed) {
         if (!s_uni[lane]) st = st ? st : 1;
         if (r.approximant == kPhenomPv2) {  // needs the time shift of S5
-          mixed_det_phase(r, s_df[lane], mreq[i]);
-          mixed_det_factors(r, mreq[i], s_ds[lane], s_ws[lane]);
+          if constexpr (ACC) {
+            acc_det_phase(r, s_df[lane], areq[i]);
+            acc_pv2_coeffs(r, s_df[lane], areq[i]);
+          } else {
+            mixed_det_phase(r, s_df[lane], mx(i));
+          }
+          mixed_det_factors(r, mx(i), s_ds[lane], s_ws[lane]);
         }
-        mixed_fold_shared_weights(mreq[i], s_wk[lane], ndet);
+        mixed_fold_shared_weights(mx(i), s_wk[lane], ndet);
+        if constexpr (ACC) acc_range(r, areq[i]);
       }
     } else {
       st = 4;
-      if (want_mixed) mreq[i] = MixedReq{};
+      if (want_mixed) mx(i) = MixedReq{};
     }
-    if (st && want_mixed) mreq[i].status = st;
+    if (st && want_mixed) mx(i).status = st;
     if (st && req) req[i].m.status = st;
     status[i] = st;
   }
@@ -656,17 +558,18 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int w
     int kcut = 0;
     if (act && !s_bad[lane] && r.m.status == 0 && s_st[lane] == 0 && s_uni[lane]) {
       const StreamDev &s0 = streams[handles[i * ndet]];
-      kcut = min(s0.N, mreq[i].n_cut - s0.n0 + 1);  // n_cut: written in S5
+      kcut = min(s0.N, mx(i).n_cut - s0.n0 + 1);  // n_cut: written in S5
     }
     tail(warp, lane, act, i, kcut);
   }
 }
 
+template <bool ACC>
 __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const GenParams *__restrict__ params, const int *__restrict__ approx, int n, const int *__restrict__ handles,
     int ndet, double T_segment, int tc_from_segment, const StreamDev *__restrict__ streams,
-    const double *__restrict__ qnm, Request *req, MixedReq *mreq, int want_mixed, int *status, const OrderArgs ord,
-    gwt::WaveF64 *w64) {
+    const double *__restrict__ qnm, Request *req, MixedReq *mreq, AccReq *areq, int want_mixed, int *status,
+    const OrderArgs ord) {
   __shared__ CoopSmem sm;
   grid_dep_trigger();  // the bin kernel may launch and wait for this grid
   // this block's requests into the work order, on the warps idle in S6 (warp
@@ -676,27 +579,34 @@ __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const int nt = act ? ord.item_count[i] : 0, i0 = act ? ord.item_start[i] : 0;
     order_append(ord, kcut, nt, i0, warp - 1, kCoopWarps - 1);
   };
-  prologue_coop_body(sm, blockIdx.x * kCoopReq, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles, ndet,
+  prologue_coop_body<ACC>(sm, blockIdx.x * kCoopReq, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles, ndet,
                      T_segment, tc_from_segment, streams, qnm, req, mreq, want_mixed, status,
-                     [] { __syncthreads(); }, tail, w64);
+                     [] { __syncthreads(); }, tail, areq);
 }
 
 
 cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
                             Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s,
-                            const OrderArgs &ord, gwt::WaveF64 *w64) {
+                            const OrderArgs &ord, AccReq *areq) {
   int grid = (n + kCoopReq - 1) / kCoopReq;
-  k_prologue_coop<<<grid, kCoopWarps * 32, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment,
-                                                   streams, qnm, req, mreq, want_mixed, status, ord, w64);
+  if (areq)
+    k_prologue_coop<true><<<grid, kCoopWarps * 32, 0, s>>>(params, approx, n, handles, ndet, T_segment,
+                                                           tc_from_segment, streams, qnm, req, nullptr, areq, 1,
+                                                           status, ord);
+  else
+    k_prologue_coop<false><<<grid, kCoopWarps * 32, 0, s>>>(params, approx, n, handles, ndet, T_segment,
+                                                            tc_from_segment, streams, qnm, req, mreq, nullptr,
+                                                            want_mixed, status, ord);
   return cudaGetLastError();
 }
 cudaError_t launch_prologue_serial(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                                    double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
-                                   Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s) {
+                                   Request *req, MixedReq *mreq, AccReq *areq, int want_mixed, int *status,
+                                   cudaStream_t s) {
   int block = 32, grid = (n + block - 1) / block;
   k_prologue<<<grid, block, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req,
-                                    mreq, want_mixed, status);
+                                    mreq, areq, want_mixed, status);
   return cudaGetLastError();
 }
 
@@ -721,8 +631,6 @@ cudaError_t launch_mcmc_repack(const double *theta, int dim, int n, int approxim
 constexpr int kBatchBlock = 256;
 static_assert(kBatchBlock == kSegBins, "one block pass covers one phase segment");
 constexpr int kMaxSegs = 32;  // segments per chunk of an item (shared buffers)
-constexpr int kMaxTile = 16384;  // FP64 form: items up to this many bins use the rotation table
-constexpr int kStatusBounds = 0x100;  // set by an item whose bins fall outside the tables; finalize reports 5
 
 // Two-level compensated reduction of NV FP32 values per thread:
 // 16-element TwoSum columns, then FP64 across columns.  Result in res[0..NV).
@@ -900,8 +808,6 @@ struct BinSmem {
   static constexpr int NV = MIXED ? NDET * kAccPerDet : 2 * NDET;
   // mixed form: segment node values and fitted phase / alpha polynomials
   static constexpr int kSegBuf = MIXED ? kMaxSegs : 1;
-  // FP64 form on uniform grids: each pass's arrival-time rotations
-  static constexpr int kRotPasses = MIXED ? 1 : kMaxTile / kBatchBlock;
   alignas(16) unsigned char req[MIXED ? sizeof(MixedReq) : sizeof(Request)];
   StreamDev st[NDET];
   double res[NV];
@@ -910,11 +816,9 @@ struct BinSmem {
   double node[kSegBuf * kSegEval], node_a[kSegBuf * kSegEval];
   SegPoly poly[kSegBuf], poly_a[kSegBuf];
   double coef[kSegBuf * 2 * kSegNodes];
-  double2 rot64[kRotPasses * NDET];
   // detector rotations: per segment pass (first bin) and per thread offset
   float2 rot_seg[kSegBuf * (MIXED ? NDET : 1)];
   float2 rot_off[(MIXED ? NDET : 1) * (MIXED ? kBatchBlock : 1)];
-  alignas(8) unsigned char w64[MIXED ? 8 : sizeof(gwt::WaveF64)];  // FP64 form: the table form's coefficients
 };
 
 // One item (iid, I) of a batch on the whole block: its partial sums into
@@ -926,7 +830,6 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
                                            Fin fin) {
   using BS = BinSmem<NDET, MIXED>;
   constexpr int NV = BS::NV;
-  constexpr int kRotPasses = BS::kRotPasses;
   unsigned char *s_req = sm.req;
   StreamDev *s_st = sm.st;
   double *s_res = sm.res;
@@ -935,7 +838,6 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
   double *s_node = sm.node, *s_node_a = sm.node_a;
   SegPoly *s_poly = sm.poly, *s_poly_a = sm.poly_a;
   double *s_coef = sm.coef;
-  double2 *s_rot64 = sm.rot64;
   float2 *s_rot_seg = sm.rot_seg, *s_rot_off = sm.rot_off;
   const int tid = threadIdx.x;
   // stage the request constants and its streams
@@ -945,14 +847,6 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
     constexpr int nw = (MIXED ? sizeof(MixedReq) : sizeof(Request)) / 4;
     for (int w = tid; w < nw; w += blockDim.x) dst[w] = __ldcg(src + w);
     if (tid < NDET) s_st[tid] = a.streams[__ldcg(a.handles + I.req * a.ndet + tid)];
-    if constexpr (!MIXED) {
-      if (a.w64) {  // the request's FP64 coefficients on the grid (IMRPhenomD, uniform grids)
-        static_assert(sizeof(gwt::WaveF64) % 4 == 0, "copied as words");
-        const unsigned *ws = (const unsigned *)(a.w64 + I.req);
-        unsigned *wd = (unsigned *)sm.w64;
-        for (int w = tid; w < (int)(sizeof(gwt::WaveF64) / 4); w += blockDim.x) wd[w] = __ldcg(ws + w);
-      }
-    }
   }
   __syncthreads();
   const int N = s_st[0].N;
@@ -972,48 +866,8 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
     double v[NV];
 #pragma unroll
     for (int j = 0; j < NV; j++) v[j] = 0.0;
-    bool uniform = true;
-#pragma unroll
-    for (int d = 0; d < NDET; d++) uniform = uniform && s_st[d].uniform_int;
-    const int npass = (kend - I.k0 + kBatchBlock - 1) / kBatchBlock;
-    if (uniform && npass <= kRotPasses) {
-      // e^{i tau f_k} = e^{i tau f_(first bin of the pass)} e^{i tau (k - first) df}
-      for (int e = tid; e < npass * NDET; e += blockDim.x) {
-        const int pass = e / NDET, d = e - pass * NDET;
-        double sn, cs;
-        sincos(r.det[d].tau * s_st[0].freqs[I.k0 + pass * kBatchBlock], &sn, &cs);
-        s_rot64[e] = make_double2(cs, sn);
-      }
-      double oc[NDET], os[NDET];
-#pragma unroll
-      for (int d = 0; d < NDET; d++) sincos(r.det[d].tau * (tid * s_st[0].df), &os[d], &oc[d]);
-      __syncthreads();
-      if (r.m.status == 0) {
-        // IMRPhenomD: the waveform from the request's coefficients and the
-        // power tables where they cover the item's bins
-        const int n0 = s_st[0].n0;
-        const bool tab = a.w64 && r.approximant == kPhenomD && n0 >= 1 && n0 + kend - 1 <= a.tables.nmax &&
-                         n0 + kend - 1 <= a.tm76d_n;
-        const gwt::WaveF64 &W = *(const gwt::WaveF64 *)sm.w64;
-        int pass = 0;
-        for (int k = I.k0 + tid; k < kend; k += blockDim.x, pass++) {
-          double rc[NDET], rs[NDET];
-#pragma unroll
-          for (int d = 0; d < NDET; d++) {
-            const double2 b = s_rot64[pass * NDET + d];
-            rc[d] = b.x * oc[d] - b.y * os[d];
-            rs[d] = b.y * oc[d] + b.x * os[d];
-          }
-          cd hp, hc;
-          if (tab) d_bin_tab(r, W, a.tables, a.tm76d, n0 + k, s_st[0].freqs[k], hp, hc);
-          else wave_bin(r, s_st[0].freqs[k], hp, hc);
-          fp64_acc_rot<NDET>(r, s_st, k, N, hp, hc, rc, rs, v);
-        }
-      }
-      __syncthreads();  // s_rot64 is rewritten by the next item
-    } else if (r.m.status == 0) {
+    if (r.m.status == 0)
       for (int k = I.k0 + tid; k < kend; k += blockDim.x) fp64_bin<NDET>(r, s_st, k, N, v);
-    }
     block_sum<NV>(v, s_dsm);
     if (tid == 0)
 #pragma unroll
@@ -1072,45 +926,13 @@ __global__ void __launch_bounds__(kBatchBlock, OCC) k_batch(const BatchArgs a) {
   __shared__ int s_iid, s_bstart[kOrderBuckets];
   const int tid = threadIdx.x;
   grid_dep_wait();  // the prologue's output
-  if (a.bucket_fill && tid < 32) {  // first position of each bucket in the work order
-    constexpr int kPerLane = (kOrderBuckets + 31) / 32;
-    int v[kPerLane], sum = 0;
-#pragma unroll
-    for (int q = 0; q < kPerLane; q++) {
-      const int b = tid * kPerLane + q;
-      v[q] = b < kOrderBuckets ? __ldcg(a.bucket_fill + b) : 0;
-      sum += v[q];
-    }
-    int incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (tid >= o) incl += y;
-    }
-    int run = incl - sum;
-#pragma unroll
-    for (int q = 0; q < kPerLane; q++) {
-      const int b = tid * kPerLane + q;
-      if (b < kOrderBuckets) s_bstart[b] = run;
-      run += v[q];
-    }
-  }
+  if (a.bucket_fill && tid < 32) order_starts(a, s_bstart);
   __syncthreads();
   for (;;) {
     if (tid == 0) {
       const int it = (int)atomicAdd(a.item_counter, 1u);
-      int iid = it;
-      if (a.bucket_fill && it < a.nitems) {  // the bucket holding position it: the last start <= it
-        int lo = 0, hi = kOrderBuckets - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (s_bstart[mid] <= it) lo = mid;
-          else hi = mid - 1;
-        }
-        iid = __ldcg(a.bucket_items + (size_t)lo * a.nitems + (it - s_bstart[lo]));
-      }
       s_item = it;
-      s_iid = iid;
+      s_iid = order_item(a, s_bstart, it);
     }
     __syncthreads();
     const int it = s_item;
@@ -1194,7 +1016,7 @@ __device__ __forceinline__ void loop_prologue(const LoopArgs &L, CoopSmem &cs, i
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < kCoopWarps)
-    prologue_coop_body(cs, slot0, warp, lane, L.dparams, L.dapprox, slot0 + k, L.dhandles, NDET, L.T_segment, 1,
+    prologue_coop_body<false>(cs, slot0, warp, lane, L.dparams, L.dapprox, slot0 + k, L.dhandles, NDET, L.T_segment, 1,
                        a.streams, L.qnm, nullptr, const_cast<MixedReq *>(a.mreq), 1, a.status,
                        [] { asm volatile("bar.sync 1, 128;" ::: "memory"); }, [](int, int, bool, int, int) {});
   __threadfence();
@@ -1424,7 +1246,7 @@ int batch_occupancy(int mixed, int ndet, int occ) {
   return nb;
 }
 
-static cudaError_t launch_dependent(const void *f, dim3 grid, dim3 block, void **args, cudaStream_t s, bool pdl) {
+cudaError_t launch_dependent(const void *f, dim3 grid, dim3 block, void **args, cudaStream_t s, bool pdl) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;

@@ -5,10 +5,12 @@
 #include <cuda_runtime.h>
 
 #include "../../include/gwgpu.h"
+#include "phenom_acc.h"
 #include "phenom_mixed.h"
 
 namespace gwk {
 
+using gwt::AccReq;
 using gwt::GenParams;
 using gwt::MixedReq;
 using gwt::Request;
@@ -31,6 +33,14 @@ struct StreamDev {
   // content key of the whitening weights (what, wscale): streams with equal
   // keys have identical weights (same grid, PSD and integration rule)
   unsigned long long wkey;
+  // FP64 form on two-float bins (phenom_acc.h; null where the stream does not
+  // qualify): W d / dscale and W / wscale as pairs, the bins' distances from
+  // (n0 + k) dfq (null: none), and the grid's spacing over its whole length
+  // (df = f[1] - f[0] carries the rounding of f there)
+  const gwt::ff4 *wd;
+  const gwt::ff *wf;
+  const float *dev;
+  double dfq;
 };
 
 struct Item {
@@ -54,19 +64,20 @@ cudaError_t launch_inner_product(const double *data, const double *psd, const do
 // The same with integration weights iw (4 w_i, times f_i ln 10 for log10F).
 cudaError_t launch_inner_product_weighted(const double *data, const double *psd, const double *resp, const double *iw,
                                           int N, double *partials, unsigned *counter, double *out, cudaStream_t s);
-// Plain form on uniform grids, IMRPhenomD: the waveform from the request's
-// FP64 coefficients on the grid (wave64_prologue) and the n-indexed power
-// tables instead of the powers, logarithm and cube root of each frequency.
-struct PlainTab {
-  gwt::WaveF64 w;
-  gwt::Tables t;
-  const double *tm76d = nullptr;  // n^(-7/6), FP64
-  int use = 0;                    // 1: the tables cover every bin of the call
-};
 // Plain form: one request, FP64, one launch.  out[0] = log L.
 cudaError_t launch_plain(const Request &r, const StreamDev *streams, int ndet, double *partials, unsigned *counter,
-                         double *out, int *status, cudaStream_t s, const PlainTab *tab = nullptr);
+                         double *out, int *status, cudaStream_t s);
+// The same on two-float bins (every stream has wd, wf; x from acc_prologue; one partial sum per block).
+cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
+                             const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
+                             cudaStream_t s);
+// One of the two: two-float bins when every stream has its pairs (and the
+// tables reach its grid), else FP64 bins.  partials: 2 kMaxDet per block.
+cudaError_t launch_plain_any(const Request &r, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
+                             const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
+                             cudaStream_t s);
 int plain_blocks(int N);
+cudaError_t plain_acc_preload();
 cudaError_t plain_preload();  // loads the plain kernels' module (function-attribute query)
 
 // Work order of a mixed batch: the prologue appends each request's items to
@@ -83,12 +94,12 @@ struct OrderArgs {
 cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
                             Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s,
-                            const OrderArgs &ord = OrderArgs(), gwt::WaveF64 *w64 = nullptr);
+                            const OrderArgs &ord = OrderArgs(), AccReq *areq = nullptr);
 // One thread per request (the reference order of the prologue); kept to check
 // the cooperative kernel against.
 cudaError_t launch_prologue_serial(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
-                            Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s);
+                            Request *req, MixedReq *mreq, AccReq *areq, int want_mixed, int *status, cudaStream_t s);
 cudaError_t launch_mcmc_repack(const double *theta, int dim, int n, int approximant, double gmst, GenParams *out,
                                int *approx_out, cudaStream_t s);
 struct BatchArgs {
@@ -111,17 +122,23 @@ struct BatchArgs {
   int *status;      // per-request working status (device memory: the bounds flag is set atomically)
   int *status_out;  // where the finalize writes each request's status (status itself, or mapped host memory)
   gwt::Tables tables;
-  // FP64 form: per-request coefficients on the grid written by the prologue
-  // (IMRPhenomD, uniform grids; null: every bin from the frequency) and the
-  // FP64 n^(-7/6) table for n <= tm76d_n
-  const gwt::WaveF64 *w64 = nullptr;
-  const double *tm76d = nullptr;
-  int tm76d_n = 0;
+  // FP64 form on two-float bins (null: every bin from its frequency, req)
+  const AccReq *areq = nullptr;
+  gwt::AccTables acc{};
+  const gwt::AccLut *lut = nullptr;
 };
 // occ: the launch shape's resident blocks per SM (mixed 3 or 4, FP64 2);
 // pdl: launched as a programmatic dependent of the kernel before it on s
 // (it starts launching while that one runs and waits for its completion).
 cudaError_t launch_batch(const BatchArgs &a, int mixed, int grid, int occ, cudaStream_t s, bool pdl);
+cudaError_t launch_dependent(const void *f, dim3 grid, dim3 block, void **args, cudaStream_t s, bool pdl);
+// The fused kernel of the FP64 form on two-float bins.
+cudaError_t launch_batch_acc(const BatchArgs &a, int grid, cudaStream_t s, bool pdl);
+int batch_acc_occupancy(int ndet);
+// Tables n <= nmax from the FP64 powers t13, tln, t34 of tab, and a stream's
+// pairs from its FP64 arrays.
+cudaError_t launch_acc_tables(const gwt::AccTables &tab, cudaStream_t s);
+cudaError_t launch_acc_stream(const StreamDev &d, bool with_dev, cudaStream_t s);
 
 int batch_default_occ(int mixed);
 int batch_block_size(int mixed);

@@ -91,8 +91,8 @@ int gwgpu_mcmc_likelihood_extrinsic_noalloc(gwgpu_context *c, const gwgpu_gen_pa
   gwt::Request r;
   gwt::request_prologue(r, gp, ap, dets, ndet, c->qnm_host.data());
   if (r.m.status) return GWGPU_EDOMAIN;  // nothing is launched; d_loglik is left as it was
-  cudaError_t e = gwk::launch_plain(r, sd, ndet, scratch, (unsigned *)(scratch + kNoAllocPartials), d_loglik,
-                                    nullptr, (cudaStream_t)stream);
+  cudaError_t e = gwk::launch_plain_any(r, sd, ndet, c->acc, c->acc_lut, scratch,
+                                        (unsigned *)(scratch + kNoAllocPartials), d_loglik, (cudaStream_t)stream);
   return e == cudaSuccess ? GWGPU_OK : GWGPU_ECUDA;
 }
 

@@ -89,6 +89,7 @@ struct ModelD {
   double phic;    // D: 2 phiRef + phi(f_ref) or phiRef; Pv2: 2 phi_aligned
   double fref;    // f_ref used in tc*(f - f_ref) (0 when shift_phase is off, D only)
   double fcut;    // 0.2 / M
+  double tcs;     // D: the tc_shift part of tcl; Pv2: 0
   int status;
 };
 

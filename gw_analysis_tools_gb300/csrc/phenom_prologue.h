@@ -387,6 +387,7 @@ GW_HD void model_d_finish_parts(ModelD &m, const PhaseConnParts &c) {
     tc_shift = Dmr + (-m.l.alpha[1] + c.a1fit) * s.M / s.eta;
   }
   m.tcl = 2 * kPi * s.tc + tc_shift;
+  m.tcs = tc_shift;
   m.A0eff = s.A0 * pow_7_6(M);
 }
 GW_HDNI void model_d_finish(ModelD &m) {
@@ -609,6 +610,7 @@ GW_HDNI void model_p_finish(ModelD &m, ModelP &pm) {
   m.fref = s.f_ref;
   m.phic = 2 * s.phi_aligned;
   m.tcl = 2 * kPi * s.tc;
+  m.tcs = 0.0;
   m.A0eff = s.A0 * pow_7_6(s.M) / (2. * sqrt(5. / (64. * kPi)));
   s.q = s.mass1 / s.mass2;
   pv2_euler_coeffs(pm.ac, pm.ec, s);

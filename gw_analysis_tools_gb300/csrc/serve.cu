@@ -117,7 +117,7 @@ namespace {
 
 size_t request_bytes(int precision, int N, int tile) {  // device scratch held by one in-flight request
   size_t items = (size_t)(N + tile - 1) / tile;
-  return (precision == GWGPU_PREC_MIXED ? sizeof(gwt::MixedReq) : sizeof(gwt::Request)) +
+  return (precision == GWGPU_PREC_MIXED ? sizeof(gwt::MixedReq) : std::max(sizeof(gwt::Request), sizeof(gwt::AccReq))) +
          items * (sizeof(double) * gwk::kAcc + sizeof(gwk::Item)) + sizeof(gwgpu_gen_params) + 64;
 }
 

@@ -1,0 +1,101 @@
+"""The FP64 form's two-float bins on the device (csrc/acc.cu): batched and plain
+log L against the oracle at the sizes where tiles, blocks and grids end, on
+grids whose frequencies are rounded, with different weights per detector, and
+with requests and streams that take another branch."""
+import numpy as np
+import pytest
+
+import gw_analysis_tools_gb300 as G
+from gw_analysis_tools_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+DETS = ("Hanford", "Livingston", "Virgo", "Kagra")
+RTOL = 1e-9  # the FP64 bound of the likelihood entry points
+
+
+def _network(ctx, oracle, T, N, ndet, same_psd=True, seed=3):
+    f = 20.0 + np.arange(N) * (1.0 / T)
+    src = W.config1_source()
+    inj = oracle.params_from_dict(dict(src, tc=T - src["tc"]))
+    rng = np.random.default_rng(seed)
+    psd = [W.analytic_psd(f) * (1.0 if same_psd else 1.0 + 0.3 * i) for i in range(ndet)]
+    data = [oracle.detector_response(f, inj, d) + np.sqrt(psd[i] * T / 4) * (rng.standard_normal(N) + 1j * rng.standard_normal(N))
+            for i, d in enumerate(DETS[:ndet])]
+    return f, data, psd, [ctx.register_data(d, f, data[i], psd[i]) for i, d in enumerate(DETS[:ndet])]
+
+
+def _close(got, ref):
+    return np.all(np.abs(np.asarray(got) - ref) <= RTOL * np.maximum(1.0, np.abs(ref)))
+
+
+@pytest.mark.parametrize("T,N,ndet,same", [(8, 2, 1, True), (8, 3, 2, True), (8, 127, 3, True), (8, 129, 4, False),
+                                           (4, 255, 3, False), (4, 257, 1, True), (16, 4095, 2, False),
+                                           (12, 4097, 3, True), (25, 9001, 3, False), (32, 32128, 2, True)])
+def test_batch_and_plain(gpu_ctx, oracle, T, N, ndet, same):
+    f, data, psd, hs = _network(gpu_ctx, oracle, T, N, ndet, same)
+    try:
+        # a near-aligned source with no in-plane spin and an extreme mass ratio beside the draws
+        src = W.config1_source()
+        d = [src, dict(src, mass1=70.0, mass2=1.2)] + W.prior_draws(5, N)
+        p = [dict(src, spin1=(0, 0, 0), spin2=(0, 0, 0)), dict(src, mass1=70.0, mass2=1.2, spin1=(0.4, 0.1, 0.2))]
+        p += W.prior_draws(5, N + 1, precessing=True)
+        draws = [x for pair in zip(d, p) for x in pair]
+        aps = [0, 1] * len(d)
+        ref = np.array([oracle.loglik(oracle.params_from_dict(x), f, list(DETS[:ndet]), data, psd, approximant=a,
+                                      T_segment=float(T)) for x, a in zip(draws, aps)])
+        for tile in (0, 256, 512):
+            gpu_ctx.set_tile(tile)
+            out, st = gpu_ctx.loglik_batch(G.params_array(draws), aps, hs, float(T), G.PREC_FP64)
+            assert np.all(st == 0) and _close(out, ref), (tile, np.abs(out - ref).max())
+        for x, a, r in zip(draws, aps, ref):
+            m = "IMRPhenomPv2" if a else "IMRPhenomD"
+            assert _close(gpu_ctx.mcmc_likelihood_extrinsic(G.gen_params(**x), m, hs, float(T)), r)
+    finally:
+        gpu_ctx.set_tile(0)
+        for h in hs:
+            gpu_ctx.release_data(h)
+
+
+def test_weighted_uniform_grid_and_bad_requests(gpu_ctx, oracle):
+    """Integration weights on a uniform grid, and requests outside the model's domain beside good ones."""
+    T, N = 8.0, 1500
+    f = 20.0 + np.arange(N) / T
+    rng = np.random.default_rng(5)
+    w = rng.uniform(0.5, 1.5, N) / T
+    psd = W.analytic_psd(f)
+    data = W.noise(f, 9)
+    h = gpu_ctx.register_data("Hanford", f, data, psd, weights=w)
+    try:
+        draws = W.prior_draws(6, 8)
+        ref = np.array([oracle.loglik_gl(oracle.params_from_dict(x), f, ["Hanford"], [data], [psd], [w], T_segment=T)
+                        for x in draws])
+        bad = [dict(draws[0], mass1=-1.0), dict(draws[1], mass1=float("nan"))]
+        out, st = gpu_ctx.loglik_batch(G.params_array(draws + bad), 0, [h], T, G.PREC_FP64)
+        assert np.all(st[:6] == 0) and _close(out[:6], ref)
+        assert np.all(st[6:] != 0) and np.all(np.isnan(out[6:]))
+    finally:
+        gpu_ctx.release_data(h)
+
+
+def test_infinite_psd_bins(gpu_ctx, oracle):
+    """A PSD of infinity takes its bin out (finite pairs); a zero PSD, whose weight is infinite, keeps the FP64
+    bins: both as the oracle."""
+    T, N = 8.0, 900
+    f = 20.0 + np.arange(N) / T
+    psd = W.analytic_psd(f)
+    psd[100:140] = np.inf
+    data = W.noise(f, 4)
+    draws = W.prior_draws(4, 2)
+    ref = np.array([oracle.loglik(oracle.params_from_dict(x), f, ["Hanford"], [data], [psd], T_segment=T) for x in draws])
+    h = gpu_ctx.register_data("Hanford", f, data, psd)
+    psd0 = psd.copy()
+    psd0[N - 1] = 0.0
+    h0 = gpu_ctx.register_data("Hanford", f, data, psd0)
+    try:
+        out, st = gpu_ctx.loglik_batch(G.params_array(draws), 0, [h], T, G.PREC_FP64)
+        assert np.all(st == 0) and _close(out, ref)
+        out, st = gpu_ctx.loglik_batch(G.params_array(draws), 0, [h0], T, G.PREC_FP64)
+        assert np.all(st == 0) and not np.any(np.isfinite(out))
+    finally:
+        gpu_ctx.release_data(h)
+        gpu_ctx.release_data(h0)
