@@ -249,8 +249,8 @@ cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet
   }
   return cudaGetLastError();
 }
-cudaError_t launch_plain_any(const Request &r, const StreamDev *streams, int ndet, const AccTables &tab,
-                             const AccLut *lut, double *partials, unsigned *counter, double *out, cudaStream_t s) {
+cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev *streams, int ndet,
+                             const AccTables &tab, const AccLut *lut, double *partials, unsigned *counter, double *out, cudaStream_t s) {
   bool acc = lut && !r.m.status && streams[0].n0 + streams[0].N - 1 <= tab.nmax;
   double ds[kMaxDet], ws[kMaxDet];
   unsigned long long wk[kMaxDet];
@@ -262,7 +262,7 @@ cudaError_t launch_plain_any(const Request &r, const StreamDev *streams, int nde
   }
   if (!acc) return launch_plain(r, streams, ndet, partials, counter, out, nullptr, s);
   AccReq x;
-  acc_prologue(r, streams[0].dfq, x, ds, ws);
+  fast_acc(r, fx, grid_const(streams[0].dfq), x, ds, ws);
   mixed_fold_shared_weights(x.m, wk, ndet);
   return launch_plain_acc(x, streams, ndet, tab, lut, partials, counter, out, s);
 }

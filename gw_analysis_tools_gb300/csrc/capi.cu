@@ -423,9 +423,12 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   std::vector<double> ip(N);  // the reciprocal PSD: the FP64 kernels multiply instead of dividing
   for (int k = 0; k < N; k++) ip[k] = 1.0 / psd[k];
   // one allocation for the stream's arrays, each on a 256-byte boundary
-  const size_t row = ((size_t)N + 31) / 32 * 32;
+  const size_t row = ((size_t)N + 31) / 32 * 32, gat = row * (weights ? 60 : 52);
   char *mem;
-  if ((st = c->dalloc((void **)&mem, row * (weights ? 60 : 52), "data stream"))) return st;
+  if ((st = c->dalloc((void **)&mem, gat + 2 * sizeof(gwt::GridConst), "data stream"))) return st;
+  const gwt::GridConst gc[2] = {gwt::grid_const(d.df), gwt::grid_const(d.dfq)};
+  cudaMemcpyAsync(mem + gat, gc, sizeof(gc), cudaMemcpyHostToDevice, c->stream);
+  d.grid = (const gwt::GridConst *)(mem + gat);
   void *pd = mem, *pf = mem + 16 * row, *pp = mem + 24 * row, *pip = mem + 32 * row, *pdh = mem + 40 * row,
        *pwh = mem + 48 * row, *piw = weights ? mem + 52 * row : nullptr;
   cudaMemcpyAsync(pip, ip.data(), 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
@@ -627,7 +630,8 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   std::memcpy(&gp, p, sizeof(gp));
   gp.tc = T_segment - gp.tc;  // mcmc_gw.cpp:2466-2473
   gwt::Request r;
-  gwt::request_prologue(r, gp, ap, dets, ndet, c->qnm_host.data());
+  gwt::FastX fx;
+  gwt::fast_request(r, fx, gp, ap, dets, ndet, c->qnm_host.data());
   void *dev;
   int nblk = gwk::plain_blocks(sd[0].N);
   int st = c->workspace(gwgpu_context::kWsPlain, sizeof(double) * ((size_t)nblk * 2 * gwt::kMaxDet + 8), &dev);
@@ -642,7 +646,7 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   if (st) return st;
   cudaError_t e = cudaHostGetDevicePointer((void **)&hd, h, 0);
   if (e != cudaSuccess) return c->fail(e, "plain result mapping");
-  e = gwk::launch_plain_any(r, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream);
+  e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream);
   if (e != cudaSuccess) return c->fail(e, "plain launch");
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return c->fail(e, "plain");

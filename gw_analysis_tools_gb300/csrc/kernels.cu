@@ -266,32 +266,6 @@ __global__ void k_prologue(const GenParams *__restrict__ params, const int *__re
   if (st && req) req[i].m.status = st;
   status[i] = st;
 }
-// Cooperative prologue: the same constants as k_prologue, with each request's
-// independent parts spread over the four warps of its block.  An FP64
-// instruction occupies a sub-partition's FP64 pipe for the same time whatever
-// the number of active lanes, so one request per lane leaves the model's
-// FP64 chain as the latency; running its independent parts on four
-// sub-partitions at once shortens that chain.  Lane j of every warp works on
-// request blockIdx.x * kCoopReq + j; shared memory holds the requests between
-// stages.  Stage plan (W0..W3 = warps):
-//   S0  W0 parameters, source;  W1/W2 detector projections (a detector per half-warp),
-//       W2 inclination factors;  W3 chirp mass and amplitude normalisation
-//   S1  W0/W3 calibration fits;  W1 D: final spin, radiated energy, ringdown frequencies /
-//       Pv2: J-frame transform;  W2 PN coefficients
-//   S2  W0 Pv2: ringdown frequencies; matching frequencies;  W1 D: phase at f_ref (inspiral);
-//       W2 D: ringdown-phase terms at f3
-//   S3  W0/W1 amplitude matching points;  D: phase connection in four pieces after them
-//       (W0 f1 terms, W1 inspiral phase, W2 inspiral derivative, W3 f2 terms);
-//       Pv2: W2 inspiral part, W1 the other parts, W3 Euler and frame constants
-//   S3b Pv2: W2 phase connection constants
-//   S4  amplitude deltas (D: W0/W1/W3, Pv2: W0/W1);  W2 D: phase connection constants,
-//       phase/time shift / Pv2: time-shift nodes 0-4;  W3 Pv2: nodes 5-9 (two
-//       nodes at a time on the half-warps)
-//   S5  W0 mixed amplitude;  W1 mixed phase;  W2 regions, D: detector factors / Pv2:
-//       angles;  W3 D: detector phases / Pv2: time shift
-//   S6  W0 Pv2: detector phases and factors; outputs;  W1-W3 the bin kernel's work order
-// (per-warp clock stamps of each stage guided the split: IMRPhenomD, warm,
-// before this split S3 20.2k / S5 22.2k / S6 13.0k cycles on the longest warp)
 // Longest-processing-time-first order for the persistent mixed kernel: an
 // item's work is its live 256-bin passes (bins below the request's cut
 // f <= 0.2/M, where the model is non-zero; beyond it a pass costs nothing), and
@@ -324,253 +298,273 @@ __device__ __forceinline__ void order_append(const OrderArgs &o, int kcut, int n
   }
 }
 
+// Cooperative prologue: the constants of a group of REQ requests on four warps.
+//
+// An FP64 instruction occupies a sub-partition's FP64 pipe for 64 cycles
+// whatever the number of active lanes, so the time is the number of FP64
+// instructions on the longest warp of each stage.  The parts of phenom_fast.h
+// are spread over the four warps (one per sub-partition), and 32 / REQ lanes
+// serve each request, so that the calibration fits, the PN coefficients, the
+// sines and cosines, the detectors and the Pv2 time-shift nodes run as lanes of
+// one instruction stream.  Lane l works on request l % REQ of the group.
+//   S0  parameters and streams into shared memory
+//   S1  every lane: masses and spins;  W0 source, Pv2: chi_p; ringdown
+//       frequencies;  W1, W2 sines and cosines of the sky, inclination and
+//       phase angles;  W3 roots and logarithms of M and f_ref, amplitude;
+//       all: calibration fits, PN coefficients
+//   S2  W0 ringdown side of the amplitude connection, detector projections;
+//       W1 powers at f2, inspiral amplitude; Pv2: Euler angle coefficients;
+//       W2 D: time shift / Pv2: J frame;  W3 f2 angle, inspiral phase, phase at f_ref
+//   S3  W0 intermediate amplitude, amplitude coefficients;  W1 connections,
+//       phase coefficients;  W2 D: detector phases / Pv2: angles;  W3 regions, D: factors
+//   S4  Pv2: W2, W3 time-shift nodes
+//   S5  W0 Pv2: detector phases and factors; status;  W1-W3 the bin kernel's work order
+// REQ: 4 where the blocks then still fit the SMs one each, else 8 or 16
+// (launch_prologue); the serving loop claims up to 16.
+constexpr int kSMs = 152;  // GB300
 constexpr int kCoopWarps = 4, kCoopReq = 16;
-// Shared state of one group of kCoopWarps warps serving kCoopReq requests.
+template <int REQ>
 struct CoopSmem {
-  Request r[kCoopReq];
-  GenParams p[kCoopReq];
-  AmpConn ac[kCoopReq];
-  PhaseConnParts pc[kCoopReq];
-  double ds[kCoopReq][kMaxDet], ws[kCoopReq][kMaxDet];  // stream scales of the mixed form
-  unsigned long long wk[kCoopReq][kMaxDet];              // and weight keys
-  double shift[kCoopReq][kPv2ShiftNodes];
-  double df[kCoopReq];
-  int st[kCoopReq], bad[kCoopReq], uni[kCoopReq];
+  Request r[REQ];
+  FastX x[REQ];
+  GenParams p[REQ];
+  GridConst g[REQ];
+  double ds[REQ][kMaxDet], ws[REQ][kMaxDet];  // stream scales
+  unsigned long long wk[REQ][kMaxDet];        // and weight keys
+  double T[REQ];                              // segment length t_c counts from
+  int det[REQ][kMaxDet];
+  int ap[REQ], st[REQ], uni[REQ], late[REQ];
+  int any_pv2;
 };
-// The cooperative prologue of requests base .. base + kCoopReq - 1 (those
-// below n) on one group of kCoopWarps warps: warp (0..3) and lane are the
-// thread's place in the group, sync() the group's barrier.  In S6, while warp
-// 0 stores the results, warps 1-3 call tail(warp, lane, act, i, kcut) with
-// kcut the end of request i's live bins (0 when it will not be evaluated);
-// tail is warp-collective.
-// ACC: the FP64 form's constants (areq) instead of the mixed form's (mreq).
-template <bool ACC, class Sync, class Tail>
-__device__ __forceinline__ void prologue_coop_body(CoopSmem &sm, int base, int warp, int lane,
+// The cooperative prologue of requests base .. base + REQ - 1 (those below n):
+// warp (0..3) and lane are the thread's place in the group, sync() the group's
+// barrier.  In S5, while warp 0 stores the results, warps 1-3 call
+// tail(warp, lane, act, i, kcut) with kcut the end of request i's live bins (0
+// when it will not be evaluated); act is set on one lane per request; tail is
+// warp-collective.  ACC: the FP64 form's constants (areq) instead of the mixed
+// form's (mreq); coef: either is wanted (else req alone).
+template <int REQ, bool ACC, class Sync, class Tail>
+__device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, int warp, int lane,
                                                    const GenParams *__restrict__ params,
                                                    const int *__restrict__ approx, int n,
                                                    const int *__restrict__ handles, int ndet, double T_segment,
                                                    int tc_from_segment, const StreamDev *__restrict__ streams,
                                                    const double *__restrict__ qnm, Request *req, MixedReq *mreq,
-                                                   int want_mixed, int *status, Sync sync, Tail tail,
-                                                   AccReq *areq = nullptr) {
-  Request *s_r = sm.r;
-  auto mx = [&](int j) -> MixedReq & {
-    if constexpr (ACC) return areq[j].m;
-    else return mreq[j];
+                                                   AccReq *areq, int coef, int *status, Sync sync, Tail tail) {
+  constexpr int G = 32 / REQ;  // lanes of a warp per request
+  const int j = lane % REQ, g = lane / REQ, i = base + j, cnt = min(REQ, n - base);
+  const bool act = j < cnt;
+  auto mx = [&](int q) -> MixedReq & {
+    if constexpr (ACC) return areq[q].m;
+    else return mreq[q];
   };
-  GenParams *s_p = sm.p;
-  AmpConn *s_ac = sm.ac;
-  PhaseConnParts *s_pc = sm.pc;
-  double(*s_ds)[kMaxDet] = sm.ds;
-  double(*s_ws)[kMaxDet] = sm.ws;
-  unsigned long long(*s_wk)[kMaxDet] = sm.wk;
-  double(*s_shift)[kPv2ShiftNodes] = sm.shift;
-  double *s_df = sm.df;
-  int *s_st = sm.st, *s_bad = sm.bad, *s_uni = sm.uni;
-  static_assert(2 * kCoopReq == 32, "two half-warps per warp share the group's requests");
-  const int i = base + lane;
-  const bool act = lane < kCoopReq && i < n;
-  // half-warp form: lanes j and j + kCoopReq both serve request j
-  const int hl = lane & (kCoopReq - 1);
-  const bool hact = base + hl < n;
-  Request &r = s_r[lane < kCoopReq ? lane : 0];
-  const GenParams &p = s_p[lane < kCoopReq ? lane : 0];
-  // S0
-  if (act && warp == 0) {
-    GenParams q = params[i];
-    const int ap = approx[i];
-    const StreamDev &s0 = streams[handles[i * ndet]];
-    // mcmc_gw.cpp:2466-2473; T_segment <= 0 selects 1/df of this request's grid
-    if (tc_from_segment) q.tc = (T_segment > 0 ? T_segment : 1.0 / s0.df) - q.tc;
-    int st = 0;
-    for (int d = 0; d < ndet; d++)
-      if (streams[handles[i * ndet + d]].N != s0.N) st = 1;
-    const bool bad = !(q.mass1 > 0) || !(q.mass2 > 0) || !(q.Luminosity_Distance > 0) || (ap != 0 && ap != 1);
-    s_p[lane] = q;
-    s_st[lane] = st;
-    s_bad[lane] = bad;
-    s_df[lane] = ACC ? s0.dfq : s0.df;
-    s_uni[lane] = s0.uniform_int;
-    r.approximant = ap;
-    r.ndet = ndet;
-    if (!bad) populate_core(r.m.s, q);
+  // S0 (through L2: the serving loop writes these arrays in the same launch)
+  {
+    static_assert(sizeof(GenParams) % 4 == 0, "copied as words");
+    constexpr int kW = sizeof(GenParams) / 4;
+    const unsigned *src = (const unsigned *)(params + base);
+    unsigned *dst = (unsigned *)sm.p;
+    for (int w = warp * 32 + lane; w < cnt * kW; w += kCoopWarps * 32) dst[w] = __ldcg(src + w);
+    if (act && g == 0) {
+      const StreamDev &s0 = streams[__ldcg(handles + i * ndet)];
+      if (warp == 0) {
+        int st = 0;
+        for (int d = 0; d < ndet; d++)
+          if (streams[__ldcg(handles + i * ndet + d)].N != s0.N) st = 1;
+        sm.st[j] = st;
+        sm.uni[j] = s0.uniform_int;
+        sm.ap[j] = __ldcg(approx + i);
+        sm.late[j] = 0;
+      }
+      if (warp == 1) {
+        const GridConst gc = s0.grid[ACC ? 1 : 0];
+        sm.g[j] = gc;
+        // mcmc_gw.cpp:2466-2473; T_segment <= 0 selects 1/df of this request's grid
+        sm.T[j] = T_segment > 0 ? T_segment : s0.grid[0].idf;
+      }
+      if (warp == 2)
+        for (int d = 0; d < ndet && d < kMaxDet; d++) {
+          const StreamDev &sd = streams[__ldcg(handles + i * ndet + d)];
+          sm.ds[j][d] = sd.dscale;
+          sm.ws[j][d] = sd.wscale;
+          sm.wk[j][d] = sd.wkey;
+          sm.det[j][d] = sd.det;
+        }
+    }
+    if (warp == 3 && lane == 0) sm.any_pv2 = 0;
   }
-  if (act && warp == 3) populate_amp(r.m.s, params[i]);
-  if (warp == 1 || warp == 2) {  // projections need only the sky position: detectors over the half-warps of warps 1, 2
-    // sky_trig with the hour angle's sincos on lanes j and the declination's
-    // on lanes j + kCoopReq at once
-    const int ih = base + hl;
-    const GenParams &q = params[min(ih, n - 1)];
-    double s1, c1, sps, cps;
-    sincos(lane < kCoopReq ? q.gmst - q.RA : q.DEC, &s1, &c1);
-    sincos(q.psi, &sps, &cps);
-    SkyTrig tr;
-    tr.sg = __shfl_sync(0xffffffffu, s1, hl);
-    tr.cg = __shfl_sync(0xffffffffu, c1, hl);
-    tr.sd = __shfl_sync(0xffffffffu, s1, hl + kCoopReq);
-    tr.cd = __shfl_sync(0xffffffffu, c1, hl + kCoopReq);
-    tr.sp = sps;
-    tr.cp = cps;
-    if (hact) {  // request hl: warp 1 detectors 0, 2 (+4k), warp 2 detectors 1, 3, half-warp by half-warp
-      Request &rh = s_r[hl];
-      if (warp == 2 && lane < kCoopReq) populate_incl(rh.m.s, q);
-      const int d0 = streams[handles[ih * ndet]].det;
-      for (int d = (warp - 1) + (lane >= kCoopReq ? 2 : 0); d < ndet && d < kMaxDet; d += 4) {
-        const StreamDev &sd = streams[handles[ih * ndet + d]];
-        const int dd = sd.det;
-        s_ds[hl][d] = sd.dscale;
-        s_ws[hl][d] = sd.wscale;
-        s_wk[hl][d] = sd.wkey;
-        antenna_trig(dd, tr, rh.det[d].fp, rh.det[d].fc);
-        rh.det[d].tau = -dtoa_trig(tr, d0, dd) * (2 * kPi);
+  sync();
+  // S1
+  Request &r = sm.r[act ? j : 0];
+  FastX &x = sm.x[act ? j : 0];
+  ModelD &m = r.m;
+  const GenParams &p = sm.p[act ? j : 0];
+  const int ap = act ? sm.ap[j] : 0;
+  const bool bad = act && (!(p.mass1 > 0) || !(p.mass2 > 0) || !(p.Luminosity_Distance > 0) || (ap != 0 && ap != 1));
+  const bool run = act && !bad, pv2 = run && ap == kPhenomPv2;
+  if (run) {
+    const FastCore k = fast_core(p);
+    if constexpr (G >= 8) {  // rows on the two warps with the least before
+      if (warp == 1)
+        for (int q = g; q < 19; q += G) fast_fit(m.l, k, q);
+      if (warp == 2)
+        for (int q = g; q < kPnRows; q += G) fast_pn(m, k, q);
+    } else {
+      for (int q = warp * G + g; q < kPnRows; q += kCoopWarps * G) fast_pn(m, k, q);
+      for (int q = (kCoopWarps - 1 - warp) * G + g; q < 19; q += kCoopWarps * G) fast_fit(m.l, k, q);
+    }
+    if (warp == 0 && g == 0) {
+      r.approximant = ap;
+      r.ndet = ndet;
+      fast_store(m.s, x, p, k);
+      if (tc_from_segment) m.s.tc = sm.T[j] - p.tc;
+      fast_fixed(m);
+      x.M34 = sqrt(k.M * sqrt(k.M));
+      if (pv2) {
+        sm.any_pv2 = 1;
+        fast_pv2_spins(m.s, p, k);
+      }
+      fast_ring(m.s, x, k, qnm);
+    }
+    if (warp == 1 || warp == 2) {
+      for (int a = (warp - 1) * G + g; a < (pv2 ? 5 : 4); a += 2 * G) {
+        const double ang = a == 0 ? p.gmst - p.RA : a == 1 ? p.DEC : a == 2 ? p.psi : a == 3 ? p.incl_angle : p.phiRef;
+        sincos(ang, &x.sn[a], &x.cn[a]);
+      }
+    }
+    if (warp == 3 && g < 2) {  // lane group 0: M, 1: f_ref
+      const double v = g == 0 ? k.M : p.f_ref, c = cbrt(v), l = log(v);
+      if (g == 0) {
+        x.cM = c;
+        x.lM = l;
+        fast_amp0(m, x, p, k);
+      } else {
+        x.cfr = c;
+        x.lfr = l;
       }
     }
   }
   sync();
-  const bool run = act && !s_bad[lane < kCoopReq ? lane : 0];
-  const bool pv2 = run && r.approximant == kPhenomPv2;
-  // S1: the calibration fits in four slots, the half-warps of warps 0 and 3
-  if ((warp == 0 || warp == 3) && hact && !s_bad[hl])
-    model_d_lambdas_slot(s_r[hl].m, (warp == 3 ? 2 : 0) + (lane >= kCoopReq ? 1 : 0));
-  if (run) {
-    if (warp == 1) {
-      if (pv2) model_p_setup(r.m, r.p, p);
-      else if (r.m.s.dep_postmerger) post_merger(r.m.s, qnm);
-      else post_merger_qnm(r.m.s, qnm, final_spin(r.m.s), EradRational0815(r.m.s.eta, r.m.s.spin1z, r.m.s.spin2z));
-    }
-    if (warp == 2) model_d_pn(r.m);
-  }
-  sync();
+  const bool lead = run && g == 0;  // one lane per request
   // S2
-  if (run && warp == 0) {
-    if (pv2) post_merger(r.m.s, qnm);
-    model_d_freqs(r.m);
+  if (lead && warp == 0) {
+    m.s.cos_incl = x.cn[3];
+    m.s.fac_incl = .5 * (1 + x.cn[3] * x.cn[3]);
+    fast_high(m, x);
   }
-  if (run && warp == 1 && !pv2) finish_fref_phase(r.m, s_pc[lane]);
-  if (run && warp == 2 && !pv2) finish_f3_terms(r.m, fpeak(r.m.s, r.m.l), s_pc[lane]);
+  if (run && warp == 0) {
+    fast_antenna(r, x, sm.det[j], g, G);
+  }
+  if (lead && warp == 1) {
+    fast_f2_powers(x);
+    fast_low_amp(m, x);
+    if (pv2) pv2_euler_coeffs(r.p.ac, r.p.ec, m.s);
+  }
+  if (lead && warp == 2) {
+    if (pv2) fast_pv2_frame(m.s, r.p, p, x);
+    else fast_time_shift(m, x);
+  }
+  if (lead && warp == 3) {
+    fast_f2_atan(m, x);
+    fast_low_phase(m, x);
+    fast_fref_phase(m, x);
+  }
   sync();
   // S3
-  if (run) {
-    if (warp == 0) {
-      d_amp_conn_low(r.m, s_ac[lane]);
-      if (!pv2) phase_conn_imr1(r.m, s_pc[lane]);
-    }
-    if (warp == 1) {
-      d_amp_conn_high(r.m, s_ac[lane]);
-      if (pv2) phase_conn_imr(r.m, s_pc[lane]);
-      else phase_conn_phins(r.m, s_pc[lane]);
-    }
-    if (warp == 2) {
-      if (pv2) {
-        phase_conn_ins(r.m, s_pc[lane]);
-      } else {
-        phase_conn_dins(r.m, s_pc[lane]);
-      }
-    }
-    if (warp == 3) {
-      if (pv2) model_p_finish(r.m, r.p);
-      else phase_conn_imr2(r.m, s_pc[lane]);
+  const double df = sm.g[act ? j : 0].df;
+  if (lead && warp == 0) {
+    fast_quartic(m, x);
+    if (req) fast_deltas(m, x);
+    if (coef) {
+      fast_amp_coeffs(m, x, sm.g[j], mx(i));
+      if constexpr (ACC) acc_amp_coeffs(r, df, areq[i]);
     }
   }
-  sync();
-  // S3b  Pv2: the phase connection constants (its time-shift nodes need them)
-  if (run && pv2 && warp == 2) phase_conn_combine(r.m, s_pc[lane]);
+  if (lead && warp == 1) {
+    fast_connect(m, x);
+    if (coef) {
+      fast_phase_coeffs(m, x, sm.g[j], mx(i));
+      if constexpr (ACC) acc_phase_coeffs(r, df, areq[i]);
+    }
+  }
+  if (run && warp == 2) {
+    if (pv2) {
+      if (g == 0) {
+        fast_pv2_finish(m, r.p, x);
+        if (coef) fast_pv2_coeffs(r, x, sm.g[j], mx(i));
+      }
+    } else {  // each lane sets the same linear constants, then takes its detectors
+      const bool known = fast_finish_d(m, x);
+      if (!known && g == 0) sm.late[j] = 1;
+      if (known && coef) {
+        if constexpr (ACC) fast_det_phase(r, df, areq[i], g, G);
+        else fast_det_phase(r, df, mreq[i], g, G);
+      }
+    }
+  }
+  if (lead && warp == 3 && coef) {
+    MixedReq &o = mx(i);
+    fast_regions(r, sm.g[j], o);
+    o.A_scale = fast_a_scale(r, sm.g[j]);
+    if (!pv2) fast_det_factors(r, o, sm.ds[j], sm.ws[j]);
+  }
   sync();
   // S4
-  if (run) {
-    if (!pv2) {
-      if (warp == 0) d_deltas(r.m, s_ac[lane], 0, 2);
-      if (warp == 1) d_deltas(r.m, s_ac[lane], 2, 4);
-      if (warp == 3) d_deltas(r.m, s_ac[lane], 4, 5);
-      if (warp == 2) {
-        phase_conn_combine(r.m, s_pc[lane]);
-        model_d_finish_parts(r.m, s_pc[lane]);
-      }
-    } else {
-      if (warp == 0) d_deltas(r.m, s_ac[lane], 0, 3);
-      if (warp == 1) d_deltas(r.m, s_ac[lane], 3, 5);
-    }
+  if (sm.any_pv2) {
+    if (pv2 && warp >= 2)
+      for (int q = (warp - 2) * G + g; q < kPv2ShiftNodes; q += 2 * G) x.node[q] = fast_pv2_node(m, x, q);
+    sync();
   }
-  if (warp == 2 || warp == 3) {  // Pv2 time-shift nodes: both half-warps, lanes j and j + kCoopReq on request j
-    const Request &rh = s_r[hl];
-    if (hact && !s_bad[hl] && rh.approximant == kPhenomPv2 && rh.m.s.shift_time) {
-      const int j1 = (warp - 1) * (kPv2ShiftNodes / 2);
-      for (int j = (warp - 2) * (kPv2ShiftNodes / 2) + (lane >= kCoopReq ? 1 : 0); j < j1; j += 2)
-        s_shift[hl][j] = pv2_shift_node(rh.m, j);
-    }
-  }
-  sync();
   // S5
-  if (run) {
-    if (warp == 3 && pv2) r.p.t_corr = r.m.s.shift_time ? pv2_shift_solve(r.m, s_shift[lane]) : 0.0;
-    if (want_mixed) {
-      MixedReq &x = mx(i);
-      const double df = s_df[lane];
-      if (warp == 0) mixed_amp_coeffs(r, df, x);
-      if (warp == 1) mixed_phase_coeffs(r, df, x);
-      if constexpr (ACC) {
-        if (warp == 0) acc_amp_coeffs(r, df, areq[i]);
-        if (warp == 1) acc_phase_coeffs(r, df, areq[i]);
-      }
-      if (warp == 2) {
-        mixed_regions(r, df, x);  // sets x.A_scale
-        if (pv2) mixed_pv2_coeffs(r, df, x);
-        else mixed_det_factors_a(r, x, x.A_scale, s_ds[lane], s_ws[lane]);
-      }
-      if (warp == 3 && !pv2) {
-        if constexpr (ACC) acc_det_phase(r, df, areq[i]);
-        else mixed_det_phase(r, df, x);
-      }
-    }
-  }
-  sync();
-  // S6
-  if (act && warp == 0) {
-    int st = s_st[lane];
-    if (!s_bad[lane]) {
-      if (r.m.status) st = 4;
-      if (req) req[i] = r;
-      if (want_mixed) {
-        if (!s_uni[lane]) st = st ? st : 1;
-        if (r.approximant == kPhenomPv2) {  // needs the time shift of S5
-          if constexpr (ACC) {
-            acc_det_phase(r, s_df[lane], areq[i]);
-            acc_pv2_coeffs(r, s_df[lane], areq[i]);
-          } else {
-            mixed_det_phase(r, s_df[lane], mx(i));
-          }
-          mixed_det_factors(r, mx(i), s_ds[lane], s_ws[lane]);
+  if (act && g == 0 && warp == 0) {
+    int st = sm.st[j];
+    if (!bad) {
+      if (pv2) r.p.t_corr = fast_pv2_time_shift(m, x);
+      else if (sm.late[j]) fast_finish_late(m);
+      if (m.status) st = 4;
+      if (coef) {
+        if (!sm.uni[j]) st = st ? st : 1;
+        if (pv2 || sm.late[j]) {
+          if constexpr (ACC) fast_det_phase(r, df, areq[i], 0, 1);
+          else fast_det_phase(r, df, mreq[i], 0, 1);
         }
-        mixed_fold_shared_weights(mx(i), s_wk[lane], ndet);
+        if (pv2) {
+          if constexpr (ACC) acc_pv2_coeffs(r, df, areq[i]);
+          fast_det_factors(r, mx(i), sm.ds[j], sm.ws[j]);
+        }
+        mixed_fold_shared_weights(mx(i), sm.wk[j], ndet);
         if constexpr (ACC) acc_range(r, areq[i]);
       }
     } else {
       st = 4;
-      if (want_mixed) mx(i) = MixedReq{};
+      if (coef) mx(i) = MixedReq{};
     }
-    if (st && want_mixed) mx(i).status = st;
-    if (st && req) req[i].m.status = st;
+    if (st && coef) mx(i).status = st;
     status[i] = st;
+    if (req) {
+      if (st) m.status = st;
+      req[i] = r;
+    }
   }
-  if (warp >= 1 && want_mixed) {
-    // a request is live when S6's status will be 0: valid parameters, model
+  if (warp >= 1 && coef) {
+    // a request is live when S5's status will be 0: valid parameters, model
     // status 0, one uniform grid length
     int kcut = 0;
-    if (act && !s_bad[lane] && r.m.status == 0 && s_st[lane] == 0 && s_uni[lane]) {
-      const StreamDev &s0 = streams[handles[i * ndet]];
-      kcut = min(s0.N, mx(i).n_cut - s0.n0 + 1);  // n_cut: written in S5
+    if (lead && m.status == 0 && sm.st[j] == 0 && sm.uni[j]) {
+      const StreamDev &s0 = streams[__ldcg(handles + i * ndet)];
+      kcut = min(s0.N, mx(i).n_cut - s0.n0 + 1);  // n_cut: written in S3
     }
-    tail(warp, lane, act, i, kcut);
+    tail(warp, lane, act && g == 0, i, kcut);
   }
 }
 
-template <bool ACC>
+template <int REQ, bool ACC>
 __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const GenParams *__restrict__ params, const int *__restrict__ approx, int n, const int *__restrict__ handles,
     int ndet, double T_segment, int tc_from_segment, const StreamDev *__restrict__ streams,
     const double *__restrict__ qnm, Request *req, MixedReq *mreq, AccReq *areq, int want_mixed, int *status,
     const OrderArgs ord) {
-  __shared__ CoopSmem sm;
+  __shared__ CoopSmem<REQ> sm;
   grid_dep_trigger();  // the bin kernel may launch and wait for this grid
   // this block's requests into the work order, on the warps idle in S6 (warp
   // w takes the tiles t = w - 1 mod 3)
@@ -579,25 +573,34 @@ __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const int nt = act ? ord.item_count[i] : 0, i0 = act ? ord.item_start[i] : 0;
     order_append(ord, kcut, nt, i0, warp - 1, kCoopWarps - 1);
   };
-  prologue_coop_body<ACC>(sm, blockIdx.x * kCoopReq, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles, ndet,
-                     T_segment, tc_from_segment, streams, qnm, req, mreq, want_mixed, status,
-                     [] { __syncthreads(); }, tail, areq);
+  prologue_coop_body<REQ, ACC>(sm, blockIdx.x * REQ, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles,
+                               ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status,
+                               [] { __syncthreads(); }, tail);
 }
 
 
+template <int REQ>
+static void launch_coop(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
+                        double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
+                        Request *req, MixedReq *mreq, AccReq *areq, int want_mixed, int *status, cudaStream_t s,
+                        const OrderArgs &ord) {
+  const int grid = (n + REQ - 1) / REQ, threads = kCoopWarps * 32;
+  if (areq)
+    k_prologue_coop<REQ, true><<<grid, threads, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment,
+                                                        streams, qnm, req, nullptr, areq, 1, status, ord);
+  else
+    k_prologue_coop<REQ, false><<<grid, threads, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment,
+                                                         streams, qnm, req, mreq, nullptr, want_mixed, status, ord);
+}
 cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
                             Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s,
                             const OrderArgs &ord, AccReq *areq) {
-  int grid = (n + kCoopReq - 1) / kCoopReq;
-  if (areq)
-    k_prologue_coop<true><<<grid, kCoopWarps * 32, 0, s>>>(params, approx, n, handles, ndet, T_segment,
-                                                           tc_from_segment, streams, qnm, req, nullptr, areq, 1,
-                                                           status, ord);
-  else
-    k_prologue_coop<false><<<grid, kCoopWarps * 32, 0, s>>>(params, approx, n, handles, ndet, T_segment,
-                                                            tc_from_segment, streams, qnm, req, mreq, nullptr,
-                                                            want_mixed, status, ord);
+  // requests per block: few enough that more lanes serve each, while the
+  // blocks find an SM each (two blocks of one SM share its FP64 pipes)
+  if (n <= 4 * kSMs) launch_coop<4>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
+  else if (n <= 8 * kSMs) launch_coop<8>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
+  else launch_coop<16>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
   return cudaGetLastError();
 }
 cudaError_t launch_prologue_serial(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
@@ -1008,17 +1011,22 @@ __device__ __forceinline__ void loop_stage(const LoopArgs &L, int slot0, int k, 
 // barrier of their own), then warp 0 publishes each request's live items
 // (tiles below its cut, at least one: a request that will not be evaluated
 // finishes through its first item with its status) in its claim word.
+__device__ __forceinline__ void loop_group_sync() {  // the barrier of warps 0-3, whose lanes may arrive apart
+  __syncwarp();
+  __barrier_sync_count(1, 128);
+}
 template <int NDET>
-__device__ __forceinline__ void loop_prologue(const LoopArgs &L, CoopSmem &cs, int slot0, int k,
+__device__ __forceinline__ void loop_prologue(const LoopArgs &L, CoopSmem<kCoopReq> &cs, int slot0, int k,
                                               unsigned long long seq0) {
   const BatchArgs &a = L.a;
   loop_stage(L, slot0, k, seq0);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < kCoopWarps)
-    prologue_coop_body<false>(cs, slot0, warp, lane, L.dparams, L.dapprox, slot0 + k, L.dhandles, NDET, L.T_segment, 1,
-                       a.streams, L.qnm, nullptr, const_cast<MixedReq *>(a.mreq), 1, a.status,
-                       [] { asm volatile("bar.sync 1, 128;" ::: "memory"); }, [](int, int, bool, int, int) {});
+    prologue_coop_body<kCoopReq, false>(cs, slot0, warp, lane, L.dparams, L.dapprox, slot0 + k, L.dhandles, NDET,
+                                        L.T_segment, 1, a.streams, L.qnm, nullptr, const_cast<MixedReq *>(a.mreq),
+                                        nullptr, 1, a.status, [] { loop_group_sync(); },
+                                        [](int, int, bool, int, int) {});
   __threadfence();
   __syncthreads();
   if (warp != 0 || lane >= k) return;
@@ -1041,7 +1049,7 @@ constexpr int kLoopPairAt = 8;          // candidate requests from which a claim
 template <int NDET>
 __global__ void __launch_bounds__(kBatchBlock, 3) k_serve_loop(const __grid_constant__ LoopArgs L) {
   using BS = BinSmem<NDET, 1>;
-  constexpr size_t kRaw = sizeof(BS) > sizeof(CoopSmem) ? sizeof(BS) : sizeof(CoopSmem);
+  constexpr size_t kRaw = sizeof(BS) > sizeof(CoopSmem<kCoopReq>) ? sizeof(BS) : sizeof(CoopSmem<kCoopReq>);
   __shared__ __align__(16) unsigned char s_raw[kRaw];
   __shared__ int s_kind, s_a, s_b;
   __shared__ unsigned long long s_seq;
@@ -1174,7 +1182,7 @@ __global__ void __launch_bounds__(kBatchBlock, 3) k_serve_loop(const __grid_cons
                             });
       }
     } else {
-      loop_prologue<NDET>(L, *(CoopSmem *)s_raw, a0, b0, seq);
+      loop_prologue<NDET>(L, *(CoopSmem<kCoopReq> *)s_raw, a0, b0, seq);
     }
     if (tid == 0) {
       const unsigned long long dt = (unsigned long long)(global_ns() - tw0);

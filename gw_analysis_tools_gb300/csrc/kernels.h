@@ -6,6 +6,7 @@
 
 #include "../../include/gwgpu.h"
 #include "phenom_acc.h"
+#include "phenom_fast.h"
 #include "phenom_mixed.h"
 
 namespace gwk {
@@ -41,6 +42,7 @@ struct StreamDev {
   const gwt::ff *wf;
   const float *dev;
   double dfq;
+  const gwt::GridConst *grid;  // of df, of dfq
 };
 
 struct Item {
@@ -73,8 +75,8 @@ cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet
                              cudaStream_t s);
 // One of the two: two-float bins when every stream has its pairs (and the
 // tables reach its grid), else FP64 bins.  partials: 2 kMaxDet per block.
-cudaError_t launch_plain_any(const Request &r, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
-                             const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
+cudaError_t launch_plain_any(const Request &r, const gwt::FastX &fx, const StreamDev *streams, int ndet,
+                             const gwt::AccTables &tab, const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
                              cudaStream_t s);
 int plain_blocks(int N);
 cudaError_t plain_acc_preload();

@@ -89,9 +89,10 @@ int gwgpu_mcmc_likelihood_extrinsic_noalloc(gwgpu_context *c, const gwgpu_gen_pa
   std::memcpy(&gp, p, sizeof(gp));
   gp.tc = T_segment - gp.tc;  // mcmc_gw.cpp:2466-2473
   gwt::Request r;
-  gwt::request_prologue(r, gp, ap, dets, ndet, c->qnm_host.data());
+  gwt::FastX fx;
+  gwt::fast_request(r, fx, gp, ap, dets, ndet, c->qnm_host.data());
   if (r.m.status) return GWGPU_EDOMAIN;  // nothing is launched; d_loglik is left as it was
-  cudaError_t e = gwk::launch_plain_any(r, sd, ndet, c->acc, c->acc_lut, scratch,
+  cudaError_t e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, scratch,
                                         (unsigned *)(scratch + kNoAllocPartials), d_loglik, (cudaStream_t)stream);
   return e == cudaSuccess ? GWGPU_OK : GWGPU_ECUDA;
 }

@@ -73,8 +73,8 @@ GW_HD uint64_t radians_q64(double ph) { return acc_turns(ph * (1.0 / (2.0 * 3.14
 
 // ---- prologue parts, after the mixed form's of the same request ----
 // Detector phases (as mixed_det_phase): t_c enters as turns, t_c f, so that the
-// whole turns of a long segment leave no rounding behind.
-GW_HD void acc_det_phase(const Request &r, double df, AccReq &x) {
+// whole turns of a long segment leave no rounding behind.  Detectors d0, d0 + step, ...
+GW_HD void acc_det_phase(const Request &r, double df, AccReq &x, int d0 = 0, int step = 1) {
   const ModelD &m = r.m;
   const bool pv2 = r.approximant == kPhenomPv2;
   const double inv2pi = 1.0 / (2.0 * kPi);
@@ -82,7 +82,7 @@ GW_HD void acc_det_phase(const Request &r, double df, AccReq &x) {
   const double c1 = pv2 ? r.p.t_corr * df : -m.tcs * df * inv2pi;
   const uint64_t q1 = acc_turns(c1) - acc_turns_prod(m.s.tc, df);
   x.tc = (float)m.s.tc;
-  for (int d = 0; d < r.ndet && d < kMaxDet; d++) {
+  for (int d = d0; d < r.ndet && d < kMaxDet; d += step) {
     double Gre, Gim;
     mixed_det_G(r, d, Gre, Gim);
     x.L0[d] = q0;

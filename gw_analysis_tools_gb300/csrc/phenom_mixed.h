@@ -461,7 +461,7 @@ GW_HD void mixed_det_G(const Request &r, int d, double &Gre, double &Gim) {
 // Detectors in two independent parts: the linear phases and projections
 // (needs the time shift), and the finalize factors (needs the amplitude
 // scale).
-GW_HD void mixed_det_phase(const Request &r, double df, MixedReq &x) {
+GW_HD void mixed_det_phase(const Request &r, double df, MixedReq &x, int d0 = 0, int step = 1) {
   const ModelD &m = r.m;
   const bool pv2 = (r.approximant == kPhenomPv2);
   // ---------------- linear phase per detector, in turns (f = n df):
@@ -471,7 +471,7 @@ GW_HD void mixed_det_phase(const Request &r, double df, MixedReq &x) {
   double c0 = (m.tcl * m.fref - m.phic) * inv2pi;
   double c1 = -m.tcl * df * inv2pi;
   if (pv2) c1 += r.p.t_corr * df;
-  for (int d = 0; d < r.ndet; d++) {
+  for (int d = d0; d < r.ndet; d += step) {
     x.det[d].L0 = turns_q64(c0);
     x.det[d].L1 = turns_q64(c1 - r.det[d].tau * df * inv2pi);
     mixed_det_G(r, d, x.det[d].Gre, x.det[d].Gim);
