@@ -262,8 +262,7 @@ cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev 
   }
   if (!acc) return launch_plain(r, streams, ndet, partials, counter, out, nullptr, s);
   AccReq x;
-  fast_acc(r, fx, grid_const(streams[0].dfq), x, ds, ws);
-  mixed_fold_shared_weights(x.m, wk, ndet);
+  fast_acc(r, fx, grid_const(streams[0].dfq), x, ds, ws, wk);
   return launch_plain_acc(x, streams, ndet, tab, lut, partials, counter, out, s);
 }
 cudaError_t plain_acc_preload() {

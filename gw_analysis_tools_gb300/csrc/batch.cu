@@ -179,8 +179,11 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   if (timing) cudaEventRecord(c->t_ev[0], L.stream);
   cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (size_t)(n + 32 + gwk::kOrderBuckets), L.stream);
   if (e != cudaSuccess) return c->fail(e, "batch counters");
-  // mixed and two-float forms: the prologue writes the work order
-  const bool ordered = form != kFormFp64 && c->order_items && !c->prologue_serial;
+  int grid = std::min(pl.nitems, persistent_grid(c->device, form, ndet, occ));
+  if (grid < 1) grid = 1;
+  // mixed and two-float forms: the prologue writes the work order, unless every
+  // item starts at once (its atomics take 3 us at the prologue's end)
+  const bool ordered = form != kFormFp64 && c->order_items && !c->prologue_serial && pl.nitems > grid;
   const int mixed = form == kFormMixed;
   gwk::OrderArgs ord;
   if (ordered) {
@@ -226,8 +229,6 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   a.areq = form == kFormAcc ? (const gwt::AccReq *)reqs : nullptr;
   a.acc = c->acc;
   a.lut = c->acc_lut;
-  int grid = std::min(pl.nitems, persistent_grid(c->device, form, ndet, occ));
-  if (grid < 1) grid = 1;
   if (form == kFormAcc) e = gwk::launch_batch_acc(a, grid, L.stream, c->pdl);
   else e = gwk::launch_batch(a, mixed, grid, occ, L.stream, c->pdl);
   if (&L == &c->lane) {

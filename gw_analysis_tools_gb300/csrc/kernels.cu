@@ -280,14 +280,14 @@ __device__ __forceinline__ int order_bucket(int kcut, int t, int tile) {
   const int lp = min(np, (live + kSegBins - 1) / kSegBins);
   return (int)((long long)(np - lp) * (kOrderBuckets - 1) / np);  // 0: all passes live
 }
-// Warp-wide: lane l appends the items t = t0, t0 + dt, ... of its request
+// Warp-wide: each lane appends the items t = t0, t0 + dt, ... of its request
 // (kcut: end of its live bins, nt items from i0) to their buckets.  Lanes that
 // draw the same bucket add to it once.  Every lane of the warp calls this
 // (nt = 0 for none).
 __device__ __forceinline__ void order_append(const OrderArgs &o, int kcut, int nt, int i0, int t0, int dt) {
   const int lane = threadIdx.x & 31;
-  const int ntmax = __reduce_max_sync(0xffffffffu, nt);
-  for (int t = t0; t < ntmax; t += dt) {
+  const int rounds = __reduce_max_sync(0xffffffffu, nt > t0 ? (nt - t0 + dt - 1) / dt : 0);
+  for (int q = 0, t = t0; q < rounds; q++, t += dt) {
     const int b = t < nt ? order_bucket(kcut, t, o.tile) : -1;
     const unsigned grp = __match_any_sync(0xffffffffu, b);
     const int leader = __ffs(grp) - 1;
@@ -298,29 +298,6 @@ __device__ __forceinline__ void order_append(const OrderArgs &o, int kcut, int n
   }
 }
 
-// Cooperative prologue: the constants of a group of REQ requests on four warps.
-//
-// An FP64 instruction occupies a sub-partition's FP64 pipe for 64 cycles
-// whatever the number of active lanes, so the time is the number of FP64
-// instructions on the longest warp of each stage.  The parts of phenom_fast.h
-// are spread over the four warps (one per sub-partition), and 32 / REQ lanes
-// serve each request, so that the calibration fits, the PN coefficients, the
-// sines and cosines, the detectors and the Pv2 time-shift nodes run as lanes of
-// one instruction stream.  Lane l works on request l % REQ of the group.
-//   S0  parameters and streams into shared memory
-//   S1  every lane: masses and spins;  W0 source, Pv2: chi_p; ringdown
-//       frequencies;  W1, W2 sines and cosines of the sky, inclination and
-//       phase angles;  W3 roots and logarithms of M and f_ref, amplitude;
-//       all: calibration fits, PN coefficients
-//   S2  W0 ringdown side of the amplitude connection, detector projections;
-//       W1 powers at f2, inspiral amplitude; Pv2: Euler angle coefficients;
-//       W2 D: time shift / Pv2: J frame;  W3 f2 angle, inspiral phase, phase at f_ref
-//   S3  W0 intermediate amplitude, amplitude coefficients;  W1 connections,
-//       phase coefficients;  W2 D: detector phases / Pv2: angles;  W3 regions, D: factors
-//   S4  Pv2: W2, W3 time-shift nodes
-//   S5  W0 Pv2: detector phases and factors; status;  W1-W3 the bin kernel's work order
-// REQ: 4 where the blocks then still fit the SMs one each, else 8 or 16
-// (launch_prologue); the serving loop claims up to 16.
 constexpr int kSMs = 152;  // GB300
 constexpr int kCoopWarps = 4, kCoopReq = 16;
 template <int REQ>
@@ -331,26 +308,29 @@ struct CoopSmem {
   GridConst g[REQ];
   double ds[REQ][kMaxDet], ws[REQ][kMaxDet];  // stream scales
   unsigned long long wk[REQ][kMaxDet];        // and weight keys
+  double f[REQ][kMaxDet][kAccPerDet];         // finalize factors
   double T[REQ];                              // segment length t_c counts from
   int det[REQ][kMaxDet];
-  int ap[REQ], st[REQ], uni[REQ], late[REQ];
+  int ap[REQ], st[REQ], uni[REQ], late[REQ], big[REQ], N[REQ], n0[REQ], ncut[REQ], item0[REQ], items[REQ];
   int any_pv2;
 };
 // The cooperative prologue of requests base .. base + REQ - 1 (those below n):
 // warp (0..3) and lane are the thread's place in the group, sync() the group's
-// barrier.  In S5, while warp 0 stores the results, warps 1-3 call
-// tail(warp, lane, act, i, kcut) with kcut the end of request i's live bins (0
-// when it will not be evaluated); act is set on one lane per request; tail is
-// warp-collective.  ACC: the FP64 form's constants (areq) instead of the mixed
+// barrier.  head(i, first, count) gives request i's items (S0).  In S6, while
+// warp 0 stores the results, warps 1-3 call tail(slot, first, count, kcut) with
+// kcut the end of the request's live bins (0 when it will not be evaluated) on
+// the slots 0 .. 3 * 32 / REQ - 1 of each request (count 0: a lane without one);
+// tail is warp-collective.  ACC: the FP64 form's constants (areq) instead of the mixed
 // form's (mreq); coef: either is wanted (else req alone).
-template <int REQ, bool ACC, class Sync, class Tail>
+template <int REQ, bool ACC, class Sync, class Head, class Tail>
 __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, int warp, int lane,
                                                    const GenParams *__restrict__ params,
                                                    const int *__restrict__ approx, int n,
                                                    const int *__restrict__ handles, int ndet, double T_segment,
                                                    int tc_from_segment, const StreamDev *__restrict__ streams,
                                                    const double *__restrict__ qnm, Request *req, MixedReq *mreq,
-                                                   AccReq *areq, int coef, int *status, Sync sync, Tail tail) {
+                                                   AccReq *areq, int coef, int *status, Sync sync, Head head,
+                                                   Tail tail) {
   constexpr int G = 32 / REQ;  // lanes of a warp per request
   const int j = lane % REQ, g = lane / REQ, i = base + j, cnt = min(REQ, n - base);
   const bool act = j < cnt;
@@ -373,6 +353,9 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
           if (streams[__ldcg(handles + i * ndet + d)].N != s0.N) st = 1;
         sm.st[j] = st;
         sm.uni[j] = s0.uniform_int;
+        sm.N[j] = s0.N;
+        sm.n0[j] = s0.n0;
+        head(i, sm.item0[j], sm.items[j]);
         sm.ap[j] = __ldcg(approx + i);
         sm.late[j] = 0;
       }
@@ -402,9 +385,38 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
   const int ap = act ? sm.ap[j] : 0;
   const bool bad = act && (!(p.mass1 > 0) || !(p.mass2 > 0) || !(p.Luminosity_Distance > 0) || (ap != 0 && ap != 1));
   const bool run = act && !bad, pv2 = run && ap == kPhenomPv2;
+  const bool lead = run && g == 0;  // one lane per request
+  if (lead && warp == 0) {
+    r.approximant = ap;
+    r.ndet = ndet;
+    m.s.pv2 = pv2;
+    fast_eta(x, p);
+    fast_fixed(m);
+    if (pv2) {
+      sm.any_pv2 = 1;
+      fast_pv2_spins(m.s, p);
+    }
+  }
+  if (lead && warp == 1) fast_inverses(x, p);
+  {
+    constexpr int kTrigWarps = G >= 4 ? 1 : 2;  // warp 2, or warps 1 and 2
+    const int slot = (2 - warp) * G + g;
+    if (run && warp <= 2 && warp > 2 - kTrigWarps)
+      for (int a = slot; a < (pv2 ? 5 : 4); a += kTrigWarps * G) {
+        const double ang = a == 0 ? p.gmst - p.RA : a == 1 ? p.DEC : a == 2 ? p.psi : a == 3 ? p.incl_angle : p.phiRef;
+        sincos(ang, &x.sn[a], &x.cn[a]);
+      }
+  }
+  if (run && warp == 3 && g < 2) {  // lane group 0: M, 1: f_ref
+    const double v = g == 0 ? (p.mass1 * kMsolSec + p.mass2 * kMsolSec) : p.f_ref, c = cbrt(v), l = log(v);
+    (g == 0 ? x.cM : x.cfr) = c;
+    (g == 0 ? x.lM : x.lfr) = l;
+  }
+  sync();
+  // S2
   if (run) {
-    const FastCore k = fast_core(p);
-    if constexpr (G >= 8) {  // rows on the two warps with the least before
+    const FastCore k = fast_core(p, x);
+    if constexpr (G >= 8) {
       if (warp == 1)
         for (int q = g; q < 19; q += G) fast_fit(m.l, k, q);
       if (warp == 2)
@@ -413,148 +425,154 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
       for (int q = warp * G + g; q < kPnRows; q += kCoopWarps * G) fast_pn(m, k, q);
       for (int q = (kCoopWarps - 1 - warp) * G + g; q < 19; q += kCoopWarps * G) fast_fit(m.l, k, q);
     }
-    if (warp == 0 && g == 0) {
-      r.approximant = ap;
-      r.ndet = ndet;
-      fast_store(m.s, x, p, k);
+    if (warp == 3) fast_antenna(r, x, sm.det[j], g, G);
+    if (lead && warp == 0) {
+      fast_store(m.s, p, k);
       if (tc_from_segment) m.s.tc = sm.T[j] - p.tc;
-      fast_fixed(m);
-      x.M34 = sqrt(k.M * sqrt(k.M));
-      if (pv2) {
-        sm.any_pv2 = 1;
-        fast_pv2_spins(m.s, p, k);
-      }
       fast_ring(m.s, x, k, qnm);
     }
-    if (warp == 1 || warp == 2) {
-      for (int a = (warp - 1) * G + g; a < (pv2 ? 5 : 4); a += 2 * G) {
-        const double ang = a == 0 ? p.gmst - p.RA : a == 1 ? p.DEC : a == 2 ? p.psi : a == 3 ? p.incl_angle : p.phiRef;
-        sincos(ang, &x.sn[a], &x.cn[a]);
-      }
+    if (lead && warp == 3) {
+      m.s.cos_incl = x.cn[3];
+      m.s.fac_incl = .5 * (1 + x.cn[3] * x.cn[3]);
+      fast_amp0(m, x, p, k);
     }
-    if (warp == 3 && g < 2) {  // lane group 0: M, 1: f_ref
-      const double v = g == 0 ? k.M : p.f_ref, c = cbrt(v), l = log(v);
-      if (g == 0) {
-        x.cM = c;
-        x.lM = l;
-        fast_amp0(m, x, p, k);
-      } else {
-        x.cfr = c;
-        x.lfr = l;
-      }
-    }
-  }
-  sync();
-  const bool lead = run && g == 0;  // one lane per request
-  // S2
-  if (lead && warp == 0) {
-    m.s.cos_incl = x.cn[3];
-    m.s.fac_incl = .5 * (1 + x.cn[3] * x.cn[3]);
-    fast_high(m, x);
-  }
-  if (run && warp == 0) {
-    fast_antenna(r, x, sm.det[j], g, G);
-  }
-  if (lead && warp == 1) {
-    fast_f2_powers(x);
-    fast_low_amp(m, x);
-    if (pv2) pv2_euler_coeffs(r.p.ac, r.p.ec, m.s);
-  }
-  if (lead && warp == 2) {
-    if (pv2) fast_pv2_frame(m.s, r.p, p, x);
-    else fast_time_shift(m, x);
-  }
-  if (lead && warp == 3) {
-    fast_f2_atan(m, x);
-    fast_low_phase(m, x);
-    fast_fref_phase(m, x);
   }
   sync();
   // S3
-  const double df = sm.g[act ? j : 0].df;
-  if (lead && warp == 0) {
-    fast_quartic(m, x);
-    if (req) fast_deltas(m, x);
-    if (coef) {
-      fast_amp_coeffs(m, x, sm.g[j], mx(i));
-      if constexpr (ACC) acc_amp_coeffs(r, df, areq[i]);
+  if (lead && warp == 0) fast_high(m, x);
+  if (run && warp == 1) {
+    for (int q = g; q < kLowRows; q += G) fast_low(m, x, q);
+    if (g == 0) fast_f2_powers(x);
+  }
+  if (run && warp == 2) {
+    if (pv2) {
+      if (g < 2) fast_pv2_frame(m.s, r.p, p, x, g);  // a lane for each of its two azimuths
+    } else if (g == 0) {
+      fast_time_shift(m, x);
     }
+  }
+  if (lead && warp == 3) {
+    fast_f2_atan(m, x);
+    if (pv2) fast_pv2_euler(r.p, m.s);
+    else fast_fref_phase(m, x);
+  }
+  sync();
+  // S4
+  const GridConst &gc = sm.g[act ? j : 0];
+  if (warp == 0) {
+    if (lead) {
+      fast_quartic(m, x);
+      if (req) fast_deltas(m, x);
+    }
+    __syncwarp();  // the quartic, from lane group 0
+    if (run && coef) {
+      for (int q = g; q < 10; q += G) fast_ins_amp(m, x, gc, mx(i), q);
+      if (g < 5) fast_int_amp(m, x, gc, mx(i), g, G);
+    }
+  }
+  if (run && warp == 1 && coef) {
+    const double A = fast_a_scale(r, gc);
+    for (int d = g; d < ndet && d < kMaxDet; d += G) fast_det_factor(r, d, A, sm.ws[j][d], sm.ds[j][d], sm.f[j][d]);
+    if (g == 0) mx(i).A_scale = A;
   }
   if (lead && warp == 1) {
     fast_connect(m, x);
     if (coef) {
-      fast_phase_coeffs(m, x, sm.g[j], mx(i));
-      if constexpr (ACC) acc_phase_coeffs(r, df, areq[i]);
+      fast_phase_coeffs(m, x, gc, mx(i));
+      fast_atan_coeffs(m, gc, mx(i));
+      if constexpr (ACC) {
+        acc_phase_coeffs(r, gc.df, areq[i]);
+        sm.big[j] = fast_range_d(m, x);
+      }
     }
   }
   if (run && warp == 2) {
     if (pv2) {
       if (g == 0) {
         fast_pv2_finish(m, r.p, x);
-        if (coef) fast_pv2_coeffs(r, x, sm.g[j], mx(i));
+        if (coef) {
+          fast_pv2_coeffs(r, x, gc, mx(i));
+          if constexpr (ACC) sm.late[j] = fast_range_p(r.p);
+        }
       }
     } else {  // each lane sets the same linear constants, then takes its detectors
       const bool known = fast_finish_d(m, x);
       if (!known && g == 0) sm.late[j] = 1;
       if (known && coef) {
-        if constexpr (ACC) fast_det_phase(r, df, areq[i], g, G);
-        else fast_det_phase(r, df, mreq[i], g, G);
+        if constexpr (ACC) fast_det_phase(r, gc.df, areq[i], g, G);
+        else fast_det_phase(r, gc.df, mreq[i], g, G);
       }
+      if (g == 0 && coef) fast_ring_amp(m, x, gc, mx(i));
     }
   }
-  if (lead && warp == 3 && coef) {
+  if (run && warp == 3 && coef) {
     MixedReq &o = mx(i);
-    fast_regions(r, sm.g[j], o);
-    o.A_scale = fast_a_scale(r, sm.g[j]);
-    if (!pv2) fast_det_factors(r, o, sm.ds[j], sm.ws[j]);
+    for (int q = g; q < 5; q += G) {
+      const int b = fast_region(m, gc, o, q);
+      if (q == 4) sm.ncut[j] = b - 1;
+    }
+    for (int q = g; q < 12; q += G) fast_ins_phase(m, x, gc, o, q);
+    if (g == 0) {
+      o.approximant = ap;
+      o.ndet = ndet;
+      o.wshared = fast_shared(sm.wk[j], ndet) ? 1 : 0;
+      if (pv2) fast_ring_amp(m, x, gc, o);
+      if constexpr (ACC) acc_amp_coeffs(r, gc.df, areq[i]);
+    }
   }
   sync();
-  // S4
+  // S5
   if (sm.any_pv2) {
     if (pv2 && warp >= 2)
       for (int q = (warp - 2) * G + g; q < kPv2ShiftNodes; q += 2 * G) x.node[q] = fast_pv2_node(m, x, q);
+    if constexpr (ACC) {
+      if (pv2 && warp == 0 && g == 0 && coef) acc_pv2_coeffs(r, gc.df, areq[i]);
+    }
     sync();
   }
-  // S5
+  // S6
+  if (run && warp == 0 && pv2) {
+    r.p.t_corr = fast_pv2_time_shift(m, x);  // the same value in every lane
+    if (coef) {
+      if constexpr (ACC) fast_det_phase(r, gc.df, areq[i], g, G);
+      else fast_det_phase(r, gc.df, mreq[i], g, G);
+    }
+  }
   if (act && g == 0 && warp == 0) {
     int st = sm.st[j];
     if (!bad) {
-      if (pv2) r.p.t_corr = fast_pv2_time_shift(m, x);
-      else if (sm.late[j]) fast_finish_late(m);
-      if (m.status) st = 4;
-      if (coef) {
-        if (!sm.uni[j]) st = st ? st : 1;
-        if (pv2 || sm.late[j]) {
-          if constexpr (ACC) fast_det_phase(r, df, areq[i], 0, 1);
-          else fast_det_phase(r, df, mreq[i], 0, 1);
+      if (!pv2 && sm.late[j]) {
+        fast_finish_late(m);
+        if (coef) {
+          if constexpr (ACC) fast_det_phase(r, gc.df, areq[i], 0, 1);
+          else fast_det_phase(r, gc.df, mreq[i], 0, 1);
         }
-        if (pv2) {
-          if constexpr (ACC) acc_pv2_coeffs(r, df, areq[i]);
-          fast_det_factors(r, mx(i), sm.ds[j], sm.ws[j]);
-        }
-        mixed_fold_shared_weights(mx(i), sm.wk[j], ndet);
-        if constexpr (ACC) acc_range(r, areq[i]);
       }
+      if (m.status) st = 4;
+      if (coef && !sm.uni[j]) st = st ? st : 1;
+      if constexpr (ACC) areq[i].fp64_phase = sm.big[j] | (pv2 ? sm.late[j] : 0);
     } else {
       st = 4;
       if (coef) mx(i) = MixedReq{};
     }
-    if (st && coef) mx(i).status = st;
+    if (coef) mx(i).status = st;
     status[i] = st;
     if (req) {
       if (st) m.status = st;
       req[i] = r;
     }
   }
+  if (run && warp == 3 && coef) {
+    const bool shared = fast_shared(sm.wk[j], ndet);
+    for (int e = g; e < kMaxDet * kAccPerDet; e += G)
+      mx(i).fc[e] = fast_factor_entry(sm.f[j], e, ndet, pv2, shared);
+  }
   if (warp >= 1 && coef) {
-    // a request is live when S5's status will be 0: valid parameters, model
+    // a request is live when its status will be 0: valid parameters, model
     // status 0, one uniform grid length
     int kcut = 0;
-    if (lead && m.status == 0 && sm.st[j] == 0 && sm.uni[j]) {
-      const StreamDev &s0 = streams[__ldcg(handles + i * ndet)];
-      kcut = min(s0.N, mx(i).n_cut - s0.n0 + 1);  // n_cut: written in S3
-    }
-    tail(warp, lane, act && g == 0, i, kcut);
+    if (run && m.status == 0 && sm.st[j] == 0 && sm.uni[j]) kcut = min(sm.N[j], sm.ncut[j] - sm.n0[j] + 1);
+    tail((warp - 1) * G + g, act ? sm.item0[j] : 0, act ? sm.items[j] : 0, kcut);
   }
 }
 
@@ -566,16 +584,17 @@ __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const OrderArgs ord) {
   __shared__ CoopSmem<REQ> sm;
   grid_dep_trigger();  // the bin kernel may launch and wait for this grid
-  // this block's requests into the work order, on the warps idle in S6 (warp
-  // w takes the tiles t = w - 1 mod 3)
-  auto tail = [&](int warp, int lane, bool act, int i, int kcut) {
-    if (!ord.fill) return;
-    const int nt = act ? ord.item_count[i] : 0, i0 = act ? ord.item_start[i] : 0;
-    order_append(ord, kcut, nt, i0, warp - 1, kCoopWarps - 1);
+  // this block's requests into the work order, on the warps idle in S6
+  auto head = [&](int i, int &first, int &count) {
+    first = ord.fill ? ord.item_start[i] : 0;
+    count = ord.fill ? ord.item_count[i] : 0;
+  };
+  auto tail = [&](int slot, int first, int count, int kcut) {
+    if (ord.fill) order_append(ord, kcut, count, first, slot, (kCoopWarps - 1) * (32 / REQ));
   };
   prologue_coop_body<REQ, ACC>(sm, blockIdx.x * REQ, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles,
                                ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status,
-                               [] { __syncthreads(); }, tail);
+                               [] { __syncthreads(); }, head, tail);
 }
 
 
@@ -1026,7 +1045,7 @@ __device__ __forceinline__ void loop_prologue(const LoopArgs &L, CoopSmem<kCoopR
     prologue_coop_body<kCoopReq, false>(cs, slot0, warp, lane, L.dparams, L.dapprox, slot0 + k, L.dhandles, NDET,
                                         L.T_segment, 1, a.streams, L.qnm, nullptr, const_cast<MixedReq *>(a.mreq),
                                         nullptr, 1, a.status, [] { loop_group_sync(); },
-                                        [](int, int, bool, int, int) {});
+                                        [](int, int &, int &) {}, [](int, int, int, int) {});
   __threadfence();
   __syncthreads();
   if (warp != 0 || lane >= k) return;

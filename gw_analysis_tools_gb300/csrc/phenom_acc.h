@@ -34,7 +34,8 @@ struct AccLut {
 
 // Largest bin count whose indices are exact in FP32.
 constexpr int kAccMaxN = 1 << 24;
-// Largest two-float phase term, in turns (acc_range).
+// Largest phase term carried in two floats, in turns: its rounding, ~4e-15 of it,
+// must stay below the FP64 series' own.
 constexpr double kAccMaxTurns = 12.0;
 
 // Constants of one request: the mixed form's (regions, FP64 phase
@@ -166,7 +167,7 @@ GW_HD void acc_range(const Request &r, AccReq &x) {
   }
   x.fp64_phase = v < kAccMaxTurns ? 0 : 1;  // also for NaN
 }
-// The whole request (host, and the plain form).
+// The whole request after request_prologue (one thread; the check of phenom_fast.h's).
 GW_HDNI int acc_prologue(const Request &r, double df, AccReq &x, const double *dscale, const double *wscale) {
   mixed_prologue(r, df, x.m, dscale, wscale);
   acc_det_phase(r, df, x);

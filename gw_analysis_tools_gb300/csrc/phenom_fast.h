@@ -27,23 +27,27 @@
 
 namespace gwt {
 
-// Literals at M f = 0.018: powers of (pi 0.018)^(1/3), ln(pi 0.018), 0.018^(1/3), ln 0.018;
-// the amplitude's sqrt(pi 40 / 192) pi^(-7/6) and sqrt(pi / 30) pi^(-7/6); the harmonics' roots.
-constexpr double kFastV2 = 0.147326742094114666947;
-constexpr double kFastV3 = 0.0565486677646162782923;
-constexpr double kFastV4 = 0.0217051689360657785201;
-constexpr double kFastV5 = 0.00833113099152339819391;
-constexpr double kFastV6 = 0.0031977518259529521925;
-constexpr double kFastV7 = 0.00122739838694045349123;
-constexpr double kFastVm5 = 120.031722105613404997;
-constexpr double kFastL = -2.8726536352365721857;
-constexpr double kFastW = 0.262074139420889660714;
+// Literals: ln 0.018, (pi 0.018)^(1/3), (pi 0.2)^(1/3), 0.2^(3/4); the amplitude's
+// sqrt(pi 40 / 192) pi^(-7/6) and sqrt(pi / 30) pi^(-7/6); the harmonics' roots.
 constexpr double kFastLx = -4.01738352108597235985;
+constexpr double kFastV = 0.383831658535502601325;
+constexpr double kFastVc = 0.85649853169451150001;
+constexpr double kFast34 = 0.299069756244244108382;
 constexpr double kFastAmp = 0.212787510139663399158;
 constexpr double kFastAmpSky = 0.0851150040558653596631;
 constexpr double kFastY2 = 0.157695782626260003015;
 constexpr double kFastY1 = 0.315391565252520006031;
 constexpr double kFastY0 = 0.386274202023189580342;
+// Rows of fast_low: coefficients of the PN terms and fits at M f = 0.014 (rows 0,
+// 1) and 0.018 (rows 2, 3: those of the series times (pi M f)^(-5/3), ln(pi M f)
+// inside), then the constant; the time shift's nodes at 2 rel = M f / (xr / 2).
+#define GWT_LOW_ROWS_LITERALS \
+  {{0.124600161600132787606, 0.0439822971502571053385, 0.0155252002707792052744, 0.00548020133246709511068, 0.00193444246261351428929, 0.0, 0.0000472387883778345077281, 0.0000113852200377848600105, 0.000002744, 0.0, 1.0}, \
+   {5.93334102857775179078, 3.14159265358979323846, 1.4785905019789719309, 0.652404920531797036986, 0.276348923230502041327, 0.0, 0.00787313139630575128802, 0.00216861334053044952582, 0.000588, 0.0, 0.0}, \
+   {17.6838825657661484188, 6.78763397456507990334, 2.60530880598924009842, 0.147326742094114666947, -1.8726536352365721857, 0.383831658535502601325, 0.018, 0.00353800088218201041964, 0.00074177482917455905034, 0.000162, 239.884266903648382923}, \
+   {-982.43792032034157882, -251.393850909817774198, -48.2464593701711129338, 5.45654600348572840543, 55.5555555555555555556, 7.10799367658338150602, 1.0, 0.262074139420889660714, 0.0686828545531999120685, 0.018, -11212.4396631232758396}}
+#define GWT_NODE34_LITERALS {1.42262352803113824098, 1.4814971108637783107, 1.53960071783900203869, 1.5969822136263238218, 1.65368435914272468323, 1.70974556228632557231, 1.76520049047833232268, 1.82008057513937784433, 1.87441443071783610951, 1.92822820546716415098}
+#define GWT_NODEINV_LITERALS {0.625, 0.592105263157894736842, 0.5625, 0.535714285714285714286, 0.511363636363636363636, 0.489130434782608695652, 0.46875, 0.45, 0.432692307692307692308, 0.416666666666666666667}
 
 // What a grid's spacing contributes: df, 1/df, df^(1/3), ln df, df^(-7/6), df^(3/4).
 struct GridConst {
@@ -59,10 +63,10 @@ struct FastCore {
 };
 // Intermediate values of one request between the parts.
 struct FastX {
-  double iM, delta, cM, lM, cfr, lfr, M34;  // M^(1/3), ln M, f_ref^(1/3), ln f_ref, M^(3/4)
+  double iM, eta, ieta, delta, cM, lM, cfr, lfr, M34;  // M^(1/3), ln M, f_ref^(1/3), ln f_ref, M^(3/4)
   double xr, xd, x3, h;                     // ringdown, damping, peak in M f; half the intermediate range
   double v1, d1, v3, d3, ins1, dins1;       // connection values (derivatives by M f)
-  double l2, i2, p2, y2, at2;               // at x2 = xr / 2: ln, 1/x2, x2^(3/4), atan argument and value
+  double l2, i2, p2, rx, at2;               // at x2 = xr / 2: ln, 1/x2, x2^(3/4); xr / xd; the atan there
   double a[5];                              // intermediate amplitude in u = (M f - xm) / h
   double phi_fref;
   int have_phi, pad;
@@ -70,17 +74,28 @@ struct FastX {
   double node[kPv2ShiftNodes];
 };
 
-GW_HDNI FastCore fast_core(const GenParams &in) {
+// The divisions and the root every part needs: eta and sqrt(1 - 4 eta) rounded
+// as the reference's (near equal masses the root shows the last bit of eta); 1/M, 1/eta.
+GW_HDNI void fast_eta(FastX &x, const GenParams &in) {
+  const double m1 = in.mass1 * kMsolSec, m2 = in.mass2 * kMsolSec, M = m1 + m2;
+  x.eta = (m1 * m2) / (M * M);
+  x.delta = sqrt(1. - 4 * x.eta);
+}
+GW_HDNI void fast_inverses(FastX &x, const GenParams &in) {
+  const double m1 = in.mass1 * kMsolSec, m2 = in.mass2 * kMsolSec, M = m1 + m2;
+  x.iM = 1. / M;
+  x.ieta = (M * M) / (m1 * m2);
+  x.M34 = sqrt(M * sqrt(M));
+}
+GW_HD FastCore fast_core(const GenParams &in, const FastX &x) {
   FastCore k;
   k.m1 = in.mass1 * kMsolSec;
   k.m2 = in.mass2 * kMsolSec;
   k.M = k.m1 + k.m2;
-  k.iM = 1. / k.M;
-  // eta and sqrt(1 - 4 eta) rounded as the reference's: near equal masses the
-  // root shows the last bit of eta
-  k.eta = (k.m1 * k.m2) / (k.M * k.M);
-  k.ieta = 1. / k.eta;
-  k.delta = sqrt(1. - 4 * k.eta);
+  k.iM = x.iM;
+  k.eta = x.eta;
+  k.ieta = x.ieta;
+  k.delta = x.delta;
   k.c1 = in.spin1[2];
   k.c2 = in.spin2[2];
   k.cs = 0.5 * (k.c1 + k.c2);
@@ -89,7 +104,7 @@ GW_HDNI FastCore fast_core(const GenParams &in) {
   k.chi_pn = chi_eff - ((38. / 113) * k.eta) * (2 * k.cs);
   return k;
 }
-GW_HD void fast_store(Source &s, FastX &x, const GenParams &in, const FastCore &k) {
+GW_HD void fast_store(Source &s, const GenParams &in, const FastCore &k) {
   s.mass1 = k.m1;
   s.mass2 = k.m2;
   s.spin1x = in.spin1[0];
@@ -115,13 +130,8 @@ GW_HD void fast_store(Source &s, FastX &x, const GenParams &in, const FastCore &
   s.shift_time = in.shift_time;
   s.shift_phase = in.shift_phase;
   s.dep_postmerger = in.dep_postmerger;
-  s.pv2 = 0;
-  s.chip = in.chip;
-  s.phip = in.phip;
   s.f1_phase = 0.018 * k.iM;
   s.f1 = 0.014 * k.iM;
-  x.iM = k.iM;
-  x.delta = k.delta;
 }
 
 // ---- tables by row ----
@@ -287,32 +297,40 @@ GW_HDNI void fast_high(ModelD &m, FastX &x) {
   x.v3 = l.gamma[0] * exp(-l.gamma[1] * y) * (iw * q);
   x.d3 = -x.v3 * iw * (l.gamma[1] + 2 * y * q);
 }
-// Inspiral amplitude and phase with their derivatives at M f = 0.014 and 0.018.
-GW_HDNI void fast_low_amp(const ModelD &m, FastX &x) {
-  // (pi 0.014)^(i/3), 0.014^((7 + i)/3)
-  const double v2 = 0.12460016160013278761, v3 = 0.043982297150257105338, v4 = 0.015525200270779205274,
-               v5 = 0.0054802013324670951107, v6 = 0.0019344424626135142893, r7 = 0.000047238788377834507728,
-               r8 = 0.000011385220037784860011, r9 = 2.744e-6, i3 = 1.0 / (3 * 0.014);
-  const double *p = m.pn_amp, *r = m.l.rho;
-  const double t2 = p[2] * v2, t3 = p[3] * v3, t4 = p[4] * v4, t5 = p[5] * v5, t6 = p[6] * v6, u7 = r[0] * r7,
-               u8 = r[1] * r8, u9 = r[2] * r9;
-  x.v1 = 1.0 + t2 + t3 + t4 + t5 + t6 + u7 + u8 + u9;
-  x.d1 = i3 * (2 * t2 + 3 * t3 + 4 * t4 + 5 * t5 + 6 * t6 + 7 * u7 + 8 * u8 + 9 * u9);
-}
-GW_HDNI void fast_low_phase(const ModelD &m, FastX &x) {
-  // v = (pi 0.018)^(1/3): v^i, ln(pi 0.018), v^-5; w = 0.018^(1/3)
-  constexpr double v2 = kFastV2, v3 = kFastV3, v4 = kFastV4, v5 = kFastV5, v6 = kFastV6, v7 = kFastV7, L = kFastL,
-                   vm5 = kFastVm5, w = kFastW, xx = 0.018, ix = 1.0 / 0.018, i3 = 1.0 / (3 * 0.018);
-  const double *p = m.pn_phase, *g = m.l.sigma;
-  const double K = m.s.k_tf2 * vm5;
-  const double t2 = p[2] * v2, t3 = p[3] * v3, t4 = p[4] * v4, t5 = (p[8] + p[9] * L) * v5,
-               t6 = (p[10] - p[11] * L) * v6, t7 = p[7] * v7;
-  const double S = 1.0 + t2 + t3 + t4 + t5 + t6 + t7;
-  const double dS = i3 * (2 * t2 + 3 * t3 + 4 * t4 + 5 * t5 + 6 * t6 + 7 * t7) + ix * (p[9] * v5 - p[11] * v6);
-  const double n = g[1] * xx + (0.75 * xx * w) * g[2] + (0.6 * xx * w * w) * g[3] + (0.5 * xx * xx) * g[4];
-  const double dn = g[1] + g[2] * w + g[3] * (w * w) + g[4] * xx;
-  x.ins1 = -kPi / 4. + K * S + m.s.inv_eta * n;
-  x.dins1 = K * (dS - (5. * i3) * S) + m.s.inv_eta * dn;
+// Inspiral amplitude and phase with their derivatives at M f = 0.014 and 0.018
+// as rows of literals: rows 0, 1 (amplitude, derivative) over pn_amp[2..6],
+// rho[0..2]; rows 2, 3 (phase, derivative) over pn_phase[2, 3, 4, 7, 8, 10] and,
+// apart, sigma[1..4].
+constexpr int kLowRows = 4, kLowPn = 6, kLowFit = 4;
+#define GWT_LOW_ROWS_INIT GWT_LOW_ROWS_LITERALS
+static const double gwt_low_rows_h[kLowRows][kLowPn + kLowFit + 1] = GWT_LOW_ROWS_INIT;
+#if defined(__CUDACC__)
+static __device__ const double gwt_low_rows_d[kLowRows][kLowPn + kLowFit + 1] = GWT_LOW_ROWS_INIT;
+#endif
+GW_HDNI void fast_low(const ModelD &m, FastX &x, int row) {
+#if defined(__CUDA_ARCH__)
+  const double *t = gwt_low_rows_d[row];
+#else
+  const double *t = gwt_low_rows_h[row];
+#endif
+  const bool amp = row < 2;
+  const double *p = amp ? m.pn_amp : m.pn_phase;
+  const double c[kLowPn] = {p[2], p[3], p[4], p[amp ? 5 : 7], p[amp ? 6 : 8], p[amp ? 1 : 10]};  // pn_amp[1] is zero
+  const double *f = amp ? m.l.rho : m.l.sigma + 1;  // rho[3] is zero
+  double s = t[kLowPn + kLowFit], n = 0.0;
+#pragma unroll
+  for (int j = 0; j < kLowPn; j++) s = fma(t[j], c[j], s);
+#pragma unroll
+  for (int j = 0; j < kLowFit; j++) n = fma(t[kLowPn + j], f[j], n);
+  if (amp) {
+    s += n;
+    if (row == 0) x.v1 = s;
+    else x.d1 = s;
+  } else {
+    s = fma(m.s.k_tf2, s, m.s.inv_eta * n);
+    if (row == 2) x.ins1 = s - kPi / 4.;
+    else x.dins1 = s;
+  }
 }
 // Intermediate and ringdown phase terms at x2 = xr / 2.
 GW_HDNI void fast_f2_powers(FastX &x) {
@@ -322,8 +340,8 @@ GW_HDNI void fast_f2_powers(FastX &x) {
   x.p2 = sqrt(x2 * sqrt(x2));
 }
 GW_HDNI void fast_f2_atan(const ModelD &m, FastX &x) {
-  x.y2 = (0.5 - m.l.alpha[5]) * x.xr / x.xd;
-  x.at2 = atan(x.y2);
+  x.rx = x.xr / x.xd;
+  x.at2 = atan((0.5 - m.l.alpha[5]) * x.rx);
 }
 // Phase at f_ref when it lies in the inspiral (have_phi).
 GW_HDNI void fast_fref_phase(const ModelD &m, FastX &x) {
@@ -362,7 +380,8 @@ GW_HDNI void fast_connect(ModelD &m, const FastX &x) {
   const double b0 = eta * x.ins1 - (b1 * x1 + b2 * l1 - b3 * (ix1 * ix1 * ix1 / 3.));
   const double x2 = 0.5 * x.xr, i2 = x.i2, i2_3 = i2 * i2 * i2;
   const double dint = b1 + b2 * i2 + b3 * (i2_3 * i2);
-  const double dmr = l.alpha[2] * (i2 * i2) + l.alpha[3] * (x.p2 * i2) + l.alpha[4] / (x.xd * (1. + x.y2 * x.y2));
+  const double y2 = (0.5 - l.alpha[5]) * x.rx;
+  const double dmr = l.alpha[2] * (i2 * i2) + l.alpha[3] * (x.p2 * i2) + l.alpha[4] / (x.xd * (1. + y2 * y2));
   const double a1 = dint - dmr;
   const double iv = b0 + b1 * x2 + b2 * x.l2 - b3 * (i2_3 * (1. / 3.));
   const double mr = a1 * x2 - l.alpha[2] * i2 + (4. / 3) * l.alpha[3] * x.p2 + l.alpha[4] * x.at2;
@@ -429,32 +448,67 @@ GW_HDNI void fast_amp0(ModelD &m, const FastX &x, const GenParams &in, const Fas
 }
 
 // ---- IMRPhenomPv2 ----
+#if defined(__CUDA_ARCH__)
+GW_HD double fast_rsqrt(double v) { return rsqrt(v); }
+#else
+GW_HD double fast_rsqrt(double v) { return 1.0 / std::sqrt(v); }
+#endif
+// Euler angle coefficients (pv2_euler_coeffs, IMRPhenomP.cpp:65-144): epsilon's
+// and, with chi_p's terms added, alpha's.
+GW_HDNI void fast_pv2_euler(ModelP &pm, const Source &s) {
+  const double iq = 1. / s.q, im2 = 1. + iq, m2 = 1. / im2, m1 = m2 * iq, d = m1 - m2;
+  const double n = m1 * m2, in = 1. / n, chil = s.chil, c2 = s.chip * s.chip;
+  const double dn = d * im2, n2 = n * n, dn2 = dn * dn, m2s = m2 * m2, dm = d * m2, cm = chil * m2s, cd = chil * dm;
+  const double c2l = chil * chil;
+  double *e = pm.ec, *a = pm.ac;
+  e[0] = -35. / 192 - (5. / 64) * dn;
+  e[1] = -in * ((15. / 128) * cd + (35. / 128) * cm);
+  e[2] = -5515. / 3072 - (4555. / 7168) * dn - n * (515. / 384 + (15. / 256) * dn2 + (175. / 256) * dn);
+  e[3] = -(35. * kPi / 48) - (5. * kPi / 16) * dn + (5. / 16) * (d * d) * chil + (5. / 3) * cd + (2545. / 1152) * cm +
+         in * ((2035. / 21504) * cd + (2995. / 9216) * cm);
+  const double q4 = (15. / 128) * dm * m2s + (35. / 128) * (m2s * m2s);  // (15 d m2^3 + 35 m2^4) / 128
+  e[4] = 4.318908476114694 + (27895885. / 2.1676032e7) * dn +
+         n * (39695. / 86016 + (1615. / 28672) * dn2 - (265. / 14336) * dn) +
+         n2 * (955. / 576 + (15. / 1024) * (dn2 * dn) + (35. / 256) * dn2 + (2725. / 3072) * dn) -
+         (kPi * in) * ((15. / 16) * cd + (35. / 16) * cm) +
+         (c2l * in) * ((375. / 256) * (dm * dm) + (1815. / 256) * (dm * m2s) + (1645. / 192) * (m2s * m2s));
+  const double in2 = in * in, m4 = m2s * m2s;
+  a[0] = e[0];
+  a[1] = e[1];
+  a[2] = e[2] - c2 * in2 * q4;
+  a[3] = e[3] - c2 * chil * (in2 * in) * m4 * ((5. / 128) * dm + (35. / 384) * m2s);
+  a[4] = e[4] + c2 * (in2 * (-(485. / 14336) * (dm * m2s) + (475. / 6144) * m4) +
+                      in * ((15. / 256) * (dm * dm) + (145. / 512) * (dm * m2s) + (575. / 1536) * m4) +
+                      (c2l - 0.25 * c2) * (in2 * in2) * m4 * q4);
+}
 // chi_p and the in-plane angular momenta (PhenomPv2_Param_Transform,
 // IMRPhenomP.cpp:1082-1210; reduced: :822-938), before the ringdown part.
-GW_HDNI void fast_pv2_spins(Source &s, const GenParams &in, const FastCore &k) {
-  s.pv2 = 1;
-  const double q = k.m1 / k.m2;
+GW_HDNI void fast_pv2_spins(Source &s, const GenParams &in) {
+  const double m1 = in.mass1 * kMsolSec, m2 = in.mass2 * kMsolSec, M = m1 + m2, im1 = 1. / m1;
+  const double q21 = m2 * im1, c1 = in.spin1[2], c2 = in.spin2[2];
+  s.chil = c1 + q21 * c2;  // (1 + q) / q chi_eff
+  const double m1_2 = m1 * m1, m2_2 = m2 * m2;
+  const double q = m1 / m2;
   s.q = q;
-  s.chil = (1.0 + q) / q * ((k.m1 * k.c1 + k.m2 * k.c2) * k.iM);
+  s.phip = in.phip;
+  s.chip = in.chip;
   if (!((in.chip + 1) > kCompThresh)) {
-    const double m1_2 = k.m1 * k.m1, m2_2 = k.m2 * k.m2;
-    const double S1 = m1_2 * sqrt(s.spin1y * s.spin1y + s.spin1x * s.spin1x);
-    const double S2 = m2_2 * sqrt(s.spin2y * s.spin2y + s.spin2x * s.spin2x);
-    const double A1 = 2 + 1.5 / q, A2 = 2 + 1.5 * q;
+    const double S1 = m1_2 * sqrt(in.spin1[1] * in.spin1[1] + in.spin1[0] * in.spin1[0]);
+    const double S2 = m2_2 * sqrt(in.spin2[1] * in.spin2[1] + in.spin2[0] * in.spin2[0]);
+    const double A1 = 2 + 1.5 * q21, A2 = 2 + 1.5 * q;
     const double a1 = A1 * S1, a2 = A2 * S2;
-    s.chip = (a2 > a1 ? a2 : a1) / (k.m2 > k.m1 ? A2 * m2_2 : A1 * m1_2);
-  } else {
-    s.chip = in.chip;
-    s.phip = in.phip;
+    s.chip = (a2 > a1 ? a2 : a1) / (m2 > m1 ? A2 * m2_2 : A1 * m1_2);
   }
-  const double f1 = k.m1 * k.iM, f2 = k.m2 * k.iM;
-  s.SP = s.chip * f1 * f1;
-  s.SL = k.c1 * f1 * f1 + k.c2 * f2 * f2;
+  const double iM2 = 1.0 / (M * M);
+  s.SP = s.chip * (m1_2 * iM2);
+  s.SL = (c1 * m1_2 + c2 * m2_2) * iM2;
 }
 // The J frame (IMRPhenomP.cpp:1130-1210): rotations by -phi_J about z, -theta_J
 // about y and kappa about z, their sines and cosines from the components that
 // define the angles.  sn/cn: of the inclination [3] and phiRef [4].
-GW_HDNI void fast_pv2_frame(Source &s, ModelP &pm, const GenParams &in, const FastX &x) {
+// part 0: all but alpha0; part 1: alpha0 (the same instructions up to the one atan2
+// each takes, for two lanes); part 2: both.
+GW_HDNI void fast_pv2_frame(Source &s, ModelP &pm, const GenParams &in, const FastX &x, int part) {
   const double m1_2 = s.mass1 * s.mass1, m2_2 = s.mass2 * s.mass2;
   const double v = 1.4645918875615231 * (x.cM * x.cfr), v2 = v * v, eta = s.eta;  // (pi M f_ref)^(1/3)
   const double L0 = s.M * s.M * (eta * (1.0 + (1.5 + eta / 6.0) * v2 + (3.375 - (19.0 * eta) / 8. - eta * eta / 24.0) * (v2 * v2))) / v;
@@ -469,31 +523,27 @@ GW_HDNI void fast_pv2_frame(Source &s, ModelP &pm, const GenParams &in, const Fa
     Jy = m1_2 * s.chip * sp;
   }
   const double Jz = L0 + m1_2 * s.spin1z + m2_2 * s.spin2z;
-  const double p2 = Jx * Jx + Jy * Jy, p = sqrt(p2), iJ = 1.0 / sqrt(p2 + Jz * Jz);
-  double cA = 1.0, sA = 0.0;
-  s.phi_aligned = 0.0;
-  if (p2 > 0) {
-    const double ip = 1.0 / p;
-    cA = Jx * ip;
-    sA = -Jy * ip;
-    s.phi_aligned = -atan2(Jy, Jx);
-  }
-  const double cB = Jz * iJ, sB = -p * iJ;
+  const double p2 = Jx * Jx + Jy * Jy, ip = p2 > 0 ? fast_rsqrt(p2) : 0.0, iJ = fast_rsqrt(p2 + Jz * Jz);
+  const double cA = p2 > 0 ? Jx * ip : 1.0, sA = -Jy * ip, cB = Jz * iJ, sB = -(p2 * ip) * iJ;
   const double si = x.sn[3], ci = x.cn[3], sr = x.sn[4], cr = x.cn[4];
   // N = (si cos(pi/2 - phiRef), si sin(pi/2 - phiRef), ci) through A and B
   double tx = si * sr, ty = si * cr, t1 = tx * cA - ty * sA;
-  double ny = tx * sA + ty * cA;
-  double nx = t1 * cB + ci * sB, nz = -t1 * sB + ci * cB;
-  const double r2 = nx * nx + ny * ny;
-  double cK = 1.0, sK = 0.0, r = 0.0;
-  if (r2 > 0) {
-    const double ir = 1.0 / sqrt(r2);
-    r = r2 * ir;
-    cK = nx * ir;
-    sK = -ny * ir;
+  const double ny = tx * sA + ty * cA;
+  const double nx = t1 * cB + ci * sB, nz = -t1 * sB + ci * cB;
+  const double r2 = nx * nx + ny * ny, ir = r2 > 0 ? fast_rsqrt(r2) : 0.0, r = r2 * ir;
+  const double cK = r2 > 0 ? nx * ir : 1.0, sK = -ny * ir;
+  // azimuths: of J in the source frame; of L = z through A, B and K
+  if (part == 2) {
+    s.phi_aligned = p2 > 0 ? -atan2(Jy, Jx) : 0.0;
+    s.alpha0 = atan2(sB * sK, sB * cK);
+  } else {
+    const double az = atan2(part ? sB * sK : Jy, part ? sB * cK : Jx);
+    if (part) {
+      s.alpha0 = az;
+      return;
+    }
+    s.phi_aligned = p2 > 0 ? -az : 0.0;
   }
-  // L = z through A, B and K: its azimuth
-  s.alpha0 = atan2(sB * sK, sB * cK);
   // X through A, B and K
   tx = -ci * sr;
   ty = -ci * cr;
@@ -501,14 +551,9 @@ GW_HDNI void fast_pv2_frame(Source &s, ModelP &pm, const GenParams &in, const Fa
   const double xy = tx * sA + ty * cA, xx = t1 * cB + si * sB, xz = -t1 * sB + si * cB;
   const double px = xx * cK - xy * sK, py = xx * sK + xy * cK;
   // zeta = atan2(X . Q, X . P), P = -y, Q = (Nz, 0, -Nx): cos and sin of 2 zeta
-  const double P = -py, Q = px * nz - xz * r, n2 = P * P + Q * Q;
-  pm.c2z = 1.0;
-  pm.s2z = 0.0;
-  if (n2 > 0) {
-    const double in2 = 1.0 / n2;
-    pm.c2z = (P * P - Q * Q) * in2;
-    pm.s2z = 2.0 * P * Q * in2;
-  }
+  const double P = -py, Q = px * nz - xz * r, n2 = P * P + Q * Q, in2 = n2 > 0 ? 1.0 / n2 : 0.0;
+  pm.c2z = n2 > 0 ? (P * P - Q * Q) * in2 : 1.0;
+  pm.s2z = 2.0 * P * Q * in2;
   // s = -2, l = 2 harmonics at theta_JN: cos = Nz, sin = r (util.cpp:1953-2333)
   const double ct = nz, st = r;
   pm.Y[0] = kFastY2 * (1.0 - ct) * (1.0 - ct);
@@ -536,9 +581,17 @@ GW_HDNI void fast_pv2_finish(ModelD &m, ModelP &pm, const FastX &x) {
 // eta) at 0.8 .. 1.2 fRD without the terms linear in f.
 GW_HDNI double fast_pv2_node(const ModelD &m, const FastX &x, int j) {
   const Lambda &l = m.l;
-  const double rel = 0.8 + j * (0.4 / (kPv2ShiftNodes - 1)), xj = rel * x.xr;
-  return -l.alpha[2] / xj + (4. / 3) * l.alpha[3] * sqrt(xj * sqrt(xj)) +
-         l.alpha[4] * atan((xj - l.alpha[5] * x.xr) / x.xd);
+  const double rel = 0.8 + j * (0.4 / (kPv2ShiftNodes - 1));
+  const double pow34[kPv2ShiftNodes] = GWT_NODE34_LITERALS, pow1[kPv2ShiftNodes] = GWT_NODEINV_LITERALS;
+  double p34 = 0.0, inv = 0.0;
+#pragma unroll
+  for (int q = 0; q < kPv2ShiftNodes; q++)
+    if (q == j) {
+      p34 = pow34[q];  // (2 rel)^(3/4)
+      inv = pow1[q];   // 1 / (2 rel)
+    }
+  return -l.alpha[2] * (x.i2 * inv) + ((4. / 3) * l.alpha[3]) * (x.p2 * p34) +
+         l.alpha[4] * atan((rel - l.alpha[5]) * x.rx);
 }
 // The natural spline's slope halfway between the middle ones of ten even
 // nodes: sum_k w_k (y_(5+k) - y_(4-k)) / spacing (exact for linear terms).
@@ -548,39 +601,48 @@ GW_HDNI double fast_pv2_time_shift(const ModelD &m, const FastX &x) {
   if (!m.s.shift_time || !(x.xr > 0)) return 0.0;
   double t = 0.0;
   for (int k = 0; k < 5; k++) t += w[k] * (x.node[5 + k] - x.node[4 - k]);
-  const double slope = m.l.alpha[1] + t * ((kPv2ShiftNodes - 1) / 0.4) / x.xr;
+  const double slope = m.l.alpha[1] + t * ((kPv2ShiftNodes - 1) / 0.4) * (0.5 * x.i2);
   return -(m.s.inv_eta * m.s.M * slope) * (1.0 / (2. * kPi));
 }
 
 // ---- the grid's coefficients (mixed_phase_coeffs, mixed_amp_coeffs, mixed_regions) ----
+// The inspiral series' coefficient j of n^((j - 5)/3), j = 0..11.
+GW_HDNI void fast_ins_phase(const ModelD &m, const FastX &x, const GridConst &g, MixedReq &o, int j) {
+  const Source &s = m.s;
+  const double cu = x.cM * g.c13, iMdf = x.iM * g.idf, K = s.k_tf2 * m.pi.PIminus_5third, *pn = m.pn_phase;
+  const double Lc = kLnPi + x.lM + g.ln;
+  // the factor of cu^(j - 5): a constant times a coefficient, without branches
+  // (lanes hold different j)
+  const double *src = j < 8 ? pn + (j == 5 ? 8 : j == 6 ? 10 : j) : m.l.sigma + (j - 7);
+  constexpr double kP1 = 1.4645918875615231, kP2 = kP1 * kP1;  // pi^(1/3)
+  double c = j == 1 ? 0.0 : 1.0;
+  c = j == 2 ? kP2 : c;
+  c = j == 3 ? kPi : c;
+  c = j == 4 ? kP1 * kPi : c;
+  c = j == 5 ? kP2 * kPi : c;
+  c = j == 6 ? kPi * kPi : c;
+  c = j == 7 ? kP1 * kPi * kPi : c;
+  c = j == 9 ? 0.75 : c;
+  c = j == 10 ? 0.6 : c;
+  c = j == 11 ? 0.5 : c;
+  const double ex = j == 5 ? pn[9] : j == 6 ? -pn[11] : 0.0;
+  const double q = (j < 8 ? K : s.inv_eta) * (c * (*src + ex * Lc)) - (j == 5 ? kPi / 4. : 0.0);
+  // ... and the power: cu^-5 = cu / (cu^3)^2, cu^3 = M df
+  const double cu2 = cu * cu, cu4 = cu2 * cu2;
+  double p = (cu * iMdf) * iMdf;
+  if (j & 1) p *= cu;
+  if (j & 2) p *= cu2;
+  if (j & 4) p *= cu4;
+  if (j & 8) p *= cu4 * cu4;
+  o.qi[j] = q * p;
+  if (j == 5) o.bi0 = K * m.pi.PI5third * pn[9];
+  if (j == 6) o.bi1 = -(K * m.pi.PIsquare) * pn[11] * cu;
+}
+// Intermediate and ringdown phase, after fast_connect.
 GW_HDNI void fast_phase_coeffs(const ModelD &m, const FastX &x, const GridConst &g, MixedReq &o) {
   const Source &s = m.s;
   const Lambda &l = m.l;
-  const double Mdf = s.M * g.df, iMdf = x.iM * g.idf, cu = x.cM * g.c13, Lx = x.lM + g.ln, Lc = kLnPi + Lx;
-  const double K = s.k_tf2 * m.pi.PIminus_5third, *pn = m.pn_phase;
-  const double icu2 = (cu * iMdf) * (cu * iMdf) * (cu * cu);  // cu^-2
-  const double icu = cu * icu2;
-  double q[12];
-  q[0] = K;
-  q[1] = 0.0;
-  q[2] = (K * m.pi.PI2third) * pn[2];
-  q[3] = (K * kPi) * pn[3];
-  q[4] = (K * m.pi.PI4third) * pn[4];
-  q[5] = (K * m.pi.PI5third) * (pn[8] + pn[9] * Lc) - kPi / 4.;
-  q[6] = (K * m.pi.PIsquare) * (pn[10] - pn[11] * Lc);
-  q[7] = (K * m.pi.PI7third) * pn[7];
-  q[8] = l.sigma[1] * s.inv_eta;
-  q[9] = (3. / 4.) * l.sigma[2] * s.inv_eta;
-  q[10] = (3. / 5.) * l.sigma[3] * s.inv_eta;
-  q[11] = (1. / 2.) * l.sigma[4] * s.inv_eta;
-  double cp = icu2 * icu2 * icu;  // cu^-5
-#pragma unroll
-  for (int j = 0; j < 12; j++) {
-    o.qi[j] = q[j] * cp;
-    cp *= cu;
-  }
-  o.bi0 = K * m.pi.PI5third * pn[9];
-  o.bi1 = -(K * m.pi.PIsquare) * pn[11] * cu;
+  const double Mdf = s.M * g.df, iMdf = x.iM * g.idf, Lx = x.lM + g.ln;
   o.pA = (l.beta[0] + l.beta[2] * Lx) * s.inv_eta;
   o.pB = l.beta[1] * Mdf * s.inv_eta;
   o.pC = l.beta[2] * s.inv_eta;
@@ -591,29 +653,36 @@ GW_HDNI void fast_phase_coeffs(const ModelD &m, const FastX &x, const GridConst 
   o.mD = (4. / 3.) * l.alpha[3] * (x.M34 * g.q34) * s.inv_eta;
   o.mE = l.alpha[4] * s.inv_eta;
   o.mEq = (float)(o.mE * (1.0 / (2.0 * 3.14159265358979323846)) * kSegFScale);
-  const double nc = l.alpha[5] * s.fRD * g.idf, nci = floor(nc);
+}
+// The atan's centre and width in bins.
+GW_HDNI void fast_atan_coeffs(const ModelD &m, const GridConst &g, MixedReq &o) {
+  const double nc = m.l.alpha[5] * m.s.fRD * g.idf, nci = floor(nc);
   o.n_c = (int)nci;
   o.ncfrac = (float)(nc - nci);
-  o.inv_nw = (float)(g.df / s.fdamp);
+  o.inv_nw = (float)(g.df / m.s.fdamp);
 }
-GW_HDNI void fast_amp_coeffs(const ModelD &m, const FastX &x, const GridConst &g, MixedReq &o) {
+// Inspiral amplitude coefficient j of n^(j/3), j = 0..9.
+GW_HDNI void fast_ins_amp(const ModelD &m, const FastX &x, const GridConst &g, MixedReq &o, int j) {
   const double cu = x.cM * g.c13, *pa = m.pn_amp;
-  const double a[10] = {1.0,
-                        0.0,
-                        pa[2] * m.pi.PI2third,
-                        pa[3] * kPi,
-                        pa[4] * m.pi.PI4third,
-                        pa[5] * m.pi.PI5third,
-                        pa[6] * m.pi.PIsquare,
-                        m.l.rho[0],
-                        m.l.rho[1],
-                        m.l.rho[2]};
+  const double *src = j < 7 ? pa + j : m.l.rho + (j - 7);
+  constexpr double kP1 = 1.4645918875615231, kP2 = kP1 * kP1;  // pi^(1/3)
   double c = 1.0;
-#pragma unroll
-  for (int j = 0; j < 10; j++) {
-    split_f(a[j] * c, o.ai[j], o.ai_lo[j]);
-    c *= cu;
-  }
+  c = j == 2 ? kP2 : c;
+  c = j == 3 ? kPi : c;
+  c = j == 4 ? kP1 * kPi : c;
+  c = j == 5 ? kP2 * kPi : c;
+  c = j == 6 ? kPi * kPi : c;
+  const double a = c * *src;
+  const double cu2 = cu * cu, cu4 = cu2 * cu2;
+  double p = 1.0;
+  if (j & 1) p *= cu;
+  if (j & 2) p *= cu2;
+  if (j & 4) p *= cu4;
+  if (j & 8) p *= cu4 * cu4;
+  split_f(a * p, o.ai[j], o.ai_lo[j]);
+}
+// Intermediate amplitude: coefficients j0, j0 + step, ... of (n - n_mid)^j.
+GW_HDNI void fast_int_amp(const ModelD &m, const FastX &x, const GridConst &g, MixedReq &o, int j0, int step) {
   // u = (n - n_m) Mdf / h, n_m the middle of the range in bins
   const double nm = 0.5 * (m.s.f1 + m.s.f3) * g.idf, nmid = floor(nm);
   o.n_mid = (int)nmid;
@@ -621,7 +690,10 @@ GW_HDNI void fast_amp_coeffs(const ModelD &m, const FastX &x, const GridConst &g
   double e[5];
   fast_shift_quartic(x.a, sc, (nmid - nm) * sc, e);
 #pragma unroll
-  for (int j = 0; j < 5; j++) split_f(e[j], o.ei[j], o.ei_lo[j]);
+  for (int j = 0; j < 5; j++)
+    if ((j - j0) % step == 0) split_f(e[j], o.ei[j], o.ei_lo[j]);
+}
+GW_HDNI void fast_ring_amp(const ModelD &m, const FastX &x, const GridConst &g, MixedReq &o) {
   const double g1 = m.l.gamma[0], g2 = m.l.gamma[1], nrd = m.s.fRD * g.idf, nrdi = floor(nrd);
   o.n_rd = (int)nrdi;
   o.mrRDfrac = (float)(nrd - nrdi);
@@ -641,17 +713,18 @@ GW_HD int fast_grid_first(double fb, const GridConst &g, bool strict) {
   for (int it = 0; it < 4 && !ok(n) && n < 2000000000; it++) n++;
   return n;
 }
-GW_HDNI void fast_regions(const Request &r, const GridConst &g, MixedReq &o) {
-  const ModelD &m = r.m;
+// Region start q = 0..4: f1, f1_phase, f3, f2_phase, the cut (last non-zero bin).
+GW_HDNI int fast_region(const ModelD &m, const GridConst &g, MixedReq &o, int q) {
   const Source &s = m.s;
-  o.approximant = r.approximant;
-  o.status = m.status;
-  o.ndet = r.ndet;
-  o.n_f1 = fast_grid_first(s.f1, g, false);
-  o.n_f1p = fast_grid_first(s.f1_phase, g, false);
-  o.n_f3 = fast_grid_first(s.f3, g, true);
-  o.n_f2p = fast_grid_first(s.f2_phase, g, true);
-  o.n_cut = fast_grid_first(m.fcut, g, true) - 1;
+  const double *fp = q == 0 ? &s.f1 : q == 1 ? &s.f1_phase : q == 2 ? &s.f3 : q == 3 ? &s.f2_phase : &m.fcut;
+  const double fb = *fp;
+  const int n = fast_grid_first(fb, g, q >= 2);
+  if (q == 0) o.n_f1 = n;
+  if (q == 1) o.n_f1p = n;
+  if (q == 2) o.n_f3 = n;
+  if (q == 3) o.n_f2p = n;
+  if (q == 4) o.n_cut = n - 1;
+  return n;
 }
 // A0eff (M df)^(-7/6) [times 1/2 for Pv2]: the powers of M cancel.
 GW_HDNI double fast_a_scale(const Request &r, const GridConst &g) {
@@ -684,12 +757,87 @@ GW_HDNI void fast_pv2_coeffs(const Request &r, const FastX &x, const GridConst &
   split_f(cw * cw, o.x2c, o.x2c_lo);
 }
 
-// Detectors d0, d0 + step, ...: projections, phases; the finalize factors.
+// Whether the phase terms that the two-float bins carry are small enough
+// (kAccMaxTurns): their largest values are at M f = 0.018, xr / 2 and the cut 0.2.
+GW_HDNI int fast_range_d(const ModelD &m, const FastX &x) {
+  const Lambda &l = m.l;
+  const double v = fabs(l.alpha[2]) * x.i2 + (4. / 3) * kFast34 * fabs(l.alpha[3]) + fabs(l.alpha[4]);
+  return v * m.s.inv_eta < kAccMaxTurns * 2 * kPi ? 0 : 1;  // 1 for NaN
+}
+GW_HDNI int fast_range_p(const ModelP &pm) {
+  // w = pi 0.018 .. pi 0.2: w^(-1/3) at the one end, w^(1/3) at the other, |ln w| < 2.9
+  constexpr double i = 1.0 / kFastV, t = kFastVc, L = 2.9;
+  const double *a = pm.ac, *e = pm.ec;
+  const double va = i * (fabs(a[2]) + i * (fabs(a[1]) + i * fabs(a[0]))) + L * fabs(a[3]) + t * fabs(a[4]);
+  const double ve = i * (fabs(e[2]) + i * (fabs(e[1]) + i * fabs(e[0]))) + L * fabs(e[3]) + t * fabs(e[4]);
+  return va < kAccMaxTurns * 2 * kPi && 2.0 * ve < kAccMaxTurns * 2 * kPi ? 0 : 1;
+}
+// Finalize factors of detector d: f[0..4] (mixed_det_factors_a).
+GW_HDNI void fast_det_factor(const Request &r, int d, double A, double w, double ds, double *f) {
+  double G1, G2;
+  mixed_det_G(r, d, G1, G2);
+  if (r.approximant == kPhenomPv2) {
+    const double h = -0.5 * A * A * w, k = A * ds;
+    f[0] = h * G1 * G1;
+    f[1] = h * G2 * G2;
+    f[2] = 2.0 * h * G1 * G2;
+    f[3] = k * G1;
+    f[4] = k * G2;
+  } else {
+    const double g = G1 * G1 + G2 * G2;
+    f[0] = -0.5 * A * A * w * g;
+    f[1] = A * ds * sqrt(g);
+    f[2] = f[3] = f[4] = 0.0;
+  }
+}
+// Entry e of the factors, the weighted |h|^2 sums folded where the detectors
+// share their weights (mixed_fold_shared_weights).
+GW_HD double fast_factor_entry(const double (*f)[kAccPerDet], int e, int ndet, bool pv2, bool shared) {
+  const int d = e / kAccPerDet, k = e - d * kAccPerDet;
+  if (d >= ndet) return 0.0;
+  if (!shared || k >= (pv2 ? 3 : 1)) return f[d][k];
+  if (d) return 0.0;
+  double v = f[0][k];
+  for (int q = 1; q < ndet; q++) v += f[q][k];
+  return v;
+}
+GW_HD bool fast_shared(const unsigned long long *wkey, int ndet) {
+  bool same = ndet > 1;
+  for (int d = 1; d < ndet; d++) same = same && wkey[d] == wkey[0];
+  return same;
+}
+// Detectors d0, d0 + step, ...: projections, phases.
+#if defined(__CUDACC__)
+// the detectors in global memory: lanes read different ones
+static __device__ const double gwt_det_tensor_g[9][9] = GWT_DET_TENSOR_INIT;
+static __device__ const double gwt_det_location_g[9][3] = GWT_DET_LOCATION_INIT;
+static __device__ const double gwt_det_geometric_g[9] = GWT_DET_GEOMETRIC_INIT;
+#endif
+#if defined(__CUDA_ARCH__)
+#define GWT_G(name) name##_g
+#else
+#define GWT_G(name) name##_h
+#endif
 GW_HDNI void fast_antenna(Request &r, const FastX &x, const int *dets, int d0, int step) {
-  const SkyTrig t{x.cn[0], x.sn[0], x.cn[1], x.sn[1], x.cn[2], x.sn[2]};
+  const double sg = x.sn[0], cg = x.cn[0], sd = x.sn[1], cd = x.cn[1], sp = x.sn[2], cp = x.cn[2];
+  const double X[3] = {-cp * sg - sp * cg * sd, -cp * cg + sp * sg * sd, sp * cd};
+  const double Y[3] = {sp * sg - cp * cg * sd, sp * cg + cp * sg * sd, cp * cd};
+  const double e0 = cd * cg, e1 = cd * -sg, e2 = sd;
   for (int d = d0; d < r.ndet && d < kMaxDet; d += step) {
-    antenna_trig(dets[d], t, r.det[d].fp, r.det[d].fc);
-    r.det[d].tau = -dtoa_trig(t, dets[0], dets[d]) * (2 * kPi);
+    const double *D = GWT_G(gwt_det_tensor)[dets[d]], geo = GWT_G(gwt_det_geometric)[dets[d]];
+    const double *l1 = GWT_G(gwt_det_location)[dets[0]], *l2 = GWT_G(gwt_det_location)[dets[d]];
+    double fp = 0.0, fc = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {  // detector_util.cpp:901-1015, 1158-1160
+      const double DX = D[i * 3] * X[0] + D[i * 3 + 1] * X[1] + D[i * 3 + 2] * X[2];
+      const double DY = D[i * 3] * Y[0] + D[i * 3 + 1] * Y[1] + D[i * 3 + 2] * Y[2];
+      fp += X[i] * DX - Y[i] * DY;
+      fc += X[i] * DY + Y[i] * DX;
+    }
+    r.det[d].fp = fp * geo;
+    r.det[d].fc = fc * geo;
+    // detector_util.cpp:760-780
+    r.det[d].tau = ((l1[0] - l2[0]) * e0 + (l1[1] - l2[1]) * e1 + (l1[2] - l2[2]) * e2) * (-2 * kPi / kC);
   }
 }
 GW_HDNI void fast_det_phase(const Request &r, double df, MixedReq &o, int d0, int step) {
@@ -698,19 +846,19 @@ GW_HDNI void fast_det_phase(const Request &r, double df, MixedReq &o, int d0, in
 GW_HDNI void fast_det_phase(const Request &r, double df, AccReq &o, int d0, int step) {
   acc_det_phase(r, df, o, d0, step);
 }
-GW_HDNI void fast_det_factors(const Request &r, MixedReq &o, const double *dscale, const double *wscale) {
-  mixed_det_factors(r, o, dscale, wscale);
-}
 
-// The parts in order (host): request_prologue and the form's coefficients.
+// The parts in order (host): request_prologue, and the FP64 form's constants.
 inline int fast_request(Request &r, FastX &x, const GenParams &in, int approximant, const int *dets, int ndet,
                         const double *qnm) {
   r.approximant = approximant;
   r.ndet = ndet;
   const bool pv2 = approximant == kPhenomPv2;
-  const FastCore k = fast_core(in);
   ModelD &m = r.m;
-  fast_store(m.s, x, in, k);
+  fast_eta(x, in);
+  fast_inverses(x, in);
+  const FastCore k = fast_core(in, x);
+  m.s.pv2 = pv2;
+  fast_store(m.s, in, k);
   fast_fixed(m);
   for (int i = 0; i < 19; i++) fast_fit(m.l, k, i);
   for (int i = 0; i < kPnRows; i++) fast_pn(m, k, i);
@@ -722,19 +870,17 @@ inline int fast_request(Request &r, FastX &x, const GenParams &in, int approxima
   x.lM = log(k.M);
   x.cfr = cbrt(in.f_ref);
   x.lfr = log(in.f_ref);
-  x.M34 = sqrt(k.M * sqrt(k.M));
   fast_amp0(m, x, in, k);
-  if (pv2) fast_pv2_spins(m.s, in, k);
+  if (pv2) fast_pv2_spins(m.s, in);
   fast_ring(m.s, x, k, qnm);
   fast_high(m, x);
-  fast_low_amp(m, x);
-  fast_low_phase(m, x);
+  for (int i = 0; i < kLowRows; i++) fast_low(m, x, i);
   fast_f2_powers(x);
   fast_f2_atan(m, x);
   fast_fref_phase(m, x);
   if (pv2) {
-    fast_pv2_frame(m.s, r.p, in, x);
-    pv2_euler_coeffs(r.p.ac, r.p.ec, m.s);
+    fast_pv2_frame(m.s, r.p, in, x, 2);
+    fast_pv2_euler(r.p, m.s);
     fast_pv2_finish(m, r.p, x);
   } else {
     fast_time_shift(m, x);
@@ -752,18 +898,29 @@ inline int fast_request(Request &r, FastX &x, const GenParams &in, int approxima
   return m.status;
 }
 inline int fast_acc(const Request &r, const FastX &x, const GridConst &g, AccReq &o, const double *dscale,
-                    const double *wscale) {
-  fast_regions(r, g, o.m);
-  o.m.A_scale = fast_a_scale(r, g);
+                    const double *wscale, const unsigned long long *wkey) {
+  const bool pv2 = r.approximant == kPhenomPv2;
+  o.m.approximant = r.approximant;
+  o.m.status = r.m.status;
+  o.m.ndet = r.ndet;
+  for (int q = 0; q < 5; q++) fast_region(r.m, g, o.m, q);
+  for (int j = 0; j < 12; j++) fast_ins_phase(r.m, x, g, o.m, j);
   fast_phase_coeffs(r.m, x, g, o.m);
-  fast_amp_coeffs(r.m, x, g, o.m);
-  if (r.approximant == kPhenomPv2) fast_pv2_coeffs(r, x, g, o.m);
-  mixed_det_factors(r, o.m, dscale, wscale);
-  acc_det_phase(r, g.df, o);
+  fast_atan_coeffs(r.m, g, o.m);
+  for (int j = 0; j < 10; j++) fast_ins_amp(r.m, x, g, o.m, j);
+  fast_int_amp(r.m, x, g, o.m, 0, 1);
+  fast_ring_amp(r.m, x, g, o.m);
+  if (pv2) fast_pv2_coeffs(r, x, g, o.m);
+  o.m.A_scale = fast_a_scale(r, g);
+  double f[kMaxDet][kAccPerDet];
+  for (int d = 0; d < r.ndet; d++) fast_det_factor(r, d, o.m.A_scale, wscale[d], dscale[d], f[d]);
+  o.m.wshared = fast_shared(wkey, r.ndet) ? 1 : 0;
+  for (int e = 0; e < kMaxDet * kAccPerDet; e++) o.m.fc[e] = fast_factor_entry(f, e, r.ndet, pv2, o.m.wshared != 0);
+  fast_det_phase(r, g.df, o, 0, 1);
   acc_phase_coeffs(r, g.df, o);
   acc_amp_coeffs(r, g.df, o);
-  if (r.approximant == kPhenomPv2) acc_pv2_coeffs(r, g.df, o);
-  acc_range(r, o);
+  if (pv2) acc_pv2_coeffs(r, g.df, o);
+  o.fp64_phase = fast_range_d(r.m, x) | (pv2 ? fast_range_p(r.p) : 0);
   return o.m.status;
 }
 

@@ -1,11 +1,12 @@
-// acc_check.cpp -- TEST BUILD ONLY: the two-float arithmetic and the bins of
-// the FP64 form built on it (two_float.h, phenom_acc.h) compiled for the host.
+// acc_check.cpp -- TEST BUILD ONLY: the two-float arithmetic, the bins of the
+// FP64 form built on it and the batched prologue (two_float.h, phenom_acc.h,
+// phenom_fast.h) compiled for the host.
 // Compiled with -ffp-contract=off: the error-free sums need every operation
 // rounded by itself.
 #include <cmath>
 #include <vector>
 
-#include "../../gw_analysis_tools_gb300/csrc/phenom_acc.h"
+#include "../../gw_analysis_tools_gb300/csrc/phenom_fast.h"
 
 using namespace gwt;
 
@@ -89,8 +90,8 @@ void gwa_worst(unsigned long long seed, int n, double *out) {
   }
 }
 
-// log L of one request on the grid f_k ~ (n0 + k) df; mode 0: as the request
-// asks, 1: with the FP64 phase series at every bin.
+// log L of one request on the grid f_k ~ (n0 + k) df.  mode bit 0: the FP64
+// phase series at every bin; bit 1: the prologue of phenom_fast.h.
 double gwa_loglik(const GenParams *pin, int approx, double T_segment, int n0, const double *f, int N, int ndet,
                   const int *dets, const double *const *data, const double *const *psd, int mode, int *fp64_phase) {
   GenParams p = *pin;
@@ -99,7 +100,9 @@ double gwa_loglik(const GenParams *pin, int approx, double T_segment, int n0, co
   std::vector<float> dev(N);
   for (int k = 0; k < N; k++) dev[k] = (float)std::fma(-(double)(n0 + k), df, f[k]);
   Request r;
-  if (request_prologue(r, p, approx, dets, ndet, qnm())) return NAN;
+  FastX fx;
+  if (mode & 2 ? fast_request(r, fx, p, approx, dets, ndet, qnm()) : request_prologue(r, p, approx, dets, ndet, qnm()))
+    return NAN;
   std::vector<std::vector<ff4>> wd(ndet);
   std::vector<std::vector<ff>> w(ndet);
   double ds[kMaxDet], ws[kMaxDet];
@@ -120,8 +123,10 @@ double gwa_loglik(const GenParams *pin, int approx, double T_segment, int n0, co
     }
   }
   AccReq x;
-  acc_prologue(r, df, x, ds, ws);
-  if (mode) x.fp64_phase = 1;
+  const unsigned long long wk[kMaxDet] = {1, 2, 3, 4};  // no shared weights
+  if (mode & 2) fast_acc(r, fx, grid_const(df), x, ds, ws, wk);
+  else acc_prologue(r, df, x, ds, ws);
+  if (mode & 1) x.fp64_phase = 1;
   if (fp64_phase) *fp64_phase = x.fp64_phase;
   std::vector<double> t13(n0 + N), tm53(n0 + N), tln(n0 + N), t34(n0 + N);
   std::vector<ff4> pw(n0 + N), ph(n0 + N), pv(n0 + N);

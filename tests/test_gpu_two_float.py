@@ -99,3 +99,29 @@ def test_infinite_psd_bins(gpu_ctx, oracle):
     finally:
         gpu_ctx.release_data(h)
         gpu_ctx.release_data(h0)
+
+
+@pytest.mark.parametrize("prec", [G.PREC_FP64, G.PREC_MIXED])
+def test_prologue_block_sizes(gpu_ctx, prec):
+    """4, 8 or 16 requests per prologue block (by the number of requests): each request as in a small batch, to
+    the bit in the mixed form (the FP64 form's tile, and with it its order of summation, follows the batch)."""
+    T = 4.0
+    f = 20.0 + np.arange(300) / T
+    psd = W.analytic_psd(f)
+    hs = [gpu_ctx.register_data(d, f, W.noise(f, 60 + i), psd) for i, d in enumerate(DETS[:2])]
+    try:
+        n = 1219
+        draws = [x for pair in zip(W.prior_draws(610, 5), W.prior_draws(610, 6, precessing=True)) for x in pair][:n]
+        aps = np.arange(n, dtype=np.int32) % 2
+        few = np.concatenate([gpu_ctx.loglik_batch(G.params_array(draws[i:i + 100]), aps[i:i + 100], hs, T, prec)[0]
+                              for i in range(0, n, 100)])
+        for m in (1, 3, 608, 609, 1216, 1217, n):
+            out, st = gpu_ctx.loglik_batch(G.params_array(draws[:m]), aps[:m], hs, T, prec)
+            assert np.all(st == 0)
+            if prec == G.PREC_MIXED:
+                assert np.array_equal(out, few[:m])
+            else:
+                assert np.all(np.abs(out - few[:m]) <= 1e-11 * np.maximum(1.0, np.abs(few[:m])))
+    finally:
+        for h in hs:
+            gpu_ctx.release_data(h)

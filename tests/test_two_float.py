@@ -68,3 +68,30 @@ def test_loglik_against_oracle(acc, oracle, T, fmax, ndet, ap):
         assert abs(other - ref) <= 1e-9 * max(1.0, abs(ref)), (d, other, ref)
         flags.append(flag)
     assert min(flags) == 0 and flags[-1] == 1
+
+
+@pytest.mark.parametrize("ap", [0, 1])
+def test_fast_prologue(acc, oracle, ap):
+    """phenom_fast.h's prologue at its branches: equal and swapped masses, f_ref past the inspiral, no time or
+    phase shift, the sky average, the other ringdown fit, aligned and reduced Pv2 spins, a face-on source."""
+    T, n0, N = 8, 160, 4000
+    f = 20.0 + np.arange(N) / T
+    dets = list(W.DETECTORS3)
+    src = W.config1_source()
+    inj = oracle.params_from_dict(dict(src, tc=T - src["tc"]))
+    data = [oracle.detector_response(f, inj, d) + W.noise(f, 15 + i) for i, d in enumerate(dets)]
+    psd = [W.analytic_psd(f)] * 3
+    kinds = [dict(), dict(mass2=36.0), dict(mass1=29.0, mass2=36.0), dict(f_ref=300.0), dict(mass1=150.0, mass2=90.0, f_ref=60.0),
+             dict(shift_time=0), dict(shift_phase=0), dict(sky_average=1), dict(dep_postmerger=1), dict(incl_angle=0.0),
+             dict(spin1=(0, 0, 0.0), spin2=(0, 0, 0.0)), dict(chip=0.4, phip=1.0), dict(mass1=80.0, mass2=5.0)]
+    for k in kinds:
+        for base in (src, W.prior_draws(1, 77, precessing=bool(ap))[0]):
+            d = dict(base, **k)
+            p = oracle.params_from_dict({a: b for a, b in d.items() if a not in ("shift_time", "shift_phase", "sky_average",
+                                                                                 "dep_postmerger", "chip", "phip")})
+            for a in ("shift_time", "shift_phase", "sky_average", "dep_postmerger", "chip", "phip"):
+                if a in d:
+                    setattr(p, a, d[a])
+            ref = oracle.loglik(p, f, dets, data, psd, approximant=ap, T_segment=T)
+            got, _ = _loglik(acc, oracle, p, ap, T, n0, f, N, dets, data, psd, mode=2)
+            assert (np.isnan(ref) and np.isnan(got)) or abs(got - ref) <= 1e-9 * max(1.0, abs(ref)), (k, got, ref)
