@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kAccBlock, 2) k_batch_acc(const BatchArgs a) {
   __shared__ __align__(16) unsigned char s_req[sizeof(AccReq)];
   __shared__ StreamDev s_st[NDET];
   __shared__ double s_red[kAccBlock / 32];
-  __shared__ int s_item, s_iid, s_bstart[kOrderBuckets];
+  __shared__ int s_item, s_iid, s_bstart[kOrderBuckets + 1];
   const int tid = threadIdx.x;
   copy_words(&lut, a.lut, sizeof(AccLut));
   grid_dep_wait();  // the prologue's output
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kAccBlock, 2) k_batch_acc(const BatchArgs a) {
       s_iid = order_item(a, s_bstart, it);
     }
     __syncthreads();
-    if (s_item >= a.nitems) break;
+    if (s_item >= (a.bucket_fill ? s_bstart[kOrderBuckets] : a.nitems)) break;
     const int iid = s_iid;
     const Item I = a.items[iid];
     static_assert(sizeof(AccReq) % 4 == 0, "copied as words");

@@ -191,6 +191,7 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
     ord.items = pl.order;
     ord.item_start = pl.item_start;
     ord.item_count = pl.item_count;
+    ord.live = (int *)(cnt + n + 32 + gwk::kOrderBuckets);
     ord.nitems = pl.nitems;
     ord.tile = pl.tile;
   }
@@ -217,7 +218,7 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   a.bucket_items = ordered ? ord.items : nullptr;
   a.nitems = pl.nitems;
   a.item_start = pl.item_start;
-  a.item_count = pl.item_count;
+  a.item_count = ordered ? ord.live : pl.item_count;
   a.tile = pl.tile;
   a.item_counter = cnt + n;
   a.req_done = cnt;
@@ -288,7 +289,7 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
   }
   size_t rq = mixed ? sizeof(gwt::MixedReq) : form == kFormAcc ? sizeof(gwt::AccReq) : sizeof(gwt::Request);
   size_t bytes = rq * n + 512 + sizeof(double) * (size_t)L.plan.nitems * gwk::kAcc + 256 +
-                 sizeof(unsigned) * (size_t)(n + 32 + gwk::kOrderBuckets);
+                 sizeof(unsigned) * (size_t)(2 * (size_t)n + 32 + gwk::kOrderBuckets);
   void *old = L.work;
   int st = lane_alloc(c, L, &L.work, &L.work_cap, bytes, "batch scratch");
   if (st) return st;

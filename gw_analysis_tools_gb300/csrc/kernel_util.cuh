@@ -35,8 +35,8 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 
-// The work order of a batch (OrderArgs): the first position of each bucket,
-// by one warp, ...
+// The work order of a batch (OrderArgs): the first position of each bucket and,
+// past the last, the number of items, by one warp, ...
 __device__ __forceinline__ void order_starts(const BatchArgs &a, int *s_bstart) {
   const int tid = threadIdx.x & 31;
   constexpr int kPerLane = (kOrderBuckets + 31) / 32;
@@ -60,11 +60,12 @@ __device__ __forceinline__ void order_starts(const BatchArgs &a, int *s_bstart) 
     if (b < kOrderBuckets) s_bstart[b] = run;
     run += v[q];
   }
+  if (tid == 31) s_bstart[kOrderBuckets] = run;
 }
 // ... and the item at position it (its own index: its partial sums' slot).
 __device__ __forceinline__ int order_item(const BatchArgs &a, const int *s_bstart, int it) {
   int iid = it;
-  if (a.bucket_fill && it < a.nitems) {  // the bucket holding position it: the last start <= it
+  if (a.bucket_fill && it < s_bstart[kOrderBuckets]) {  // the bucket holding position it: the last start <= it
     int lo = 0, hi = kOrderBuckets - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;

@@ -585,14 +585,18 @@ __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
   __shared__ CoopSmem<REQ> sm;
   grid_dep_trigger();  // the bin kernel may launch and wait for this grid
   // this block's requests into the work order, on the warps idle in S6
+  const int base = blockIdx.x * REQ;
   auto head = [&](int i, int &first, int &count) {
     first = ord.fill ? ord.item_start[i] : 0;
     count = ord.fill ? ord.item_count[i] : 0;
   };
   auto tail = [&](int slot, int first, int count, int kcut) {
-    if (ord.fill) order_append(ord, kcut, count, first, slot, (kCoopWarps - 1) * (32 / REQ));
+    if (!ord.fill) return;
+    const int live = count ? max(1, min(count, (kcut + ord.tile - 1) / ord.tile)) : 0;
+    if (slot == 0 && count) ord.live[base + (threadIdx.x & 31) % REQ] = live;
+    order_append(ord, kcut, live, first, slot, (kCoopWarps - 1) * (32 / REQ));
   };
-  prologue_coop_body<REQ, ACC>(sm, blockIdx.x * REQ, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles,
+  prologue_coop_body<REQ, ACC>(sm, base, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles,
                                ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status,
                                [] { __syncthreads(); }, head, tail);
 }
@@ -945,7 +949,7 @@ template <int NDET, int MIXED, int OCC>
 __global__ void __launch_bounds__(kBatchBlock, OCC) k_batch(const BatchArgs a) {
   __shared__ int s_item;
   __shared__ BinSmem<NDET, MIXED> sm;
-  __shared__ int s_iid, s_bstart[kOrderBuckets];
+  __shared__ int s_iid, s_bstart[kOrderBuckets + 1];
   const int tid = threadIdx.x;
   grid_dep_wait();  // the prologue's output
   if (a.bucket_fill && tid < 32) order_starts(a, s_bstart);
@@ -958,7 +962,7 @@ __global__ void __launch_bounds__(kBatchBlock, OCC) k_batch(const BatchArgs a) {
     }
     __syncthreads();
     const int it = s_item;
-    if (it >= a.nitems) break;
+    if (it >= (a.bucket_fill ? s_bstart[kOrderBuckets] : a.nitems)) break;
     const int iid = s_iid;  // the item's own index: its partials' slot
     batch_item<NDET, MIXED>(a, iid, a.items[iid], sm, [&](int req, double ll, int st) {
       a.out[req] = ll;

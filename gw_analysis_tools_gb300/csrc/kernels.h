@@ -82,14 +82,16 @@ int plain_blocks(int N);
 cudaError_t plain_acc_preload();
 cudaError_t plain_preload();  // loads the plain kernels' module (function-attribute query)
 
-// Work order of a mixed batch: the prologue appends each request's items to
-// the bucket of their live 256-bin passes (bucket 0: all live) as soon as it
-// knows the request's cut; the bin kernel takes items bucket by bucket.
+// Work order of a batch: the prologue appends each request's live items (those
+// that start below its cut; at least one, which reports the status) to the bucket
+// of their live 256-bin passes (bucket 0: all live) as soon as it knows the cut
+// and writes their number; the bin kernel takes items bucket by bucket.
 constexpr int kOrderBuckets = 65;
 struct OrderArgs {
   int *fill = nullptr;          // kOrderBuckets counters (zeroed before the prologue); nullptr: no ordering
   int *items = nullptr;         // bucket b's items at items[b * nitems ...]
   const int *item_start = nullptr, *item_count = nullptr;  // per request: first item, number of items
+  int *live = nullptr;          // per request: live items (the first ones)
   int nitems = 0, tile = 0;
 };
 // Batched: prologue (one thread per request) then the fused bin kernel.
@@ -115,7 +117,7 @@ struct BatchArgs {
   const int *bucket_items;  // partials stay indexed by item
   int nitems;
   const int *item_start;  // per request
-  const int *item_count;
+  const int *item_count;  // (with a work order: the live items alone)
   int tile;               // bins per item
   unsigned *item_counter;  // dynamic item scheduler (zeroed before launch)
   unsigned *req_done;      // per request finished-item counters (zeroed before launch)
