@@ -237,8 +237,26 @@ int gwf_ref_run(gwgpu_context *c, const GenParams *params, int n, int method, in
     a.psd[d] = s->dev.psd;
   }
   const int nk = order >= 4 ? 4 : 2;
-  const int N = s0->dev.N, tile = 2048, ntiles = (N + tile - 1) / tile;
-  const int chunk = std::min(n, 1024);
+  const int N = s0->dev.N, chunk = std::min(n, 1024);
+  const size_t smem = sizeof(double) * (size_t)(2 * kDim + 1) * ndet * kRefBlock;
+  static int attr_set = 0, nsm = 0;
+  if (!attr_set) {
+    cudaFuncSetAttribute(k_fref_main, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double) * (2 * kDim + 1) * kMaxDet * kRefBlock));
+    cudaDeviceProp pr;
+    cudaGetDeviceProperties(&pr, c->device);
+    nsm = pr.multiProcessorCount;
+    attr_set = 1;
+  }
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fref_main, kRefBlock, smem);
+  // Bins per item: 2,048 where the sources alone fill the chip.  A pass of 128
+  // bins takes 0.7 ms (44 waveforms a bin at order 4), so the one or two sources
+  // that the moment form leaves here (a cut between the steps) take an item per
+  // pass: one source on 32,608 bins 11 -> 1.5 ms
+  const long long slots = (long long)nsm * std::max(per_sm, 1);
+  long long tile_l = ((long long)N * chunk / (2 * slots) + kRefBlock - 1) / kRefBlock * kRefBlock;
+  const int tile = (int)std::min(2048LL, std::max((long long)kRefBlock, tile_l)), ntiles = (N + tile - 1) / tile;
   auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const size_t b_par = align(sizeof(GenParams) * chunk), b_req = align(sizeof(Request) * (size_t)chunk * kDim * nk),
                b_rs = align(sizeof(RefSrc) * chunk), b_part = align(sizeof(double) * (size_t)chunk * ntiles * kPairs),
@@ -278,17 +296,6 @@ int gwf_ref_run(gwgpu_context *c, const GenParams *params, int n, int method, in
   a.df = s0->host_freqs[1] - s0->host_freqs[0];
   a.partials = dpart;
   a.fisher = dfish;
-  const size_t smem = sizeof(double) * (size_t)(2 * kDim + 1) * ndet * kRefBlock;
-  static int attr_set = 0, per_sm = 0, nsm = 0;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_fref_main, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(double) * (2 * kDim + 1) * kMaxDet * kRefBlock));
-    cudaDeviceProp pr;
-    cudaGetDeviceProperties(&pr, c->device);
-    nsm = pr.multiProcessorCount;
-    attr_set = 1;
-  }
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fref_main, kRefBlock, smem);
   for (int s0i = 0; s0i < n; s0i += chunk) {
     const int m = std::min(chunk, n - s0i);
     cudaMemcpyAsync(dparams, params + s0i, sizeof(GenParams) * m, cudaMemcpyHostToDevice, c->stream);
@@ -300,7 +307,7 @@ int gwf_ref_run(gwgpu_context *c, const GenParams *params, int n, int method, in
     a.nsrc = m;
     a.src_done = dcnt;
     a.item_counter = dcnt + m;
-    const int grid = std::min(m * ntiles, nsm * std::max(per_sm, 1));
+    const int grid = (int)std::min((long long)m * ntiles, slots);
     k_fref_main<<<grid, kRefBlock, smem, c->stream>>>(a);
     k_fref_finish<<<(m + 63) / 64, 64, 0, c->stream>>>(m, drs, add_prior, dfish, cov ? dcov : nullptr, dstat);
     cudaError_t e = cudaGetLastError();
