@@ -29,6 +29,9 @@
 // the FP64 values, i.e. the reference's maximum.  A pair with more than
 // kCand candidates (a flat spectrum) sends the batch to the FP64 transforms
 // (also selected by GWGPU_MAXLL=fp64).
+//
+// On uniform grids the waveform, the products g and the refinement's sums run on
+// pairs of FP32 numbers (phenom_acc.h): as FP64 they were 70 % of the time.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -336,6 +339,116 @@ __global__ void k_mx_prep(const Request *__restrict__ req, const double2 *__rest
   }
 }
 
+// k_mx_prep for the intrinsic mode on uniform grids: the waveform and the products
+// in two floats (g as pairs), a tile of kPrepTile bins per block.
+// Bound by memory: per pair and bin 16 B of data read and 16 + 8 B written (the
+// padding of a Bluestein row another 8 B per entry); 128 IMRPhenomD requests on
+// 3 x 32,128 bins against the FP64 bins: see run_search.
+constexpr int kPrepTile = 2048;
+template <bool UN>
+__global__ void __launch_bounds__(kBlock) k_mx_prep_ff(const gwt::AccReq *__restrict__ areq, int ndet,
+                                                       const StreamDev *__restrict__ streams,
+                                                       const int *__restrict__ handles, const gwt::AccTables tb,
+                                                       const gwt::AccLut *__restrict__ glut, int N, int ld, int blue,
+                                                       const float2 *__restrict__ chirp_tab, gwt::ff4 *__restrict__ g,
+                                                       float2 *__restrict__ a32, double *__restrict__ part) {
+  using namespace gwt;
+  constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1;
+  __shared__ AccLut lut;
+  __shared__ __align__(16) unsigned char s_req[sizeof(AccReq)];
+  __shared__ StreamDev s_st[kMaxDet];
+  __shared__ ff s_sc[kMaxDet];
+  __shared__ double s_hs[kMaxDet], s_red[kWarps];
+  const int r = blockIdx.y, tid = threadIdx.x;
+  const AccReq &x = *(const AccReq *)s_req;
+  for (int w = tid; w < (int)(sizeof(AccLut) / 4); w += kBlock) ((unsigned *)&lut)[w] = ((const unsigned *)glut)[w];
+  for (int w = tid; w < (int)(sizeof(AccReq) / 4); w += kBlock) ((unsigned *)s_req)[w] = ((const unsigned *)(areq + r))[w];
+  if (tid < ndet) s_st[tid] = streams[handles[(size_t)r * ndet + tid]];
+  __syncthreads();
+  if (tid < ndet) {  // the streams' pairs are W d / dscale and W / wscale, W = (4 df_s / 3) s_k / S_k
+    const StreamDev &st = s_st[tid];
+    const double A = x.m.A_scale;
+    s_sc[tid] = ff_split(A * (3.0 * st.dscale / st.simpson_df));
+    s_hs[tid] = A * A * st.wscale * (3.0 / (4.0 * st.simpson_df));
+  }
+  __syncthreads();
+  const int n0 = s_st[0].n0, k0 = blockIdx.x * kPrepTile, k1 = min(k0 + kPrepTile, ld);
+  const float *dev = s_st[0].dev;
+  const bool ok = x.m.status == 0;
+  ff acc[kMaxDet * NS];
+#pragma unroll
+  for (int j = 0; j < kMaxDet * NS; j++) acc[j] = ff{0.f, 0.f};
+  for (int k = k0 + tid; k < k1; k += kBlock) {
+    if (k >= N) {
+#pragma unroll
+      for (int dd = 0; dd < kMaxDet; dd++)
+        if (dd < ndet)
+          for (int u = 0; u < NP; u++) a32[((size_t)(r * ndet + dd) * NP + u) * ld + k] = make_float2(0.f, 0.f);
+      continue;
+    }
+    ff pr, pi, cr, ci;
+    const uint64_t qd = dev && ok ? acc_dev_turns(x, __ldg(dev + k)) : 0;
+    if (ok) acc_wave<UN>(x, n0 + k, qd, tb, lut, pr, pi, cr, ci);
+    else pr = pi = cr = ci = ff{0.f, 0.f};
+    const float2 ch = blue ? __ldg(chirp_tab + k) : make_float2(1.f, 0.f);
+    const float is = k == 0 || k == N - 1 ? 1.0f : (k & 1) ? 0.25f : 0.5f;  // 1 / s_k
+    const ff hh = ff_norm(ff_add(ff_sqr(pr), ff_sqr(pi)));
+    ff cc, hc;
+    if constexpr (UN) {
+      cc = ff_norm(ff_add(ff_sqr(cr), ff_sqr(ci)));
+      hc = ff_norm(ff_add(ff_mul(pr, cr), ff_mul(pi, ci)));
+    }
+#pragma unroll
+    for (int dd = 0; dd < kMaxDet; dd++) {
+      if (dd >= ndet) break;
+      const size_t q = (size_t)(r * ndet + dd) * NP;
+      const ff4 w = acc_ld(s_st[dd].wd + k);
+      const float2 wv = __ldg((const float2 *)s_st[dd].wf + k);
+      const ff wk{wv.x, wv.y}, sc{s_sc[dd].h * is, s_sc[dd].l * is};
+      const ff dr = ff_norm(ff_mul(ff{w.ch, w.cl}, sc)), di = ff_norm(ff_mul(ff{w.sh, w.sl}, sc));
+      auto product = [&](ff hr, ff hi, size_t row, ff &nn) {  // 4 conj(d) h / S
+        const ff vr = ff_norm(ff_add(ff_mul(dr, hr), ff_mul(di, hi))), vi = ff_norm(ff_sub(ff_mul(dr, hi), ff_mul(di, hr)));
+        g[row * N + k] = ff4{vr.h, vr.l, vi.h, vi.l};
+        a32[row * ld + k] = make_float2(vr.h * ch.x - vi.h * ch.y, vr.h * ch.y + vi.h * ch.x);
+        ff_acc(nn, ff_add(ff_sqr(vr), ff_sqr(vi)));
+      };
+      ff_acc(acc[dd * NS], ff_mul(wk, hh));
+      if constexpr (UN) {
+        ff_acc(acc[dd * NS + 1], ff_mul(wk, cc));
+        ff_acc(acc[dd * NS + 2], ff_mul(wk, hc));
+        product(pr, pi, q, acc[dd * NS + 3]);
+        product(cr, ci, q + 1, acc[dd * NS + 4]);
+      } else {
+        product(pr, pi, q, acc[dd * NS + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int dd = 0; dd < kMaxDet; dd++) {
+    if (dd >= ndet) break;
+#pragma unroll
+    for (int j = 0; j < NS; j++) {
+      ff v = acc[dd * NS + j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        v = ff_add(v, ff{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});
+      __syncthreads();  // the previous sum's warps have been read
+      if ((tid & 31) == 0) s_red[tid >> 5] = ff_value(v);
+      __syncthreads();
+      if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < kWarps; w++) t += s_red[w];
+        part[((size_t)(r * ndet + dd) * NS + j) * gridDim.x + blockIdx.x] = j < (UN ? 3 : 1) ? t * s_hs[dd] : t;
+      }
+    }
+  }
+}
+
+// The Bluestein chirp e^{-i pi k^2/N}, k < N, in FP32.
+__global__ void k_chirp_tab(float2 *__restrict__ t, int N) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) t[k] = chirp32(k, N);
+}
+
 __global__ void k_chirp_mul32(float2 *__restrict__ a, const float2 *__restrict__ B, int M, long long total) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -442,13 +555,16 @@ __global__ void k_mx_cand(const float2 *__restrict__ C, const double *__restrict
 // twiddle of n = 256 j + i as e^{-2 pi i (256 j k mod N)/N} e^{-2 pi i (i k mod N)/N}
 // (both phases reduced exactly in integers).  candval = |G_k|^2 (aligned) or
 // lambda (unaligned).  Persistent over the (pair, candidate) slots.
-template <bool UN>
-__global__ void k_mx_refine(const double2 *__restrict__ g64, int N, int pairs, const int *__restrict__ cand,
+// FF: the rows and the twiddle table as pairs of FP32 numbers, the sums over a
+// thread's bins in two floats.
+template <bool UN, bool FF>
+__global__ void k_mx_refine(const void *__restrict__ rows, int N, int pairs, const int *__restrict__ cand,
                             const int *__restrict__ ncand, const double *__restrict__ sums,
                             const StreamDev *__restrict__ streams, const int *__restrict__ handles,
                             double *__restrict__ candval) {
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1, NV = UN ? 4 : 2;
   extern __shared__ double2 s_wj[];
+  gwt::ff4 *s_wf = (gwt::ff4 *)s_wj;
   __shared__ double s_red[NV][kWarps];
   const int nj = (N + kBlock - 1) / kBlock;
   // slot s = (candidate ci, pair q) with ci major, so that the first
@@ -462,7 +578,12 @@ __global__ void k_mx_refine(const double2 *__restrict__ g64, int N, int pairs, c
       const long long t = ((long long)j * kBlock % N) * k % N;
       double sn, cs;
       sincospi(2.0 * (double)t / (double)N, &sn, &cs);
-      s_wj[j] = make_double2(cs, -sn);
+      if constexpr (FF) {
+        const gwt::ff a = gwt::ff_split(cs), b = gwt::ff_split(-sn);
+        s_wf[j] = gwt::ff4{a.h, a.l, b.h, b.l};
+      } else {
+        s_wj[j] = make_double2(cs, -sn);
+      }
     }
     double2 wi;
     {
@@ -477,8 +598,36 @@ __global__ void k_mx_refine(const double2 *__restrict__ g64, int N, int pairs, c
     for (int u = 0; u < NV; u++) v[u] = 0.0;
     // this thread's bins n = 256 j + i: sum_j g_n e^{-2 pi i 256 j k/N}, then
     // one product with e^{-2 pi i i k/N}
-    const double2 *row = g64 + ((size_t)q * NP) * N;
-    for (int j = 0; j < nj; j++) {
+    if constexpr (FF) {
+      using namespace gwt;
+      const ff4 *row = (const ff4 *)rows + ((size_t)q * NP) * N;
+      ff s[NV];
+#pragma unroll
+      for (int u = 0; u < NV; u++) s[u] = ff{0.f, 0.f};
+      for (int j = 0; j < nj; j++) {
+        const int n = j * kBlock + threadIdx.x;
+        if (n >= N) break;
+        const ff4 w = s_wf[j];
+        const ff wr{w.ch, w.cl}, wim{w.sh, w.sl};
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+          const ff4 x = acc_ld(row + (size_t)u * N + n);
+          const ff xr{x.ch, x.cl}, xi{x.sh, x.sl};
+          ff_acc(s[2 * u], ff_sub(ff_mul(xr, wr), ff_mul(xi, wim)));
+          ff_acc(s[2 * u + 1], ff_add(ff_mul(xr, wim), ff_mul(xi, wr)));
+        }
+        if ((j & 31) == 31)  // 32 terms to FP64: a longer two-float sum would lose digits
+#pragma unroll
+          for (int u = 0; u < NV; u++) {
+            v[u] += ff_value(s[u]);
+            s[u] = ff{0.f, 0.f};
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < NV; u++) v[u] += ff_value(s[u]);
+    }
+    const double2 *row = (const double2 *)rows + ((size_t)q * NP) * N;
+    for (int j = 0; !FF && j < nj; j++) {
       const int n = j * kBlock + threadIdx.x;
       if (n >= N) break;
       const double2 w = s_wj[j];
@@ -599,13 +748,14 @@ int xform_len(int N, int *blue) {
 
 // The Bluestein kernel for N, FFT_M(b)/M in FP64 (kWsChirp) and FP32
 // (kWsChirp32), and the search's error scale M max|B|, kept until N changes.
-int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const float2 **B32) {
+int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const float2 **B32, const float2 **tab) {
   void *kb, *kb32;
   int st = c->workspace(gwgpu_context::kWsChirp, 16 * (size_t)M + 256, &kb);
   if (st) return st;
-  if ((st = c->workspace(gwgpu_context::kWsChirp32, 8 * (size_t)M, &kb32))) return st;
+  if ((st = c->workspace(gwgpu_context::kWsChirp32, 8 * ((size_t)M + N), &kb32))) return st;
   *B64 = (const double2 *)kb;
   *B32 = (const float2 *)kb32;
+  *tab = *B32 + M;
   if (c->chirp_n == N) return GWGPU_OK;
   int p1;
   if ((st = gwfft::plan(c, gwfft::kZ2Z, M, 1, &p1))) return st;
@@ -615,6 +765,7 @@ int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const floa
   double *dmax = (double *)((char *)kb + 16 * (size_t)M);
   k_absmax<<<1, kBlock, 0, c->stream>>>((const double2 *)kb, M, dmax);
   k_to_f32<<<gb, kBlock, 0, c->stream>>>((const double2 *)kb, (float2 *)kb32, M);
+  k_chirp_tab<<<gb, kBlock, 0, c->stream>>>((float2 *)kb32 + M, N);
   double bmax = 0;
   cudaMemcpyAsync(&bmax, dmax, 8, cudaMemcpyDeviceToHost, c->stream);
   cudaError_t e = cudaStreamSynchronize(c->stream);
@@ -627,6 +778,7 @@ int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const floa
 // What both entry points hand to the pipeline (device pointers).
 struct MxIn {
   const Request *req = nullptr;               // requests (intrinsic mode), or null
+  const gwt::AccReq *areq = nullptr;          // the same for the search on two-float bins, or null
   const double2 *rp = nullptr, *rc = nullptr;  // responses per pair, rows of N, when req is null
   const StreamDev *streams = nullptr;
   const int *handles = nullptr;                // [n * ndet]
@@ -642,7 +794,8 @@ int run_fp64(gwgpu_context *c, const MxIn &in, double *out, int *status) {
   const int ld = xform_len(in.N, &blue);
   const double2 *B64 = nullptr;
   const float2 *B32 = nullptr;
-  int st = blue ? ensure_chirp(c, in.N, ld, &B64, &B32) : GWGPU_OK;
+  const float2 *ctab = nullptr;
+  int st = blue ? ensure_chirp(c, in.N, ld, &B64, &B32, &ctab) : GWGPU_OK;
   if (st) return st;
   int plan;  // fetched last: a new plan may reset the cache (cufft_rt.cu)
   if ((st = gwfft::plan(c, gwfft::kZ2Z, ld, rows, &plan))) return st;
@@ -688,16 +841,17 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   int blue;
   const int ld = xform_len(in.N, &blue);
   const double2 *B64 = nullptr;
-  const float2 *B32 = nullptr;
+  const float2 *B32 = nullptr, *ctab = nullptr;
   double kscale = std::sqrt((double)in.N);
   int st = GWGPU_OK;
   if (blue) {
-    if ((st = ensure_chirp(c, in.N, ld, &B64, &B32))) return st;
+    if ((st = ensure_chirp(c, in.N, ld, &B64, &B32, &ctab))) return st;
     kscale = c->chirp_kscale;
   }
   int plan;  // fetched last: a new plan may reset the cache (cufft_rt.cu)
   if ((st = gwfft::plan(c, gwfft::kC2C, ld, rows, &plan))) return st;
-  const int nblk = (ld + kBlock - 1) / kBlock;
+  const bool two = in.areq != nullptr;  // two-float bins
+  const int per = two ? kPrepTile : kBlock, nblk = (ld + per - 1) / per;
   const size_t o_g = 0, o_a = up256(16 * (size_t)rows * in.N), o_h = o_a + up256(8 * (size_t)rows * ld),
                o_s = o_h + up256(8 * (size_t)pairs * ns * nblk), o_c = o_s + up256(8 * (size_t)pairs * ns),
                o_nc = o_c + up256(4 * (size_t)pairs * kCand), o_v = o_nc + up256(4 * (size_t)pairs),
@@ -711,7 +865,13 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   int *cand = (int *)(b + o_c), *ncand = (int *)(b + o_nc), *ovf = (int *)(b + o_o);
   cudaMemsetAsync(ovf, 0, 4, c->stream);
   const dim3 grid(nblk, in.n);
-  if (in.un)
+  if (two && in.un)
+    k_mx_prep_ff<true><<<grid, kBlock, 0, c->stream>>>(in.areq, in.ndet, in.streams, in.handles, c->acc, c->acc_lut,
+                                                        in.N, ld, blue, ctab, (gwt::ff4 *)g64, a32, hh);
+  else if (two)
+    k_mx_prep_ff<false><<<grid, kBlock, 0, c->stream>>>(in.areq, in.ndet, in.streams, in.handles, c->acc, c->acc_lut,
+                                                         in.N, ld, blue, ctab, (gwt::ff4 *)g64, a32, hh);
+  else if (in.un)
     k_mx_prep<true><<<grid, kBlock, 0, c->stream>>>(in.req, in.rp, in.rc, in.ndet, in.streams, in.handles, in.N, ld,
                                                      blue, g64, a32, hh);
   else
@@ -741,17 +901,19 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   const int nj = (in.N + kBlock - 1) / kBlock;
   const size_t smem = 16 * (size_t)nj;
   const int gr = std::min(pairs * kCand, 152 * 8);
+  auto refine = [&](auto kern) {
+    if (smem > 48 * 1024)
+      cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<gr, kBlock, smem, c->stream>>>(g64, in.N, pairs, cand, ncand, sums, in.streams, in.handles, cv);
+  };
   if (in.un) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mx_refine<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_mx_refine<true><<<gr, kBlock, smem, c->stream>>>(g64, in.N, pairs, cand, ncand, sums, in.streams, in.handles,
-                                                        cv);
+    if (two) refine(k_mx_refine<true, true>);
+    else refine(k_mx_refine<true, false>);
     k_mx_final<true><<<(in.n + 127) / 128, 128, 0, c->stream>>>(cv, ncand, sums, in.n, in.ndet, in.streams,
                                                                  in.handles, in.req_status, out, status);
   } else {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_mx_refine<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_mx_refine<false><<<gr, kBlock, smem, c->stream>>>(g64, in.N, pairs, cand, ncand, sums, in.streams,
-                                                         in.handles, cv);
+    if (two) refine(k_mx_refine<false, true>);
+    else refine(k_mx_refine<false, false>);
     k_mx_final<false><<<(in.n + 127) / 128, 128, 0, c->stream>>>(cv, ncand, sums, in.n, in.ndet, in.streams,
                                                                   in.handles, in.req_status, out, status);
   }
@@ -759,11 +921,19 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   return e == cudaSuccess ? GWGPU_OK : c->fail(e, "maximised likelihood launch");
 }
 
-int maxll_run(gwgpu_context *c, const MxIn &in, double *out, int *status) {
-  if (!c->maxll_fp64 && (in.N + kBlock - 1) / kBlock <= kMaxTwiddleRows) {
+bool search_fits(const gwgpu_context *c, int N) { return !c->maxll_fp64 && (N + kBlock - 1) / kBlock <= kMaxTwiddleRows; }
+
+// *searched: false when only the FP64 transforms' inputs (in.req) will do.
+int maxll_run(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *searched = nullptr) {
+  if (searched) *searched = true;
+  if (search_fits(c, in.N)) {
     bool fb = false;
     int st = run_search(c, in, out, status, &fb);
     if (st || !fb) return st;
+  }
+  if (in.areq && !in.req) {
+    *searched = false;
+    return GWGPU_OK;
   }
   return run_fp64(c, in, out, status);
 }
@@ -849,7 +1019,8 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
   }
   const int pairs = n * ndet;
   const size_t o_p = 0, o_a = up256(sizeof(gwgpu_gen_params) * n), o_h = o_a + up256(4 * (size_t)n),
-               o_req = o_h + up256(4 * (size_t)pairs), o_out = o_req + up256(sizeof(Request) * n),
+               o_req = o_h + up256(4 * (size_t)pairs),
+               o_out = o_req + up256(std::max(sizeof(Request), sizeof(gwt::AccReq)) * n),
                o_st = o_out + up256(8 * (size_t)n), total = o_st + up256(4 * (size_t)n);
   void *dev;
   int st = c->workspace(gwgpu_context::kWsMaxll, total, &dev);
@@ -869,21 +1040,35 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
   cudaMemcpyAsync(b + o_p, hp.data(), sizeof(gwgpu_gen_params) * n, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(b + o_a, ap.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(b + o_h, handles, 4 * (size_t)pairs, cudaMemcpyHostToDevice, c->stream);
-  cudaError_t e = gwk::launch_prologue((const gwt::GenParams *)(b + o_p), (const int *)(b + o_a), n,
-                                       (const int *)(b + o_h), ndet, 0.0, 0, c->streams_dev, c->qnm_dev,
-                                       (Request *)(b + o_req), nullptr, 0, (int *)(b + o_st), c->stream);
-  if (e != cudaSuccess) return c->fail(e, "maximised likelihood prologue");
+  // two-float bins when every stream has its pairs; a search that gives up on
+  // them leaves the FP64 transforms, which take the requests themselves
+  bool two = c->acc_lut && search_fits(c, N);
+  for (int i = 0; i < pairs && two; i++) {
+    const StreamDev &sd = c->get_stream(handles[i])->dev;
+    two = sd.wd && sd.n0 + sd.N - 1 <= c->acc.nmax;
+  }
   int *dst = (int *)(b + o_st);
-  MxIn in;
-  in.req = (const Request *)(b + o_req);
-  in.streams = c->streams_dev;
-  in.handles = (const int *)(b + o_h);
-  in.req_status = dst;
-  in.n = n;
-  in.ndet = ndet;
-  in.N = N;
-  in.un = un;
-  if ((st = maxll_run(c, in, (double *)(b + o_out), dst))) return st;
+  cudaError_t e;
+  for (;;) {
+    e = gwk::launch_prologue((const gwt::GenParams *)(b + o_p), (const int *)(b + o_a), n, (const int *)(b + o_h),
+                             ndet, 0.0, 0, c->streams_dev, c->qnm_dev, two ? nullptr : (Request *)(b + o_req), nullptr,
+                             0, dst, c->stream, gwk::OrderArgs(), two ? (gwt::AccReq *)(b + o_req) : nullptr);
+    if (e != cudaSuccess) return c->fail(e, "maximised likelihood prologue");
+    MxIn in;
+    if (two) in.areq = (const gwt::AccReq *)(b + o_req);
+    else in.req = (const Request *)(b + o_req);
+    in.streams = c->streams_dev;
+    in.handles = (const int *)(b + o_h);
+    in.req_status = dst;
+    in.n = n;
+    in.ndet = ndet;
+    in.N = N;
+    in.un = un;
+    bool searched = true;
+    if ((st = maxll_run(c, in, (double *)(b + o_out), dst, &searched))) return st;
+    if (searched) break;
+    two = false;
+  }
   std::vector<int> hs(n);
   cudaMemcpyAsync(loglik, b + o_out, 8 * (size_t)n, cudaMemcpyDeviceToHost, c->stream);
   cudaMemcpyAsync(hs.data(), dst, 4 * (size_t)n, cudaMemcpyDeviceToHost, c->stream);

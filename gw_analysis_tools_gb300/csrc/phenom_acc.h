@@ -44,6 +44,7 @@ constexpr double kAccMaxTurns = 12.0;
 struct AccReq {
   MixedReq m;
   uint64_t L0[kMaxDet], L1[kMaxDet];  // linear phase of each detector, turns 2^64: L0 + L1 n
+  uint64_t B0, B1;                    // the same without a detector's delay and projection phase
   uint64_t pR0, pR1;                  // intermediate phase: its constant and linear terms
   uint64_t mR0, mR1;                  // ringdown phase: the same
   uint64_t mEq;                       // ringdown: mE / kTurnTab (mE atan at the table angles)
@@ -54,6 +55,7 @@ struct AccReq {
   uint64_t alQ, epQ;
   ff us[4];                           // 1/s = us0 i + us1 t + us2 n + us3 (the Wigner angle)
   ff y2p, y1p, y0p, y2m, y1m;         // harmonics: sums and differences of Y_m and Y_-m
+  ff c2z, s2z;                        // polarisation rotation
   float tc;                           // model's t_c, for bins off the line n df (acc_dev_turns)
   int fp64_phase;                     // 1: terms too large for two floats; every bin takes the FP64 series
 };
@@ -83,6 +85,8 @@ GW_HD void acc_det_phase(const Request &r, double df, AccReq &x, int d0 = 0, int
   const double c1 = pv2 ? r.p.t_corr * df : -m.tcs * df * inv2pi;
   const uint64_t q1 = acc_turns(c1) - acc_turns_prod(m.s.tc, df);
   x.tc = (float)m.s.tc;
+  x.B0 = q0;
+  x.B1 = q1;
   for (int d = d0; d < r.ndet && d < kMaxDet; d += step) {
     double Gre, Gim;
     mixed_det_G(r, d, Gre, Gim);
@@ -146,6 +150,8 @@ GW_HD void acc_pv2_coeffs(const Request &r, double df, AccReq &x) {
   x.y0p = ff_split(2.0 * kSqrt6 * 0.25 * Y[2]);
   x.y2m = ff_split(Y[0] - Y[4]);
   x.y1m = ff_split(-Y[1] - Y[3]);
+  x.c2z = ff_split(r.p.c2z);
+  x.s2z = ff_split(r.p.s2z);
 }
 // Whether the terms that the bins carry in two floats are small enough: their
 // rounding, ~4e-15 of the largest, must stay below the FP64 series' own.
@@ -299,11 +305,38 @@ GW_HD void acc_bin_d(const AccReq &x, int n, uint64_t qd, const AccTables &tb, c
     ff_acc(acc[2 * d + 1], ff_mul(a, v));
   }
 }
-// IMRPhenomPv2 bin: five sums per detector (mixed_bin_p's).  With cb, sb the
-// cosine and sine of beta, the twist-up reads
+// The IMRPhenomPv2 twist-up factors of bin n.  With cb, sb the cosine and sine of beta,
 //   h+ = p2 (1 + cb^2)/2 cos 2a + p1 sb cb cos a + p0 sb^2 + i (p2 cb sin 2a + p1 sb sin a)
 //   hx = i (m2 cb cos 2a + m1 sb cos a) - (m2 (1 + cb^2)/2 sin 2a + m1 sb cb sin a)
 // (the half-angle products of IMRPhenomP.cpp:665-715 collected by e^{i k alpha}).
+GW_HD void acc_twist(const AccReq &x, int n, const AccTables &tb, const AccLut &lut, ff t, uint64_t al, ff &hpr,
+                     ff &hpi, ff &hcr, ff &hci) {
+  const ff4 iw = acc_ld(tb.pv + n);
+  ff u = ff_add(ff_mul(x.us[0], ff{iw.ch, iw.cl}), ff_mul(x.us[1], t));
+  u = ff_norm(ff_add(ff_add(u, ff_mulf(x.us[2], (float)n)), x.us[3]));
+  ff cb, sb;
+  if (fabsf(u.h) < 1e9f) {
+    sb = ff_rsqrt(ff_norm(ff_addf(ff_sqr(u), 1.0f)));
+    cb = ff_norm(ff_mul(u.h < 0.0f ? ff_neg(u) : u, sb));
+  } else {  // beta below 1e-9; NaN stays NaN
+    sb = ff{f_rcp(fabsf(u.h)), 0.0f};
+    cb = ff{u.h == u.h ? 1.0f : u.h, 0.0f};
+  }
+  ff ca, sa;
+  ff_turns_sincos(al, lut.turn, ca, sa);
+  const ff s2 = ff_norm(ff_mul(ff{2.0f * sa.h, 2.0f * sa.l}, ca));
+  const ff ss = ff_sqr(sa);
+  const ff c2 = ff_norm(ff_addf(ff{-2.0f * ss.h, -2.0f * ss.l}, 1.0f));
+  const ff cc = ff_norm(ff_sqr(cb));
+  const ff hc2{0.5f * cc.h, 0.5f * cc.l};
+  const ff uu = ff_norm(ff_addf(hc2, 0.5f)), sc = ff_norm(ff_mul(sb, cb)), sq = ff_norm(ff_sqr(sb));
+  hpr = ff_norm(ff_add(ff_add(ff_mul(ff_norm(ff_mul(x.y2p, uu)), c2), ff_mul(ff_norm(ff_mul(x.y1p, sc)), ca)),
+                       ff_mul(x.y0p, sq)));
+  hpi = ff_norm(ff_add(ff_mul(ff_norm(ff_mul(x.y2p, cb)), s2), ff_mul(ff_norm(ff_mul(x.y1p, sb)), sa)));
+  hci = ff_norm(ff_add(ff_mul(ff_norm(ff_mul(x.y2m, cb)), c2), ff_mul(ff_norm(ff_mul(x.y1m, sb)), ca)));
+  hcr = ff_norm(ff_neg(ff_add(ff_mul(ff_norm(ff_mul(x.y2m, uu)), s2), ff_mul(ff_norm(ff_mul(x.y1m, sc)), sa))));
+}
+// IMRPhenomPv2 bin: five sums per detector (mixed_bin_p's).
 template <int NDET>
 GW_HD void acc_bin_p(const AccReq &x, int n, uint64_t qd, const AccTables &tb, const AccLut &lut, const ff4 *wd, const ff *w,
                      bool wshared, ff *acc) {
@@ -313,32 +346,7 @@ GW_HD void acc_bin_p(const AccReq &x, int n, uint64_t qd, const AccTables &tb, c
   uint64_t al;
   const uint64_t ph = qd + acc_phase<true>(x, n, tb, lut, t, al);
   ff hpr, hpi, hcr, hci;
-  {
-    const ff4 iw = acc_ld(tb.pv + n);
-    ff u = ff_add(ff_mul(x.us[0], ff{iw.ch, iw.cl}), ff_mul(x.us[1], t));
-    u = ff_norm(ff_add(ff_add(u, ff_mulf(x.us[2], (float)n)), x.us[3]));
-    ff cb, sb;
-    if (fabsf(u.h) < 1e9f) {
-      sb = ff_rsqrt(ff_norm(ff_addf(ff_sqr(u), 1.0f)));
-      cb = ff_norm(ff_mul(u.h < 0.0f ? ff_neg(u) : u, sb));
-    } else {  // beta below 1e-9; NaN stays NaN
-      sb = ff{f_rcp(fabsf(u.h)), 0.0f};
-      cb = ff{u.h == u.h ? 1.0f : u.h, 0.0f};
-    }
-    ff ca, sa;
-    ff_turns_sincos(al, lut.turn, ca, sa);
-    const ff s2 = ff_norm(ff_mul(ff{2.0f * sa.h, 2.0f * sa.l}, ca));
-    const ff ss = ff_sqr(sa);
-    const ff c2 = ff_norm(ff_addf(ff{-2.0f * ss.h, -2.0f * ss.l}, 1.0f));
-    const ff cc = ff_norm(ff_sqr(cb));
-    const ff hc2{0.5f * cc.h, 0.5f * cc.l};
-    const ff uu = ff_norm(ff_addf(hc2, 0.5f)), sc = ff_norm(ff_mul(sb, cb)), sq = ff_norm(ff_sqr(sb));
-    hpr = ff_norm(ff_add(ff_add(ff_mul(ff_norm(ff_mul(x.y2p, uu)), c2), ff_mul(ff_norm(ff_mul(x.y1p, sc)), ca)),
-                         ff_mul(x.y0p, sq)));
-    hpi = ff_norm(ff_add(ff_mul(ff_norm(ff_mul(x.y2p, cb)), s2), ff_mul(ff_norm(ff_mul(x.y1p, sb)), sa)));
-    hci = ff_norm(ff_add(ff_mul(ff_norm(ff_mul(x.y2m, cb)), c2), ff_mul(ff_norm(ff_mul(x.y1m, sb)), ca)));
-    hcr = ff_norm(ff_neg(ff_add(ff_mul(ff_norm(ff_mul(x.y2m, uu)), s2), ff_mul(ff_norm(ff_mul(x.y1m, sc)), sa))));
-  }
+  acc_twist(x, n, tb, lut, t, al, hpr, hpi, hcr, hci);
   const ff aa = ff_norm(ff_sqr(a));
   const ff spp = ff_norm(ff_mul(aa, ff_norm(ff_add(ff_sqr(hpr), ff_sqr(hpi)))));
   const ff scc = ff_norm(ff_mul(aa, ff_norm(ff_add(ff_sqr(hcr), ff_sqr(hci)))));
@@ -357,6 +365,37 @@ GW_HD void acc_bin_p(const AccReq &x, int n, uint64_t qd, const AccTables &tb, c
     const ff qi = ff_norm(ff_mul(a, ff_norm(ff_add(ff_mul(dr, s), ff_mul(di, c)))));
     ff_acc(acc[kAccPerDet * d + 3], ff_add(ff_mul(qr, hpr), ff_mul(qi, hpi)));
     ff_acc(acc[kAccPerDet * d + 4], ff_add(ff_mul(qr, hcr), ff_mul(qi, hci)));
+  }
+}
+
+// The model's polarisations / A_scale at bin n (zero beyond the cut): IMRPhenomD
+// h+ = h (1 + cos^2 iota)/2 and hx = -i h cos iota are left to the caller as h;
+// IMRPhenomPv2 h+, hx.
+template <bool PV2>
+GW_HD void acc_wave(const AccReq &x, int n, uint64_t qd, const AccTables &tb, const AccLut &lut, ff &pr, ff &pi,
+                    ff &cr, ff &ci) {
+  pr = pi = cr = ci = ff{0.f, 0.f};
+  if (n > x.m.n_cut) return;
+  const ff4 p = acc_ld(tb.pw + n);
+  const ff t{p.ch, p.cl};
+  const ff a = acc_amp(x, n, t, ff{p.sh, p.sl}, lut);
+  uint64_t al;
+  const uint64_t ph = qd + acc_phase<PV2>(x, n, tb, lut, t, al) + x.B0 + x.B1 * (uint64_t)n;
+  ff c, s;
+  ff_turns_sincos(ph, lut.turn, c, s);
+  const ff er = ff_norm(ff_mul(a, c)), ei = ff_norm(ff_neg(ff_mul(a, s)));  // a e^{-i psi}
+  if constexpr (!PV2) {
+    pr = er;
+    pi = ei;
+  } else {
+    ff hpr, hpi, hcr, hci;
+    acc_twist(x, n, tb, lut, t, al, hpr, hpi, hcr, hci);
+    const ff tpr = ff_norm(ff_sub(ff_mul(hpr, er), ff_mul(hpi, ei))), tpi = ff_norm(ff_add(ff_mul(hpr, ei), ff_mul(hpi, er)));
+    const ff txr = ff_norm(ff_sub(ff_mul(hcr, er), ff_mul(hci, ei))), txi = ff_norm(ff_add(ff_mul(hcr, ei), ff_mul(hci, er)));
+    pr = ff_norm(ff_add(ff_mul(x.c2z, tpr), ff_mul(x.s2z, txr)));
+    pi = ff_norm(ff_add(ff_mul(x.c2z, tpi), ff_mul(x.s2z, txi)));
+    cr = ff_norm(ff_sub(ff_mul(x.c2z, txr), ff_mul(x.s2z, tpr)));
+    ci = ff_norm(ff_sub(ff_mul(x.c2z, txi), ff_mul(x.s2z, tpi)));
   }
 }
 

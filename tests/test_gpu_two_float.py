@@ -125,3 +125,20 @@ def test_prologue_block_sizes(gpu_ctx, prec):
     finally:
         for h in hs:
             gpu_ctx.release_data(h)
+
+
+@pytest.mark.parametrize("T,N,ndet", [(8, 90, 1), (8, 2047, 2), (4, 2048, 1), (8, 2049, 4), (12, 5003, 3)])
+@pytest.mark.parametrize("ap", [0, 1])
+def test_maximized(gpu_ctx, oracle, T, N, ndet, ap):
+    """The maximised likelihood's two-float bins at tile edges, odd lengths and a rounded grid."""
+    f, data, psd, hs = _network(gpu_ctx, oracle, T, N, ndet)
+    try:
+        draws = [W.config1_source(), dict(W.config1_source(), spin1=(0.3, 0.1, 0.2))] + W.prior_draws(3, N, precessing=bool(ap))
+        bad = dict(draws[0], mass1=-3.0)
+        ref = np.array([oracle.maximized_loglik_intrinsic(d, f, data, psd, approximant=ap) for d in draws])
+        out, st = gpu_ctx.maximized_loglik_batch(G.params_array(draws + [bad]), hs, ap)
+        assert np.all(st[:-1] == 0) and st[-1] != 0 and np.isnan(out[-1])
+        assert _close(out[:-1], ref), np.abs(out[:-1] - ref)
+    finally:
+        for h in hs:
+            gpu_ctx.release_data(h)
