@@ -169,7 +169,7 @@ __global__ void k_chirp_mul(double2 *__restrict__ g, const double2 *__restrict__
   }
 }
 
-// Sum of v over the block (every thread gets it).
+// Sum of v over the block (every thread gets it; s_tmp: one double per warp).
 __device__ double block_sum(double v, double *s_tmp) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -177,7 +177,7 @@ __device__ double block_sum(double v, double *s_tmp) {
   if ((threadIdx.x & 31) == 0) s_tmp[threadIdx.x >> 5] = v;
   __syncthreads();
   double t = 0.0;
-  for (int w = 0; w < kWarps; w++) t += s_tmp[w];
+  for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s_tmp[w];
   return t;
 }
 
@@ -255,7 +255,7 @@ __global__ void k_maxll_reduce(const double2 *__restrict__ G, const double *__re
 // ======================================================= FP32 search path
 constexpr int kCand = 32;              // candidates per pair
 constexpr double kTau = 4e-5;          // FP32 transform error / (||a||_2 * kscale), with a 4x margin
-constexpr int kMaxTwiddleRows = 12288; // shared twiddle table of the FP64 refinement: N <= 256 * this
+constexpr int kMaxTwiddleRows = 12288; // shared twiddle table of the refinement: N <= 256 * this
 
 // e^{-i pi m^2 / N} in FP32 (phase reduced exactly in integers).
 __device__ __forceinline__ float2 chirp32(long long m, int N) {
@@ -342,11 +342,16 @@ __global__ void k_mx_prep(const Request *__restrict__ req, const double2 *__rest
 // k_mx_prep for the intrinsic mode on uniform grids: the waveform and the products
 // in two floats (g as pairs), a tile of kPrepTile bins per block.
 // Bound by memory: per pair and bin 16 B of data read and 16 + 8 B written (the
-// padding of a Bluestein row another 8 B per entry); 128 IMRPhenomD requests on
-// 3 x 32,128 bins against the FP64 bins: see run_search.
+// padding of a Bluestein row another 8 B per entry).  128 IMRPhenomD requests on
+// 3 x 32,128 bins: 1,480 -> 131 us against the FP64 bins; bins beyond a
+// request's cut only write their zeros (242 -> 131 us).
 constexpr int kPrepTile = 2048;
+// Bins of the grid below the model's cut (0 for a request outside its domain).
+__device__ __forceinline__ int live_bins(const gwt::AccReq &x, int n0, int N) {
+  return x.m.status ? 0 : max(0, min(N, x.m.n_cut - n0 + 1));
+}
 template <bool UN>
-__global__ void __launch_bounds__(kBlock) k_mx_prep_ff(const gwt::AccReq *__restrict__ areq, int ndet,
+__global__ void __launch_bounds__(kBlock, UN ? 1 : 3) k_mx_prep_ff(const gwt::AccReq *__restrict__ areq, int ndet,
                                                        const StreamDev *__restrict__ streams,
                                                        const int *__restrict__ handles, const gwt::AccTables tb,
                                                        const gwt::AccLut *__restrict__ glut, int N, int ld, int blue,
@@ -358,38 +363,38 @@ __global__ void __launch_bounds__(kBlock) k_mx_prep_ff(const gwt::AccReq *__rest
   __shared__ __align__(16) unsigned char s_req[sizeof(AccReq)];
   __shared__ StreamDev s_st[kMaxDet];
   __shared__ ff s_sc[kMaxDet];
-  __shared__ double s_hs[kMaxDet], s_red[kWarps];
+  __shared__ double s_hs[kMaxDet], s_red[kMaxDet * NS][kWarps];
   const int r = blockIdx.y, tid = threadIdx.x;
   const AccReq &x = *(const AccReq *)s_req;
-  for (int w = tid; w < (int)(sizeof(AccLut) / 4); w += kBlock) ((unsigned *)&lut)[w] = ((const unsigned *)glut)[w];
-  for (int w = tid; w < (int)(sizeof(AccReq) / 4); w += kBlock) ((unsigned *)s_req)[w] = ((const unsigned *)(areq + r))[w];
+  const int k0 = blockIdx.x * kPrepTile, k1 = min(k0 + kPrepTile, ld);
   if (tid < ndet) s_st[tid] = streams[handles[(size_t)r * ndet + tid]];
   __syncthreads();
+  // bins below the model's cut; g is neither written nor read beyond them
+  const int n0 = s_st[0].n0, kcut = live_bins(areq[r], n0, N);
+  if (k0 < kcut) {
+    for (int w = tid; w < (int)(sizeof(AccLut) / 4); w += kBlock) ((unsigned *)&lut)[w] = ((const unsigned *)glut)[w];
+    for (int w = tid; w < (int)(sizeof(AccReq) / 4); w += kBlock)
+      ((unsigned *)s_req)[w] = ((const unsigned *)(areq + r))[w];
+  }
   if (tid < ndet) {  // the streams' pairs are W d / dscale and W / wscale, W = (4 df_s / 3) s_k / S_k
     const StreamDev &st = s_st[tid];
-    const double A = x.m.A_scale;
+    const double A = areq[r].m.A_scale;
     s_sc[tid] = ff_split(A * (3.0 * st.dscale / st.simpson_df));
     s_hs[tid] = A * A * st.wscale * (3.0 / (4.0 * st.simpson_df));
   }
   __syncthreads();
-  const int n0 = s_st[0].n0, k0 = blockIdx.x * kPrepTile, k1 = min(k0 + kPrepTile, ld);
   const float *dev = s_st[0].dev;
-  const bool ok = x.m.status == 0;
   ff acc[kMaxDet * NS];
 #pragma unroll
   for (int j = 0; j < kMaxDet * NS; j++) acc[j] = ff{0.f, 0.f};
   for (int k = k0 + tid; k < k1; k += kBlock) {
-    if (k >= N) {
-#pragma unroll
-      for (int dd = 0; dd < kMaxDet; dd++)
-        if (dd < ndet)
-          for (int u = 0; u < NP; u++) a32[((size_t)(r * ndet + dd) * NP + u) * ld + k] = make_float2(0.f, 0.f);
+    if (k >= kcut) {
+      for (int q = r * ndet * NP; q < (r + 1) * ndet * NP; q++) a32[(size_t)q * ld + k] = make_float2(0.f, 0.f);
       continue;
     }
     ff pr, pi, cr, ci;
-    const uint64_t qd = dev && ok ? acc_dev_turns(x, __ldg(dev + k)) : 0;
-    if (ok) acc_wave<UN>(x, n0 + k, qd, tb, lut, pr, pi, cr, ci);
-    else pr = pi = cr = ci = ff{0.f, 0.f};
+    const uint64_t qd = dev ? acc_dev_turns(x, __ldg(dev + k)) : 0;
+    acc_wave<UN>(x, n0 + k, qd, tb, lut, pr, pi, cr, ci);
     const float2 ch = blue ? __ldg(chirp_tab + k) : make_float2(1.f, 0.f);
     const float is = k == 0 || k == N - 1 ? 1.0f : (k & 1) ? 0.25f : 0.5f;  // 1 / s_k
     const ff hh = ff_norm(ff_add(ff_sqr(pr), ff_sqr(pi)));
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_prep_ff(const gwt::AccReq *__rest
         const ff vr = ff_norm(ff_add(ff_mul(dr, hr), ff_mul(di, hi))), vi = ff_norm(ff_sub(ff_mul(dr, hi), ff_mul(di, hr)));
         g[row * N + k] = ff4{vr.h, vr.l, vi.h, vi.l};
         a32[row * ld + k] = make_float2(vr.h * ch.x - vi.h * ch.y, vr.h * ch.y + vi.h * ch.x);
-        ff_acc(nn, ff_add(ff_sqr(vr), ff_sqr(vi)));
+        nn.h = fmaf(vr.h, vr.h, fmaf(vi.h, vi.h, nn.h));  // |g|^2 for the search's error bound
       };
       ff_acc(acc[dd * NS], ff_mul(wk, hh));
       if constexpr (UN) {
@@ -432,15 +437,15 @@ __global__ void __launch_bounds__(kBlock) k_mx_prep_ff(const gwt::AccReq *__rest
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
         v = ff_add(v, ff{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});
-      __syncthreads();  // the previous sum's warps have been read
-      if ((tid & 31) == 0) s_red[tid >> 5] = ff_value(v);
-      __syncthreads();
-      if (tid == 0) {
-        double t = 0.0;
-        for (int w = 0; w < kWarps; w++) t += s_red[w];
-        part[((size_t)(r * ndet + dd) * NS + j) * gridDim.x + blockIdx.x] = j < (UN ? 3 : 1) ? t * s_hs[dd] : t;
-      }
+      if ((tid & 31) == 0) s_red[dd * NS + j][tid >> 5] = ff_value(v);
     }
+  }
+  __syncthreads();
+  if (tid < ndet * NS) {
+    double t = 0.0;
+    for (int w = 0; w < kWarps; w++) t += s_red[tid][w];
+    const int j = tid % NS;
+    part[((size_t)r * ndet * NS + tid) * gridDim.x + blockIdx.x] = j < (UN ? 3 : 1) ? t * s_hs[tid / NS] : t;
   }
 }
 
@@ -465,21 +470,21 @@ __device__ float block_max(float v, float *s_tmp) {
   if ((threadIdx.x & 31) == 0) s_tmp[threadIdx.x >> 5] = v;
   __syncthreads();
   float t = s_tmp[0];
-  for (int w = 1; w < kWarps; w++) t = fmaxf(t, s_tmp[w]);
+  for (int w = 1; w < (int)(blockDim.x >> 5); w++) t = fmaxf(t, s_tmp[w]);
   return t;
 }
 
 // One block per pair: the sums (Simpson sums scaled, |g|^2 raw, kept for the
 // refinement), the FP32 score of every k < N with its error bound, and the
 // candidates k whose score plus bound reaches the largest score minus bound.
+constexpr int kCandBlock = 1024;  // few pairs leave the chip short of loads in flight otherwise
 template <bool UN>
-__global__ void k_mx_cand(const float2 *__restrict__ C, const double *__restrict__ part, int nblk, int N, int ld,
+__global__ void __launch_bounds__(kCandBlock) k_mx_cand(const float2 *__restrict__ C, const double *__restrict__ part, int nblk, int N, int ld,
                           int ndet, const StreamDev *__restrict__ streams, const int *__restrict__ handles,
                           const int *__restrict__ req_status, double kscale, double *__restrict__ sums,
                           int *__restrict__ cand, int *__restrict__ ncand, int *__restrict__ overflow) {
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1;
-  __shared__ double s_tmp[kWarps];
-  __shared__ float s_tmpf[kWarps];
+  __shared__ float s_tmpf[kCandBlock / 32], s_scale[5];
   __shared__ int s_cnt;
   const int q = blockIdx.x, r = q / ndet;
   if (req_status && req_status[r]) {  // outside the model domain: no candidates, the result is NaN
@@ -488,27 +493,38 @@ __global__ void k_mx_cand(const float2 *__restrict__ C, const double *__restrict
   }
   const StreamDev &st = streams[handles[q]];
   const double df = st.freqs[1] - st.freqs[0];
-  double sm[NS];
+  // the sums and the scores' scales, on one warp (the FP64 pipe's time counts for
+  // every warp that repeats them)
+  if (threadIdx.x < 32) {
+    double sm[NS];
 #pragma unroll
-  for (int j = 0; j < NS; j++) {
-    double t = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) t += part[((size_t)q * NS + j) * nblk + b];
-    t = block_sum(t, s_tmp);
-    sm[j] = (UN ? j < 3 : j < 1) ? 4.0 * t * df / 3.0 : t;
+    for (int j = 0; j < NS; j++) {
+      double t = 0.0;
+      for (int b = threadIdx.x; b < nblk; b += 32) t += part[((size_t)q * NS + j) * nblk + b];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      sm[j] = (UN ? j < 3 : j < 1) ? 4.0 * t * df / 3.0 : t;
+    }
+    if (threadIdx.x == 0) {
+      for (int j = 0; j < NS; j++) sums[(size_t)q * NS + j] = sm[j];
+      s_cnt = 0;
+      if (UN) {
+        const float I = (float)(sm[2] / (sqrt(sm[0]) * sqrt(sm[1])));
+        const double ap = df / sqrt(sm[0]), ac = df / sqrt(sm[1]);
+        s_scale[0] = (float)ap;
+        s_scale[1] = (float)ac;
+        s_scale[2] = I;
+        s_scale[3] = (float)fmax((double)(float)ap * kTau * kscale * sqrt(sm[NS - 2]),
+                                 (double)(float)ac * kTau * kscale * sqrt(sm[NS - 1]));
+        s_scale[4] = 1.f / (1.f - fabsf(I));
+      } else {
+        s_scale[0] = (float)(kTau * kscale * sqrt(sm[1]));
+      }
+    }
   }
-  if (threadIdx.x < NS) sums[(size_t)q * NS + threadIdx.x] = sm[threadIdx.x];
-  if (threadIdx.x == 0) s_cnt = 0;
+  __syncthreads();
   // score and bound of bin k
-  float ap = 1.f, ac = 1.f, I = 0.f, eps = 0.f, E = 0.f, inv1mI = 1.f;
-  if (UN) {
-    ap = (float)(df / sqrt(sm[0]));
-    ac = (float)(df / sqrt(sm[1]));
-    I = (float)(sm[2] / (sqrt(sm[0]) * sqrt(sm[1])));
-    eps = (float)fmax(ap * kTau * kscale * sqrt(sm[3]), ac * kTau * kscale * sqrt(sm[4]));
-    inv1mI = 1.f / (1.f - fabsf(I));
-  } else {
-    E = (float)(kTau * kscale * sqrt(sm[1]));
-  }
+  const float ap = s_scale[0], ac = s_scale[1], I = s_scale[2], eps = s_scale[3], inv1mI = s_scale[4], E = s_scale[0];
   auto score = [&](int k, float &lo, float &hi) {
     if (!UN) {
       const float2 v = C[(size_t)q * ld + k];
@@ -529,21 +545,26 @@ __global__ void k_mx_cand(const float2 *__restrict__ C, const double *__restrict
       hi = lam + D;
     }
   };
-  float L = -INFINITY;
+  float L = -INFINITY, H = -INFINITY;  // H: the largest upper bound of this thread's bins
+  bool nan = false;
+#pragma unroll 4
   for (int k = threadIdx.x; k < N; k += blockDim.x) {
     float lo, hi;
     score(k, lo, hi);
     L = fmaxf(L, lo);
+    H = fmaxf(H, hi);
+    nan = nan || hi != hi;
   }
   L = block_max(L, s_tmpf);
-  for (int k = threadIdx.x; k < N; k += blockDim.x) {
-    float lo, hi;
-    score(k, lo, hi);
-    if (hi >= L || hi != hi) {  // NaN scores are candidates too
-      const int i = atomicAdd(&s_cnt, 1);
-      if (i < kCand) cand[(size_t)q * kCand + i] = k;
+  if (H >= L || nan)
+    for (int k = threadIdx.x; k < N; k += blockDim.x) {
+      float lo, hi;
+      score(k, lo, hi);
+      if (hi >= L || hi != hi) {  // NaN scores are candidates too
+        const int i = atomicAdd(&s_cnt, 1);
+        if (i < kCand) cand[(size_t)q * kCand + i] = k;
+      }
     }
-  }
   __syncthreads();
   if (threadIdx.x == 0) {
     ncand[q] = min(s_cnt, kCand);
@@ -551,20 +572,142 @@ __global__ void k_mx_cand(const float2 *__restrict__ C, const double *__restrict
   }
 }
 
+// Fewer candidates for the refinement (two-float rows): the direct sum of each in
+// FP32, four at a time so that a row is read once for them.  Sums of 16 products
+// (FP32 twiddles, within 2^-22) join a two-float total, so each |G_k| is off by at
+// most 32 2^-24 ||g||_1 <= 32 2^-24 sqrt(N) ||g||_2 -- a few percent of the
+// transform's bound -- and the same interval test leaves those that may still be
+// the maximum.  One block per pair; pairs with one candidate have nothing to do.
+constexpr int kScreen = 4;
+template <bool UN>
+__global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict__ rows,
+                                                      const gwt::AccReq *__restrict__ areq, int ndet, int N,
+                                                      const StreamDev *__restrict__ streams,
+                                                      const int *__restrict__ handles, const double *__restrict__ sums,
+                                                      int *__restrict__ cand, int *__restrict__ ncand) {
+  using namespace gwt;
+  constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1;
+  extern __shared__ float2 s_tw[];  // [kScreen][nj]
+  __shared__ double s_part[kScreen * NP * 2][kWarps];
+  __shared__ float s_lo[kCand], s_hi[kCand];
+  __shared__ int s_k[kCand], s_keep;
+  const int q = blockIdx.x, tid = threadIdx.x, nc = ncand[q];
+  if (nc <= 1) return;
+  const StreamDev &st = streams[handles[q]];
+  const int nl = live_bins(areq[q / ndet], streams[handles[q - q % ndet]].n0, N), nj = (N + kBlock - 1) / kBlock;
+  if (tid < nc) s_k[tid] = cand[(size_t)q * kCand + tid];
+  if (tid == 0) s_keep = 0;
+  auto twiddle = [&](unsigned long long m) {  // e^{-2 pi i m / N}, m < N
+    float s, c;
+    q64_sincospi(((m << 32) / (unsigned)N) << 32, &s, &c);
+    return make_float2(c, -s);
+  };
+  const double *sm = sums + (size_t)q * NS;
+  const double unit = 32.0 / 16777216.0 * sqrt((double)N);
+  for (int c0 = 0; c0 < nc; c0 += kScreen) {
+    const int mc = min(kScreen, nc - c0);
+    __syncthreads();
+    for (int e = tid; e < mc * nj; e += kBlock) {
+      const int c = e / nj, j = e - c * nj;
+      s_tw[e] = twiddle(((unsigned long long)j * kBlock % N) * s_k[c0 + c] % N);
+    }
+    __syncthreads();
+    ff tot[kScreen * NP * 2];
+#pragma unroll
+    for (int u = 0; u < kScreen * NP * 2; u++) tot[u] = ff{0.f, 0.f};
+    const ff4 *row = rows + (size_t)q * NP * N;
+    for (int j0 = 0; j0 * kBlock < nl; j0 += 16) {
+      float a[kScreen * NP * 2];
+#pragma unroll
+      for (int u = 0; u < kScreen * NP * 2; u++) a[u] = 0.f;
+#pragma unroll 8
+      for (int j = j0; j < j0 + 16; j++) {
+        const int n = j * kBlock + tid;
+        const bool in = n < nl;
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+          const ff4 x = in ? acc_ld(row + (size_t)p * N + n) : ff4{0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int c = 0; c < kScreen; c++) {
+            const float2 w = s_tw[in && c < mc ? c * nj + j : 0];
+            float &re = a[(c * NP + p) * 2], &im = a[(c * NP + p) * 2 + 1];
+            re = fmaf(x.ch, w.x, fmaf(-x.sh, w.y, re));
+            im = fmaf(x.ch, w.y, fmaf(x.sh, w.x, im));
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kScreen * NP * 2; u++) ff_acc(tot[u], ff{a[u], 0.f});
+    }
+#pragma unroll
+    for (int c = 0; c < kScreen; c++) {
+      const float2 w = twiddle(c < mc ? (unsigned long long)tid * s_k[c0 + c] % N : 0);
+#pragma unroll
+      for (int p = 0; p < NP; p++) {
+        const ff re = tot[(c * NP + p) * 2], im = tot[(c * NP + p) * 2 + 1];
+        ff v[2] = {two_sum(fmaf(re.h, w.x, -(im.h * w.y)), 0.f), two_sum(fmaf(re.h, w.y, im.h * w.x), 0.f)};
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+            v[u] = ff_add(v[u], ff{__shfl_xor_sync(0xffffffffu, v[u].h, o), __shfl_xor_sync(0xffffffffu, v[u].l, o)});
+          if ((tid & 31) == 0) s_part[(c * NP + p) * 2 + u][tid >> 5] = ff_value(v[u]);
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < mc) {
+      double G[NP * 2];
+#pragma unroll
+      for (int u = 0; u < NP * 2; u++) {
+        G[u] = 0.0;
+        for (int w = 0; w < kWarps; w++) G[u] += s_part[tid * NP * 2 + u][w];
+      }
+      double lo, hi;
+      if (!UN) {
+        const double mag = sqrt(G[0] * G[0] + G[1] * G[1]), E = unit * sqrt(sm[1]);
+        lo = mag - E;
+        hi = mag + E;
+      } else {
+        const double df = st.freqs[1] - st.freqs[0], ap = df / sqrt(sm[0]), ac = df / sqrt(sm[1]);
+        const double I = sm[2] / (sqrt(sm[0]) * sqrt(sm[1]));
+        const double eps = fmax(ap * unit * sqrt(sm[3]), ac * unit * sqrt(sm[4]));
+        const double rpx = ap * G[0], rpy = ap * G[1], rcx = ac * G[NP * 2 - 2], rcy = ac * G[NP * 2 - 1];
+        const double p2 = rpx * rpx + rpy * rpy, c2 = rcx * rcx + rcy * rcy, gam = rpx * rcx + rpy * rcy;
+        const double lam = (p2 + c2 - 2 * gam * I +
+                            sqrt(fmax((p2 - c2) * (p2 - c2) + 4. * (I * p2 - gam) * (I * c2 - gam), 0.0))) / (1. - I * I);
+        // k_mx_cand's bound on lambda with this error
+        const double D = 2. * (4. * (sqrt(p2) + sqrt(c2) + 2. * eps) * eps + 4. * eps * eps) / (1. - fabs(I)) +
+                         1e-5 * fabs(lam);
+        lo = lam - D;
+        hi = lam + D;
+      }
+      // outward to FP32
+      s_lo[c0 + tid] = (float)lo - fabsf((float)lo) * 2.4e-7f;
+      s_hi[c0 + tid] = (float)hi + fabsf((float)hi) * 2.4e-7f;
+    }
+  }
+  __syncthreads();
+  if (tid < nc) {
+    float L = -INFINITY;
+    for (int c = 0; c < nc; c++) L = fmaxf(L, s_lo[c]);
+    if (!(s_hi[tid] < L)) cand[(size_t)q * kCand + atomicAdd(&s_keep, 1)] = s_k[tid];
+  }
+  __syncthreads();
+  if (tid == 0) ncand[q] = s_keep;
+}
+
 // G_k of the candidate rows exactly in FP64: sum_n g_n e^{-2 pi i nk/N}, the
 // twiddle of n = 256 j + i as e^{-2 pi i (256 j k mod N)/N} e^{-2 pi i (i k mod N)/N}
 // (both phases reduced exactly in integers).  candval = |G_k|^2 (aligned) or
 // lambda (unaligned).  Persistent over the (pair, candidate) slots.
-// FF: the rows and the twiddle table as pairs of FP32 numbers, the sums over a
-// thread's bins in two floats.
-template <bool UN, bool FF>
-__global__ void k_mx_refine(const void *__restrict__ rows, int N, int pairs, const int *__restrict__ cand,
+template <bool UN>
+__global__ void k_mx_refine(const double2 *__restrict__ g64, int N, int pairs, const int *__restrict__ cand,
                             const int *__restrict__ ncand, const double *__restrict__ sums,
                             const StreamDev *__restrict__ streams, const int *__restrict__ handles,
                             double *__restrict__ candval) {
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1, NV = UN ? 4 : 2;
   extern __shared__ double2 s_wj[];
-  gwt::ff4 *s_wf = (gwt::ff4 *)s_wj;
   __shared__ double s_red[NV][kWarps];
   const int nj = (N + kBlock - 1) / kBlock;
   // slot s = (candidate ci, pair q) with ci major, so that the first
@@ -578,12 +721,7 @@ __global__ void k_mx_refine(const void *__restrict__ rows, int N, int pairs, con
       const long long t = ((long long)j * kBlock % N) * k % N;
       double sn, cs;
       sincospi(2.0 * (double)t / (double)N, &sn, &cs);
-      if constexpr (FF) {
-        const gwt::ff a = gwt::ff_split(cs), b = gwt::ff_split(-sn);
-        s_wf[j] = gwt::ff4{a.h, a.l, b.h, b.l};
-      } else {
-        s_wj[j] = make_double2(cs, -sn);
-      }
+      s_wj[j] = make_double2(cs, -sn);
     }
     double2 wi;
     {
@@ -598,36 +736,8 @@ __global__ void k_mx_refine(const void *__restrict__ rows, int N, int pairs, con
     for (int u = 0; u < NV; u++) v[u] = 0.0;
     // this thread's bins n = 256 j + i: sum_j g_n e^{-2 pi i 256 j k/N}, then
     // one product with e^{-2 pi i i k/N}
-    if constexpr (FF) {
-      using namespace gwt;
-      const ff4 *row = (const ff4 *)rows + ((size_t)q * NP) * N;
-      ff s[NV];
-#pragma unroll
-      for (int u = 0; u < NV; u++) s[u] = ff{0.f, 0.f};
-      for (int j = 0; j < nj; j++) {
-        const int n = j * kBlock + threadIdx.x;
-        if (n >= N) break;
-        const ff4 w = s_wf[j];
-        const ff wr{w.ch, w.cl}, wim{w.sh, w.sl};
-#pragma unroll
-        for (int u = 0; u < NP; u++) {
-          const ff4 x = acc_ld(row + (size_t)u * N + n);
-          const ff xr{x.ch, x.cl}, xi{x.sh, x.sl};
-          ff_acc(s[2 * u], ff_sub(ff_mul(xr, wr), ff_mul(xi, wim)));
-          ff_acc(s[2 * u + 1], ff_add(ff_mul(xr, wim), ff_mul(xi, wr)));
-        }
-        if ((j & 31) == 31)  // 32 terms to FP64: a longer two-float sum would lose digits
-#pragma unroll
-          for (int u = 0; u < NV; u++) {
-            v[u] += ff_value(s[u]);
-            s[u] = ff{0.f, 0.f};
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < NV; u++) v[u] += ff_value(s[u]);
-    }
-    const double2 *row = (const double2 *)rows + ((size_t)q * NP) * N;
-    for (int j = 0; !FF && j < nj; j++) {
+    const double2 *row = g64 + ((size_t)q * NP) * N;
+    for (int j = 0; j < nj; j++) {
       const int n = j * kBlock + threadIdx.x;
       if (n >= N) break;
       const double2 w = s_wj[j];
@@ -671,6 +781,112 @@ __global__ void k_mx_refine(const void *__restrict__ rows, int N, int pairs, con
         const double ap = df / sqrt(sm[0]), ac = df / sqrt(sm[1]);
         const double I = sm[2] / (sqrt(sm[0]) * sqrt(sm[1]));
         const double rpx = ap * G[0], rpy = ap * G[1], rcx = ac * G[2], rcy = ac * G[3];
+        const double p2 = rpx * rpx + rpy * rpy, c2 = rcx * rcx + rcy * rcy, gam = rpx * rcx + rpy * rcy;
+        candval[it] =
+            (p2 + c2 - 2 * gam * I + sqrt((p2 - c2) * (p2 - c2) + 4. * (I * p2 - gam) * (I * c2 - gam))) / (1. - I * I);
+      }
+    }
+  }
+}
+
+// k_mx_refine on two-float rows: the twiddles from their exact fixed-point turns,
+// products and sums in two floats, bins beyond the cut left out.  Few blocks have
+// work (a candidate or two per pair), so a thread keeps eight loads in flight.
+template <bool UN>
+__global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restrict__ rows,
+                                                         const gwt::AccReq *__restrict__ areq, int ndet,
+                                                         const gwt::AccLut *__restrict__ glut, int N, int pairs,
+                                                         const int *__restrict__ cand, const int *__restrict__ ncand,
+                                                         const double *__restrict__ sums,
+                                                         const StreamDev *__restrict__ streams,
+                                                         const int *__restrict__ handles, double *__restrict__ candval) {
+  using namespace gwt;
+  constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1, NV = 2 * NP;
+  extern __shared__ double2 s_wj[];
+  ff4 *s_wf = (ff4 *)s_wj, *s_turn = s_wf + (N + kBlock - 1) / kBlock;
+  __shared__ double s_red[NV][kWarps];
+  const int nj = (N + kBlock - 1) / kBlock, tid = threadIdx.x;
+  bool loaded = false;
+  for (int sl = blockIdx.x; sl < pairs * kCand; sl += gridDim.x) {
+    const int q = sl % pairs, ci = sl / pairs, it = q * kCand + ci;
+    if (ci >= ncand[q]) continue;
+    const unsigned k = (unsigned)cand[it];
+    __syncthreads();  // the previous slot's table has been read
+    if (!loaded) {
+      for (int w = tid; w < kTurnTab; w += kBlock) s_turn[w] = acc_ld(glut->turn + w);
+      __syncthreads();
+      loaded = true;
+    }
+    auto twiddle = [&](unsigned long long m, ff &c, ff &s) {  // e^{-2 pi i m / N}, m < N: m / N 2^64 in two quotients
+      const unsigned long long a = (m << 32) / (unsigned)N, rem = (m << 32) - a * (unsigned)N;
+      ff_turns_sincos(0ull - ((a << 32) + (rem << 32) / (unsigned)N), s_turn, c, s);
+    };
+    for (int j = tid; j < nj; j += kBlock) {
+      ff c, s;
+      twiddle(((unsigned long long)j * kBlock % N) * k % N, c, s);
+      s_wf[j] = ff4{c.h, c.l, s.h, s.l};
+    }
+    ff wc, ws;
+    twiddle((unsigned long long)tid * k % N, wc, ws);
+    __syncthreads();
+    const int nl = live_bins(areq[q / ndet], streams[handles[q - q % ndet]].n0, N);
+    const ff4 *row = rows + ((size_t)q * NP) * N;
+    // this thread's bins n = 256 j + i: sum_j g_n e^{-2 pi i 256 j k/N}, then
+    // one product with e^{-2 pi i i k/N}
+    ff v[NV];
+#pragma unroll
+    for (int u = 0; u < NV; u++) v[u] = ff{0.f, 0.f};
+    for (int j0 = 0; j0 * kBlock < nl; j0 += 8) {
+      ff4 x[8][NP];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int n = (j0 + j) * kBlock + tid;
+#pragma unroll
+        for (int u = 0; u < NP; u++) x[j][u] = n < nl ? acc_ld(row + (size_t)u * N + n) : ff4{0.f, 0.f, 0.f, 0.f};
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const ff4 w = s_wf[j0 + j < nj ? j0 + j : 0];
+        const ff wr{w.ch, w.cl}, wi{w.sh, w.sl};
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+          const ff xr{x[j][u].ch, x[j][u].cl}, xi{x[j][u].sh, x[j][u].sl};
+          ff_acc(v[2 * u], ff_sub(ff_mul(xr, wr), ff_mul(xi, wi)));
+          ff_acc(v[2 * u + 1], ff_add(ff_mul(xr, wi), ff_mul(xi, wr)));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < NV; u++) v[u] = ff_norm(v[u]);  // the low part stays an ulp of the sum
+    }
+#pragma unroll
+    for (int u = 0; u < NV; u += 2) {
+      ff p[2] = {ff_norm(ff_sub(ff_mul(v[u], wc), ff_mul(v[u + 1], ws))),
+                 ff_norm(ff_add(ff_mul(v[u], ws), ff_mul(v[u + 1], wc)))};
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          p[e] = ff_add(p[e], ff{__shfl_xor_sync(0xffffffffu, p[e].h, o), __shfl_xor_sync(0xffffffffu, p[e].l, o)});
+        if ((tid & 31) == 0) s_red[u + e][tid >> 5] = ff_value(p[e]);
+      }
+    }
+    __syncthreads();
+    if (tid == 0) {
+      double G[NV];
+#pragma unroll
+      for (int u = 0; u < NV; u++) {
+        G[u] = 0.0;
+        for (int w = 0; w < kWarps; w++) G[u] += s_red[u][w];
+      }
+      if (!UN) {
+        candval[it] = G[0] * G[0] + G[1] * G[1];
+      } else {
+        const double *sm = sums + (size_t)q * NS;
+        const StreamDev &st = streams[handles[q]];
+        const double df = st.freqs[1] - st.freqs[0];
+        const double ap = df / sqrt(sm[0]), ac = df / sqrt(sm[1]);
+        const double I = sm[2] / (sqrt(sm[0]) * sqrt(sm[1]));
+        const double rpx = ap * G[0], rpy = ap * G[1], rcx = ac * G[NV - 2], rcy = ac * G[NV - 1];
         const double p2 = rpx * rpx + rpy * rpy, c2 = rcx * rcx + rcy * rcy, gam = rpx * rcx + rpy * rcy;
         candval[it] =
             (p2 + c2 - 2 * gam * I + sqrt((p2 - c2) * (p2 - c2) + 4. * (I * p2 - gam) * (I * c2 - gam))) / (1. - I * I);
@@ -833,8 +1049,12 @@ int run_fp64(gwgpu_context *c, const MxIn &in, double *out, int *status) {
   return e == cudaSuccess ? GWGPU_OK : c->fail(e, "maximised likelihood launch");
 }
 
-// The FP32 search and FP64 refinement; *fallback set when a pair had more
-// candidates than kCand (nothing written to out then).
+// The FP32 search and its refinement; *fallback set when a pair had more
+// candidates than kCand (nothing written to out then).  128 IMRPhenomD requests
+// on 3 x 32,128 bins, device time by kernel: products 131, transforms and chirp
+// 434, candidates 56 (132 with its FP64 sums on every warp), screen 45 and
+// two-float refinement 71 (389 for FP64 sums of every candidate over the whole
+// row), result 9 us; the transforms' memory traffic is the largest part left.
 int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *fallback) {
   const int np = in.un ? 2 : 1, ns = in.un ? 5 : 2, pairs = in.n * in.ndet, rows = pairs * np;
   *fallback = false;
@@ -885,10 +1105,10 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
     if ((st = gwfft::exec_c2c(c, plan, a32, a32, gwfft::kInverse, c->stream))) return st;
   }
   if (in.un)
-    k_mx_cand<true><<<pairs, kBlock, 0, c->stream>>>(a32, hh, nblk, in.N, ld, in.ndet, in.streams, in.handles,
+    k_mx_cand<true><<<pairs, kCandBlock, 0, c->stream>>>(a32, hh, nblk, in.N, ld, in.ndet, in.streams, in.handles,
                                                       in.req_status, kscale, sums, cand, ncand, ovf);
   else
-    k_mx_cand<false><<<pairs, kBlock, 0, c->stream>>>(a32, hh, nblk, in.N, ld, in.ndet, in.streams, in.handles,
+    k_mx_cand<false><<<pairs, kCandBlock, 0, c->stream>>>(a32, hh, nblk, in.N, ld, in.ndet, in.streams, in.handles,
                                                        in.req_status, kscale, sums, cand, ncand, ovf);
   int h_ovf = 0;
   cudaMemcpyAsync(&h_ovf, ovf, 4, cudaMemcpyDeviceToHost, c->stream);
@@ -901,22 +1121,40 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   const int nj = (in.N + kBlock - 1) / kBlock;
   const size_t smem = 16 * (size_t)nj;
   const int gr = std::min(pairs * kCand, 152 * 8);
+  if (two) {
+    const size_t tw = sizeof(float2) * (size_t)kScreen * nj;
+    auto screen = [&](auto kern) {
+      if (tw > 48 * 1024) cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tw);
+      kern<<<pairs, kBlock, tw, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, in.N, in.streams, in.handles,
+                                              sums, cand, ncand);
+    };
+    if (tw <= 200 * 1024) {  // longer rows keep every candidate
+      if (in.un) screen(k_mx_screen<true>);
+      else screen(k_mx_screen<false>);
+    }
+  }
   auto refine = [&](auto kern) {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kern<<<gr, kBlock, smem, c->stream>>>(g64, in.N, pairs, cand, ncand, sums, in.streams, in.handles, cv);
   };
-  if (in.un) {
-    if (two) refine(k_mx_refine<true, true>);
-    else refine(k_mx_refine<true, false>);
+  const size_t smem_ff = smem + sizeof(gwt::ff4) * gwt::kTurnTab;
+  auto refine_ff = [&](auto kern) {
+    if (smem_ff > 48 * 1024)
+      cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ff);
+    kern<<<gr, kBlock, smem_ff, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, c->acc_lut, in.N, pairs, cand,
+                                             ncand, sums, in.streams, in.handles, cv);
+  };
+  if (two && in.un) refine_ff(k_mx_refine_ff<true>);
+  else if (two) refine_ff(k_mx_refine_ff<false>);
+  else if (in.un) refine(k_mx_refine<true>);
+  else refine(k_mx_refine<false>);
+  if (in.un)
     k_mx_final<true><<<(in.n + 127) / 128, 128, 0, c->stream>>>(cv, ncand, sums, in.n, in.ndet, in.streams,
                                                                  in.handles, in.req_status, out, status);
-  } else {
-    if (two) refine(k_mx_refine<false, true>);
-    else refine(k_mx_refine<false, false>);
+  else
     k_mx_final<false><<<(in.n + 127) / 128, 128, 0, c->stream>>>(cv, ncand, sums, in.n, in.ndet, in.streams,
                                                                   in.handles, in.req_status, out, status);
-  }
   e = cudaGetLastError();
   return e == cudaSuccess ? GWGPU_OK : c->fail(e, "maximised likelihood launch");
 }
@@ -1042,7 +1280,7 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
   cudaMemcpyAsync(b + o_h, handles, 4 * (size_t)pairs, cudaMemcpyHostToDevice, c->stream);
   // two-float bins when every stream has its pairs; a search that gives up on
   // them leaves the FP64 transforms, which take the requests themselves
-  bool two = c->acc_lut && search_fits(c, N);
+  bool two = c->acc_lut && search_fits(c, N) && N <= kBlock * (kMaxTwiddleRows - gwt::kTurnTab);
   for (int i = 0; i < pairs && two; i++) {
     const StreamDev &sd = c->get_stream(handles[i])->dev;
     two = sd.wd && sd.n0 + sd.N - 1 <= c->acc.nmax;
