@@ -26,8 +26,10 @@
 
 #include "../../include/gwgpu.h"
 #include "capi_internal.h"
+#include "fisher_ff.h"
 #include "fisher_math.h"
 #include "fisher_ref.h"
+#include "kernel_util.cuh"
 #include "kernels.h"
 
 namespace gwf {
@@ -37,6 +39,7 @@ using gwk::StreamDev;
 constexpr int kBlock = 128;
 constexpr int kStatusBounds = 0x100;  // set by a tile whose bins fall outside the tables
 constexpr int kStatusRedo = 10;       // five-point source left to the reference algorithm (never returned)
+constexpr int kStatusFp64 = 11;       // a source that two floats cannot hold, left to the FP64 sums (never returned)
 
 // ------------------------------------------------------------- batched form
 __global__ void k_fisher_slots(const GenParams *__restrict__ params, int nsrc, int method, const int *__restrict__ dets,
@@ -47,13 +50,39 @@ __global__ void k_fisher_slots(const GenParams *__restrict__ params, int nsrc, i
   fisher_slot(params[g / kSlots], g % kSlots, method, dets, ndet, df, epsilon, step_mode, qnm, out[g]);
 }
 
-__global__ void k_fisher_setup(const GenParams *__restrict__ params, int nsrc, int method, int ndet, double epsilon,
-                               int step_mode, int order, const SlotOut *__restrict__ slots, FisherSrc *out,
-                               int *status) {
-  int src = blockIdx.x * blockDim.x + threadIdx.x;
-  if (src >= nsrc) return;
-  status[src] =
-      fisher_setup(params[src], method, ndet, epsilon, step_mode, order, slots + (size_t)src * kSlots, out[src]);
+// One warp per source: lane 0 the head, a lane per waveform pair, then a lane
+// per extrinsic row, and with FF the pairs' two-float coefficients.  Bound by
+// the latency of one lane's chain (11 perturbed parameters, the pairs' two-float
+// coefficients); 256 sources x 3 detectors 68 us, one thread per source 292.
+template <bool FF>
+__global__ void __launch_bounds__(32) k_fisher_setup(const GenParams *__restrict__ params, int method, int ndet,
+                                                     double epsilon, int step_mode, int order,
+                                                     const SlotOut *__restrict__ slots, FisherSrc *out, FfSrc *ffout,
+                                                     int *status) {
+  const int src = blockIdx.x, lane = threadIdx.x;
+  const SlotOut *S = slots + (size_t)src * kSlots;
+  FisherSrc &F = out[src];
+  if (lane == 0) {
+    fisher_setup_head(params[src], method, epsilon, step_mode, S, F);
+    status[src] = F.status;
+  }
+  __syncwarp();
+  if (lane < kIntr) fisher_setup_pair(S, lane, F);
+  for (int j = lane; j < ndet * (kCheap + 1); j += 32) {
+    const int d = j / (kCheap + 1), i = j % (kCheap + 1);
+    if (i < kCheap) fisher_setup_row(S, order, d, i, F);
+    else fisher_setup_det(S, order, d, F);
+  }
+  __syncwarp();
+  if (lane == 0) fisher_setup_route(order, F);
+  if constexpr (FF) {
+    FfSrc &X = ffout[src];
+    bool ok = true;
+    if (lane < kIntr) ok = ff_pair(F, lane, X.q[lane]);
+    else if (lane == kIntr) ok = ff_centre(F, X);
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) X.ok = ok;
+  }
 }
 
 struct FisherArgs {
@@ -74,6 +103,11 @@ struct FisherArgs {
   gwt::Tables tab;
   const double *tm76d;
   int tm76d_n;              // tm76d valid for n <= tm76d_n
+  // two-float sums: the sources' coefficients, the power tables, the weights
+  const FfSrc *ff;
+  gwt::AccTables acc;
+  const gwt::AccLut *lut;
+  const gwt::ff *wf[kMaxDet];
   unsigned *item_counter, *src_done;
   double *partials;  // items * kMaxDet * kSums
   double *fisher, *cov;
@@ -202,6 +236,148 @@ __global__ void __launch_bounds__(kBlock, 3) k_fisher_main(const FisherArgs a) {
       a.status[src] = st;
     }
     __syncthreads();
+  }
+}
+
+// Sums 0..31 of v over the warp, in two floats: lane l is left with sum l.
+__device__ __forceinline__ ff warp_sums(ff (&v)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int j = 0; j < o; j++) {
+      const bool up = lane & o;
+      const ff keep = up ? v[j + o] : v[j], send = up ? v[j] : v[j + o];
+      v[j] = ff_norm(ff_add(keep, ff{__shfl_xor_sync(0xffffffffu, send.h, o), __shfl_xor_sync(0xffffffffu, send.l, o)}));
+    }
+  return v[0];
+}
+// A pair's difference in FP64 (bins that ff_pair_q leaves).
+__device__ __noinline__ double2 pair_fp64(const FisherSrc *F, int q, int n, double t, double r, double lnn, double t34,
+                                          double m76) {
+  double2 v;
+  fisher_pair_q<double>(*F, q, n, t, r, lnn, t34, m76, 0.f, wave64_amp(F->w0, n, t, m76), v.x, v.y);
+  return v;
+}
+
+// The moment sums of the calls that take no inverse, in two floats.  An item is
+// a tile of one source under one weight stream; a thread's sums run over
+// kFfTile / kBlock terms, short enough for a two-float sum, the rest of the way
+// up goes through one transposed warp sum and FP64.
+// FP64 bins occupy the FP64 pipe for 64 cycles an instruction; here a bin is
+// ~1,900 FP32 instructions (the differences of four pairs ~1,100, products and
+// sums ~500), bound by their issue: 256 sources on 32,128 bins 5740 -> 745 us.
+// Where the inverse is wanted too the sums stay FP64: it magnifies them by the
+// matrix's condition number.
+constexpr int kFfTile = 2048;
+__global__ void __launch_bounds__(kBlock, 3) k_fisher_ff(const __grid_constant__ FisherArgs a) {
+  __shared__ int s_item, s_last;
+  __shared__ FfSrc S;
+  __shared__ gwt::AccLut lut;
+  __shared__ double s_red[kBlock / 32][32];
+  __shared__ double s_sum[kMaxDet * kSums];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  {
+    const unsigned *p = (const unsigned *)a.lut;
+    for (int w = tid; w < (int)(sizeof(gwt::AccLut) / 4); w += kBlock) ((unsigned *)&lut)[w] = p[w];
+  }
+  const int per = a.ntiles * a.nw, nitems = a.nsrc * per;
+  for (;;) {
+    if (tid == 0) s_item = (int)atomicAdd(a.item_counter, 1u);
+    __syncthreads();
+    const int it = s_item;
+    if (it >= nitems) break;
+    const int src = it / per, w = it % per / a.ntiles, tile = it % a.ntiles;
+    const FisherSrc &F = a.src[src];
+    const int k0 = tile * kFfTile;
+    int k1 = min(k0 + kFfTile, a.N);
+    const bool in_tables = a.n0 >= 1 && a.n0 + k1 - 1 <= a.tab.nmax && a.n0 + k1 - 1 <= a.tm76d_n &&
+                           a.n0 + k1 - 1 <= a.acc.nmax;
+    if (!in_tables && tid == 0) atomicOr(a.status + src, kStatusBounds);
+    const bool run = F.status == 0 && !F.needs_ref && in_tables && a.ff[src].ok;
+    k1 = run ? min(k1, F.n_cut_any - a.n0 + 1) : k0;
+    double *part = a.partials + ((size_t)(src * a.ntiles + tile) * kMaxDet + w) * kSums;
+    if (k0 < k1) {
+      const unsigned *p = (const unsigned *)(a.ff + src);
+      for (int j = tid; j < (int)(sizeof(FfSrc) / 4); j += kBlock) ((unsigned *)&S)[j] = p[j];
+      __syncthreads();
+      ff acc[32];
+#pragma unroll
+      for (int j = 0; j < 32; j++) acc[j] = ff{0.f, 0.f};
+      for (int k = k0 + tid; k < k1; k += kBlock) {
+        const int n = a.n0 + k;
+        const FfBin b = ff_bin(a.acc, n);
+        const ff a0 = ff_amp0(S, n, b, lut);
+        ff qr[kIntr], qi[kIntr];
+        unsigned left = 0;
+#pragma unroll
+        for (int q = 0; q < kIntr; q++)
+          if (!ff_pair_q(S.q[q], S.n_mid, n, b, lut, a0, qr[q], qi[q])) left |= 1u << q;
+        while (left) {
+          const int q = __ffs(left) - 1;
+          left &= left - 1;
+          const double2 v = pair_fp64(&F, q, n, a.tab.t13[n], a.tab.tm53[n], a.tab.tln[n], a.tab.t34[n], a.tm76d[n]);
+#pragma unroll
+          for (int j = 0; j < kIntr; j++)
+            if (j == q) {
+              qr[j] = ff_split(v.x);
+              qi[j] = ff_split(v.y);
+            }
+        }
+        ff_accumulate(a.wf[w][k], a0, b.n, qr, qi, acc);
+      }
+      s_red[warp][lane] = ff_value(warp_sums(acc, lane));
+      __syncthreads();
+      if (tid < kSums) {
+        double s = 0;
+        for (int j = 0; j < kBlock / 32; j++) s += s_red[j][tid];
+        part[tid] = s;
+      }
+    } else if (tid < kSums) {
+      part[tid] = 0.0;
+    }
+    // the source's last tile adds the tiles in their order and assembles Gamma
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      s_last = atomicAdd(a.src_done + src, 1u) == (unsigned)per - 1;
+    }
+    __syncthreads();
+    if (!s_last) continue;
+    __threadfence();
+    bool fin = a.ff[src].ok;
+    for (int j = tid; j < a.nw * kSums; j += kBlock) {
+      const int i = j % kSums;
+      double s = 0;
+      for (int t = 0; t < a.ntiles; t++)
+        s += __ldcg(&a.partials[((size_t)(src * a.ntiles + t) * kMaxDet + j / kSums) * kSums + i]);
+      if (!isfinite(s)) fin = false;
+      if (i == 1 || (i >= 13 && ((i - 13) & 2))) s *= a.df;  // the bin number to its frequency
+      if (i == 2) s *= a.df * a.df;
+      s_sum[j] = s;
+    }
+    fin = __syncthreads_and(fin);
+    int st = F.status;
+    if (__ldcg(a.status + src) & kStatusBounds) st = 5;
+    if (tid < kDim * (kDim + 1) / 2) {
+      int i = 0, j = tid;
+      while (j > i) j -= ++i;
+      const double g = st ? __longlong_as_double(0x7ff8000000000000ll)
+                          : fisher_element(F, s_sum, a.ndet, a.wslot, a.wscale, a.fisher_df_ratio, i, j);
+      double *G = a.fisher + (size_t)src * kDim * kDim;
+      G[i * kDim + j] = G[j * kDim + i] = g;
+    }
+    __syncthreads();
+    if (tid == 0) a.status[src] = st ? st : (F.needs_ref ? kStatusRedo : (fin ? 0 : kStatusFp64));
+  }
+}
+
+template <bool ACC64>
+void launch_main(const FisherArgs &a, int nw, int grid, cudaStream_t s) {
+  switch (nw) {
+    case 1: k_fisher_main<1, ACC64><<<grid, kBlock, 0, s>>>(a); break;
+    case 2: k_fisher_main<2, ACC64><<<grid, kBlock, 0, s>>>(a); break;
+    case 3: k_fisher_main<3, ACC64><<<grid, kBlock, 0, s>>>(a); break;
+    default: k_fisher_main<4, ACC64><<<grid, kBlock, 0, s>>>(a); break;
   }
 }
 
@@ -420,13 +596,18 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   // the FP64 n^(-7/6) table
   int st = c->ensure_tm76d(s0->dev.n0 + s0->dev.N);
   if (st) return st;
-  const int N = s0->dev.N, tile = 4096, ntiles = (N + tile - 1) / tile;
+  // Two-float sums for the FP64 calls without an inverse, on streams that have
+  // their two-float weights.
+  bool two_float = acc64 && !covariance;
+  for (const auto *s : ws) two_float = two_float && s->dev.wf != nullptr;
+  const int N = s0->dev.N, tile = two_float ? kFfTile : 4096, ntiles = (N + tile - 1) / tile;
   const double df = s0->dev.df;
   // chunk sources to bound the scratch
   const int chunk = std::min(n, 2048);
   size_t bytes = sizeof(GenParams) * chunk + sizeof(SlotOut) * (size_t)chunk * kSlots + sizeof(FisherSrc) * chunk +
                  sizeof(double) * (size_t)chunk * ntiles * kMaxDet * kSums + sizeof(double) * (size_t)chunk * 2 * kDim * kDim +
-                 sizeof(int) * (chunk + 8) + sizeof(unsigned) * (chunk + 8) + 1024;
+                 sizeof(int) * (chunk + 8) + sizeof(unsigned) * (chunk + 8) + sizeof(FfSrc) * (two_float ? chunk : 0) +
+                 2048;
   void *dev;
   st = c->workspace(gwgpu_context::kWsFisher + 10, bytes, &dev);
   if (st) return st;
@@ -447,6 +628,8 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   int *dstat = (int *)p;
   p = align(p + sizeof(int) * (chunk + 8));
   unsigned *cnt = (unsigned *)p;
+  p = align(p + sizeof(unsigned) * (chunk + 8));
+  FfSrc *ffs = (FfSrc *)p;
   int *dwslot, *ddets;
   void *small;
   st = c->workspace(gwgpu_context::kWsFisher + 11, 256, &small);
@@ -464,7 +647,11 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
     a.ipsd[w] = ws[w]->dev.ipsd;
     a.iw[w] = ws[w]->dev.iw;
     a.c3[w] = 4. * ws[w]->dev.simpson_df / 3.;
+    a.wf[w] = ws[w]->dev.wf;
   }
+  a.ff = ffs;
+  a.acc = c->acc;
+  a.lut = c->acc_lut;
   a.n0 = s0->dev.n0;
   a.N = N;
   a.tile = tile;
@@ -475,23 +662,28 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   a.tab = c->tables;
   a.tm76d = c->tm76d;
   a.tm76d_n = c->tm76d_n;
-  static int grid_cache = 0;
+  static int grid_cache = 0, grid_ff = 0;
   if (!grid_cache) {
     cudaDeviceProp pr;
     cudaGetDeviceProperties(&pr, c->device);
     int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fisher_ff, kBlock, 0);
+    grid_ff = pr.multiProcessorCount * std::max(per, 1);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fisher_main<1, false>, kBlock, 0);
     grid_cache = pr.multiProcessorCount * std::max(per, 1);
   }
   for (int s0i = 0; s0i < n; s0i += chunk) {
     int m = std::min(chunk, n - s0i);
     cudaMemcpyAsync(dparams, params + s0i, sizeof(GenParams) * m, cudaMemcpyHostToDevice, c->stream);
-    cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (m + 8), c->stream);
     int tot = m * kSlots;
     k_fisher_slots<<<(tot + 63) / 64, 64, 0, c->stream>>>(dparams, m, method, ddets, ndet, df, epsilon, step_mode,
                                                           c->qnm_dev, slots);
-    k_fisher_setup<<<(m + 63) / 64, 64, 0, c->stream>>>(dparams, m, method, ndet, epsilon, step_mode, order, slots,
-                                                        srcs, dstat);
+    if (two_float)
+      k_fisher_setup<true><<<m, 32, 0, c->stream>>>(dparams, method, ndet, epsilon, step_mode, order, slots, srcs, ffs,
+                                                    dstat);
+    else
+      k_fisher_setup<false><<<m, 32, 0, c->stream>>>(dparams, method, ndet, epsilon, step_mode, order, slots, srcs,
+                                                     nullptr, dstat);
     a.src = srcs;
     a.nsrc = m;
     a.item_counter = cnt + m;
@@ -500,34 +692,28 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
     a.fisher = dfish;
     a.cov = covariance ? dcov : nullptr;
     a.status = dstat;
-    int grid = std::min(m * ntiles, grid_cache);
-    switch (nw) {
-      case 1:
-        if (acc64) k_fisher_main<1, true><<<grid, kBlock, 0, c->stream>>>(a);
-        else k_fisher_main<1, false><<<grid, kBlock, 0, c->stream>>>(a);
-        break;
-      case 2:
-        if (acc64) k_fisher_main<2, true><<<grid, kBlock, 0, c->stream>>>(a);
-        else k_fisher_main<2, false><<<grid, kBlock, 0, c->stream>>>(a);
-        break;
-      case 3:
-        if (acc64) k_fisher_main<3, true><<<grid, kBlock, 0, c->stream>>>(a);
-        else k_fisher_main<3, false><<<grid, kBlock, 0, c->stream>>>(a);
-        break;
-      default:
-        if (acc64) k_fisher_main<4, true><<<grid, kBlock, 0, c->stream>>>(a);
-        else k_fisher_main<4, false><<<grid, kBlock, 0, c->stream>>>(a);
-        break;
+    std::vector<int> hs(m);
+    cudaError_t e = cudaSuccess;
+    for (bool again = two_float;; again = false) {
+      cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (m + 8), c->stream);
+      int grid = std::min(m * ntiles * (again ? nw : 1), again ? grid_ff : grid_cache);
+      if (again) k_fisher_ff<<<grid, kBlock, 0, c->stream>>>(a);
+      else if (acc64) launch_main<true>(a, nw, grid, c->stream);
+      else launch_main<false>(a, nw, grid, c->stream);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return c->fail(e, "fisher batch launch");
+      cudaMemcpyAsync(hs.data(), dstat, sizeof(int) * m, cudaMemcpyDeviceToHost, c->stream);
+      cudaMemcpyAsync(fisher + (size_t)s0i * kDim * kDim, dfish, sizeof(double) * m * kDim * kDim,
+                      cudaMemcpyDeviceToHost, c->stream);
+      if (!again) break;
+      e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess) return c->fail(e, "fisher batch");
+      // a source beyond what two floats hold: the chunk again with FP64 sums
+      if (std::find(hs.begin(), hs.end(), kStatusFp64) == hs.end()) break;
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return c->fail(e, "fisher batch launch");
-    cudaMemcpyAsync(fisher + (size_t)s0i * kDim * kDim, dfish, sizeof(double) * m * kDim * kDim,
-                    cudaMemcpyDeviceToHost, c->stream);
     if (covariance)
       cudaMemcpyAsync(covariance + (size_t)s0i * kDim * kDim, dcov, sizeof(double) * m * kDim * kDim,
                       cudaMemcpyDeviceToHost, c->stream);
-    std::vector<int> hs(m);
-    cudaMemcpyAsync(hs.data(), dstat, sizeof(int) * m, cudaMemcpyDeviceToHost, c->stream);
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return c->fail(e, "fisher batch");
     // Sources whose matrix the sums leave indefinite (a normalised smallest

@@ -29,6 +29,7 @@ struct SlotOut {
 struct WaveDiff {
   double qi[12], bi0, bi1, pA, pB, pC, pD, mA, mB, mC, mD, phic;
   double ai[10], ei[5];
+  double yw, yc;  // the ringdown atan's argument: y+ - y- = (yw n + yc) divisor
 };
 
 struct FisherSrc {
@@ -162,6 +163,8 @@ GW_HD void wave_diff(const WaveF64 &p, const WaveF64 &m, double sp, double sm, i
   d.mC = (p.mC - m.mC) * inv;
   d.mD = (p.mD - m.mD) * inv;
   d.phic = (p.phic - m.phic) * inv;
+  d.yw = (p.inv_nw - m.inv_nw) * inv;
+  d.yc = -p.nc * d.yw - (p.nc - m.nc) * inv * m.inv_nw;
   for (int j = 0; j < 10; j++) d.ai[j] = (p.ai[j] * sp - m.ai[j] * sm) * inv;
   double ep[5], em[5];
   recentre_ei(p, H, ep);
@@ -169,8 +172,11 @@ GW_HD void wave_diff(const WaveF64 &p, const WaveF64 &m, double sp, double sm, i
   for (int j = 0; j < 5; j++) d.ei[j] = (ep[j] * sp - em[j] * sm) * inv;
 }
 
-GW_HDNI int fisher_setup(const GenParams &in, int method, int ndet, double epsilon, int step_mode, int order,
-                         const SlotOut *S, FisherSrc &F) {
+// The set-up in parts that separate threads can take: the parameters and
+// divisors, a waveform pair, an extrinsic parameter of a detector, a detector's
+// own projection, and what the source is left to.
+GW_HD void fisher_setup_head(const GenParams &in, int method, double epsilon, int step_mode, const SlotOut *S,
+                             FisherSrc &F) {
   fisher_unpack(in, method, F.v, F.logf);
   int st = 0;
   for (int s = 0; s < kSlots; s++) st |= S[s].status;
@@ -188,93 +194,97 @@ GW_HDNI int fisher_setup(const GenParams &in, int method, int ndet, double epsil
     // difference is taken waveform by waveform.
     F.exact[q] = q == 1 && (0.25 - F.v[8]) < 1000.0 * F.div[8];
   }
+  F.status = st;
   F.w0 = S[0].w;
   F.n_cut_any = F.w0.n_cut;
   for (int s = 1; s < kSlots; s++) F.n_cut_any = F.n_cut_any > S[s].w.n_cut ? F.n_cut_any : S[s].w.n_cut;
+}
+GW_HD void fisher_setup_pair(const SlotOut *S, int k, FisherSrc &F) {
   const double A0 = S[0].w.A_scale;
-  for (int k = 0; k < kIntr; k++) {
-    int i = 7 + k;
-    F.wp[k] = S[1 + 2 * i].w;
-    F.wm[k] = S[2 + 2 * i].w;
-    F.sp[k] = F.wp[k].A_scale / A0;
-    F.sm[k] = F.wm[k].A_scale / A0;
-    F.amp_lk[k] = log((F.wp[k].mrK * F.sp[k]) / (F.wm[k].mrK * F.sm[k]));
-    wave_diff(F.wp[k], F.wm[k], F.sp[k], F.sm[k], F.w0.n_mid, F.idiv[k], F.wd[k]);
+  int i = 7 + k;
+  F.wp[k] = S[1 + 2 * i].w;
+  F.wm[k] = S[2 + 2 * i].w;
+  F.sp[k] = F.wp[k].A_scale / A0;
+  F.sm[k] = F.wm[k].A_scale / A0;
+  F.amp_lk[k] = log((F.wp[k].mrK * F.sp[k]) / (F.wm[k].mrK * F.sm[k]));
+  wave_diff(F.wp[k], F.wm[k], F.sp[k], F.sm[k], F.w0.n_mid, F.idiv[k], F.wd[k]);
+}
+GW_HD void fisher_setup_row(const SlotOut *S, int order, int d, int i, FisherSrc &F) {
+  const double A0 = S[0].w.A_scale, g0r = S[0].Gre[d], g0i = S[0].Gim[d];
+  const SlotOut &P = S[1 + 2 * i], &Mn = S[2 + 2 * i];
+  double dv = F.div[i];
+  double ar = 0, ai = 0, br = 0, bi = 0;
+  if (i <= 3) {  // RA, DEC, psi, iota: dG + i G f dtau
+    ar = (P.Gre[d] - Mn.Gre[d]) / dv;
+    ai = (P.Gim[d] - Mn.Gim[d]) / dv;
+    double dt = (P.tau[d] - Mn.tau[d]) / dv;
+    br = -g0i * dt;  // i G dtau
+    bi = g0r * dt;
+  } else if (i == 4) {  // phiRef: i G dphic
+    double dph = (P.w.phic - Mn.w.phic) / dv;
+    ar = -g0i * dph;
+    ai = g0r * dph;
+  } else if (i == 5) {  // tc: i G dtcl (f - fref)
+    double dt = (P.w.tcl - Mn.w.tcl) / dv;
+    double fr = S[0].w.fref;
+    br = -g0i * dt;
+    bi = g0r * dt;
+    ar = g0i * dt * fr;
+    ai = -g0r * dt * fr;
+  } else {  // D_L: G dA/A
+    double rel = (P.w.A_scale - Mn.w.A_scale) / (dv * A0);
+    ar = g0r * rel;
+    ai = g0i * rel;
   }
-  for (int d = 0; d < ndet; d++) {
-    double g0r = S[0].Gre[d], g0i = S[0].Gim[d];
-    F.G0re[d] = g0r;
-    F.G0im[d] = g0i;
-    for (int i = 0; i < kCheap; i++) {
-      const SlotOut &P = S[1 + 2 * i], &Mn = S[2 + 2 * i];
-      double dv = F.div[i];
-      double ar = 0, ai = 0, br = 0, bi = 0;
-      if (i <= 3) {  // RA, DEC, psi, iota: dG + i G f dtau
-        ar = (P.Gre[d] - Mn.Gre[d]) / dv;
-        ai = (P.Gim[d] - Mn.Gim[d]) / dv;
-        double dt = (P.tau[d] - Mn.tau[d]) / dv;
-        br = -g0i * dt;  // i G dtau
-        bi = g0r * dt;
-      } else if (i == 4) {  // phiRef: i G dphic
-        double dph = (P.w.phic - Mn.w.phic) / dv;
-        ar = -g0i * dph;
-        ai = g0r * dph;
-      } else if (i == 5) {  // tc: i G dtcl (f - fref)
-        double dt = (P.w.tcl - Mn.w.tcl) / dv;
-        double fr = S[0].w.fref;
-        br = -g0i * dt;
-        bi = g0r * dt;
-        ar = g0i * dt * fr;
-        ai = -g0r * dt * fr;
-      } else {  // D_L: G dA/A
-        double rel = (P.w.A_scale - Mn.w.A_scale) / (dv * A0);
-        ar = g0r * rel;
-        ai = g0i * rel;
-      }
-      if (F.logf[i]) {
-        ar *= F.v[i];
-        ai *= F.v[i];
-        br *= F.v[i];
-        bi *= F.v[i];
-      }
-      if (order == 4) {
-        // Five-point rule (fisher.cpp:426-458): the reference shifts t_c by
-        // the detector's arrival time at the +-2 eps steps instead of
-        // rotating by e^{-2 pi i DTOA f}, so those two responses carry the
-        // extra constant phase phq = -tau f_ref.  To second order in the step
-        // the five-point difference is then kappa r' + c r with
-        // kappa = (4 - e^{i phq}) / 3 and c = -(i/3) e^{i phq} d(phq)/d(theta)
-        // = (i/3) e^{i phq} f_ref dtau (the sky position only); kappa = 1 and
-        // c = 0 at the reference detector (tau = 0).  Here a' = kappa a + c G0
-        // and b' = kappa b; the intrinsic rows take kappa G0 below.
-        const double phq = -S[0].tau[d] * S[0].w.fref;
-        double sq, cq;
-        sincos(phq, &sq, &cq);
-        const double kr = (4.0 - cq) / 3.0, ki = -sq / 3.0;
-        double dt = i <= 3 ? (P.tau[d] - Mn.tau[d]) / dv : 0.0;
-        if (F.logf[i]) dt *= F.v[i];
-        const double cr = -sq * S[0].w.fref * dt / 3.0, ci = cq * S[0].w.fref * dt / 3.0;
-        const double ar2 = kr * ar - ki * ai + (cr * g0r - ci * g0i), ai2 = kr * ai + ki * ar + (cr * g0i + ci * g0r);
-        const double br2 = kr * br - ki * bi, bi2 = kr * bi + ki * br;
-        ar = ar2;
-        ai = ai2;
-        br = br2;
-        bi = bi2;
-      }
-      F.ar[d][i] = ar;
-      F.ai[d][i] = ai;
-      F.br[d][i] = br;
-      F.bi[d][i] = bi;
-    }
-    if (order == 4) {  // the intrinsic derivatives: kappa G0 q
-      const double phq = -S[0].tau[d] * S[0].w.fref;
-      double sq, cq;
-      sincos(phq, &sq, &cq);
-      const double kr = (4.0 - cq) / 3.0, ki = -sq / 3.0;
-      F.G0re[d] = kr * g0r - ki * g0i;
-      F.G0im[d] = kr * g0i + ki * g0r;
-    }
+  if (F.logf[i]) {
+    ar *= F.v[i];
+    ai *= F.v[i];
+    br *= F.v[i];
+    bi *= F.v[i];
   }
+  if (order == 4) {
+    // Five-point rule (fisher.cpp:426-458): the reference shifts t_c by
+    // the detector's arrival time at the +-2 eps steps instead of
+    // rotating by e^{-2 pi i DTOA f}, so those two responses carry the
+    // extra constant phase phq = -tau f_ref.  To second order in the step
+    // the five-point difference is then kappa r' + c r with
+    // kappa = (4 - e^{i phq}) / 3 and c = -(i/3) e^{i phq} d(phq)/d(theta)
+    // = (i/3) e^{i phq} f_ref dtau (the sky position only); kappa = 1 and
+    // c = 0 at the reference detector (tau = 0).  Here a' = kappa a + c G0
+    // and b' = kappa b; the intrinsic rows take kappa G0 below.
+    const double phq = -S[0].tau[d] * S[0].w.fref;
+    double sq, cq;
+    sincos(phq, &sq, &cq);
+    const double kr = (4.0 - cq) / 3.0, ki = -sq / 3.0;
+    double dt = i <= 3 ? (P.tau[d] - Mn.tau[d]) / dv : 0.0;
+    if (F.logf[i]) dt *= F.v[i];
+    const double cr = -sq * S[0].w.fref * dt / 3.0, ci = cq * S[0].w.fref * dt / 3.0;
+    const double ar2 = kr * ar - ki * ai + (cr * g0r - ci * g0i), ai2 = kr * ai + ki * ar + (cr * g0i + ci * g0r);
+    const double br2 = kr * br - ki * bi, bi2 = kr * bi + ki * br;
+    ar = ar2;
+    ai = ai2;
+    br = br2;
+    bi = bi2;
+  }
+  F.ar[d][i] = ar;
+  F.ai[d][i] = ai;
+  F.br[d][i] = br;
+  F.bi[d][i] = bi;
+}
+GW_HD void fisher_setup_det(const SlotOut *S, int order, int d, FisherSrc &F) {
+  const double g0r = S[0].Gre[d], g0i = S[0].Gim[d];
+  F.G0re[d] = g0r;
+  F.G0im[d] = g0i;
+  if (order == 4) {  // the intrinsic derivatives: kappa G0 q
+    const double phq = -S[0].tau[d] * S[0].w.fref;
+    double sq, cq;
+    sincos(phq, &sq, &cq);
+    const double kr = (4.0 - cq) / 3.0, ki = -sq / 3.0;
+    F.G0re[d] = kr * g0r - ki * g0i;
+    F.G0im[d] = kr * g0i + ki * g0r;
+  }
+}
+GW_HD void fisher_setup_route(int order, FisherSrc &F) {
   // The five-point rule's +-2 eps waveforms are not among the slots: a pair
   // that the moment form takes bin by bin (eta at 1/4, a waveform's cut inside
   // the pair) is left to the reference algorithm.
@@ -283,8 +293,17 @@ GW_HDNI int fisher_setup(const GenParams &in, int method, int ndet, double epsil
     for (int q = 0; q < kIntr; q++)
       if (F.onesided[q] || F.exact[q] || F.wp[q].n_cut != F.w0.n_cut || F.wm[q].n_cut != F.w0.n_cut) F.needs_ref = 1;
   }
-  F.status = st;
-  return st;
+}
+GW_HDNI int fisher_setup(const GenParams &in, int method, int ndet, double epsilon, int step_mode, int order,
+                         const SlotOut *S, FisherSrc &F) {
+  fisher_setup_head(in, method, epsilon, step_mode, S, F);
+  for (int k = 0; k < kIntr; k++) fisher_setup_pair(S, k, F);
+  for (int d = 0; d < ndet; d++) {
+    for (int i = 0; i < kCheap; i++) fisher_setup_row(S, order, d, i, F);
+    fisher_setup_det(S, order, d, F);
+  }
+  fisher_setup_route(order, F);
+  return F.status;
 }
 
 
@@ -330,7 +349,9 @@ GW_HD double fisher_phase_deriv(const FisherSrc &F, int q, int n, double t, doub
     if (n >= p.n_f2p && n >= m.n_f2p) {  // ringdown: the atan pair as in wave64_phase_diff
       const double nd = (double)n;
       const double yp = (nd - p.nc) * p.inv_nw, ym = (nd - m.nc) * m.inv_nw;
-      const double z = (yp - ym) / (1.0 + yp * ym);
+      // y+ - y- from the coefficients' differences: their own difference keeps
+      // only 1e-16 / step of it
+      const double z = (d.yw * nd + d.yc) * F.div[7 + q] / (1.0 + yp * ym);
       if (fabs(z) < 1e-3) {
         const double z2 = z * z;
         const double datan = z * (1.0 - z2 * ((1.0 / 3.0) - z2 * 0.2));  // atan z to z^5
@@ -366,38 +387,42 @@ GW_HD void fisher_q_exact(const FisherSrc &F, int q, int n, double t, double r, 
   qi = (T)(im * F.idiv[q]);
 }
 
-// One bin: the intrinsic differences q = (r+ - r-) e^{i Phi0} / (G divisor) of
-// the four waveform pairs, for the moment sums.  With h half the phase step
+// The difference of pair q at bin n: q = (r+ - r-) e^{i Phi0} / (G divisor).
+// With h half the phase step
 // (Phi+ - Phi-) / 2 and the mean phase offset of the pair second order in the
 // step, a central pair is exactly (A+ - A-) cos h - i (A+ + A-) sin h; cos h and
 // sin h / h by their series (h stays below 1e-2 for the steps used).  A
 // one-sided pair (eta at 1/4, + the centre) is A0 - A- e^{2ih}.
+template <typename T>
+GW_HD void fisher_pair_q(const FisherSrc &F, int q, int n, double t, double r, double lnn, double t34, double m76,
+                         float m76f, double amp0, T &qr, T &qi) {
+  if (F.exact[q] || amp0 == 0.0 || n > F.wp[q].n_cut || n > F.wm[q].n_cut) {
+    fisher_q_exact(F, q, n, t, r, lnn, t34, m76, qr, qi);
+    return;
+  }
+  const T damp = fisher_amp_deriv<T>(F, q, n, t, m76, m76f);      // (A+ - A-) / divisor
+  const double dph = fisher_phase_deriv(F, q, n, t, r, lnn, t34);  // (Phi+ - Phi-) / divisor
+  const double h = 0.5 * dph * F.div[7 + q];
+  const double h2 = h * h;
+  if (!F.onesided[q]) {
+    qr = damp * (T)(1.0 - h2 * (0.5 - h2 * (1.0 / 24.0)));
+    qi = (T)(-amp0 * dph * (1.0 - h2 * ((1.0 / 6.0) - h2 * (1.0 / 120.0))));
+  } else {
+    const double am = amp0 - (double)damp * F.div[7 + q];
+    double s2, c2;
+    sincos(2.0 * h, &s2, &c2);
+    qr = (T)((amp0 - am * c2) * F.idiv[q]);
+    qi = (T)(-am * s2 * F.idiv[q]);
+  }
+}
+// One bin: the centre's amplitude and the four pairs, for the moment sums.
 template <typename T>
 GW_HD bool fisher_bin_q(const FisherSrc &F, int n, double t, double r, double lnn, double t34, double m76,
                         float m76f, T &a0, T *qr, T *qi) {
   if (n > F.n_cut_any) return false;
   const double amp0 = wave64_amp(F.w0, n, t, m76);
   a0 = (T)amp0;
-  for (int q = 0; q < kIntr; q++) {
-    if (F.exact[q] || amp0 == 0.0 || n > F.wp[q].n_cut || n > F.wm[q].n_cut) {
-      fisher_q_exact(F, q, n, t, r, lnn, t34, m76, qr[q], qi[q]);
-      continue;
-    }
-    const T damp = fisher_amp_deriv<T>(F, q, n, t, m76, m76f);      // (A+ - A-) / divisor
-    const double dph = fisher_phase_deriv(F, q, n, t, r, lnn, t34);  // (Phi+ - Phi-) / divisor
-    const double h = 0.5 * dph * F.div[7 + q];
-    const double h2 = h * h;
-    if (!F.onesided[q]) {
-      qr[q] = damp * (T)(1.0 - h2 * (0.5 - h2 * (1.0 / 24.0)));
-      qi[q] = (T)(-amp0 * dph * (1.0 - h2 * ((1.0 / 6.0) - h2 * (1.0 / 120.0))));
-    } else {
-      const double am = amp0 - (double)damp * F.div[7 + q];
-      double s2, c2;
-      sincos(2.0 * h, &s2, &c2);
-      qr[q] = (T)((amp0 - am * c2) * F.idiv[q]);
-      qi[q] = (T)(-am * s2 * F.idiv[q]);
-    }
-  }
+  for (int q = 0; q < kIntr; q++) fisher_pair_q(F, q, n, t, r, lnn, t34, m76, m76f, amp0, qr[q], qi[q]);
   return true;
 }
 GW_HD void fisher_accumulate(float wh, float a0, float fk, const float *qr, const float *qi, KSum *A) {
@@ -433,60 +458,51 @@ GW_HD void fisher_accumulate64(double wh, double a0, double fk, const double *qr
     A[13 + 4 * i + 3] += wa * qi[i] * fk;
   }
 }
-// FP64 assembly of Gamma from the moment sums Ssum[w * kSums + j] of each
-// weight stream; wscale[w] * ratio restores the whitening scale and the
+// Element (i >= j) of Gamma from the moment sums Ssum[w * kSums + j] of each
+// weight stream, in FP64; wscale[w] * ratio restores the whitening scale and the
 // Simpson step of calculate_fisher_elements (fisher.cpp:2704-2781).
-GW_HDNI void fisher_assemble(const FisherSrc &F, const double *Ssum, int ndet, const int *wslot, const double *wscale,
-                         double ratio, double *Gm) {
-  for (int j = 0; j < kDim * kDim; j++) Gm[j] = 0;
+GW_HD double fisher_element(const FisherSrc &F, const double *Ssum, int ndet, const int *wslot, const double *wscale,
+                            double ratio, int i, int j) {
   const double A0 = F.w0.A_scale;
+  double g = 0;
   for (int d = 0; d < ndet; d++) {
     const int w = wslot[d];
     const double *Sv = Ssum + w * kSums;
     const double c = A0 * A0 * wscale[w] * ratio;
-    const double M0 = Sv[0], M1 = Sv[1], M2 = Sv[2];
-    const double gr = F.G0re[d], gi = F.G0im[d], g2 = gr * gr + gi * gi;
-    // cheap x cheap
-    for (int i = 0; i < kCheap; i++)
-      for (int j = 0; j <= i; j++) {
-        double aiR = F.ar[d][i], aiI = F.ai[d][i], biR = F.br[d][i], biI = F.bi[d][i];
-        double ajR = F.ar[d][j], ajI = F.ai[d][j], bjR = F.br[d][j], bjI = F.bi[d][j];
-        double t0 = aiR * ajR + aiI * ajI;                            // Re(a_i a_j*)
-        double t1 = (aiR * bjR + aiI * bjI) + (biR * ajR + biI * ajI);  // Re(a_i b_j* + b_i a_j*)
-        double t2 = biR * bjR + biI * bjI;
-        Gm[i * kDim + j] += c * (t0 * M0 + t1 * M1 + t2 * M2);
-      }
-    // intrinsic x intrinsic
-    int o = 3;
-    for (int ii = 0; ii < kIntr; ii++)
-      for (int jj = ii; jj < kIntr; jj++) {
-        double val = c * g2 * Sv[o++];
-        int I = 7 + jj, J = 7 + ii;  // I >= J
-        Gm[I * kDim + J] += val;
-      }
-    // intrinsic x cheap: Re[G conj(a_j) S_i + G conj(b_j) T_i]
-    for (int ii = 0; ii < kIntr; ii++) {
-      double Sr = Sv[13 + 4 * ii], Si = Sv[14 + 4 * ii], Tr = Sv[15 + 4 * ii], Ti = Sv[16 + 4 * ii];
-      for (int j = 0; j < kCheap; j++) {
-        double ajR = F.ar[d][j], ajI = F.ai[d][j], bjR = F.br[d][j], bjI = F.bi[d][j];
-        // G conj(a_j) = (gr + i gi)(ajR - i ajI)
-        double car = gr * ajR + gi * ajI, cai = gi * ajR - gr * ajI;
-        double cbr = gr * bjR + gi * bjI, cbi = gi * bjR - gr * bjI;
-        double val = (car * Sr - cai * Si) + (cbr * Tr - cbi * Ti);
-        Gm[(7 + ii) * kDim + j] += c * val;
-      }
+    const double gr = F.G0re[d], gi = F.G0im[d];
+    const double ajR = F.ar[d][j % kCheap], ajI = F.ai[d][j % kCheap];  // read where j < kCheap
+    const double bjR = F.br[d][j % kCheap], bjI = F.bi[d][j % kCheap];
+    if (i < kCheap) {  // cheap x cheap
+      const double aiR = F.ar[d][i], aiI = F.ai[d][i], biR = F.br[d][i], biI = F.bi[d][i];
+      const double t0 = aiR * ajR + aiI * ajI;                            // Re(a_i a_j*)
+      const double t1 = (aiR * bjR + aiI * bjI) + (biR * ajR + biI * ajI);  // Re(a_i b_j* + b_i a_j*)
+      const double t2 = biR * bjR + biI * bjI;
+      g += c * (t0 * Sv[0] + t1 * Sv[1] + t2 * Sv[2]);
+    } else if (j < kCheap) {  // intrinsic x cheap: Re[G conj(a_j) S_i + G conj(b_j) T_i]
+      const double *X = Sv + 13 + 4 * (i - kCheap);
+      // G conj(a_j) = (gr + i gi)(ajR - i ajI)
+      const double car = gr * ajR + gi * ajI, cai = gi * ajR - gr * ajI;
+      const double cbr = gr * bjR + gi * bjI, cbi = gi * bjR - gr * bjI;
+      const double val = (car * X[0] - cai * X[1]) + (cbr * X[2] - cbi * X[3]);
+      g += c * val;
+    } else {  // intrinsic x intrinsic: Q is stored by rows of its upper triangle
+      const int ii = j - kCheap, jj = i - kCheap, o = 3 + ii * kIntr - ii * (ii - 1) / 2 + (jj - ii);
+      const double g2 = gr * gr + gi * gi;
+      const double val = c * g2 * Sv[o];
+      g += val;
     }
   }
-  // log factor of M_c (parameter 7) on the intrinsic block
-  if (F.logf[7]) {
-    for (int j = 0; j < kDim; j++) {
-      if (j == 7) Gm[7 * kDim + 7] *= F.v[7] * F.v[7];
-      else if (j < 7) Gm[7 * kDim + j] *= F.v[7];
-      else Gm[j * kDim + 7] *= F.v[7];
-    }
+  if (F.logf[7]) {  // log factor of M_c (parameter 7) on the intrinsic block
+    if (i == 7 && j == 7) g *= F.v[7] * F.v[7];
+    else if (i == 7 || j == 7) g *= F.v[7];
   }
+  return g;
+}
+GW_HDNI void fisher_assemble(const FisherSrc &F, const double *Ssum, int ndet, const int *wslot, const double *wscale,
+                             double ratio, double *Gm) {
   for (int i = 0; i < kDim; i++)
-    for (int j = 0; j < i; j++) Gm[j * kDim + i] = Gm[i * kDim + j];
+    for (int j = 0; j <= i; j++)
+      Gm[i * kDim + j] = Gm[j * kDim + i] = fisher_element(F, Ssum, ndet, wslot, wscale, ratio, i, j);
 }
 
 }  // namespace gwf

@@ -184,8 +184,11 @@ __global__ void __launch_bounds__(kRefBlock) k_fref_main(const RefArgs a) {
 
 // MCMC_fisher_transformations (mcmc_gw.cpp:2136-2160), non-intrinsic
 // IMRPhenomD: the prior widths added to the diagonal.
-__constant__ double c_prior_diag[kDim] = {1. / (4 * kPi * kPi), 1. / 4, 1. / (4 * kPi * kPi), 1. / 4,
-                                          1. / (4 * kPi * kPi), 1. / (.01), 0., 0., 1. / .25, 1. / 4, 1. / 4};
+GW_HD double prior_diag(int i) {
+  const double w[kDim] = {1. / (4 * kPi * kPi), 1. / 4, 1. / (4 * kPi * kPi), 1. / 4, 1. / (4 * kPi * kPi), 1. / (.01),
+                          0., 0., 1. / .25, 1. / 4, 1. / 4};
+  return w[i];
+}
 
 __global__ void k_fref_finish(int nsrc, const RefSrc *__restrict__ rs, int add_prior, double *fisher, double *cov,
                               int *status) {
@@ -194,7 +197,7 @@ __global__ void k_fref_finish(int nsrc, const RefSrc *__restrict__ rs, int add_p
   double *F = fisher + (size_t)src * kDim * kDim;
   int st = rs[src].status;
   if (add_prior)
-    for (int i = 0; i < kDim; i++) F[i * kDim + i] += c_prior_diag[i];
+    for (int i = 0; i < kDim; i++) F[i * kDim + i] += prior_diag(i);
   if (st) {
     for (int j = 0; j < kDim * kDim; j++) F[j] = NAN;
   }
@@ -342,11 +345,9 @@ int gwgpu_fisher_batch_ex(gwgpu_context *c, const gwgpu_gen_params *params, int 
     int st = gwf_moment_run(c, params, n, opt->method, opt->order, handles, ndet, opt->epsilon, opt->step_mode, fisher,
                             covariance, status, opt->precision == GWGPU_PREC_FP64);
     if (st || !opt->add_prior) return st;
-    double prior[kDim];
-    cudaMemcpyFromSymbol(prior, c_prior_diag, sizeof(prior));
     for (int i = 0; i < n; i++) {  // the prior diagonal, then the inverse again
       double *F = fisher + (size_t)i * kDim * kDim;
-      for (int k = 0; k < kDim; k++) F[k * kDim + k] += prior[k];
+      for (int k = 0; k < kDim; k++) F[k * kDim + k] += prior_diag(k);
       if (covariance) {
         double *C = covariance + (size_t)i * kDim * kDim;
         const bool bad = status && status[i] == GWGPU_EDOMAIN;
@@ -392,15 +393,8 @@ int gwgpu_mcmc_fisher_batch(gwgpu_context *c, const double *theta, int dim, int 
   int st = gwf_moment_run(c, (const gwgpu_gen_params *)hp.data(), n, GWGPU_FISHER_MCMC_IMRPHENOMD, 4, handles, ndet,
                           1e-8, GWGPU_FISHER_STEP_ABSOLUTE, fisher, nullptr, ks.data(), true);
   if (st) return st;
-  double prior[kDim];
-  {
-    std::lock_guard<std::mutex> lk(c->mu);
-    cudaSetDevice(c->device);
-    cudaError_t e = cudaMemcpyFromSymbol(prior, c_prior_diag, sizeof(prior));
-    if (e != cudaSuccess) return c->fail(e, "prior diagonal");
-  }
   for (int i = 0; i < n; i++)
-    for (int k = 0; k < kDim; k++) fisher[(size_t)i * kDim * kDim + k * kDim + k] += prior[k];
+    for (int k = 0; k < kDim; k++) fisher[(size_t)i * kDim * kDim + k * kDim + k] += prior_diag(k);
   if (status)
     for (int i = 0; i < n; i++) status[i] = ks[i];
   return GWGPU_OK;

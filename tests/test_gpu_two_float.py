@@ -142,3 +142,33 @@ def test_maximized(gpu_ctx, oracle, T, N, ndet, ap):
     finally:
         for h in hs:
             gpu_ctx.release_data(h)
+
+
+@pytest.mark.parametrize("T,N,ndet,same", [(8, 2, 1, True), (8, 127, 2, False), (1, 2047, 3, True), (1, 2049, 4, False),
+                                           (8, 8113, 3, True)])
+@pytest.mark.parametrize("order,eps,mode", [(2, 1e-6, 1), (4, 1e-8, 0), (2, 3e-4, 1)])
+def test_fisher_moments(gpu_ctx, T, N, ndet, same, order, eps, mode):
+    """The two-float moment sums against the FP64 ones on the same coefficients
+    (a call with a source that two floats cannot hold, a ringdown beyond 2^24
+    bins, takes FP64 sums): every region, boundary bins and cuts inside the grid,
+    equal masses, steps beyond the series.  A bin's phase difference is a sum of
+    at most 14 products with 2^-47 of the largest each, whose largest exceeds the
+    sum by less than 100: below 1e-11."""
+    f = (np.arange(N) + 10 * T) / T
+    psd = W.analytic_psd(f)
+    hs = [gpu_ctx.register_data(d, f, np.zeros(f.size, complex), psd if same else psd * (1 + 0.3 * i + f / 500.0))
+          for i, d in enumerate(DETS[:ndet])]
+    draws = W.prior_draws(9, 91)
+    draws += [dict(draws[0], mass1=30.0, mass2=30.0 * (1 - 1e-5)), dict(draws[1], mass1=20.0, mass2=20.0),
+              dict(draws[2], mass1=300.0, mass2=200.0), dict(draws[3], mass1=1.6, mass2=1.2)]
+    kw = dict(order=order, epsilon=eps, step_mode=mode, precision=G.PREC_FP64, algorithm=G.FISHER_MOMENTS,
+              covariance=False)
+    got, _, st = gpu_ctx.fisher_batch_ex(G.params_array(draws), 1, hs, **kw)
+    ref, _, sr = gpu_ctx.fisher_batch_ex(G.params_array(draws + [dict(draws[3], mass1=2e-6, mass2=1e-6)]), 1, hs, **kw)
+    assert np.array_equal(st, sr[:-1]) and np.all(st == 0)
+    assert N < 100 or np.any(got != ref[:-1])
+    for i, d in enumerate(draws):
+        s = np.sqrt(np.maximum(np.diag(ref[i]), 1e-300))
+        assert np.max(np.abs(got[i] - ref[i]) / np.outer(s, s)) <= 1e-11, (i, d)
+    for h in hs:
+        gpu_ctx.release_data(h)
