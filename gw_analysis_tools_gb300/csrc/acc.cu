@@ -70,12 +70,12 @@ __device__ __forceinline__ double acc_reduce(const AccReq &x, const ff *acc, dou
   for (int d = 0; d < NDET; d++)
 #pragma unroll
     for (int j = 0; j < NA; j++) {
-      const ff t = warp_sum_ff(acc[d * NA + j]);
-      if (lane == 0) v += x.m.fc[d * kAccPerDet + j] * ff_value(t);
+      const double t = ff_value(warp_sum_ff(acc[d * NA + j]));
+      if (lane == 0 && t != 0.0) v += x.m.fc[d * kAccPerDet + j] * t;  // an infinite factor: only with bins
     }
   if (lane == 0) s_red[warp] = v;
   __syncthreads();
-  double r = 0.0;
+  double r = x.bad;
   if (threadIdx.x == 0)
     for (int w = 0; w < nw; w++) r += s_red[w];
   return r;

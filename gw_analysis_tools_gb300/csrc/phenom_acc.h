@@ -57,6 +57,7 @@ struct AccReq {
   ff y2p, y1p, y0p, y2m, y1m;         // harmonics: sums and differences of Y_m and Y_-m
   ff c2z, s2z;                        // polarisation rotation
   float tc;                           // model's t_c, for bins off the line n df (acc_dev_turns)
+  float bad;                          // NaN when a linear phase is (turns cannot hold it), else 0; joins the result
   int fp64_phase;                     // 1: terms too large for two floats; every bin takes the FP64 series
 };
 
@@ -85,6 +86,7 @@ GW_HD void acc_det_phase(const Request &r, double df, AccReq &x, int d0 = 0, int
   const double c1 = pv2 ? r.p.t_corr * df : -m.tcs * df * inv2pi;
   const uint64_t q1 = acc_turns(c1) - acc_turns_prod(m.s.tc, df);
   x.tc = (float)m.s.tc;
+  x.bad = (float)(0.0 * (m.s.tc * m.fref + m.tcs * m.fref - m.phic + c1));
   x.B0 = q0;
   x.B1 = q1;
   for (int d = d0; d < r.ndet && d < kMaxDet; d += step) {
@@ -378,7 +380,8 @@ GW_HD void acc_wave(const AccReq &x, int n, uint64_t qd, const AccTables &tb, co
   if (n > x.m.n_cut) return;
   const ff4 p = acc_ld(tb.pw + n);
   const ff t{p.ch, p.cl};
-  const ff a = acc_amp(x, n, t, ff{p.sh, p.sl}, lut);
+  ff a = acc_amp(x, n, t, ff{p.sh, p.sl}, lut);
+  a.h += x.bad;
   uint64_t al;
   const uint64_t ph = qd + acc_phase<PV2>(x, n, tb, lut, t, al) + x.B0 + x.B1 * (uint64_t)n;
   ff c, s;

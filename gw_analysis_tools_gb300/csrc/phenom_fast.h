@@ -791,15 +791,18 @@ GW_HDNI void fast_det_factor(const Request &r, int d, double A, double w, double
   }
 }
 // Entry e of the factors, the weighted |h|^2 sums folded where the detectors
-// share their weights (mixed_fold_shared_weights).
+// share their weights (mixed_fold_shared_weights).  An infinite factor of the
+// Pv2 cross sum Re(h+ hx*), of either sign, gives way to those of |h+|^2 and
+// |hx|^2: log L goes to -inf with |h|^2.
 GW_HD double fast_factor_entry(const double (*f)[kAccPerDet], int e, int ndet, bool pv2, bool shared) {
   const int d = e / kAccPerDet, k = e - d * kAccPerDet;
   if (d >= ndet) return 0.0;
-  if (!shared || k >= (pv2 ? 3 : 1)) return f[d][k];
-  if (d) return 0.0;
-  double v = f[0][k];
-  for (int q = 1; q < ndet; q++) v += f[q][k];
-  return v;
+  double v = f[d][k];
+  if (shared && k < (pv2 ? 3 : 1)) {
+    if (d) return 0.0;
+    for (int q = 1; q < ndet; q++) v += f[q][k];
+  }
+  return pv2 && k == 2 && !(fabs(f[d][0]) < 1e300) && f[d][0] == f[d][0] ? 0.0 : v;
 }
 GW_HD bool fast_shared(const unsigned long long *wkey, int ndet) {
   bool same = ndet > 1;

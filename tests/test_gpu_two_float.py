@@ -77,6 +77,23 @@ def test_weighted_uniform_grid_and_bad_requests(gpu_ctx, oracle):
         gpu_ctx.release_data(h)
 
 
+@pytest.mark.parametrize("ap,key,val,want", [
+    (0, "tc", float("nan"), "nan"), (1, "tc", float("nan"), "nan"), (0, "tc", float("inf"), "nan"),
+    (0, "phiRef", float("nan"), "nan"), (0, "f_ref", float("nan"), "nan"), (0, "f_ref", 0.0, "nan"),
+    (1, "RA", float("nan"), "nan"), (0, "Luminosity_Distance", 1e-300, "-inf"), (1, "Luminosity_Distance", 1e-300, "-inf")])
+def test_non_finite_parameters(gpu_ctx, ap, key, val, want):
+    """A phase that is not a number reaches log L though angles are integers; an infinite
+    amplitude squared outweighs the finite cross term."""
+    f = 20.0 + np.arange(4000) / 8.0
+    psd = W.analytic_psd(f)
+    hs = [gpu_ctx.register_data(d, f, W.noise(f, 9 + i), psd) for i, d in enumerate(DETS[:2])]
+    x = dict(W.prior_draws(1, 8, precessing=bool(ap))[0], **{key: val})
+    out, st = gpu_ctx.loglik_batch(G.params_array([x]), ap, hs, 8.0, G.PREC_FP64)
+    assert np.array_equal(out, [float(want)], equal_nan=True) and st[0] == 0
+    for h in hs:
+        gpu_ctx.release_data(h)
+
+
 def test_infinite_psd_bins(gpu_ctx, oracle):
     """A PSD of infinity takes its bin out (finite pairs); a zero PSD, whose weight is infinite, keeps the FP64
     bins: both as the oracle."""
