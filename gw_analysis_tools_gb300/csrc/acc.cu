@@ -6,11 +6,13 @@
 // and amplitude 200; per SM and second that leaves DRAM and L2 idle (a
 // detector bin is 16 B of data and, once for shared weights, 8 B, from L2).
 // Against the FP64 bins they took the place of (FP64 pipe full): 512
-// IMRPhenomD requests on 3 x 32,128 bins 4,165 -> 333 us a call, 64
-// IMRPhenomPv2 requests on 2 x 32,448 bins 961 -> 174 us, the one-request call
-// on 3 x 32,128 bins 38.4 -> 23 us (Pv2, 3 x 16,224 bins: 48 -> 27 us), with
-// an error against 64-bit references of 1e-13 instead of 2e-13 (t_c's turns
-// leave no rounding behind).
+// IMRPhenomD requests on 3 x 32,128 bins 4,170 -> 283 us a call, 64
+// IMRPhenomPv2 requests on 2 x 32,448 bins 973 -> 103 us, the one-request call
+// on 3 x 32,128 bins 38.4 -> 22 us (Pv2, 3 x 16,224 bins: 48 -> 26 us), with
+// an error against 64-bit references of 7e-14 instead of 2e-13 (t_c's turns
+// leave no rounding behind).  512 requests on 3 x 3,000 quadrature nodes
+// 745 -> 111 us (bins 70, prologue 31): the powers of each node are tabulated
+// at registration, its linear phases 128-bit products.
 #include <cstdint>
 
 #include "kernel_util.cuh"
@@ -35,9 +37,10 @@ __device__ __forceinline__ ff warp_sum_ff(ff v) {
 }
 
 // Bins k0, k0 + step, ... < k1 of one request into acc.
+// (nodes: x's grid where it is not uniform; beyond the cut a node adds nothing).
 template <int NDET, bool PV2>
 __device__ __forceinline__ void acc_bins(const AccReq &x, const StreamDev *st, const AccTables &tb, const AccLut &lut,
-                                         int k0, int k1, int step, ff *acc) {
+                                         const AccNodes *nodes, int k0, int k1, int step, ff *acc) {
   const int n0 = st[0].n0;
   const bool wsh = x.m.wshared != 0;
   const float *dev = st[0].dev;
@@ -52,9 +55,18 @@ __device__ __forceinline__ void acc_bins(const AccReq &x, const StreamDev *st, c
         w[d] = ff{v.x, v.y};
       }
     }
-    const uint64_t qd = dev ? acc_dev_turns(x, __ldg(dev + k)) : 0;
-    if constexpr (PV2) acc_bin_p<NDET>(x, n0 + k, qd, tb, lut, wd, w, wsh, acc);
-    else acc_bin_d<NDET>(x, n0 + k, qd, tb, lut, wd, w, wsh, acc);
+    if (nodes) {
+      const int64_t f = __ldg((const long long *)st[0].freqs + k);
+      if (f > x.fcut) continue;
+      const float2 v = __ldg((const float2 *)nodes->x + k);
+      const AccNode b{k, f, __ldg((const long long *)nodes->X + k), ff{v.x, v.y}, 0};
+      if constexpr (PV2) acc_bin_p<NDET>(x, b, nodes->tb, lut, wd, w, wsh, acc);
+      else acc_bin_d<NDET>(x, b, nodes->tb, lut, wd, w, wsh, acc);
+      continue;
+    }
+    const AccBin b{n0 + k, dev ? acc_dev_turns(x, __ldg(dev + k)) : 0};
+    if constexpr (PV2) acc_bin_p<NDET>(x, b, tb, lut, wd, w, wsh, acc);
+    else acc_bin_d<NDET>(x, b, tb, lut, wd, w, wsh, acc);
   }
 }
 
@@ -83,19 +95,21 @@ __device__ __forceinline__ double acc_reduce(const AccReq &x, const ff *acc, dou
 // Bins k0, k0 + blockDim.x .. below kend on the whole block; the result in thread 0.
 template <int NDET>
 __device__ __forceinline__ double acc_block(const AccReq &x, const StreamDev *st, const AccTables &tb,
-                                            const AccLut &lut, int k0, int kend, double *s_red) {
-  const int kcut = min(kend, x.m.n_cut - st[0].n0 + 1);  // the model is zero beyond the cut
+                                            const AccLut &lut, const AccNodes *nodes, int k0, int kend,
+                                            double *s_red) {
+  // the model is zero beyond the cut
+  const int kcut = nodes ? kend : min(kend, x.m.n_cut - st[0].n0 + 1);
   if (x.m.approximant == kPhenomPv2) {
     ff acc[NDET * kAccPerDet];
 #pragma unroll
     for (int j = 0; j < NDET * kAccPerDet; j++) acc[j] = ff{0.f, 0.f};
-    acc_bins<NDET, true>(x, st, tb, lut, k0 + threadIdx.x, kcut, blockDim.x, acc);
+    acc_bins<NDET, true>(x, st, tb, lut, nodes, k0 + threadIdx.x, kcut, blockDim.x, acc);
     return acc_reduce<NDET, true>(x, acc, s_red);
   }
   ff acc[NDET * 2];
 #pragma unroll
   for (int j = 0; j < NDET * 2; j++) acc[j] = ff{0.f, 0.f};
-  acc_bins<NDET, false>(x, st, tb, lut, k0 + threadIdx.x, kcut, blockDim.x, acc);
+  acc_bins<NDET, false>(x, st, tb, lut, nodes, k0 + threadIdx.x, kcut, blockDim.x, acc);
   return acc_reduce<NDET, false>(x, acc, s_red);
 }
 
@@ -106,12 +120,15 @@ __device__ __forceinline__ void copy_words(void *dst, const void *src, int bytes
 // ------------------------------------------------------------------- batch
 // Persistent over the items in work order (as k_batch): an item is a tile of
 // one request's bins, its partial sum one double; the block that finishes a
-// request's last item adds them in item order.
-template <int NDET>
+// request's last item adds them in item order.  NODES: some requests' grids are
+// not uniform (a kernel of its own, so that batches without them keep their
+// code small).
+template <int NDET, bool NODES>
 __global__ void __launch_bounds__(kAccBlock, 2) k_batch_acc(const BatchArgs a) {
   __shared__ AccLut lut;
   __shared__ __align__(16) unsigned char s_req[sizeof(AccReq)];
   __shared__ StreamDev s_st[NDET];
+  __shared__ AccNodes s_nodes;
   __shared__ double s_red[kAccBlock / 32];
   __shared__ int s_item, s_iid, s_bstart[kOrderBuckets + 1];
   const int tid = threadIdx.x;
@@ -131,12 +148,20 @@ __global__ void __launch_bounds__(kAccBlock, 2) k_batch_acc(const BatchArgs a) {
     const Item I = a.items[iid];
     static_assert(sizeof(AccReq) % 4 == 0, "copied as words");
     copy_words(s_req, a.areq + I.req, sizeof(AccReq));
-    if (tid < NDET) s_st[tid] = a.streams[__ldcg(a.handles + I.req * a.ndet + tid)];
+    if (tid < NDET) {
+      StreamDev s = a.streams[__ldcg(a.handles + I.req * a.ndet + tid)];
+      if (NODES && s.node) {
+        s.wd = s.node->wd;
+        s.wf = s.node->wf;
+        if (tid == 0) s_nodes = *s.node;
+      }
+      s_st[tid] = s;
+    }
     __syncthreads();
     const AccReq &x = *(const AccReq *)s_req;
     const int kend = min(I.k0 + a.tile, s_st[0].N);
     double v = 0.0;
-    if (x.m.status == 0) v = acc_block<NDET>(x, s_st, a.acc, lut, I.k0, kend, s_red);
+    if (x.m.status == 0) v = acc_block<NDET>(x, s_st, a.acc, lut, NODES && s_st[0].node ? &s_nodes : nullptr, I.k0, kend, s_red);
     if (tid == 0) a.partials[iid] = v;
     if (arrive_last(a.req_done + I.req, (unsigned)__ldcg(a.item_count + I.req)) && tid == 0) {
       const int i0 = __ldcg(a.item_start + I.req), ic = __ldcg(a.item_count + I.req), st = x.m.status;
@@ -167,7 +192,7 @@ __global__ void __launch_bounds__(kPlainBlock) k_plain_acc(const __grid_constant
   if (k0 < x.m.n_cut - ps.s[0].n0 + 1) {
     copy_words(&lut, glut, sizeof(AccLut));
     __syncthreads();
-    v = acc_block<NDET>(x, ps.s, tb, lut, k0, min(k0 + kPlainBlock, N), s_red);
+    v = acc_block<NDET>(x, ps.s, tb, lut, nullptr, k0, min(k0 + kPlainBlock, N), s_red);
   }
   if (tid == 0) partials[blockIdx.x] = v;
   if (arrive_last(counter, gridDim.x)) {
@@ -211,26 +236,47 @@ __global__ void k_acc_stream(const StreamDev d, int with_dev) {
   }
 }
 
-const void *acc_fn(int ndet) {
-  switch (ndet) {
-    case 1: return (const void *)k_batch_acc<1>;
-    case 2: return (const void *)k_batch_acc<2>;
-    case 3: return (const void *)k_batch_acc<3>;
-    case 4: return (const void *)k_batch_acc<4>;
+// The same for a grid of nodes.
+__global__ void k_acc_nodes(const StreamDev d, const AccNodes a) {
+  const double idf = 1.0 / d.dfq;  // a power of two
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < d.N; k += gridDim.x * blockDim.x) {
+    const double x = d.freqs[k] * idf, t = cbrt(x), ln = log(x), q = sqrt(x * sqrt(x));
+    const_cast<ff4 *>(a.tb.pw)[k] = two_pairs(t, pow_m7_6(x));
+    const_cast<ff4 *>(a.tb.ph)[k] = two_pairs(1.0 / x, q);
+    const_cast<ff4 *>(a.tb.pv)[k] = two_pairs(1.0 / t, ln);
+    const_cast<double *>(a.tb.t13)[k] = t;
+    const_cast<double *>(a.tb.tm53)[k] = 1.0 / (x * (t * t));
+    const_cast<double *>(a.tb.tln)[k] = ln;
+    const_cast<double *>(a.tb.t34)[k] = q;
+    const_cast<int64_t *>(a.X)[k] = (int64_t)llrint(x * 4398046511104.0);  // 2^kNodeBits
+    const_cast<ff *>(a.x)[k] = ff_split(x);
+  }
+}
+
+const void *acc_fn(int ndet, bool nodes) {
+  switch (ndet + (nodes ? kMaxDet : 0)) {
+    case 1: return (const void *)k_batch_acc<1, false>;
+    case 2: return (const void *)k_batch_acc<2, false>;
+    case 3: return (const void *)k_batch_acc<3, false>;
+    case 4: return (const void *)k_batch_acc<4, false>;
+    case kMaxDet + 1: return (const void *)k_batch_acc<1, true>;
+    case kMaxDet + 2: return (const void *)k_batch_acc<2, true>;
+    case kMaxDet + 3: return (const void *)k_batch_acc<3, true>;
+    case kMaxDet + 4: return (const void *)k_batch_acc<4, true>;
     default: return nullptr;
   }
 }
 
 }  // namespace
 
-int batch_acc_occupancy(int ndet) {
+int batch_acc_occupancy(int ndet, bool nodes) {
   int nb = 0;
-  const void *f = acc_fn(ndet);
+  const void *f = acc_fn(ndet, nodes);
   if (!f || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, kAccBlock, 0) != cudaSuccess) return 1;
   return nb;
 }
-cudaError_t launch_batch_acc(const BatchArgs &a, int grid, cudaStream_t s, bool pdl) {
-  const void *f = acc_fn(a.ndet);
+cudaError_t launch_batch_acc(const BatchArgs &a, bool nodes, int grid, cudaStream_t s, bool pdl) {
+  const void *f = acc_fn(a.ndet, nodes);
   if (!f) return cudaErrorInvalidValue;
   void *args[] = {(void *)&a};
   return launch_dependent(f, dim3(grid), dim3(kAccBlock), args, s, pdl);
@@ -275,6 +321,14 @@ cudaError_t plain_acc_preload() {
 }
 cudaError_t launch_acc_tables(const AccTables &tab, cudaStream_t s) {
   k_acc_tables<<<(tab.nmax + 255) / 256, 256, 0, s>>>(tab);
+  return cudaGetLastError();
+}
+cudaError_t launch_acc_nodes(const StreamDev &d, const AccNodes &a, cudaStream_t s) {
+  StreamDev t = d;
+  t.wd = a.wd;
+  t.wf = a.wf;
+  k_acc_nodes<<<(d.N + 255) / 256, 256, 0, s>>>(d, a);
+  k_acc_stream<<<(d.N + 255) / 256, 256, 0, s>>>(t, 0);
   return cudaGetLastError();
 }
 cudaError_t launch_acc_stream(const StreamDev &d, bool with_dev, cudaStream_t s) {

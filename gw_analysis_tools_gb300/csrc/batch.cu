@@ -58,15 +58,17 @@ static int choose_occ(gwgpu_context *c, int mixed, const std::string &key) {
   return gwk::batch_default_occ(1);
 }
 
-enum { kFormFp64 = 0, kFormMixed = 1, kFormAcc = 2 };  // FP64 bins, mixed, FP64 form on two-float bins
+// FP64 bins, mixed, FP64 form on two-float bins, the same where some grids are not uniform
+enum { kFormFp64 = 0, kFormMixed = 1, kFormAcc = 2, kFormNodes = 3 };
+static bool two_float(int form) { return form == kFormAcc || form == kFormNodes; }
 
 static int persistent_grid(int device, int form, int ndet, int occ) {
-  static int cache[3][gwt::kMaxDet + 1][5] = {{{0}}};
+  static int cache[4][gwt::kMaxDet + 1][5] = {{{0}}};
   int &g = cache[form][ndet][occ & 3];
   if (g) return g;
   cudaDeviceProp p;
   cudaGetDeviceProperties(&p, device);
-  int per_sm = form == kFormAcc ? gwk::batch_acc_occupancy(ndet) : gwk::batch_occupancy(form, ndet, occ);
+  int per_sm = two_float(form) ? gwk::batch_acc_occupancy(ndet, form == kFormNodes) : gwk::batch_occupancy(form, ndet, occ);
   if (per_sm < 1) per_sm = 1;
   g = p.multiProcessorCount * per_sm;
   return g;
@@ -199,12 +201,12 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
     e = gwk::launch_prologue_serial((const gwt::GenParams *)d_params, d_approx, n, pl.handles, ndet, T_segment, 1,
                                     c->streams_dev, c->qnm_dev, form == kFormFp64 ? (gwt::Request *)reqs : nullptr,
                                     mixed ? (gwt::MixedReq *)reqs : nullptr,
-                                    form == kFormAcc ? (gwt::AccReq *)reqs : nullptr, mixed, d_status, L.stream);
+                                    two_float(form) ? (gwt::AccReq *)reqs : nullptr, mixed, d_status, L.stream);
   else
     e = gwk::launch_prologue((const gwt::GenParams *)d_params, d_approx, n, pl.handles, ndet, T_segment, 1,
                              c->streams_dev, c->qnm_dev, form == kFormFp64 ? (gwt::Request *)reqs : nullptr,
                              mixed ? (gwt::MixedReq *)reqs : nullptr, mixed, d_status, L.stream, ord,
-                             form == kFormAcc ? (gwt::AccReq *)reqs : nullptr);
+                             two_float(form) ? (gwt::AccReq *)reqs : nullptr);
   if (e != cudaSuccess) return c->fail(e, "prologue launch");
   if (timing) cudaEventRecord(c->t_ev[1], L.stream);
   gwk::BatchArgs a;
@@ -227,10 +229,10 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   a.status = d_status;
   a.status_out = status_out ? status_out : d_status;
   a.tables = c->tables;
-  a.areq = form == kFormAcc ? (const gwt::AccReq *)reqs : nullptr;
+  a.areq = two_float(form) ? (const gwt::AccReq *)reqs : nullptr;
   a.acc = c->acc;
   a.lut = c->acc_lut;
-  if (form == kFormAcc) e = gwk::launch_batch_acc(a, grid, L.stream, c->pdl);
+  if (two_float(form)) e = gwk::launch_batch_acc(a, form == kFormNodes, grid, L.stream, c->pdl);
   else e = gwk::launch_batch(a, mixed, grid, occ, L.stream, c->pdl);
   if (&L == &c->lane) {
     c->last_shape[0] = pl.tile;
@@ -263,18 +265,22 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
     L.shape.epoch = c->streams_epoch;
     L.shape.mixed = mixed;
     L.shape.acc = !mixed && c->acc_lut;
+    L.shape.nodes = false;
     L.shape.bins = 0;
     for (size_t i = 0; i < nh; i++) {
-      const gwgpu_context::Stream *s = c->get_stream(h_handles[i]);
-      L.shape.acc = L.shape.acc && s && s->dev.wd && s->dev.n0 + s->dev.N - 1 <= c->acc.nmax;
+      const gwgpu_context::Stream *s = c->get_stream(h_handles[i]), *s0 = c->get_stream(h_handles[i - i % ndet]);
+      // a request's detectors: all on bins of a uniform grid or all on nodes
+      const bool node = s && s->dev.node, bin = s && s->dev.wd && s->dev.n0 + s->dev.N - 1 <= c->acc.nmax;
+      L.shape.acc = L.shape.acc && s0 && (bin || node) && node == (s0->dev.node != nullptr);
+      L.shape.nodes = L.shape.nodes || node;
       if (s && i % ndet == 0) L.shape.bins += s->dev.N;
     }
   }
-  const int form = mixed ? kFormMixed : L.shape.acc ? kFormAcc : kFormFp64;
+  const int form = mixed ? kFormMixed : !L.shape.acc ? kFormFp64 : L.shape.nodes ? kFormNodes : kFormAcc;
   if (tile <= 0) {
     tile = choose_tile(c, mixed, L.tk);
-    if (form == kFormAcc && c->tile_override <= 0 && !c->tuned.count(L.tk))
-      tile = acc_tile(L.shape.bins, persistent_grid(c->device, kFormAcc, ndet, 0));
+    if (two_float(form) && c->tile_override <= 0 && !c->tuned.count(L.tk))
+      tile = acc_tile(L.shape.bins, persistent_grid(c->device, form, ndet, 0));
   }
   const int occ = choose_occ(c, mixed, L.tk);
   bool replanned = false;
@@ -287,7 +293,7 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
     L.plan.valid = true;
     replanned = true;
   }
-  size_t rq = mixed ? sizeof(gwt::MixedReq) : form == kFormAcc ? sizeof(gwt::AccReq) : sizeof(gwt::Request);
+  size_t rq = mixed ? sizeof(gwt::MixedReq) : two_float(form) ? sizeof(gwt::AccReq) : sizeof(gwt::Request);
   size_t bytes = rq * n + 512 + sizeof(double) * (size_t)L.plan.nitems * gwk::kAcc + 256 +
                  sizeof(unsigned) * (size_t)(2 * (size_t)n + 32 + gwk::kOrderBuckets);
   void *old = L.work;

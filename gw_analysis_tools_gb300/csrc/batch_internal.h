@@ -51,7 +51,8 @@ struct Lane {
   struct Shape {
     std::vector<int> handles;
     int n = -1, ndet = -1, mixed = -1;
-    bool acc = false;     // FP64 form: every stream has its two-float pairs
+    bool acc = false;
+  bool nodes = false;     // FP64 form: every stream has its two-float pairs
     long long bins = 0;   // over all requests
     uint64_t epoch = ~0ull;
   } shape;

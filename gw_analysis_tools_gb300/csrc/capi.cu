@@ -171,18 +171,22 @@ int gwgpu_context::ensure_tm76d(int nmax) {
   return GWGPU_OK;
 }
 
+int gwgpu_context::ensure_lut() {
+  if (acc_lut) return GWGPU_OK;
+  std::vector<gwt::AccLut> h(1);
+  gwt::ff_fill_tables(h[0].turn, h[0].ex);
+  void *p;
+  int st = dalloc(&p, sizeof(gwt::AccLut), "sine table");
+  if (st) return st;
+  cudaError_t e = cudaMemcpy(p, h.data(), sizeof(gwt::AccLut), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return fail(e, "sine table");
+  acc_lut = (gwt::AccLut *)p;
+  return GWGPU_OK;
+}
 int gwgpu_context::ensure_acc(int nmax) {
   int st = ensure_tables(nmax);
+  if (!st) st = ensure_lut();
   if (st) return st;
-  if (!acc_lut) {
-    std::vector<gwt::AccLut> h(1);
-    gwt::ff_fill_tables(h[0].turn, h[0].ex);
-    void *p;
-    if ((st = dalloc(&p, sizeof(gwt::AccLut), "sine table"))) return st;
-    cudaError_t e = cudaMemcpy(p, h.data(), sizeof(gwt::AccLut), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return fail(e, "sine table");
-    acc_lut = (gwt::AccLut *)p;
-  }
   if (nmax <= acc.nmax) return GWGPU_OK;
   const size_t n1 = (size_t)std::max(nmax, std::min(tables.nmax, std::max(2 * acc.nmax, 1 << 16))) + 1;
   void *p;
@@ -367,6 +371,38 @@ static void acc_stream(gwgpu_context *c, gwgpu_context::Stream &s, const double 
   s.mem.push_back(p);
 }
 
+// The same for a grid that is not uniform (phenom_acc.h, AccNodes; d.dfq its
+// scale): positive finite frequencies within the range of the bin tables, in
+// nodes_bytes of device memory at p.
+static size_t nodes_bytes(size_t row) { return 120 * row + sizeof(gwt::AccNodes); }
+static bool nodes_fit(const StreamDev &d, const double *freqs) {
+  for (int k = 0; k < d.N; k++)
+    if (!(freqs[k] > 0x1p-20 * d.dfq && freqs[k] < 0x1p20 * d.dfq)) return false;
+  return true;
+}
+static int acc_nodes(gwgpu_context *c, StreamDev &d, size_t row, char *p) {
+  gwt::AccNodes a;
+  a.wd = (const gwt::ff4 *)p;
+  a.tb.pw = a.wd + row;
+  a.tb.ph = a.wd + 2 * row;
+  a.tb.pv = a.wd + 3 * row;
+  a.tb.t13 = (const double *)(a.wd + 4 * row);
+  a.tb.tm53 = a.tb.t13 + row;
+  a.tb.tln = a.tb.t13 + 2 * row;
+  a.tb.t34 = a.tb.t13 + 3 * row;
+  a.X = (const int64_t *)(a.tb.t13 + 4 * row);
+  a.x = (const gwt::ff *)(a.tb.t13 + 5 * row);
+  a.wf = (const gwt::ff *)(a.tb.t13 + 6 * row);
+  a.tb.nmax = d.N - 1;
+  cudaError_t e = gwk::launch_acc_nodes(d, a, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(p + 120 * row, &a, sizeof(a), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return c->fail(e, "two-float stream");
+  d.node = (const gwt::AccNodes *)(p + 120 * row);
+  return GWGPU_OK;
+}
+
 // One detector stream; weights (GAUSSLEG) or null (Simpson's rule).
 static int register_stream(gwgpu_context *c, const char *detector, const double *freqs, int N, const double *data,
                            const double *psd, const double *weights, int log10F, int *handle) {
@@ -393,6 +429,11 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   d.n0 = (int)std::llround(n0f);
   d.dfq = (freqs[N - 1] - freqs[0]) / (N - 1);
   d.uniform_int = uniform && d.n0 >= 1 && std::fabs(n0f - d.n0) < 1e-6 && (d.n0 + (double)N) < 1.5e9;
+  if (!d.uniform_int) {
+    double fmax = 0;
+    for (int k = 0; k < N; k++) fmax = std::fmax(fmax, freqs[k]);
+    d.dfq = fmax > 0 && std::isfinite(fmax) ? std::ldexp(1.0, std::ilogb(fmax) - 19) : 1.0;
+  }
   // integration weights: Simpson's rule, (4 df/3) s_k (util.h:844-856), or the
   // GAUSSLEG branch, 4 w_k (times f_k ln 10 for log10F) (mcmc_gw.cpp:820-862);
   // whitening for the mixed form W_k = weight_k / S_k
@@ -424,8 +465,15 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   for (int k = 0; k < N; k++) ip[k] = 1.0 / psd[k];
   // one allocation for the stream's arrays, each on a 256-byte boundary
   const size_t row = ((size_t)N + 31) / 32 * 32, gat = row * (weights ? 60 : 52);
+  const size_t nat = gat + 2 * sizeof(gwt::GridConst);
+  bool nodes = !d.uniform_int && finite && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
   char *mem;
-  if ((st = c->dalloc((void **)&mem, gat + 2 * sizeof(gwt::GridConst), "data stream"))) return st;
+  st = c->dalloc((void **)&mem, nat + (nodes ? nodes_bytes(row) : 0), "data stream");
+  if (st && nodes) {  // without them the stream keeps the FP64 bins
+    nodes = false;
+    st = c->dalloc((void **)&mem, nat, "data stream");
+  }
+  if (st) return st;
   const gwt::GridConst gc[2] = {gwt::grid_const(d.df), gwt::grid_const(d.dfq)};
   cudaMemcpyAsync(mem + gat, gc, sizeof(gc), cudaMemcpyHostToDevice, c->stream);
   d.grid = (const gwt::GridConst *)(mem + gat);
@@ -472,6 +520,9 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     st = c->ensure_tables(d.n0 + N);
     if (st) return st;
     if (finite) acc_stream(c, s, freqs);
+  } else if (nodes && (st = acc_nodes(c, s.dev, row, mem + nat))) {
+    c->dfree(mem);
+    return st;
   }
   c->streams.push_back(s);
   *handle = (int)c->streams.size() - 1;

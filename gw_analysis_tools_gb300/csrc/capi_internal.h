@@ -83,6 +83,7 @@ struct gwgpu_context {
   int ensure_tables(int nmax);
   int ensure_tm76d(int nmax);
   int ensure_acc(int nmax);
+  int ensure_lut();
   int sync_streams_table();
   const Stream *get_stream(int handle) const;
   unsigned *counter(int i);

@@ -244,7 +244,7 @@ __global__ void k_prologue(const GenParams *__restrict__ params, const int *__re
     if (r.m.status) st = 4;
     if (req) req[i] = r;
     if (want_mixed || areq) {
-      if (!s0.uniform_int) st = st ? st : 1;
+      if (!s0.uniform_int && !(areq && s0.node)) st = st ? st : 1;
       double ds[kMaxDet], ws[kMaxDet];
       unsigned long long wk[kMaxDet];
       for (int d = 0; d < ndet; d++) {
@@ -252,8 +252,10 @@ __global__ void k_prologue(const GenParams *__restrict__ params, const int *__re
         ws[d] = streams[handles[i * ndet + d]].wscale;
         wk[d] = streams[handles[i * ndet + d]].wkey;
       }
-      if (areq) acc_prologue(r, s0.dfq, areq[i], ds, ws);
-      else mixed_prologue(r, s0.df, mreq[i], ds, ws);
+      if (areq) {
+        acc_prologue(r, s0.dfq, areq[i], ds, ws);
+        if (s0.node) acc_node_coeffs(r, s0.dfq, areq[i]);
+      } else mixed_prologue(r, s0.df, mreq[i], ds, ws);
       mixed_fold_shared_weights(areq ? areq[i].m : mreq[i], wk, ndet);
     }
   } else {
@@ -352,7 +354,7 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
         for (int d = 0; d < ndet; d++)
           if (streams[__ldcg(handles + i * ndet + d)].N != s0.N) st = 1;
         sm.st[j] = st;
-        sm.uni[j] = s0.uniform_int;
+        sm.uni[j] = s0.uniform_int ? 1 : ACC && s0.node ? 2 : 0;  // bins, nodes, neither
         sm.N[j] = s0.N;
         sm.n0[j] = s0.n0;
         head(i, sm.item0[j], sm.items[j]);
@@ -550,6 +552,9 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
       }
       if (m.status) st = 4;
       if (coef && !sm.uni[j]) st = st ? st : 1;
+      if constexpr (ACC) {
+        if (sm.uni[j] == 2) acc_node_coeffs(r, gc.df, areq[i]);
+      }
       if constexpr (ACC) areq[i].fp64_phase = sm.big[j] | (pv2 ? sm.late[j] : 0);
     } else {
       st = 4;
@@ -571,7 +576,8 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
     // a request is live when its status will be 0: valid parameters, model
     // status 0, one uniform grid length
     int kcut = 0;
-    if (run && m.status == 0 && sm.st[j] == 0 && sm.uni[j]) kcut = min(sm.N[j], sm.ncut[j] - sm.n0[j] + 1);
+    if (run && m.status == 0 && sm.st[j] == 0 && sm.uni[j])
+      kcut = sm.uni[j] == 2 ? sm.N[j] : min(sm.N[j], sm.ncut[j] - sm.n0[j] + 1);
     tail((warp - 1) * G + g, act ? sm.item0[j] : 0, act ? sm.items[j] : 0, kcut);
   }
 }

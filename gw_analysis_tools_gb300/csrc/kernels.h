@@ -43,6 +43,7 @@ struct StreamDev {
   const float *dev;
   double dfq;
   const gwt::GridConst *grid;  // of df, of dfq
+  const gwt::AccNodes *node;   // grids that are not uniform: the same by node (dfq the nodes' scale), or null
 };
 
 struct Item {
@@ -137,11 +138,12 @@ struct BatchArgs {
 cudaError_t launch_batch(const BatchArgs &a, int mixed, int grid, int occ, cudaStream_t s, bool pdl);
 cudaError_t launch_dependent(const void *f, dim3 grid, dim3 block, void **args, cudaStream_t s, bool pdl);
 // The fused kernel of the FP64 form on two-float bins.
-cudaError_t launch_batch_acc(const BatchArgs &a, int grid, cudaStream_t s, bool pdl);
-int batch_acc_occupancy(int ndet);
+cudaError_t launch_batch_acc(const BatchArgs &a, bool nodes, int grid, cudaStream_t s, bool pdl);
+int batch_acc_occupancy(int ndet, bool nodes);
 // Tables n <= nmax from the FP64 powers t13, tln, t34 of tab, and a stream's
 // pairs from its FP64 arrays.
 cudaError_t launch_acc_tables(const gwt::AccTables &tab, cudaStream_t s);
+cudaError_t launch_acc_nodes(const StreamDev &d, const gwt::AccNodes &a, cudaStream_t s);
 cudaError_t launch_acc_stream(const StreamDev &d, bool with_dev, cudaStream_t s);
 
 int batch_default_occ(int mixed);

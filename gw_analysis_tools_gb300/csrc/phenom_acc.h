@@ -12,6 +12,9 @@
 // phase, ~1e-12 rad.
 #pragma once
 
+#include <cstring>
+#include <type_traits>
+
 #include "phenom_mixed.h"
 #include "two_float.h"
 
@@ -24,6 +27,18 @@ struct AccTables {
   const ff4 *pv;       // n^(-1/3), ln n
   const double *t13, *tm53, *tln, *t34;  // n^(1/3), n^(-5/3), ln n, n^(3/4)
   int nmax;            // valid for 1 <= n <= nmax
+};
+
+// A grid of any other spacing (quadrature nodes): bins at x = f / df, df the
+// power of two that puts the highest frequency in [2^19, 2^20); the weights and
+// data products as on uniform grids, the tables by the bin's index.
+constexpr int kNodeBits = 42;
+struct AccNodes {
+  const ff4 *wd;
+  const ff *wf;
+  AccTables tb;
+  const int64_t *X;  // x 2^kNodeBits
+  const ff *x;
 };
 
 // Sine/cosine and exponential tables (shared memory in the kernels).
@@ -58,6 +73,13 @@ struct AccReq {
   ff c2z, s2z;                        // polarisation rotation
   float tc;                           // model's t_c, for bins off the line n df (acc_dev_turns)
   float bad;                          // NaN when a linear phase is (turns cannot hold it), else 0; joins the result
+  // On nodes (acc_node_coeffs): slopes of the linear phases in turns per bin
+  // 2^(node_shift + 64 - kNodeBits), region boundaries as the bits of the
+  // frequencies (f positive: ordered as integers), n_rd and n_c whole
+  int64_t nS[kMaxDet], nP, nM;
+  int64_t f1, f1p, f3, f2p, fcut;
+  ff nrd, nc;
+  int node_shift;
   int fp64_phase;                     // 1: terms too large for two floats; every bin takes the FP64 series
 };
 
@@ -116,6 +138,41 @@ GW_HD void acc_phase_coeffs(const Request &r, double df, AccReq &x) {
 GW_HD void acc_amp_coeffs(const Request &r, double df, AccReq &x) {
   const double nrd = r.m.s.fRD / df;
   x.rdfrac = ff_split(nrd - floor(nrd));
+}
+GW_HD int64_t acc_bits(double v) {
+  int64_t b;
+  memcpy(&b, &v, 8);
+  return b;
+}
+// What nodes need beside the above (df: their scale), the linear phases first:
+// a slope of at most 2^62 in size against x 2^kNodeBits, a 128-bit product.
+GW_HDNI void acc_node_coeffs(const Request &r, double df, AccReq &x) {
+  const ModelD &m = r.m;
+  const double inv2pi = 1.0 / (2.0 * kPi);
+  const double c1 = r.approximant == kPhenomPv2 ? r.p.t_corr * df : -m.tcs * df * inv2pi, tc = m.s.tc * df;
+  double tau[kMaxDet], big = 0.0;
+  for (int d = 0; d < r.ndet && d < kMaxDet; d++) {
+    tau[d] = r.det[d].tau * df * inv2pi;
+    big = fmax(big, fabs(tau[d]));
+  }
+  const double pB = x.m.pB * inv2pi, mB = x.m.mB * inv2pi;
+  big += fabs(c1) + fabs(tc) + fabs(pB) + fabs(mB);
+  int a = big > 0.0 && big < 1e300 ? 61 - ilogb(big) : 85;
+  a = a > 85 ? 85 : a < 23 ? 23 : a;
+  // beyond 2^38 turns per bin no digit of a bin's phase is left
+  const double sc = big < 274877906944.0 ? ldexp(1.0, a) : 0.0;
+  for (int d = 0; d < r.ndet && d < kMaxDet; d++)
+    x.nS[d] = gw_llrint(c1 * sc) - gw_llrint(tc * sc) - gw_llrint(tau[d] * sc);
+  x.nP = gw_llrint(pB * sc);
+  x.nM = gw_llrint(mB * sc);
+  x.node_shift = a + kNodeBits - 64;
+  x.f1 = acc_bits(m.s.f1);
+  x.f1p = acc_bits(m.s.f1_phase);
+  x.f3 = acc_bits(m.s.f3);
+  x.f2p = acc_bits(m.s.f2_phase);
+  x.fcut = acc_bits(m.fcut);
+  x.nrd = ff_split(m.s.fRD / df);
+  x.nc = ff_split(m.l.alpha[5] * m.s.fRD / df);
 }
 // Pv2, after mixed_pv2_coeffs and mixed_phase_coeffs: epsilon joins the
 // inspiral phase series (the same powers of n), the rest in turns.
@@ -203,46 +260,117 @@ GW_HD ff4 acc_ld(const ff4 *p) {
   return *p;
 #endif
 }
-// The FP64 phase of bin n in turns 2^64 without the linear terms (Pv2: with
+// A bin of a uniform grid (qd: its acc_dev_turns) and a node (f's bits, x 2^kNodeBits,
+// x; sl: the slope of its phase region).  The functions below take either.
+struct AccBin {
+  int n;
+  uint64_t qd;
+};
+struct AccNode {
+  int k;
+  int64_t f, X;
+  ff x;
+  int64_t sl;
+};
+GW_HD int acc_at(const AccBin &b) { return b.n; }
+GW_HD int acc_at(const AccNode &b) { return b.k; }
+GW_HD bool acc_ins_amp(const AccReq &x, const AccBin &b) { return b.n < x.m.n_f1; }
+GW_HD bool acc_ins_amp(const AccReq &x, const AccNode &b) { return b.f < x.f1; }
+GW_HD bool acc_ring_amp(const AccReq &x, const AccBin &b) { return b.n >= x.m.n_f3; }
+GW_HD bool acc_ring_amp(const AccReq &x, const AccNode &b) { return b.f > x.f3; }
+GW_HD bool acc_ins_phase(const AccReq &x, const AccBin &b) { return b.n < x.m.n_f1p; }
+GW_HD bool acc_ins_phase(const AccReq &x, const AccNode &b) { return b.f < x.f1p; }
+GW_HD bool acc_ring_phase(const AccReq &x, const AccBin &b) { return b.n >= x.m.n_f2p; }
+GW_HD bool acc_ring_phase(const AccReq &x, const AccNode &b) { return b.f > x.f2p; }
+// The bin's distance from a position, n0 + frac or whole.
+GW_HD ff acc_from(const AccBin &b, int n0, ff frac, ff) {
+  ff xx = two_sum((float)(b.n - n0), -frac.h);
+  xx.l = f_sub(xx.l, frac.l);
+  return xx;
+}
+GW_HD ff acc_from(const AccNode &b, int, ff, ff whole) { return ff_norm(ff_sub(b.x, whole)); }
+GW_HD ff acc_times(ff a, const AccBin &b, int n0) { return ff_mulf(a, (float)(b.n - n0)); }
+GW_HD ff acc_times(ff a, const AccNode &b, int n0) { return ff_mul(a, n0 ? ff_norm(ff_addf(b.x, -(float)n0)) : b.x); }
+// S X 2^-s modulo one turn.
+GW_HD uint64_t acc_node_turns(int64_t S, int64_t X, int s) {
+#if defined(__CUDA_ARCH__)
+  const uint64_t hi = (uint64_t)__mul64hi(S, X), lo = (uint64_t)S * (uint64_t)X;
+#else
+  const __int128 p = (__int128)S * X;
+  const uint64_t hi = (uint64_t)(p >> 64), lo = (uint64_t)p;
+#endif
+  return (hi << (64 - s)) | (lo >> s);  // 1 <= s <= 63
+}
+// Detector d's linear phase (a node's with its region's slope).
+GW_HD uint64_t acc_linear(const AccReq &x, const AccBin &b, int d) { return x.L0[d] + x.L1[d] * (uint64_t)b.n; }
+GW_HD uint64_t acc_linear(const AccReq &x, const AccNode &b, int d) {
+  return x.L0[d] + acc_node_turns(x.nS[d] + b.sl, b.X, x.node_shift);
+}
+GW_HD uint64_t acc_region_slope(const AccBin &b, uint64_t per_bin, int64_t) { return per_bin * (uint64_t)b.n; }
+GW_HD uint64_t acc_region_slope(AccNode &b, uint64_t, int64_t sl) {
+  b.sl = sl;
+  return 0;
+}
+GW_HD uint64_t acc_offset(const AccBin &b) { return b.qd; }
+GW_HD uint64_t acc_offset(const AccNode &) { return 0; }
+
+// The FP64 phase of a bin in turns 2^64 without the linear terms (Pv2: with
 // 2 epsilon), and alpha.
-template <bool PV2>
-GW_HD uint64_t acc_phase64(const AccReq &x, int n, const AccTables &tb, const AccLut &lut, uint64_t &al) {
+template <bool PV2, class B>
+GW_HD uint64_t acc_phase64(const AccReq &x, B &b, const AccTables &tb, const AccLut &lut, uint64_t &al) {
   const MixedReq &m = x.m;
+  const int n = acc_at(b);
   const double t = acc_ld(tb.t13 + n), r = acc_ld(tb.tm53 + n), lnn = acc_ld(tb.tln + n);
-  if (PV2) al = radians_q64(mixed_pv2_alpha(m, n, t, r, lnn));
-  if (n < m.n_f1p) return radians_q64(mixed_phase_d(m, n, t, r, lnn, 0.0));
+  double nd, eps = 0.0;
+  if constexpr (std::is_same<B, AccBin>::value) {
+    nd = (double)n;
+    if (PV2) al = radians_q64(mixed_pv2_alpha(m, n, t, r, lnn));
+    if (acc_ins_phase(x, b)) return radians_q64(mixed_phase_d(m, n, t, r, lnn, 0.0));
+    if (PV2) eps = mixed_pv2_eps(m, n, t, r, lnn);
+  } else {
+    nd = (double)b.X * (1.0 / 4398046511104.0);
+    b.sl = 0;
+    if (PV2) {
+      const double *a = m.ea, *e = m.ee;
+      al = radians_q64(r * (a[0] * t * t + a[1] * nd + a[2] * nd * t) + a[3] + a[4] * t + a[5] * lnn);
+      eps = r * (e[0] * t * t + e[1] * nd + e[2] * nd * t) + e[3] + e[4] * t + e[5] * lnn;
+    }
+    if (acc_ins_phase(x, b)) {
+      double p = m.qi[11];
+      for (int j = 10; j >= 0; j--) p = p * t + m.qi[j];
+      return radians_q64(r * p + lnn * (m.bi0 + m.bi1 * t));
+    }
+  }
   double ph;
   uint64_t q = 0;
-  if (n >= m.n_f2p) {
-    const double nd = (double)n;
+  if (acc_ring_phase(x, b)) {
     // the atan by its two-float form, |mE| ~ 1
-    ff xx = two_sum((float)(n - m.n_c), -x.ncfrac.h), d;
-    xx.l -= x.ncfrac.l;
-    const int i = ff_atan(ff_norm(ff_mul(xx, x.inv_nw)), lut.turn, d);
+    ff d;
+    const int i = ff_atan(ff_norm(ff_mul(acc_from(b, m.n_c, x.ncfrac, x.nc), x.inv_nw)), lut.turn, d);
     ph = m.mA + m.mB * nd - m.mC * (r * t * t) + m.mD * acc_ld(tb.t34 + n) + m.mE * ff_value(d);
     q = x.mEq * (uint64_t)(int64_t)i;
   } else {
-    ph = m.pA + m.pB * (double)n + m.pC * lnn - m.pD * (r * r * t);
+    ph = m.pA + m.pB * nd + m.pC * lnn - m.pD * (r * r * t);
   }
-  if (PV2) ph += 2.0 * mixed_pv2_eps(m, n, t, r, lnn);
+  if (PV2) ph += 2.0 * eps;
   return q + radians_q64(ph);
 }
-template <bool PV2>
-GW_HD uint64_t acc_phase(const AccReq &x, int n, const AccTables &tb, const AccLut &lut, ff t, uint64_t &al) {
+template <bool PV2, class B>
+GW_HD uint64_t acc_phase(const AccReq &x, B &b, const AccTables &tb, const AccLut &lut, ff t, uint64_t &al) {
   const MixedReq &m = x.m;
-  if (n < m.n_f1p || x.fp64_phase) return acc_phase64<PV2>(x, n, tb, lut, al);
+  const int n = acc_at(b);
+  if (acc_ins_phase(x, b) || x.fp64_phase) return acc_phase64<PV2>(x, b, tb, lut, al);
   uint64_t q;
-  if (n >= m.n_f2p) {
+  if (acc_ring_phase(x, b)) {
     const ff4 w = acc_ld(tb.ph + n);
-    ff xx = two_sum((float)(n - m.n_c), -x.ncfrac.h), d;
-    xx.l = f_sub(xx.l, x.ncfrac.l);
-    const int i = ff_atan(ff_norm(ff_mul(xx, x.inv_nw)), lut.turn, d);
+    ff d;
+    const int i = ff_atan(ff_norm(ff_mul(acc_from(b, m.n_c, x.ncfrac, x.nc), x.inv_nw)), lut.turn, d);
     ff v = ff_add(ff_mul(x.cD, ff{w.sh, w.sl}), ff_mul(x.cC, ff{w.ch, w.cl}));
     v = ff_add(v, ff_mul(x.cE, d));
-    q = x.mR0 + x.mR1 * (uint64_t)n + x.mEq * (uint64_t)(int64_t)i + ff_turns_q64(ff_norm(v));
+    q = x.mR0 + acc_region_slope(b, x.mR1, x.nM) + x.mEq * (uint64_t)(int64_t)i + ff_turns_q64(ff_norm(v));
   } else {
     const double r = acc_ld(tb.tm53 + n);
-    q = x.pR0 + x.pR1 * (uint64_t)n +
+    q = x.pR0 + acc_region_slope(b, x.pR1, x.nP) +
         radians_q64(m.pC * acc_ld(tb.tln + n) - m.pD * (r * r * acc_ld(tb.t13 + n)));
   }
   if (PV2) {
@@ -257,25 +385,24 @@ GW_HD uint64_t acc_phase(const AccReq &x, int n, const AccTables &tb, const AccL
   }
   return q;
 }
-// Amplitude / A_scale of bin n (below the cut): mixed_amp's formulas.
-GW_HD ff acc_amp(const AccReq &x, int n, ff t, ff m76, const AccLut &lut) {
+// Amplitude / A_scale of a bin (below the cut): mixed_amp's formulas.
+template <class B>
+GW_HD ff acc_amp(const AccReq &x, const B &b, ff t, ff m76, const AccLut &lut) {
   const MixedReq &m = x.m;
   ff a;
-  if (n < m.n_f1) {
+  if (acc_ins_amp(x, b)) {
     a = acc_pair(m.ai, m.ai_lo, 9);
 #pragma unroll
     for (int j = 8; j >= 0; j--) a = ff_add(ff_mul(a, t), acc_pair(m.ai, m.ai_lo, j));
-  } else if (n >= m.n_f3) {
-    ff xx = two_sum((float)(n - m.n_rd), -x.rdfrac.h);
-    xx.l = f_sub(xx.l, x.rdfrac.l);
+  } else if (acc_ring_amp(x, b)) {
+    const ff xx = acc_from(b, m.n_rd, x.rdfrac, x.nrd);
     const ff z = ff_norm(ff_neg(ff_mul(ff{m.mrExp, m.mrExp_lo}, xx)));
     const ff den = ff_norm(ff_add(ff_sqr(xx), ff{m.mrG2, m.mrG2_lo}));
     a = ff_div(ff_norm(ff_mul(ff_exp(z, lut.ex), ff{m.mrK, m.mrK_lo})), den);
   } else {
-    const float h = (float)(n - m.n_mid);
     a = acc_pair(m.ei, m.ei_lo, 4);
 #pragma unroll
-    for (int j = 3; j >= 0; j--) a = ff_add(ff_mulf(a, h), acc_pair(m.ei, m.ei_lo, j));
+    for (int j = 3; j >= 0; j--) a = ff_add(acc_times(a, b, m.n_mid), acc_pair(m.ei, m.ei_lo, j));
   }
   return ff_norm(ff_mul(ff_norm(a), m76));
 }
@@ -286,22 +413,22 @@ GW_HD uint64_t acc_dev_turns(const AccReq &x, float dev) {
   return (uint64_t)(int64_t)f_to_int(f_mul(f_mul(-x.tc, dev), 36028797018963968.0f)) << 9;  // 2^-55 turns
 }
 
-// IMRPhenomD bin (qd: its acc_dev_turns): acc[2 d] weighted |h|^2 (detector 0 only when the detectors
+// IMRPhenomD bin: acc[2 d] weighted |h|^2 (detector 0 only when the detectors
 // share their weights), acc[2 d + 1] Re(d* h e^{i phi_d}).  wd: the detector
 // streams at this bin, W d (re, im); w: W.
-template <int NDET>
-GW_HD void acc_bin_d(const AccReq &x, int n, uint64_t qd, const AccTables &tb, const AccLut &lut, const ff4 *wd, const ff *w,
+template <int NDET, class B>
+GW_HD void acc_bin_d(const AccReq &x, B b, const AccTables &tb, const AccLut &lut, const ff4 *wd, const ff *w,
                      bool wshared, ff *acc) {
-  const ff4 p = acc_ld(tb.pw + n);
+  const ff4 p = acc_ld(tb.pw + acc_at(b));
   const ff t{p.ch, p.cl};
-  const ff a = acc_amp(x, n, t, ff{p.sh, p.sl}, lut);
+  const ff a = acc_amp(x, b, t, ff{p.sh, p.sl}, lut);
   uint64_t al;
-  const uint64_t ph = qd + acc_phase<false>(x, n, tb, lut, t, al);
+  const uint64_t ph = acc_offset(b) + acc_phase<false>(x, b, tb, lut, t, al);
   const ff aa = ff_norm(ff_sqr(a));
 #pragma unroll
   for (int d = 0; d < NDET; d++) {
     ff c, s;
-    ff_turns_sincos(ph + x.L0[d] + x.L1[d] * (uint64_t)n, lut.turn, c, s);
+    ff_turns_sincos(ph + acc_linear(x, b, d), lut.turn, c, s);
     if (d == 0 || !wshared) ff_acc(acc[2 * d], ff_mul(w[d], aa));
     const ff v = ff_sub(ff_mul(ff{wd[d].ch, wd[d].cl}, c), ff_mul(ff{wd[d].sh, wd[d].sl}, s));
     ff_acc(acc[2 * d + 1], ff_mul(a, v));
@@ -311,11 +438,12 @@ GW_HD void acc_bin_d(const AccReq &x, int n, uint64_t qd, const AccTables &tb, c
 //   h+ = p2 (1 + cb^2)/2 cos 2a + p1 sb cb cos a + p0 sb^2 + i (p2 cb sin 2a + p1 sb sin a)
 //   hx = i (m2 cb cos 2a + m1 sb cos a) - (m2 (1 + cb^2)/2 sin 2a + m1 sb cb sin a)
 // (the half-angle products of IMRPhenomP.cpp:665-715 collected by e^{i k alpha}).
-GW_HD void acc_twist(const AccReq &x, int n, const AccTables &tb, const AccLut &lut, ff t, uint64_t al, ff &hpr,
+template <class B>
+GW_HD void acc_twist(const AccReq &x, const B &b, const AccTables &tb, const AccLut &lut, ff t, uint64_t al, ff &hpr,
                      ff &hpi, ff &hcr, ff &hci) {
-  const ff4 iw = acc_ld(tb.pv + n);
+  const ff4 iw = acc_ld(tb.pv + acc_at(b));
   ff u = ff_add(ff_mul(x.us[0], ff{iw.ch, iw.cl}), ff_mul(x.us[1], t));
-  u = ff_norm(ff_add(ff_add(u, ff_mulf(x.us[2], (float)n)), x.us[3]));
+  u = ff_norm(ff_add(ff_add(u, acc_times(x.us[2], b, 0)), x.us[3]));
   ff cb, sb;
   if (fabsf(u.h) < 1e9f) {
     sb = ff_rsqrt(ff_norm(ff_addf(ff_sqr(u), 1.0f)));
@@ -339,16 +467,16 @@ GW_HD void acc_twist(const AccReq &x, int n, const AccTables &tb, const AccLut &
   hcr = ff_norm(ff_neg(ff_add(ff_mul(ff_norm(ff_mul(x.y2m, uu)), s2), ff_mul(ff_norm(ff_mul(x.y1m, sc)), sa))));
 }
 // IMRPhenomPv2 bin: five sums per detector (mixed_bin_p's).
-template <int NDET>
-GW_HD void acc_bin_p(const AccReq &x, int n, uint64_t qd, const AccTables &tb, const AccLut &lut, const ff4 *wd, const ff *w,
+template <int NDET, class B>
+GW_HD void acc_bin_p(const AccReq &x, B b, const AccTables &tb, const AccLut &lut, const ff4 *wd, const ff *w,
                      bool wshared, ff *acc) {
-  const ff4 p = acc_ld(tb.pw + n);
+  const ff4 p = acc_ld(tb.pw + acc_at(b));
   const ff t{p.ch, p.cl};
-  const ff a = acc_amp(x, n, t, ff{p.sh, p.sl}, lut);
+  const ff a = acc_amp(x, b, t, ff{p.sh, p.sl}, lut);
   uint64_t al;
-  const uint64_t ph = qd + acc_phase<true>(x, n, tb, lut, t, al);
+  const uint64_t ph = acc_offset(b) + acc_phase<true>(x, b, tb, lut, t, al);
   ff hpr, hpi, hcr, hci;
-  acc_twist(x, n, tb, lut, t, al, hpr, hpi, hcr, hci);
+  acc_twist(x, b, tb, lut, t, al, hpr, hpi, hcr, hci);
   const ff aa = ff_norm(ff_sqr(a));
   const ff spp = ff_norm(ff_mul(aa, ff_norm(ff_add(ff_sqr(hpr), ff_sqr(hpi)))));
   const ff scc = ff_norm(ff_mul(aa, ff_norm(ff_add(ff_sqr(hcr), ff_sqr(hci)))));
@@ -356,7 +484,7 @@ GW_HD void acc_bin_p(const AccReq &x, int n, uint64_t qd, const AccTables &tb, c
 #pragma unroll
   for (int d = 0; d < NDET; d++) {
     ff c, s;
-    ff_turns_sincos(ph + x.L0[d] + x.L1[d] * (uint64_t)n, lut.turn, c, s);
+    ff_turns_sincos(ph + acc_linear(x, b, d), lut.turn, c, s);
     if (d == 0 || !wshared) {
       ff_acc(acc[kAccPerDet * d + 0], ff_mul(w[d], spp));
       ff_acc(acc[kAccPerDet * d + 1], ff_mul(w[d], scc));
@@ -378,12 +506,13 @@ GW_HD void acc_wave(const AccReq &x, int n, uint64_t qd, const AccTables &tb, co
                     ff &cr, ff &ci) {
   pr = pi = cr = ci = ff{0.f, 0.f};
   if (n > x.m.n_cut) return;
+  AccBin b{n, qd};
   const ff4 p = acc_ld(tb.pw + n);
   const ff t{p.ch, p.cl};
-  ff a = acc_amp(x, n, t, ff{p.sh, p.sl}, lut);
+  ff a = acc_amp(x, b, t, ff{p.sh, p.sl}, lut);
   a.h += x.bad;
   uint64_t al;
-  const uint64_t ph = qd + acc_phase<PV2>(x, n, tb, lut, t, al) + x.B0 + x.B1 * (uint64_t)n;
+  const uint64_t ph = qd + acc_phase<PV2>(x, b, tb, lut, t, al) + x.B0 + x.B1 * (uint64_t)n;
   ff c, s;
   ff_turns_sincos(ph, lut.turn, c, s);
   const ff er = ff_norm(ff_mul(a, c)), ei = ff_norm(ff_neg(ff_mul(a, s)));  // a e^{-i psi}
@@ -392,7 +521,7 @@ GW_HD void acc_wave(const AccReq &x, int n, uint64_t qd, const AccTables &tb, co
     pi = ei;
   } else {
     ff hpr, hpi, hcr, hci;
-    acc_twist(x, n, tb, lut, t, al, hpr, hpi, hcr, hci);
+    acc_twist(x, b, tb, lut, t, al, hpr, hpi, hcr, hci);
     const ff tpr = ff_norm(ff_sub(ff_mul(hpr, er), ff_mul(hpi, ei))), tpi = ff_norm(ff_add(ff_mul(hpr, ei), ff_mul(hpi, er)));
     const ff txr = ff_norm(ff_sub(ff_mul(hcr, er), ff_mul(hci, ei))), txi = ff_norm(ff_add(ff_mul(hcr, ei), ff_mul(hci, er)));
     pr = ff_norm(ff_add(ff_mul(x.c2z, tpr), ff_mul(x.s2z, txr)));

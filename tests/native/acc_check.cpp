@@ -42,9 +42,9 @@ static void bins(const AccReq &x, int n0, int N, const AccTables &tb, const std:
         a[d] = wd[d][k];
         b[d] = w[d][k];
       }
-      const uint64_t qd = acc_dev_turns(x, dev[k]);
-      if (pv2) acc_bin_p<NDET>(x, n, qd, tb, lut(), a, b, false, acc);
-      else acc_bin_d<NDET>(x, n, qd, tb, lut(), a, b, false, acc);
+      const AccBin bin{n, acc_dev_turns(x, dev[k])};
+      if (pv2) acc_bin_p<NDET>(x, bin, tb, lut(), a, b, false, acc);
+      else acc_bin_d<NDET>(x, bin, tb, lut(), a, b, false, acc);
     }
     for (int d = 0; d < NDET; d++)
       for (int j = 0; j < na; j++) sums[d * kAccPerDet + j] += ff_value(acc[d * na + j]);

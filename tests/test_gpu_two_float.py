@@ -189,3 +189,57 @@ def test_fisher_moments(gpu_ctx, T, N, ndet, same, order, eps, mode):
         assert np.max(np.abs(got[i] - ref[i]) / np.outer(s, s)) <= 1e-11, (i, d)
     for h in hs:
         gpu_ctx.release_data(h)
+
+
+@pytest.mark.parametrize("N,ndet,log10F", [(2, 1, False), (255, 2, False), (257, 3, True), (1537, 4, False), (3001, 3, False)])
+@pytest.mark.parametrize("ap", [0, 1])
+def test_nodes(gpu_ctx, oracle, N, ndet, log10F, ap):
+    """Grids that are not uniform: Gauss-Chebyshev nodes in frequency or its logarithm, in any order,
+    reaching beyond the cut, in one batch with a uniform grid; the coarsest and finest node spacing, a
+    source with the cut inside the grid, and one whose phase falls back to FP64."""
+    th = np.pi * (np.arange(N) + 0.5) / N
+    x, w = -np.cos(th), np.pi / N * np.sin(th)
+    lo, hi = (np.log10(12.0), np.log10(1900.0)) if log10F else (12.0, 1900.0)
+    f, w = lo + 0.5 * (hi - lo) * (x + 1), 0.5 * (hi - lo) * w
+    f = 10.0 ** f if log10F else f
+    perm = np.random.default_rng(N).permutation(N)
+    f, w = np.ascontiguousarray(f[perm]), np.ascontiguousarray(w[perm])
+    psd = [W.analytic_psd(f) * (1.0 if ndet == 3 else 1 + 0.3 * i) for i in range(ndet)]
+    rng = np.random.default_rng(3)
+    data = [np.sqrt(4.0 * q) * (rng.standard_normal(N) + 1j * rng.standard_normal(N)) for q in psd]
+    hs = [gpu_ctx.register_data(d, f, data[i], psd[i], weights=w, log10F=log10F) for i, d in enumerate(DETS[:ndet])]
+    T = 16.0
+    _, udata, upsd, uh = _network(gpu_ctx, oracle, 16, 300, ndet)
+    uf = 20.0 + np.arange(300) / 16.0
+    src = W.config1_source()
+    draws = W.prior_draws(6, 40 + N, precessing=bool(ap)) + [src, dict(src, mass1=150.0, mass2=90.0),
+                                                             dict(src, mass1=70.0, mass2=1.2)]
+    p = [oracle.params_from_dict(d) for d in draws]
+    ref = np.array([oracle.loglik_gl(q, f, DETS[:ndet], data, psd, [w] * ndet, log10F=log10F, approximant=ap,
+                                     T_segment=T) for q in p])
+    out, st = gpu_ctx.loglik_batch(G.params_array(draws), ap, hs, T, G.PREC_FP64)
+    assert np.all(st == 0) and _close(out, ref)
+    mix, st = gpu_ctx.loglik_batch(G.params_array(draws + draws), ap, np.array([hs] * len(draws) + [uh] * len(draws)), T,
+                                   G.PREC_FP64)
+    uni, _ = gpu_ctx.loglik_batch(G.params_array(draws), ap, uh, T, G.PREC_FP64)
+    assert np.all(st == 0) and _close(mix[:len(draws)], ref) and _close(mix[len(draws):], uni)
+    for h in hs + uh:
+        gpu_ctx.release_data(h)
+
+
+def test_offset_and_odd_grids(gpu_ctx, oracle):
+    """Simpson's rule on a uniform grid that starts between multiples of its spacing (nodes), and grids
+    that keep the FP64 bins: a zero frequency."""
+    f = 20.03 + np.arange(1500) / 8.0
+    psd, data = W.analytic_psd(f), W.noise(f, 4)
+    draws = W.prior_draws(5, 12)
+    h = gpu_ctx.register_data("Virgo", f, data, psd)
+    ref = np.array([oracle.loglik(oracle.params_from_dict(d), f, ["Virgo"], [data], [psd], T_segment=8.0) for d in draws])
+    out, st = gpu_ctx.loglik_batch(G.params_array(draws), 0, [h], 8.0, G.PREC_FP64)
+    gpu_ctx.release_data(h)
+    assert np.all(st == 0) and _close(out, ref)
+    f = np.concatenate([[0.0], 30.0 + np.sort(np.random.default_rng(1).uniform(0, 100, 99))])
+    h = gpu_ctx.register_data("Virgo", f, np.zeros(100, complex), W.analytic_psd(f + 1), weights=np.ones(100))
+    out, st = gpu_ctx.loglik_batch(G.params_array(draws), 0, [h], 8.0, G.PREC_FP64)
+    gpu_ctx.release_data(h)
+    assert np.all(st == 0) and out.shape == (5,)
