@@ -15,7 +15,7 @@ BUILDDIR = os.path.join(HERE, "_build")
 LIB = os.path.join(LIBDIR, "libgwgpu.so")
 DROPIN_SRC = os.path.join(HERE, "dropin", "gwat_dropin.cpp")
 DROPIN_LIB = os.path.join(LIBDIR, "libgwat_dropin.so")
-SOURCES = ["kernels.cu", "acc.cu", "capi.cu", "batch.cu", "fisher.cu", "fisher_ref.cu", "serve.cu", "noalloc.cu", "maxll.cu", "cufft_rt.cu", "ingest.cu"]
+SOURCES = ["kernels.cu", "acc.cu", "capi.cu", "batch.cu", "fisher.cu", "fisher_ref.cu", "serve.cu", "noalloc.cu", "maxll.cu", "conv.cu", "cufft_rt.cu", "ingest.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # host code: no multiply-add contraction, so that it rounds the same on x86 and Arm hosts
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2,-ffp-contract=off", "--expt-relaxed-constexpr"]

@@ -60,6 +60,7 @@ struct gwgpu_context {
   int last_shape[3] = {0, 0, 0};         // tile, blocks per SM, grid of the last context-stream batch
   bool use_graphs = true;
   int chirp_n = 0;                 // grid length whose Bluestein kernel the kWsChirp workspace holds
+  bool chirp_conv = false;         // conv.cu's tables follow that kernel's FP32 copy
   double chirp_kscale = 0;         // M max|B| of that kernel (the FP32 search's error scale)
   bool maxll_fp64 = false;         // maximised likelihood: FP64 transforms only (no FP32 search)
   bool prologue_serial = false;    // batched prologue: one thread per request instead of the cooperative kernel

@@ -44,6 +44,7 @@
 
 #include "../../include/gwgpu.h"
 #include "capi_internal.h"
+#include "conv.h"
 #include "cufft_rt.h"
 #include "kernels.h"
 
@@ -340,11 +341,12 @@ __global__ void k_mx_prep(const Request *__restrict__ req, const double2 *__rest
 }
 
 // k_mx_prep for the intrinsic mode on uniform grids: the waveform and the products
-// in two floats (g as pairs), a tile of kPrepTile bins per block.
+// in two floats (g as pairs), a tile of kPrepTile bins per block; a32's rows are
+// padded with zeros up to pad.
 // Bound by memory: per pair and bin 16 B of data read and 16 + 8 B written (the
 // padding of a Bluestein row another 8 B per entry).  128 IMRPhenomD requests on
-// 3 x 32,128 bins: 1,480 -> 131 us against the FP64 bins; bins beyond a
-// request's cut only write their zeros (242 -> 131 us).
+// 3 x 32,128 bins: 1,480 -> 103 us against the FP64 bins; bins beyond a
+// request's cut only write their zeros (242 -> 131 us), the padding none.
 constexpr int kPrepTile = 2048;
 // Bins of the grid below the model's cut (0 for a request outside its domain).
 __device__ __forceinline__ int live_bins(const gwt::AccReq &x, int n0, int N) {
@@ -354,8 +356,9 @@ template <bool UN>
 __global__ void __launch_bounds__(kBlock, UN ? 1 : 3) k_mx_prep_ff(const gwt::AccReq *__restrict__ areq, int ndet,
                                                        const StreamDev *__restrict__ streams,
                                                        const int *__restrict__ handles, const gwt::AccTables tb,
-                                                       const gwt::AccLut *__restrict__ glut, int N, int ld, int blue,
-                                                       const float2 *__restrict__ chirp_tab, gwt::ff4 *__restrict__ g,
+                                                       const gwt::AccLut *__restrict__ glut, int N, int ld, int pad,
+                                                       int blue, const float2 *__restrict__ chirp_tab,
+                                                       gwt::ff4 *__restrict__ g,
                                                        float2 *__restrict__ a32, double *__restrict__ part) {
   using namespace gwt;
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1;
@@ -366,7 +369,7 @@ __global__ void __launch_bounds__(kBlock, UN ? 1 : 3) k_mx_prep_ff(const gwt::Ac
   __shared__ double s_hs[kMaxDet], s_red[kMaxDet * NS][kWarps];
   const int r = blockIdx.y, tid = threadIdx.x;
   const AccReq &x = *(const AccReq *)s_req;
-  const int k0 = blockIdx.x * kPrepTile, k1 = min(k0 + kPrepTile, ld);
+  const int k0 = blockIdx.x * kPrepTile, k1 = min(k0 + kPrepTile, pad);
   if (tid < ndet) s_st[tid] = streams[handles[(size_t)r * ndet + tid]];
   __syncthreads();
   // bins below the model's cut; g is neither written nor read beyond them
@@ -963,16 +966,23 @@ int xform_len(int N, int *blue) {
 }
 
 // The Bluestein kernel for N, FFT_M(b)/M in FP64 (kWsChirp) and FP32
-// (kWsChirp32), and the search's error scale M max|B|, kept until N changes.
-int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const float2 **B32, const float2 **tab) {
+// (kWsChirp32), and the search's error scale M max|B|, kept until N changes; in
+// FP32 also the chirp, and conv.cu's tables (*conv; null where it has no kernels
+// for M or there is no memory for them).
+int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const float2 **B32, const float2 **tab,
+                 void **conv = nullptr) {
   void *kb, *kb32;
+  const size_t b32 = up256(8 * ((size_t)M + N)), bconv = gwk::conv_table_bytes(M);
   int st = c->workspace(gwgpu_context::kWsChirp, 16 * (size_t)M + 256, &kb);
   if (st) return st;
-  if ((st = c->workspace(gwgpu_context::kWsChirp32, 8 * ((size_t)M + N), &kb32))) return st;
+  if (c->chirp_n != N) c->chirp_conv = bconv && c->workspace(gwgpu_context::kWsChirp32, b32 + bconv, &kb32) == GWGPU_OK;
+  if ((st = c->workspace(gwgpu_context::kWsChirp32, b32 + (c->chirp_conv ? bconv : 0), &kb32))) return st;
   *B64 = (const double2 *)kb;
   *B32 = (const float2 *)kb32;
   *tab = *B32 + M;
+  if (conv) *conv = c->chirp_conv ? (char *)kb32 + b32 : nullptr;
   if (c->chirp_n == N) return GWGPU_OK;
+  c->chirp_n = 0;
   int p1;
   if ((st = gwfft::plan(c, gwfft::kZ2Z, M, 1, &p1))) return st;
   const int gb = std::min((M + kBlock - 1) / kBlock, 1024);
@@ -982,6 +992,7 @@ int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const floa
   k_absmax<<<1, kBlock, 0, c->stream>>>((const double2 *)kb, M, dmax);
   k_to_f32<<<gb, kBlock, 0, c->stream>>>((const double2 *)kb, (float2 *)kb32, M);
   k_chirp_tab<<<gb, kBlock, 0, c->stream>>>((float2 *)kb32 + M, N);
+  if (c->chirp_conv) gwk::launch_conv_tables((const float2 *)kb32, M, (char *)kb32 + b32, c->stream);
   double bmax = 0;
   cudaMemcpyAsync(&bmax, dmax, 8, cudaMemcpyDeviceToHost, c->stream);
   cudaError_t e = cudaStreamSynchronize(c->stream);
@@ -1051,10 +1062,10 @@ int run_fp64(gwgpu_context *c, const MxIn &in, double *out, int *status) {
 
 // The FP32 search and its refinement; *fallback set when a pair had more
 // candidates than kCand (nothing written to out then).  128 IMRPhenomD requests
-// on 3 x 32,128 bins, device time by kernel: products 131, transforms and chirp
-// 434, candidates 56 (132 with its FP64 sums on every warp), screen 45 and
+// on 3 x 32,128 bins, device time by kernel: products 103, transforms and chirp
+// 209 (conv.cu; 434 with library transforms), candidates 56 (132 with its FP64 sums on every warp), screen 45 and
 // two-float refinement 71 (389 for FP64 sums of every candidate over the whole
-// row), result 9 us; the transforms' memory traffic is the largest part left.
+// row), result 10 us.
 int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *fallback) {
   const int np = in.un ? 2 : 1, ns = in.un ? 5 : 2, pairs = in.n * in.ndet, rows = pairs * np;
   *fallback = false;
@@ -1064,14 +1075,15 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   const float2 *B32 = nullptr, *ctab = nullptr;
   double kscale = std::sqrt((double)in.N);
   int st = GWGPU_OK;
+  void *conv = nullptr;
   if (blue) {
-    if ((st = ensure_chirp(c, in.N, ld, &B64, &B32, &ctab))) return st;
+    if ((st = ensure_chirp(c, in.N, ld, &B64, &B32, &ctab, &conv))) return st;
     kscale = c->chirp_kscale;
   }
-  int plan;  // fetched last: a new plan may reset the cache (cufft_rt.cu)
-  if ((st = gwfft::plan(c, gwfft::kC2C, ld, rows, &plan))) return st;
+  int plan = 0;  // fetched last: a new plan may reset the cache (cufft_rt.cu)
+  if (!conv && (st = gwfft::plan(c, gwfft::kC2C, ld, rows, &plan))) return st;
   const bool two = in.areq != nullptr;  // two-float bins
-  const int per = two ? kPrepTile : kBlock, nblk = (ld + per - 1) / per;
+  const int pad = conv ? in.N : ld, per = two ? kPrepTile : kBlock, nblk = (pad + per - 1) / per;
   const size_t o_g = 0, o_a = up256(16 * (size_t)rows * in.N), o_h = o_a + up256(8 * (size_t)rows * ld),
                o_s = o_h + up256(8 * (size_t)pairs * ns * nblk), o_c = o_s + up256(8 * (size_t)pairs * ns),
                o_nc = o_c + up256(4 * (size_t)pairs * kCand), o_v = o_nc + up256(4 * (size_t)pairs),
@@ -1087,18 +1099,23 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   const dim3 grid(nblk, in.n);
   if (two && in.un)
     k_mx_prep_ff<true><<<grid, kBlock, 0, c->stream>>>(in.areq, in.ndet, in.streams, in.handles, c->acc, c->acc_lut,
-                                                        in.N, ld, blue, ctab, (gwt::ff4 *)g64, a32, hh);
+                                                        in.N, ld, pad, blue, ctab, (gwt::ff4 *)g64, a32, hh);
   else if (two)
     k_mx_prep_ff<false><<<grid, kBlock, 0, c->stream>>>(in.areq, in.ndet, in.streams, in.handles, c->acc, c->acc_lut,
-                                                         in.N, ld, blue, ctab, (gwt::ff4 *)g64, a32, hh);
+                                                         in.N, ld, pad, blue, ctab, (gwt::ff4 *)g64, a32, hh);
   else if (in.un)
     k_mx_prep<true><<<grid, kBlock, 0, c->stream>>>(in.req, in.rp, in.rc, in.ndet, in.streams, in.handles, in.N, ld,
                                                      blue, g64, a32, hh);
   else
     k_mx_prep<false><<<grid, kBlock, 0, c->stream>>>(in.req, in.rp, in.rc, in.ndet, in.streams, in.handles, in.N, ld,
                                                       blue, g64, a32, hh);
-  if ((st = gwfft::exec_c2c(c, plan, a32, a32, gwfft::kForward, c->stream))) return st;
-  if (blue) {
+  if (conv) {
+    cudaError_t ce = gwk::launch_conv(a32, rows, in.N, ld, gwk::conv_tables_at(conv, ld), c->stream);
+    if (ce != cudaSuccess) return c->fail(ce, "maximised likelihood transform");
+  } else if ((st = gwfft::exec_c2c(c, plan, a32, a32, gwfft::kForward, c->stream))) {
+    return st;
+  }
+  if (blue && !conv) {
     const long long tot = (long long)rows * ld;
     const int gb = (int)std::min<long long>((tot + kBlock - 1) / kBlock, 152 * 16);
     k_chirp_mul32<<<gb, kBlock, 0, c->stream>>>(a32, B32, ld, tot);

@@ -243,3 +243,21 @@ def test_offset_and_odd_grids(gpu_ctx, oracle):
     out, st = gpu_ctx.loglik_batch(G.params_array(draws), 0, [h], 8.0, G.PREC_FP64)
     gpu_ctx.release_data(h)
     assert np.all(st == 0) and out.shape == (5,)
+
+
+@pytest.mark.parametrize("N", [4099, 8191, 8209, 16411, 32771, 65537, 131101])
+@pytest.mark.parametrize("ap", [0, 1])
+def test_maximized_transform_lengths(gpu_ctx, oracle, N, ap):
+    """Every padded length of the row convolution (2^14 .. 2^18, and one on each side), the grid mostly
+    just beyond a power of two: the maximum over the lags against the oracle's FP64 transform."""
+    T = max(4, N // 1500)
+    f = 20.0 + np.arange(N) / T
+    psd = W.analytic_psd(f)
+    data = [W.noise(f, 6 + i) for i in range(2)]
+    hs = [gpu_ctx.register_data(d, f, data[i], psd) for i, d in enumerate(DETS[:2])]
+    draws = W.prior_draws(3, N, precessing=bool(ap))
+    ref = np.array([oracle.maximized_loglik_intrinsic(d, f, data, [psd] * 2, approximant=ap) for d in draws])
+    out, st = gpu_ctx.maximized_loglik_batch(G.params_array(draws), hs, ap)
+    for h in hs:
+        gpu_ctx.release_data(h)
+    assert np.all(st == 0) and _close(out, ref)
