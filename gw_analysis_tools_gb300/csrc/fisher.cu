@@ -50,24 +50,42 @@ __global__ void k_fisher_slots(const GenParams *__restrict__ params, int nsrc, i
   fisher_slot(params[g / kSlots], g % kSlots, method, dets, ndet, df, epsilon, step_mode, qnm, out[g]);
 }
 
-// One warp per source: lane 0 the head, a lane per waveform pair, then a lane
-// per extrinsic row, and with FF the pairs' two-float coefficients.  Bound by
-// the latency of one lane's chain (11 perturbed parameters, the pairs' two-float
-// coefficients); 256 sources x 3 detectors 68 us, one thread per source 292.
+// One warp per source: a lane per divisor, eight per waveform pair, then a lane
+// per extrinsic row, and with FF the pairs' two-float coefficients the same way.
+// Bound by the latency of a lane's FP64 chain; 256 sources x 3 detectors: 63
+// us, one thread per source 292.
 template <bool FF>
 __global__ void __launch_bounds__(32) k_fisher_setup(const GenParams *__restrict__ params, int method, int ndet,
                                                      double epsilon, int step_mode, int order,
                                                      const SlotOut *__restrict__ slots, FisherSrc *out, FfSrc *ffout,
                                                      int *status) {
   const int src = blockIdx.x, lane = threadIdx.x;
+  const unsigned all = 0xffffffffu;
   const SlotOut *S = slots + (size_t)src * kSlots;
   FisherSrc &F = out[src];
+  // the waveforms: centre, + and - of the four pairs
+  constexpr int kW = sizeof(WaveF64) / 4;
+  static_assert(sizeof(WaveF64) % 4 == 0, "copied as words");
+#pragma unroll
+  for (int j = 0; j < 1 + 2 * kIntr; j++) {
+    const unsigned *x = (const unsigned *)&S[j ? 14 + j : 0].w;
+    unsigned *y = (unsigned *)(j == 0 ? &F.w0 : j & 1 ? &F.wp[j / 2] : &F.wm[j / 2 - 1]);
+    for (int w = lane; w < kW; w += 32) y[w] = x[w];
+  }
+  const bool slot = lane < kSlots;
+  const int st = (int)__reduce_or_sync(all, slot ? (unsigned)S[lane].status : 0u);
+  const int cut = __reduce_max_sync(all, slot ? S[lane].w.n_cut : S[0].w.n_cut);
   if (lane == 0) {
-    fisher_setup_head(params[src], method, epsilon, step_mode, S, F);
-    status[src] = F.status;
+    fisher_unpack(params[src], method, F.v, F.logf);
+    F.status = status[src] = st;
+    F.n_cut_any = cut;
   }
   __syncwarp();
-  if (lane < kIntr) fisher_setup_pair(S, lane, F);
+  if (lane < kDim) fisher_setup_div(epsilon, step_mode, lane, F);
+  __syncwarp();
+  if (lane < kIntr) fisher_setup_rule(epsilon, step_mode, lane, F);
+  __syncwarp();
+  fisher_setup_pair(F.w0.A_scale, lane / 8, F, lane % 8, 8);
   for (int j = lane; j < ndet * (kCheap + 1); j += 32) {
     const int d = j / (kCheap + 1), i = j % (kCheap + 1);
     if (i < kCheap) fisher_setup_row(S, order, d, i, F);
@@ -77,10 +95,9 @@ __global__ void __launch_bounds__(32) k_fisher_setup(const GenParams *__restrict
   if (lane == 0) fisher_setup_route(order, F);
   if constexpr (FF) {
     FfSrc &X = ffout[src];
-    bool ok = true;
-    if (lane < kIntr) ok = ff_pair(F, lane, X.q[lane]);
-    else if (lane == kIntr) ok = ff_centre(F, X);
-    ok = __all_sync(0xffffffffu, ok);
+    bool ok = ff_pair(F, lane / 8, X.q[lane / 8], lane % 8, 8);
+    if (lane == 1) ok = ff_centre(F, X) && ok;
+    ok = __all_sync(all, ok);
     if (lane == 0) X.ok = ok;
   }
 }
@@ -265,11 +282,12 @@ __device__ __noinline__ double2 pair_fp64(const FisherSrc *F, int q, int n, doub
 // up goes through one transposed warp sum and FP64.
 // FP64 bins occupy the FP64 pipe for 64 cycles an instruction; here a bin is
 // ~1,900 FP32 instructions (the differences of four pairs ~1,100, products and
-// sums ~500), bound by their issue: 256 sources on 32,128 bins 5740 -> 745 us.
+// sums ~500), bound by their issue: 256 sources on 32,128 bins 5740 -> 560 us
+// (745 with the four pairs' code unrolled at three blocks an SM).
 // Where the inverse is wanted too the sums stay FP64: it magnifies them by the
 // matrix's condition number.
 constexpr int kFfTile = 2048;
-__global__ void __launch_bounds__(kBlock, 3) k_fisher_ff(const __grid_constant__ FisherArgs a) {
+__global__ void __launch_bounds__(kBlock, 4) k_fisher_ff(const __grid_constant__ FisherArgs a) {
   __shared__ int s_item, s_last;
   __shared__ FfSrc S;
   __shared__ gwt::AccLut lut;
@@ -308,19 +326,20 @@ __global__ void __launch_bounds__(kBlock, 3) k_fisher_ff(const __grid_constant__
         const FfBin b = ff_bin(a.acc, n);
         const ff a0 = ff_amp0(S, n, b, lut);
         ff qr[kIntr], qi[kIntr];
-        unsigned left = 0;
-#pragma unroll
-        for (int q = 0; q < kIntr; q++)
-          if (!ff_pair_q(S.q[q], S.n_mid, n, b, lut, a0, qr[q], qi[q])) left |= 1u << q;
-        while (left) {
-          const int q = __ffs(left) - 1;
-          left &= left - 1;
-          const double2 v = pair_fp64(&F, q, n, a.tab.t13[n], a.tab.tm53[n], a.tab.tln[n], a.tab.t34[n], a.tm76d[n]);
+        // one copy of the pair's code: four of them exceed the instruction cache
+#pragma unroll 1
+        for (int q = 0; q < kIntr; q++) {
+          ff vr, vi;
+          if (!ff_pair_q(S.q[q], S.n_mid, n, b, lut, a0, vr, vi)) {
+            const double2 v = pair_fp64(&F, q, n, a.tab.t13[n], a.tab.tm53[n], a.tab.tln[n], a.tab.t34[n], a.tm76d[n]);
+            vr = ff_split(v.x);
+            vi = ff_split(v.y);
+          }
 #pragma unroll
           for (int j = 0; j < kIntr; j++)
             if (j == q) {
-              qr[j] = ff_split(v.x);
-              qi[j] = ff_split(v.y);
+              qr[j] = vr;
+              qi[j] = vi;
             }
         }
         ff_accumulate(a.wf[w][k], a0, b.n, qr, qi, acc);

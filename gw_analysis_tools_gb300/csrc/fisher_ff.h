@@ -81,10 +81,16 @@ GW_HD bool ff_centre(const FisherSrc &F, FfSrc &S) {
   ok &= ff_set_pos(S.rd, w.nrd);
   return ok && w.n_mid > -16777216 && w.n_mid < 16777216;
 }
-GW_HD bool ff_pair(const FisherSrc &F, int q, FfPair &P) {
+// Of step threads part takes every step-th of the series, the first the rest.
+GW_HD bool ff_pair(const FisherSrc &F, int q, FfPair &P, int part, int step) {
   const WaveF64 &p = F.wp[q], &m = F.wm[q];
   const WaveDiff &d = F.wd[q];
   const double inv = F.idiv[q], div = F.div[7 + q];
+  bool ok = true;
+  for (int j = part; j < 12; j += step) ok &= ff_set(P.qi[j], j == 5 ? d.qi[5] - d.phic : d.qi[j]);
+  for (int j = part; j < 10; j += step) ok &= ff_set(P.ai[j], d.ai[j]);
+  for (int j = part; j < 5; j += step) ok &= ff_set(P.ei[j], d.ei[j]);
+  if (part) return ok;
   P.n_cut = imin(imin(p.n_cut, m.n_cut), F.w0.n_cut);
   P.slow = F.exact[q] || F.onesided[q];
   P.a1 = imin(p.n_f1, m.n_f1);
@@ -96,8 +102,7 @@ GW_HD bool ff_pair(const FisherSrc &F, int q, FfPair &P) {
   P.b3 = imin(p.n_f2p, m.n_f2p);
   P.b4 = imax(p.n_f2p, m.n_f2p);
   P.div = (float)div;
-  bool ok = ff_set(P.hdiv, 0.5 * div);
-  for (int j = 0; j < 12; j++) ok &= ff_set(P.qi[j], j == 5 ? d.qi[5] - d.phic : d.qi[j]);
+  ok &= ff_set(P.hdiv, 0.5 * div);
   ok &= ff_set(P.bi0, d.bi0);
   ok &= ff_set(P.bi1, d.bi1);
   ok &= ff_set(P.pA, d.pA - d.phic);
@@ -108,8 +113,6 @@ GW_HD bool ff_pair(const FisherSrc &F, int q, FfPair &P) {
   ok &= ff_set(P.mB, d.mB);
   ok &= ff_set(P.mC, -d.mC);
   ok &= ff_set(P.mD, d.mD);
-  for (int j = 0; j < 10; j++) ok &= ff_set(P.ai[j], d.ai[j]);
-  for (int j = 0; j < 5; j++) ok &= ff_set(P.ei[j], d.ei[j]);
   ok &= ff_set(P.K, m.mrK * F.sm[q]);
   ok &= ff_set(P.ex, m.mrExp);
   ok &= ff_set(P.gm, m.mrG2);

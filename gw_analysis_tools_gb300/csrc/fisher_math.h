@@ -149,9 +149,19 @@ GW_HD void recentre_ei(const WaveF64 &x, int H, double *e) {
     e[k] = acc;
   }
 }
-// The differences, times inv = 1 / (the difference's divisor).
-GW_HD void wave_diff(const WaveF64 &p, const WaveF64 &m, double sp, double sm, int H, double inv, WaveDiff &d) {
-  for (int j = 0; j < 12; j++) d.qi[j] = (p.qi[j] - m.qi[j]) * inv;
+// The differences, times inv = 1 / (the difference's divisor).  Of step threads
+// part takes every step-th of the series and its share of the rest.
+GW_HD void wave_diff(const WaveF64 &p, const WaveF64 &m, double sp, double sm, int H, double inv, WaveDiff &d,
+                     int part = 0, int step = 1) {
+  for (int j = part; j < 12; j += step) d.qi[j] = (p.qi[j] - m.qi[j]) * inv;
+  for (int j = part; j < 10; j += step) d.ai[j] = (p.ai[j] * sp - m.ai[j] * sm) * inv;
+  if (part == step - 1) {
+    double ep[5], em[5];
+    recentre_ei(p, H, ep);
+    recentre_ei(m, H, em);
+    for (int j = 0; j < 5; j++) d.ei[j] = (ep[j] * sp - em[j] * sm) * inv;
+  }
+  if (part) return;
   d.bi0 = (p.bi0 - m.bi0) * inv;
   d.bi1 = (p.bi1 - m.bi1) * inv;
   d.pA = (p.pA - m.pA) * inv;
@@ -165,49 +175,33 @@ GW_HD void wave_diff(const WaveF64 &p, const WaveF64 &m, double sp, double sm, i
   d.phic = (p.phic - m.phic) * inv;
   d.yw = (p.inv_nw - m.inv_nw) * inv;
   d.yc = -p.nc * d.yw - (p.nc - m.nc) * inv * m.inv_nw;
-  for (int j = 0; j < 10; j++) d.ai[j] = (p.ai[j] * sp - m.ai[j] * sm) * inv;
-  double ep[5], em[5];
-  recentre_ei(p, H, ep);
-  recentre_ei(m, H, em);
-  for (int j = 0; j < 5; j++) d.ei[j] = (ep[j] * sp - em[j] * sm) * inv;
 }
 
-// The set-up in parts that separate threads can take: the parameters and
-// divisors, a waveform pair, an extrinsic parameter of a detector, a detector's
-// own projection, and what the source is left to.
-GW_HD void fisher_setup_head(const GenParams &in, int method, double epsilon, int step_mode, const SlotOut *S,
-                             FisherSrc &F) {
-  fisher_unpack(in, method, F.v, F.logf);
-  int st = 0;
-  for (int s = 0; s < kSlots; s++) st |= S[s].status;
-  for (int i = 0; i < kDim; i++) {
-    double eps = fisher_step(F.v, i, epsilon, step_mode);
-    double tmp[kDim];
-    F.div[i] = fisher_perturb(F.v, i, 1, eps, tmp);
-  }
-  for (int q = 0; q < kIntr; q++) {
-    F.idiv[q] = 1.0 / F.div[7 + q];
-    F.onesided[q] = F.div[7 + q] == fisher_step(F.v, 7 + q, epsilon, step_mode);
-    // The waveform depends on eta through sqrt(1 - 4 eta) (the component
-    // masses): within a few thousand steps of eta = 1/4 the pair's mean phase
-    // and amplitude offsets are no longer second order in the step, and the
-    // difference is taken waveform by waveform.
-    F.exact[q] = q == 1 && (0.25 - F.v[8]) < 1000.0 * F.div[8];
-  }
-  F.status = st;
-  F.w0 = S[0].w;
-  F.n_cut_any = F.w0.n_cut;
-  for (int s = 1; s < kSlots; s++) F.n_cut_any = F.n_cut_any > S[s].w.n_cut ? F.n_cut_any : S[s].w.n_cut;
+// The set-up in parts that separate threads can take: a parameter's divisor, a
+// waveform pair's rule and its differences (after the copies of its waveforms),
+// an extrinsic parameter of a detector, a detector's own projection, and what the
+// source is left to.
+GW_HD void fisher_setup_div(double epsilon, int step_mode, int i, FisherSrc &F) {
+  double tmp[kDim];
+  F.div[i] = fisher_perturb(F.v, i, 1, fisher_step(F.v, i, epsilon, step_mode), tmp);
 }
-GW_HD void fisher_setup_pair(const SlotOut *S, int k, FisherSrc &F) {
-  const double A0 = S[0].w.A_scale;
-  int i = 7 + k;
-  F.wp[k] = S[1 + 2 * i].w;
-  F.wm[k] = S[2 + 2 * i].w;
-  F.sp[k] = F.wp[k].A_scale / A0;
-  F.sm[k] = F.wm[k].A_scale / A0;
-  F.amp_lk[k] = log((F.wp[k].mrK * F.sp[k]) / (F.wm[k].mrK * F.sm[k]));
-  wave_diff(F.wp[k], F.wm[k], F.sp[k], F.sm[k], F.w0.n_mid, F.idiv[k], F.wd[k]);
+GW_HD void fisher_setup_rule(double epsilon, int step_mode, int q, FisherSrc &F) {
+  F.idiv[q] = 1.0 / F.div[7 + q];
+  F.onesided[q] = F.div[7 + q] == fisher_step(F.v, 7 + q, epsilon, step_mode);
+  // The waveform depends on eta through sqrt(1 - 4 eta) (the component
+  // masses): within a few thousand steps of eta = 1/4 the pair's mean phase
+  // and amplitude offsets are no longer second order in the step, and the
+  // difference is taken waveform by waveform.
+  F.exact[q] = q == 1 && (0.25 - F.v[8]) < 1000.0 * F.div[8];
+}
+GW_HD void fisher_setup_pair(double A0, int k, FisherSrc &F, int part = 0, int step = 1) {
+  const double sp = F.wp[k].A_scale / A0, sm = F.wm[k].A_scale / A0;
+  if (part == 0) {
+    F.sp[k] = sp;
+    F.sm[k] = sm;
+    F.amp_lk[k] = log((F.wp[k].mrK * sp) / (F.wm[k].mrK * sm));
+  }
+  wave_diff(F.wp[k], F.wm[k], sp, sm, F.w0.n_mid, F.idiv[k], F.wd[k], part, step);
 }
 GW_HD void fisher_setup_row(const SlotOut *S, int order, int d, int i, FisherSrc &F) {
   const double A0 = S[0].w.A_scale, g0r = S[0].Gre[d], g0i = S[0].Gim[d];
@@ -296,8 +290,21 @@ GW_HD void fisher_setup_route(int order, FisherSrc &F) {
 }
 GW_HDNI int fisher_setup(const GenParams &in, int method, int ndet, double epsilon, int step_mode, int order,
                          const SlotOut *S, FisherSrc &F) {
-  fisher_setup_head(in, method, epsilon, step_mode, S, F);
-  for (int k = 0; k < kIntr; k++) fisher_setup_pair(S, k, F);
+  fisher_unpack(in, method, F.v, F.logf);
+  F.status = 0;
+  F.w0 = S[0].w;
+  F.n_cut_any = F.w0.n_cut;
+  for (int s = 0; s < kSlots; s++) {
+    F.status |= S[s].status;
+    F.n_cut_any = F.n_cut_any > S[s].w.n_cut ? F.n_cut_any : S[s].w.n_cut;
+  }
+  for (int i = 0; i < kDim; i++) fisher_setup_div(epsilon, step_mode, i, F);
+  for (int k = 0; k < kIntr; k++) {
+    F.wp[k] = S[15 + 2 * k].w;
+    F.wm[k] = S[16 + 2 * k].w;
+    fisher_setup_rule(epsilon, step_mode, k, F);
+    fisher_setup_pair(S[0].w.A_scale, k, F);
+  }
   for (int d = 0; d < ndet; d++) {
     for (int i = 0; i < kCheap; i++) fisher_setup_row(S, order, d, i, F);
     fisher_setup_det(S, order, d, F);
