@@ -20,8 +20,11 @@
 // Work layout: a set-up kernel builds the model constants of every perturbed
 // parameter set (one thread per source, parameter and step); the main kernel
 // is persistent over (source, bin tile) items; each thread evaluates one bin's
-// 2 or 4 perturbed waveforms per parameter, writes that bin's derivatives to
-// shared memory, and then the block's first 66 threads each accumulate one
+// perturbed waveforms (the model once for the 14 or 28 steps of the extrinsic
+// parameters, and for each of the 8 or 16 others; bound by the FP64 pipe, one
+// source on 3 x 32,608 bins at order 4 from 850 to 500 us by it, with the
+// rotations by arrival times that a step leaves alone kept over the steps),
+// writes that bin's derivatives to shared memory, and then the block's first 66 threads each accumulate one
 // Gram pair over the block's bins.  The last tile of a source sums the tiles'
 // partials in a fixed order (the same result every run).
 #include <cuda_runtime.h>
@@ -125,6 +128,18 @@ __global__ void __launch_bounds__(kRefBlock) k_fref_main(const RefArgs a) {
       const double f = live ? a.freqs[kb] : 0.0;
       for (int d = 0; d < a.ndet; d++)
         wsm[d * kRefBlock + tid] = live ? simpson_weight(kb, a.N) / a.psd[d][kb] : 0.0;
+      // the steps of the extrinsic parameters share the model's amplitude and
+      // phase, and those that leave the distance, t_c and phi_ref the waveform
+      double ma = 0.0, mph = 0.0, la = 0.0, lt = 0.0, lp = 0.0;
+      cd h{0., 0.};
+      bool have = false;
+      // ... and the rotations by a detector's arrival time where it stays: at
+      // +-eps (e^{i tau f}) and at +-2 eps (e^{i tau (f - f_ref)})
+      double rt[2][kMaxDet];
+      cd rot[2][kMaxDet];
+#pragma unroll
+      for (int d = 0; d < kMaxDet; d++) rt[0][d] = rt[1][d] = 0.0;
+      if (live && f <= R[0].m.fcut) d_bin_model(R[0].m, f, ma, mph);
       for (int i = 0; i < kDim; i++) {
         cd sum[kMaxDet];
         for (int d = 0; d < kMaxDet; d++) sum[d] = cd{0., 0.};
@@ -132,15 +147,33 @@ __global__ void __launch_bounds__(kRefBlock) k_fref_main(const RefArgs a) {
           for (int s = 0; s < a.nk; s++) {
             const Request &r = R[i * a.nk + s];
             cd hp, hc;
-            wave_bin(r, f, hp, hc);
+            if (i >= kCheap) {
+              wave_bin(r, f, hp, hc);
+            } else if (f > r.m.fcut) {
+              hp = hc = cd{0., 0.};
+            } else {
+              if (!have || r.m.A0eff != la || r.m.tcl != lt || r.m.phic != lp) h = d_bin_wave(r.m, f, ma, mph);
+              have = true;
+              la = r.m.A0eff;
+              lt = r.m.tcl;
+              lp = r.m.phic;
+              d_bin_pol(r.m, h, hp, hc);
+            }
             const double w = fdw[s];
-            for (int d = 0; d < a.ndet; d++) {
+#pragma unroll
+            for (int d = 0; d < kMaxDet; d++) {
+              if (d >= a.ndet) break;
               cd x = response_bin(r.det[d], hp, hc, f, false);
               const double tau = r.det[d].tau;
               if (tau != 0.0) {  // a detector other than the reference one
-                double sn, cs;
-                sincos(s < 2 ? tau * f : tau * (f - r.m.fref), &sn, &cs);
-                x = cmul(x, cd{cs, sn});
+                const bool near = s < 2;
+                if (tau != (near ? rt[0][d] : rt[1][d])) {
+                  cd e;
+                  sincos(near ? tau * f : tau * (f - r.m.fref), &e.im, &e.re);
+                  if (near) rt[0][d] = tau, rot[0][d] = e;
+                  else rt[1][d] = tau, rot[1][d] = e;
+                }
+                x = cmul(x, near ? rot[0][d] : rot[1][d]);
               }
               sum[d].re += w * x.re;
               sum[d].im += w * x.im;
@@ -254,9 +287,9 @@ int gwf_ref_run(gwgpu_context *c, const GenParams *params, int n, int method, in
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fref_main, kRefBlock, smem);
   // Bins per item: 2,048 where the sources alone fill the chip.  A pass of 128
-  // bins takes 0.7 ms (44 waveforms a bin at order 4), so the one or two sources
-  // that the moment form leaves here (a cut between the steps) take an item per
-  // pass: one source on 32,608 bins 11 -> 1.5 ms
+  // bins takes 0.25 ms, so the one or two sources that the moment form leaves here
+  // (a cut between the steps, eta near 1/4) take an item per pass: one source on
+  // 32,608 bins 4 -> 0.5 ms
   const long long slots = (long long)nsm * std::max(per_sm, 1);
   long long tile_l = ((long long)N * chunk / (2 * slots) + kRefBlock - 1) / kRefBlock * kRefBlock;
   const int tile = (int)std::min(2048LL, std::max((long long)kRefBlock, tile_l)), ntiles = (N + tile - 1) / tile;

@@ -41,13 +41,9 @@ GW_HD double build_phase_bin(double f, const ModelD &m, const Pows &p) {
   return phase_int(f, s, m.l);
 }
 
-// IMRPhenomD: h+ and hx at one frequency.
-GW_HD void d_bin(const ModelD &m, double f, cd &hp, cd &hc) {
-  if (f > m.fcut) {
-    hp = cd{0., 0.};
-    hc = cd{0., 0.};
-    return;
-  }
+// IMRPhenomD, the part that the masses and spins fix: the amplitude / A0eff and
+// the phase without its linear terms, at f <= m.fcut.
+GW_HD void d_bin_model(const ModelD &m, double f, double &a, double &phase) {
   double M = m.s.M;
   Pows p;
   if (f < m.s.f1_phase) {
@@ -56,16 +52,33 @@ GW_HD void d_bin(const ModelD &m, double f, cd &hp, cd &hc) {
     p.MFsixth = sqrt(cbrt(M * f));
     p.MF7sixth = pow_int(p.MFsixth, 7);
   }
-  double amp = (m.A0eff * build_amp(f, m, p));
-  double phase = build_phase_bin(f, m, p);
+  a = build_amp(f, m, p);
+  phase = build_phase_bin(f, m, p);
+}
+// e^{-i phase} of it.
+GW_HD cd d_bin_wave(const ModelD &m, double f, double a, double phase) {
+  const double amp = m.A0eff * a;
   phase -= (m.tcl * (f - m.fref) + m.phic);
   double sn, cs;
   sincos(phase, &sn, &cs);
-  cd h{amp * cs, -(amp * sn)};
+  return cd{amp * cs, -(amp * sn)};
+}
+GW_HD void d_bin_pol(const ModelD &m, cd h, cd &hp, cd &hc) {
   const double ci = m.s.cos_incl;
   hc = cd{h.im * ci, -h.re * ci};  // (-i h) cos(iota)
   const double fac = m.s.fac_incl;
   hp = cd{h.re * fac, h.im * fac};
+}
+// IMRPhenomD: h+ and hx at one frequency.
+GW_HD void d_bin(const ModelD &m, double f, cd &hp, cd &hc) {
+  if (f > m.fcut) {
+    hp = cd{0., 0.};
+    hc = cd{0., 0.};
+    return;
+  }
+  double a, phase;
+  d_bin_model(m, f, a, phase);
+  d_bin_pol(m, d_bin_wave(m, f, a, phase), hp, hc);
 }
 
 // Twist-up factors (IMRPhenomP.cpp:696-715) with the harmonics real (phi = 0).
