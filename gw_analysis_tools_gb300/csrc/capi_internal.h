@@ -27,7 +27,7 @@ struct gwgpu_context {
   };
   enum { kWsWave = 0, kWsInner, kWsPlain, kWsBatch, kWsBatchItems, kWsFisher, kWsServe, kWsMaxll, kWsIngest, kWsChirp, kWsChirp32, kWsMaxllRun,
          kWsFisherRef = 40 };
-  enum { kHwsPlain = 0, kHwsBatch, kHwsFisher, kHwsInner };
+  enum { kHwsPlain = 0, kHwsBatch, kHwsFisher, kHwsInner, kHwsMaxll };
 
   int device = 0;
   size_t budget = 0, in_use = 0;

@@ -525,9 +525,12 @@ __global__ void __launch_bounds__(kCandBlock) k_mx_cand(const float2 *__restrict
       }
     }
   }
-  __syncthreads();
-  // score and bound of bin k
-  const float ap = s_scale[0], ac = s_scale[1], I = s_scale[2], eps = s_scale[3], inv1mI = s_scale[4], E = s_scale[0];
+  // score and bound of bin k; the aligned form's bound is the same at every bin and
+  // joins after the scan, which then does not wait for the sums
+  if (UN) __syncthreads();
+  const float ap = UN ? s_scale[0] : 0.f, ac = UN ? s_scale[1] : 0.f, I = UN ? s_scale[2] : 0.f,
+              eps = UN ? s_scale[3] : 0.f, inv1mI = UN ? s_scale[4] : 0.f;
+  float E = 0.f;
   auto score = [&](int k, float &lo, float &hi) {
     if (!UN) {
       const float2 v = C[(size_t)q * ld + k];
@@ -559,6 +562,11 @@ __global__ void __launch_bounds__(kCandBlock) k_mx_cand(const float2 *__restrict
     nan = nan || hi != hi;
   }
   L = block_max(L, s_tmpf);
+  if (!UN) {
+    E = s_scale[0];
+    L -= E;
+    H += E;
+  }
   if (H >= L || nan)
     for (int k = threadIdx.x; k < N; k += blockDim.x) {
       float lo, hi;
@@ -581,9 +589,9 @@ __global__ void __launch_bounds__(kCandBlock) k_mx_cand(const float2 *__restrict
 // most 32 2^-24 ||g||_1 <= 32 2^-24 sqrt(N) ||g||_2 -- a few percent of the
 // transform's bound -- and the same interval test leaves those that may still be
 // the maximum.  One block per pair; pairs with one candidate have nothing to do.
-constexpr int kScreen = 4;
+constexpr int kScreen = 4, kScreenBlock = 1024;
 template <bool UN>
-__global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict__ rows,
+__global__ void __launch_bounds__(kScreenBlock, 1) k_mx_screen(const gwt::ff4 *__restrict__ rows,
                                                       const gwt::AccReq *__restrict__ areq, int ndet, int N,
                                                       const StreamDev *__restrict__ streams,
                                                       const int *__restrict__ handles, const double *__restrict__ sums,
@@ -591,10 +599,10 @@ __global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict
   using namespace gwt;
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1;
   extern __shared__ float2 s_tw[];  // [kScreen][nj]
-  __shared__ double s_part[kScreen * NP * 2][kWarps];
+  __shared__ double s_part[kScreen * NP * 2][kScreenBlock / 32];
   __shared__ float s_lo[kCand], s_hi[kCand];
   __shared__ int s_k[kCand], s_keep;
-  const int q = blockIdx.x, tid = threadIdx.x, nc = ncand[q];
+  const int q = blockIdx.x, tid = threadIdx.x, bin = tid % kBlock, nc = ncand[q];
   if (nc <= 1) return;
   const StreamDev &st = streams[handles[q]];
   const int nl = live_bins(areq[q / ndet], streams[handles[q - q % ndet]].n0, N), nj = (N + kBlock - 1) / kBlock;
@@ -610,7 +618,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict
   for (int c0 = 0; c0 < nc; c0 += kScreen) {
     const int mc = min(kScreen, nc - c0);
     __syncthreads();
-    for (int e = tid; e < mc * nj; e += kBlock) {
+    for (int e = tid; e < mc * nj; e += kScreenBlock) {
       const int c = e / nj, j = e - c * nj;
       s_tw[e] = twiddle(((unsigned long long)j * kBlock % N) * s_k[c0 + c] % N);
     }
@@ -619,13 +627,13 @@ __global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict
 #pragma unroll
     for (int u = 0; u < kScreen * NP * 2; u++) tot[u] = ff{0.f, 0.f};
     const ff4 *row = rows + (size_t)q * NP * N;
-    for (int j0 = 0; j0 * kBlock < nl; j0 += 16) {
+    for (int j0 = tid / kBlock * 16; j0 * kBlock < nl; j0 += kScreenBlock / kBlock * 16) {
       float a[kScreen * NP * 2];
 #pragma unroll
       for (int u = 0; u < kScreen * NP * 2; u++) a[u] = 0.f;
 #pragma unroll 8
       for (int j = j0; j < j0 + 16; j++) {
-        const int n = j * kBlock + tid;
+        const int n = j * kBlock + bin;
         const bool in = n < nl;
 #pragma unroll
         for (int p = 0; p < NP; p++) {
@@ -644,7 +652,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict
     }
 #pragma unroll
     for (int c = 0; c < kScreen; c++) {
-      const float2 w = twiddle(c < mc ? (unsigned long long)tid * s_k[c0 + c] % N : 0);
+      const float2 w = twiddle(c < mc ? (unsigned long long)bin * s_k[c0 + c] % N : 0);
 #pragma unroll
       for (int p = 0; p < NP; p++) {
         const ff re = tot[(c * NP + p) * 2], im = tot[(c * NP + p) * 2 + 1];
@@ -664,7 +672,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_screen(const gwt::ff4 *__restrict
 #pragma unroll
       for (int u = 0; u < NP * 2; u++) {
         G[u] = 0.0;
-        for (int w = 0; w < kWarps; w++) G[u] += s_part[tid * NP * 2 + u][w];
+        for (int w = 0; w < kScreenBlock / 32; w++) G[u] += s_part[tid * NP * 2 + u][w];
       }
       double lo, hi;
       if (!UN) {
@@ -793,10 +801,13 @@ __global__ void k_mx_refine(const double2 *__restrict__ g64, int N, int pairs, c
 }
 
 // k_mx_refine on two-float rows: the twiddles from their exact fixed-point turns,
-// products and sums in two floats, bins beyond the cut left out.  Few blocks have
-// work (a candidate or two per pair), so a thread keeps eight loads in flight.
+// products and sums in two floats, bins beyond the cut left out.  A candidate or two
+// per pair have work, a few per SM: a block takes two rows of 256 bins at a time, so
+// that the last ones end together, and a thread keeps eight loads in flight (384
+// rows of 32,128 bins: 46 us; blocks of 256 threads, two an SM, 71).
+constexpr int kRefineBlock = 512;
 template <bool UN>
-__global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restrict__ rows,
+__global__ void __launch_bounds__(kRefineBlock, 2) k_mx_refine_ff(const gwt::ff4 *__restrict__ rows,
                                                          const gwt::AccReq *__restrict__ areq, int ndet,
                                                          const gwt::AccLut *__restrict__ glut, int N, int pairs,
                                                          const int *__restrict__ cand, const int *__restrict__ ncand,
@@ -807,8 +818,9 @@ __global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restr
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1, NV = 2 * NP;
   extern __shared__ double2 s_wj[];
   ff4 *s_wf = (ff4 *)s_wj, *s_turn = s_wf + (N + kBlock - 1) / kBlock;
-  __shared__ double s_red[NV][kWarps];
-  const int nj = (N + kBlock - 1) / kBlock, tid = threadIdx.x;
+  __shared__ double s_red[NV][kRefineBlock / 32];
+  constexpr int kLoads = UN ? 4 : 8;  // in flight per thread
+  const int nj = (N + kBlock - 1) / kBlock, tid = threadIdx.x, bin = tid % kBlock;
   bool loaded = false;
   for (int sl = blockIdx.x; sl < pairs * kCand; sl += gridDim.x) {
     const int q = sl % pairs, ci = sl / pairs, it = q * kCand + ci;
@@ -816,7 +828,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restr
     const unsigned k = (unsigned)cand[it];
     __syncthreads();  // the previous slot's table has been read
     if (!loaded) {
-      for (int w = tid; w < kTurnTab; w += kBlock) s_turn[w] = acc_ld(glut->turn + w);
+      for (int w = tid; w < kTurnTab; w += kRefineBlock) s_turn[w] = acc_ld(glut->turn + w);
       __syncthreads();
       loaded = true;
     }
@@ -824,13 +836,13 @@ __global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restr
       const unsigned long long a = (m << 32) / (unsigned)N, rem = (m << 32) - a * (unsigned)N;
       ff_turns_sincos(0ull - ((a << 32) + (rem << 32) / (unsigned)N), s_turn, c, s);
     };
-    for (int j = tid; j < nj; j += kBlock) {
+    for (int j = tid; j < nj; j += kRefineBlock) {
       ff c, s;
       twiddle(((unsigned long long)j * kBlock % N) * k % N, c, s);
       s_wf[j] = ff4{c.h, c.l, s.h, s.l};
     }
     ff wc, ws;
-    twiddle((unsigned long long)tid * k % N, wc, ws);
+    twiddle((unsigned long long)bin * k % N, wc, ws);
     __syncthreads();
     const int nl = live_bins(areq[q / ndet], streams[handles[q - q % ndet]].n0, N);
     const ff4 *row = rows + ((size_t)q * NP) * N;
@@ -839,16 +851,16 @@ __global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restr
     ff v[NV];
 #pragma unroll
     for (int u = 0; u < NV; u++) v[u] = ff{0.f, 0.f};
-    for (int j0 = 0; j0 * kBlock < nl; j0 += 8) {
-      ff4 x[8][NP];
+    for (int j0 = tid / kBlock * kLoads; j0 * kBlock < nl; j0 += kRefineBlock / kBlock * kLoads) {
+      ff4 x[kLoads][NP];
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int n = (j0 + j) * kBlock + tid;
+      for (int j = 0; j < kLoads; j++) {
+        const int n = (j0 + j) * kBlock + bin;
 #pragma unroll
         for (int u = 0; u < NP; u++) x[j][u] = n < nl ? acc_ld(row + (size_t)u * N + n) : ff4{0.f, 0.f, 0.f, 0.f};
       }
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
+      for (int j = 0; j < kLoads; j++) {
         const ff4 w = s_wf[j0 + j < nj ? j0 + j : 0];
         const ff wr{w.ch, w.cl}, wi{w.sh, w.sl};
 #pragma unroll
@@ -879,7 +891,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_refine_ff(const gwt::ff4 *__restr
 #pragma unroll
       for (int u = 0; u < NV; u++) {
         G[u] = 0.0;
-        for (int w = 0; w < kWarps; w++) G[u] += s_red[u][w];
+        for (int w = 0; w < kRefineBlock / 32; w++) G[u] += s_red[u][w];
       }
       if (!UN) {
         candval[it] = G[0] * G[0] + G[1] * G[1];
@@ -1012,6 +1024,12 @@ struct MxIn {
   const int *req_status = nullptr;             // per request, or null
   int n = 0, ndet = 0, N = 0;
   bool un = false;
+  // the results and the search's overflow flag (*overflow, on the host at
+  // *h_overflow once copied) go to the host in one copy
+  void *results = nullptr, *h_results = nullptr;
+  size_t result_bytes = 0;
+  int *overflow = nullptr;
+  const volatile int *h_overflow = nullptr;
 };
 
 // The FP64 transforms: prep, FFT_M (Bluestein) or FFT_N, reduction.
@@ -1063,9 +1081,10 @@ int run_fp64(gwgpu_context *c, const MxIn &in, double *out, int *status) {
 // The FP32 search and its refinement; *fallback set when a pair had more
 // candidates than kCand (nothing written to out then).  128 IMRPhenomD requests
 // on 3 x 32,128 bins, device time by kernel: products 103, transforms and chirp
-// 209 (conv.cu; 434 with library transforms), candidates 56 (132 with its FP64 sums on every warp), screen 45 and
-// two-float refinement 71 (389 for FP64 sums of every candidate over the whole
-// row), result 10 us.
+// 209 (conv.cu; 434 with library transforms), candidates 55 (132 with its FP64 sums on every warp), screen 31 and
+// two-float refinement 46 (389 for FP64 sums of every candidate over the whole
+// row), result 9 us; one copy each way through pinned memory and one
+// synchronisation at the end: the overflow flag travels with the results.
 int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *fallback) {
   const int np = in.un ? 2 : 1, ns = in.un ? 5 : 2, pairs = in.n * in.ndet, rows = pairs * np;
   *fallback = false;
@@ -1087,14 +1106,14 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   const size_t o_g = 0, o_a = up256(16 * (size_t)rows * in.N), o_h = o_a + up256(8 * (size_t)rows * ld),
                o_s = o_h + up256(8 * (size_t)pairs * ns * nblk), o_c = o_s + up256(8 * (size_t)pairs * ns),
                o_nc = o_c + up256(4 * (size_t)pairs * kCand), o_v = o_nc + up256(4 * (size_t)pairs),
-               o_o = o_v + up256(8 * (size_t)pairs * kCand), total = o_o + 256;
+               total = o_v + up256(8 * (size_t)pairs * kCand);
   void *dev;
   if ((st = c->workspace(gwgpu_context::kWsMaxllRun, total, &dev))) return st;
   char *b = (char *)dev;
   double2 *g64 = (double2 *)(b + o_g);
   float2 *a32 = (float2 *)(b + o_a);
   double *hh = (double *)(b + o_h), *sums = (double *)(b + o_s), *cv = (double *)(b + o_v);
-  int *cand = (int *)(b + o_c), *ncand = (int *)(b + o_nc), *ovf = (int *)(b + o_o);
+  int *cand = (int *)(b + o_c), *ncand = (int *)(b + o_nc), *ovf = in.overflow;
   cudaMemsetAsync(ovf, 0, 4, c->stream);
   const dim3 grid(nblk, in.n);
   if (two && in.un)
@@ -1127,14 +1146,6 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   else
     k_mx_cand<false><<<pairs, kCandBlock, 0, c->stream>>>(a32, hh, nblk, in.N, ld, in.ndet, in.streams, in.handles,
                                                        in.req_status, kscale, sums, cand, ncand, ovf);
-  int h_ovf = 0;
-  cudaMemcpyAsync(&h_ovf, ovf, 4, cudaMemcpyDeviceToHost, c->stream);
-  cudaError_t e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return c->fail(e, "maximised likelihood search");
-  if (h_ovf) {
-    *fallback = true;
-    return GWGPU_OK;
-  }
   const int nj = (in.N + kBlock - 1) / kBlock;
   const size_t smem = 16 * (size_t)nj;
   const int gr = std::min(pairs * kCand, 152 * 8);
@@ -1142,7 +1153,7 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
     const size_t tw = sizeof(float2) * (size_t)kScreen * nj;
     auto screen = [&](auto kern) {
       if (tw > 48 * 1024) cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tw);
-      kern<<<pairs, kBlock, tw, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, in.N, in.streams, in.handles,
+      kern<<<pairs, kScreenBlock, tw, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, in.N, in.streams, in.handles,
                                               sums, cand, ncand);
     };
     if (tw <= 200 * 1024) {  // longer rows keep every candidate
@@ -1159,7 +1170,7 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   auto refine_ff = [&](auto kern) {
     if (smem_ff > 48 * 1024)
       cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ff);
-    kern<<<gr, kBlock, smem_ff, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, c->acc_lut, in.N, pairs, cand,
+    kern<<<gr, kRefineBlock, smem_ff, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, c->acc_lut, in.N, pairs, cand,
                                              ncand, sums, in.streams, in.handles, cv);
   };
   if (two && in.un) refine_ff(k_mx_refine_ff<true>);
@@ -1172,13 +1183,21 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   else
     k_mx_final<false><<<(in.n + 127) / 128, 128, 0, c->stream>>>(cv, ncand, sums, in.n, in.ndet, in.streams,
                                                                   in.handles, in.req_status, out, status);
-  e = cudaGetLastError();
-  return e == cudaSuccess ? GWGPU_OK : c->fail(e, "maximised likelihood launch");
+  // the last candidates of a pair with too many of them were left out: its
+  // results, computed from the others, are not used
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return c->fail(e, "maximised likelihood launch");
+  cudaMemcpyAsync(in.h_results, in.results, in.result_bytes, cudaMemcpyDeviceToHost, c->stream);
+  e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return c->fail(e, "maximised likelihood");
+  *fallback = *in.h_overflow != 0;
+  return GWGPU_OK;
 }
 
 bool search_fits(const gwgpu_context *c, int N) { return !c->maxll_fp64 && (N + kBlock - 1) / kBlock <= kMaxTwiddleRows; }
 
-// *searched: false when only the FP64 transforms' inputs (in.req) will do.
+// The results on the host (in.h_results); *searched: false when only the FP64
+// transforms' inputs (in.req) will do.
 int maxll_run(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *searched = nullptr) {
   if (searched) *searched = true;
   if (search_fits(c, in.N)) {
@@ -1190,7 +1209,11 @@ int maxll_run(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *
     *searched = false;
     return GWGPU_OK;
   }
-  return run_fp64(c, in, out, status);
+  int st = run_fp64(c, in, out, status);
+  if (st) return st;
+  cudaMemcpyAsync(in.h_results, in.results, in.result_bytes, cudaMemcpyDeviceToHost, c->stream);
+  cudaError_t e = cudaStreamSynchronize(c->stream);
+  return e == cudaSuccess ? GWGPU_OK : c->fail(e, "maximised likelihood");
 }
 
 // One pair from host arrays: hp (and hc when unaligned) given.
@@ -1230,10 +1253,14 @@ int maximized_single(gwgpu_context *c, const double *data, const double *psd, co
   in.ndet = 1;
   in.N = N;
   in.un = un;
+  double h[2];  // the result, the flag
+  in.results = res;
+  in.h_results = h;
+  in.result_bytes = sizeof(h);
+  in.overflow = (int *)(res + 1);
+  in.h_overflow = (const int *)(h + 1);
   if ((st = maxll_run(c, in, res, nullptr))) return st;
-  cudaMemcpyAsync(out, res, 8, cudaMemcpyDeviceToHost, c->stream);
-  cudaError_t e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return c->fail(e, "maximised likelihood");
+  *out = h[0];
   return GWGPU_OK;
 }
 
@@ -1276,25 +1303,35 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
   const size_t o_p = 0, o_a = up256(sizeof(gwgpu_gen_params) * n), o_h = o_a + up256(4 * (size_t)n),
                o_req = o_h + up256(4 * (size_t)pairs),
                o_out = o_req + up256(std::max(sizeof(Request), sizeof(gwt::AccReq)) * n),
-               o_st = o_out + up256(8 * (size_t)n), total = o_st + up256(4 * (size_t)n);
+               o_st = o_out + 8 * (size_t)n, o_ovf = o_st + 4 * (size_t)n, total = o_ovf + 4;
   void *dev;
   int st = c->workspace(gwgpu_context::kWsMaxll, total, &dev);
   if (st) return st;
   char *b = (char *)dev;
+  // inputs and results by one copy each through pinned memory
+  char *h;
+  if ((st = c->pinned(gwgpu_context::kHwsMaxll, o_req + total - o_out, (void **)&h))) return st;
   // the sampler's intrinsic mode fixes the extrinsic parameters
   // (IMRPhenomD: mcmc_gw.cpp:2614-2620, 2645-2651; IMRPhenomPv2: 2693-2699)
-  std::vector<gwgpu_gen_params> hp(params, params + n);
-  for (auto &p : hp) {
+  gwgpu_gen_params *hp = (gwgpu_gen_params *)(h + o_p);
+  for (int i = 0; i < n; i++) {
+    gwgpu_gen_params &p = hp[i];
+    p = params[i];
     p.RA = p.DEC = p.psi = 0;
     p.phiRef = 1;
     p.f_ref = un ? 20 : 10;
     p.incl_angle = 0;
     p.tc = 1;
+    ((int *)(h + o_a))[i] = un ? gwt::kPhenomPv2 : gwt::kPhenomD;
   }
-  std::vector<int> ap(n, un ? gwt::kPhenomPv2 : gwt::kPhenomD);
-  cudaMemcpyAsync(b + o_p, hp.data(), sizeof(gwgpu_gen_params) * n, cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(b + o_a, ap.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(b + o_h, handles, 4 * (size_t)pairs, cudaMemcpyHostToDevice, c->stream);
+  std::memcpy(h + o_h, handles, 4 * (size_t)pairs);
+  struct Drain {  // the pinned inputs are read by then, on every way out
+    cudaStream_t s;
+    ~Drain() {
+      if (s) cudaStreamSynchronize(s);
+    }
+  } drain{c->stream};
+  cudaMemcpyAsync(b, h, o_req, cudaMemcpyHostToDevice, c->stream);
   // two-float bins when every stream has its pairs; a search that gives up on
   // them leaves the FP64 transforms, which take the requests themselves
   bool two = c->acc_lut && search_fits(c, N) && N <= kBlock * (kMaxTwiddleRows - gwt::kTurnTab);
@@ -1319,16 +1356,19 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
     in.ndet = ndet;
     in.N = N;
     in.un = un;
+    in.results = b + o_out;
+    in.h_results = h + o_req;
+    in.result_bytes = total - o_out;
+    in.overflow = (int *)(b + o_ovf);
+    in.h_overflow = (const int *)(h + o_req + (o_ovf - o_out));
     bool searched = true;
     if ((st = maxll_run(c, in, (double *)(b + o_out), dst, &searched))) return st;
     if (searched) break;
     two = false;
   }
-  std::vector<int> hs(n);
-  cudaMemcpyAsync(loglik, b + o_out, 8 * (size_t)n, cudaMemcpyDeviceToHost, c->stream);
-  cudaMemcpyAsync(hs.data(), dst, 4 * (size_t)n, cudaMemcpyDeviceToHost, c->stream);
-  e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return c->fail(e, "maximised likelihood");
+  drain.s = nullptr;
+  std::memcpy(loglik, h + o_req, 8 * (size_t)n);
+  const int *hs = (const int *)(h + o_req + (o_st - o_out));
   if (status)
     for (int i = 0; i < n; i++) status[i] = gwk::status_code(hs[i]);
   return GWGPU_OK;
