@@ -338,37 +338,19 @@ size_t gwgpu_context_bytes_in_use(gwgpu_context *c) { return c ? c->in_use : 0; 
 
 // ------------------------------------------------------------ data registry
 // The two-float pairs of a registered stream with finite weights on a uniform
-// grid (FP64 form, phenom_acc.h).  Without the memory for them the stream
-// keeps the FP64 bins.
-static void acc_stream(gwgpu_context *c, gwgpu_context::Stream &s, const double *freqs) {
-  StreamDev &d = s.dev;
-  if ((long long)d.n0 + d.N > gwt::kAccMaxN || c->ensure_acc(d.n0 + d.N) != GWGPU_OK) {
-    c->last_error.clear();
-    return;
-  }
+// grid (FP64 form, phenom_acc.h), in 28 bytes per bin at p.  Without the memory
+// for them the stream keeps the FP64 bins.
+static cudaError_t acc_stream(gwgpu_context *c, StreamDev &d, const double *freqs, size_t row, char *p) {
   // f_k = (n0 + k) dfq to the last bit when the product is exact (dfq with 24
   // zero bits at its end) and equal; a grid that is not carries its distances
   int ex;
   const double mant = std::ldexp(std::frexp(d.dfq, &ex), 29);
   bool exact = mant == std::floor(mant);
   for (int k = 0; k < d.N && exact; k++) exact = (double)(d.n0 + k) * d.dfq == freqs[k];
-  void *p;
-  if (c->dalloc(&p, (exact ? 24 : 28) * (size_t)d.N, "two-float stream") != GWGPU_OK) {
-    c->last_error.clear();
-    return;
-  }
-  StreamDev t = d;
-  t.wd = (const gwt::ff4 *)p;
-  t.wf = (const gwt::ff *)(t.wd + d.N);
-  t.dev = exact ? nullptr : (const float *)(t.wf + d.N);
-  cudaError_t e = gwk::launch_acc_stream(t, !exact, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) {
-    c->dfree(p);
-    return;
-  }
-  d = t;
-  s.mem.push_back(p);
+  d.wd = (const gwt::ff4 *)p;
+  d.wf = (const gwt::ff *)(d.wd + row);
+  d.dev = exact ? nullptr : (const float *)(d.wf + row);
+  return gwk::launch_acc_stream(d, !exact, c->stream);
 }
 
 // The same for a grid that is not uniform (phenom_acc.h, AccNodes; d.dfq its
@@ -380,7 +362,7 @@ static bool nodes_fit(const StreamDev &d, const double *freqs) {
     if (!(freqs[k] > 0x1p-20 * d.dfq && freqs[k] < 0x1p20 * d.dfq)) return false;
   return true;
 }
-static int acc_nodes(gwgpu_context *c, StreamDev &d, size_t row, char *p) {
+static cudaError_t acc_nodes(gwgpu_context *c, StreamDev &d, size_t row, char *p) {
   gwt::AccNodes a;
   a.wd = (const gwt::ff4 *)p;
   a.tb.pw = a.wd + row;
@@ -395,12 +377,9 @@ static int acc_nodes(gwgpu_context *c, StreamDev &d, size_t row, char *p) {
   a.wf = (const gwt::ff *)(a.tb.t13 + 6 * row);
   a.tb.nmax = d.N - 1;
   cudaError_t e = gwk::launch_acc_nodes(d, a, c->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(p + 120 * row, &a, sizeof(a), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return c->fail(e, "two-float stream");
+  if (e == cudaSuccess) e = cudaMemcpyAsync(p + 120 * row, &a, sizeof(a), cudaMemcpyHostToDevice, c->stream);
   d.node = (const gwt::AccNodes *)(p + 120 * row);
-  return GWGPU_OK;
+  return e;
 }
 
 // One detector stream; weights (GAUSSLEG) or null (Simpson's rule).
@@ -466,14 +445,18 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   // one allocation for the stream's arrays, each on a 256-byte boundary
   const size_t row = ((size_t)N + 31) / 32 * 32, gat = row * (weights ? 60 : 52);
   const size_t nat = gat + 2 * sizeof(gwt::GridConst);
+  // two-float arrays, by bin or by node, behind them
+  bool pairs = d.uniform_int && finite && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
   bool nodes = !d.uniform_int && finite && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
+  const size_t more = pairs ? 28 * row : nodes ? nodes_bytes(row) : 0;
   char *mem;
-  st = c->dalloc((void **)&mem, nat + (nodes ? nodes_bytes(row) : 0), "data stream");
-  if (st && nodes) {  // without them the stream keeps the FP64 bins
-    nodes = false;
+  st = c->dalloc((void **)&mem, nat + more, "data stream");
+  if (st && more) {  // without them the stream keeps the FP64 bins
+    pairs = nodes = false;
     st = c->dalloc((void **)&mem, nat, "data stream");
   }
   if (st) return st;
+  c->last_error.clear();
   const gwt::GridConst gc[2] = {gwt::grid_const(d.df), gwt::grid_const(d.dfq)};
   cudaMemcpyAsync(mem + gat, gc, sizeof(gc), cudaMemcpyHostToDevice, c->stream);
   d.grid = (const gwt::GridConst *)(mem + gat);
@@ -486,11 +469,6 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   cudaMemcpyAsync(pp, psd, 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(pdh, dh.data(), 8 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(pwh, wh.data(), 4 * (size_t)N, cudaMemcpyHostToDevice, c->stream);
-  cudaError_t e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) {
-    c->dfree(mem);
-    return c->fail(e, "data upload");
-  }
   d.freqs = (const double *)pf;
   d.data = (const double *)pd;
   d.psd = (const double *)pp;
@@ -498,16 +476,26 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   d.dhat = (const float *)pdh;
   d.what = (const float *)pwh;
   d.iw = (const double *)piw;
+  cudaError_t e = pairs ? acc_stream(c, d, freqs, row, mem + nat) : nodes ? acc_nodes(c, d, row, mem + nat) : cudaSuccess;
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) {
+    c->dfree(mem);
+    return c->fail(e, "data upload");
+  }
   s.live = true;
   s.mem = {mem};
   s.host_freqs.assign(freqs, freqs + N);
   uint64_t hsh = 1469598103934665603ull;
-  const unsigned char *pb = (const unsigned char *)psd;
-  for (size_t i = 0; i < 8 * (size_t)N; i++) hsh = (hsh ^ pb[i]) * 1099511628211ull;
-  if (weights) {
-    const unsigned char *wb = (const unsigned char *)iw.data();
-    for (size_t i = 0; i < 8 * (size_t)N; i++) hsh = (hsh ^ wb[i]) * 1099511628211ull;
-  }
+  auto mix = [&](const double *v) {
+    for (int k = 0; k < N; k++) {
+      uint64_t w;
+      std::memcpy(&w, v + k, 8);
+      hsh = (hsh ^ w) * 1099511628211ull;
+      hsh ^= hsh >> 29;
+    }
+  };
+  mix(psd);
+  if (weights) mix(iw.data());
   s.psd_hash = hsh ^ (uint64_t)N;
   {  // the weights follow from the PSD, the integration rule and the grid
     uint64_t gk = s.psd_hash;
@@ -516,11 +504,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     for (size_t i = 0; i < sizeof(gv); i++) gk = (gk ^ gb[i]) * 1099511628211ull;
     s.dev.wkey = gk;
   }
-  if (d.uniform_int) {
-    st = c->ensure_tables(d.n0 + N);
-    if (st) return st;
-    if (finite) acc_stream(c, s, freqs);
-  } else if (nodes && (st = acc_nodes(c, s.dev, row, mem + nat))) {
+  if (d.uniform_int && (st = c->ensure_tables(d.n0 + N))) {
     c->dfree(mem);
     return st;
   }
