@@ -6,12 +6,12 @@
 // and amplitude 200; per SM and second that leaves DRAM and L2 idle (a
 // detector bin is 16 B of data and, once for shared weights, 8 B, from L2).
 // Against the FP64 bins they took the place of (FP64 pipe full): 512
-// IMRPhenomD requests on 3 x 32,128 bins 4,170 -> 283 us a call, 64
+// IMRPhenomD requests on 3 x 32,128 bins 4,170 -> 256 us a call, 64
 // IMRPhenomPv2 requests on 2 x 32,448 bins 973 -> 103 us, the one-request call
 // on 3 x 32,128 bins 38.4 -> 22 us (Pv2, 3 x 16,224 bins: 48 -> 26 us), with
 // an error against 64-bit references of 7e-14 instead of 2e-13 (t_c's turns
 // leave no rounding behind).  512 requests on 3 x 3,000 quadrature nodes
-// 745 -> 111 us (bins 70, prologue 31): the powers of each node are tabulated
+// 745 -> 100 us (prologue 31): the powers of each node are tabulated
 // at registration, its linear phases 128-bit products.
 #include <cstdint>
 
@@ -23,7 +23,11 @@ using namespace gwt;
 
 namespace {
 
-constexpr int kAccBlock = 256;
+// Blocks of 128 threads, five an SM (96 registers; a few spills from three detectors on): the reduction at an
+// item's end then holds up a fifth of the SM's warps instead of half.  512
+// IMRPhenomD requests on 3 x 32,128 bins: 250 us; two blocks of 256 threads 285,
+// three 254, six of 128 255, ten of 64 265.
+constexpr int kAccBlock = 128;
 constexpr int kPlainBlock = 128;
 
 __device__ __forceinline__ ff shfl_down_ff(ff v, int o) {
@@ -119,12 +123,12 @@ __device__ __forceinline__ void copy_words(void *dst, const void *src, int bytes
 
 // ------------------------------------------------------------------- batch
 // Persistent over the items in work order (as k_batch): an item is a tile of
-// one request's bins, its partial sum one double; the block that finishes a
-// request's last item adds them in item order.  NODES: some requests' grids are
+// one request's bins, its partial sum one double; a warp of the block that finishes
+// a request's last item adds them in a fixed order.  NODES: some requests' grids are
 // not uniform (a kernel of its own, so that batches without them keep their
 // code small).
 template <int NDET, bool NODES>
-__global__ void __launch_bounds__(kAccBlock, 2) k_batch_acc(const BatchArgs a) {
+__global__ void __launch_bounds__(kAccBlock, 5) k_batch_acc(const BatchArgs a) {
   __shared__ AccLut lut;
   __shared__ __align__(16) unsigned char s_req[sizeof(AccReq)];
   __shared__ StreamDev s_st[NDET];
@@ -163,12 +167,15 @@ __global__ void __launch_bounds__(kAccBlock, 2) k_batch_acc(const BatchArgs a) {
     double v = 0.0;
     if (x.m.status == 0) v = acc_block<NDET>(x, s_st, a.acc, lut, NODES && s_st[0].node ? &s_nodes : nullptr, I.k0, kend, s_red);
     if (tid == 0) a.partials[iid] = v;
-    if (arrive_last(a.req_done + I.req, (unsigned)__ldcg(a.item_count + I.req)) && tid == 0) {
+    if (arrive_last(a.req_done + I.req, (unsigned)__ldcg(a.item_count + I.req)) && tid < 32) {
       const int i0 = __ldcg(a.item_start + I.req), ic = __ldcg(a.item_count + I.req), st = x.m.status;
       double ll = 0.0;
-      for (int q = 0; q < ic; q++) ll += __ldcg(a.partials + i0 + q);
-      a.out[I.req] = st ? __longlong_as_double(0x7ff8000000000000ll) : ll;
-      a.status_out[I.req] = st;
+      for (int q = tid; q < ic; q += 32) ll += __ldcg(a.partials + i0 + q);
+      ll = warp_sum(ll);
+      if (tid == 0) {
+        a.out[I.req] = st ? __longlong_as_double(0x7ff8000000000000ll) : ll;
+        a.status_out[I.req] = st;
+      }
     }
     __syncthreads();
   }
