@@ -582,6 +582,9 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
   }
 }
 
+// Bound by dependency waits and instruction fetch (2,450 instructions a warp, run
+// once; FP64 pipe 27 %): 512 IMRPhenomD requests 47 -> 27 us, 64 IMRPhenomPv2 100 ->
+// 43 us against stages of inlined FP64 code at 16 requests a block.
 template <int REQ, bool ACC>
 __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const GenParams *__restrict__ params, const int *__restrict__ approx, int n, const int *__restrict__ handles,
@@ -627,7 +630,10 @@ cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, c
                             const OrderArgs &ord, AccReq *areq) {
   // requests per block: few enough that more lanes serve each, while the
   // blocks find an SM each (two blocks of one SM share its FP64 pipes)
-  if (n <= 4 * kSMs) launch_coop<4>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
+  // (512 IMRPhenomD requests, prologue: 4 per block 27 us, 2 31, 8 30, 16 37; the
+  // call of 16 chains: 2 per block 82.4 us, 1 84.6, 4 84.0)
+  if (n <= 2 * kSMs) launch_coop<2>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
+  else if (n <= 4 * kSMs) launch_coop<4>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
   else if (n <= 8 * kSMs) launch_coop<8>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
   else launch_coop<16>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, want_mixed, status, s, ord);
   return cudaGetLastError();

@@ -120,7 +120,7 @@ def test_infinite_psd_bins(gpu_ctx, oracle):
 
 @pytest.mark.parametrize("prec", [G.PREC_FP64, G.PREC_MIXED])
 def test_prologue_block_sizes(gpu_ctx, prec):
-    """4, 8 or 16 requests per prologue block (by the number of requests): each request as in a small batch, to
+    """2, 4, 8 or 16 requests per prologue block (by the number of requests): each request as in a small batch, to
     the bit in the mixed form (the FP64 form's tile, and with it its order of summation, follows the batch)."""
     T = 4.0
     f = 20.0 + np.arange(300) / T
@@ -132,7 +132,7 @@ def test_prologue_block_sizes(gpu_ctx, prec):
         aps = np.arange(n, dtype=np.int32) % 2
         few = np.concatenate([gpu_ctx.loglik_batch(G.params_array(draws[i:i + 100]), aps[i:i + 100], hs, T, prec)[0]
                               for i in range(0, n, 100)])
-        for m in (1, 3, 608, 609, 1216, 1217, n):
+        for m in (1, 3, 304, 305, 608, 609, 1216, 1217, n):
             out, st = gpu_ctx.loglik_batch(G.params_array(draws[:m]), aps[:m], hs, T, prec)
             assert np.all(st == 0)
             if prec == G.PREC_MIXED:
