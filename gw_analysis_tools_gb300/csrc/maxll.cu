@@ -345,7 +345,8 @@ __global__ void k_mx_prep(const Request *__restrict__ req, const double2 *__rest
 // padded with zeros up to pad.
 // Bound by memory: per pair and bin 16 B of data read and 16 + 8 B written (the
 // padding of a Bluestein row another 8 B per entry).  128 IMRPhenomD requests on
-// 3 x 32,128 bins: 1,480 -> 103 us against the FP64 bins; bins beyond a
+// 3 x 32,128 bins: 1,480 -> 97 us against the FP64 bins at
+// four blocks an SM (three: 103; Pv2, 48 requests on 3 x 15,680, two: 57, one: 81); bins beyond a
 // request's cut only write their zeros (242 -> 131 us), the padding none.
 constexpr int kPrepTile = 2048;
 // Bins of the grid below the model's cut (0 for a request outside its domain).
@@ -353,7 +354,7 @@ __device__ __forceinline__ int live_bins(const gwt::AccReq &x, int n0, int N) {
   return x.m.status ? 0 : max(0, min(N, x.m.n_cut - n0 + 1));
 }
 template <bool UN>
-__global__ void __launch_bounds__(kBlock, UN ? 1 : 3) k_mx_prep_ff(const gwt::AccReq *__restrict__ areq, int ndet,
+__global__ void __launch_bounds__(kBlock, UN ? 2 : 4) k_mx_prep_ff(const gwt::AccReq *__restrict__ areq, int ndet,
                                                        const StreamDev *__restrict__ streams,
                                                        const int *__restrict__ handles, const gwt::AccTables tb,
                                                        const gwt::AccLut *__restrict__ glut, int N, int ld, int pad,
