@@ -343,8 +343,8 @@ __global__ void k_mx_prep(const Request *__restrict__ req, const double2 *__rest
 // k_mx_prep for the intrinsic mode on uniform grids: the waveform and the products
 // in two floats (g as pairs), a tile of kPrepTile bins per block; a32's rows are
 // padded with zeros up to pad.
-// Bound by memory: per pair and bin 16 B of data read and 16 + 8 B written (the
-// padding of a Bluestein row another 8 B per entry).  128 IMRPhenomD requests on
+// Bound by memory: per pair and bin 16 B of data read and 16 + 8 B written (for a
+// library transform the padding of a Bluestein row another 8 B per entry).  128 IMRPhenomD requests on
 // 3 x 32,128 bins: 1,480 -> 97 us against the FP64 bins at
 // four blocks an SM (three: 103; Pv2, 48 requests on 3 x 15,680, two: 57, one: 81); bins beyond a
 // request's cut only write their zeros (242 -> 131 us), the padding none.
@@ -1081,7 +1081,7 @@ int run_fp64(gwgpu_context *c, const MxIn &in, double *out, int *status) {
 
 // The FP32 search and its refinement; *fallback set when a pair had more
 // candidates than kCand (nothing written to out then).  128 IMRPhenomD requests
-// on 3 x 32,128 bins, device time by kernel: products 103, transforms and chirp
+// on 3 x 32,128 bins, device time by kernel: products 97, transforms and chirp
 // 209 (conv.cu; 434 with library transforms), candidates 55 (132 with its FP64 sums on every warp), screen 31 and
 // two-float refinement 46 (389 for FP64 sums of every candidate over the whole
 // row), result 9 us; one copy each way through pinned memory and one
