@@ -337,8 +337,8 @@ void *gwgpu_context_stream(gwgpu_context *c) { return c ? (void *)c->stream : nu
 size_t gwgpu_context_bytes_in_use(gwgpu_context *c) { return c ? c->in_use : 0; }
 
 // ------------------------------------------------------------ data registry
-// The two-float pairs of a registered stream with finite weights on a uniform
-// grid (FP64 form, phenom_acc.h), in 28 bytes per bin at p.  Without the memory
+// The two-float pairs of a registered stream with finite weights on a grid of n
+// dfq (FP64 form, phenom_acc.h), in 28 bytes per bin at p.  Without the memory
 // for them the stream keeps the FP64 bins.
 static cudaError_t acc_stream(gwgpu_context *c, StreamDev &d, const double *freqs, size_t row, char *p) {
   // f_k = (n0 + k) dfq to the last bit when the product is exact (dfq with 24
@@ -353,9 +353,9 @@ static cudaError_t acc_stream(gwgpu_context *c, StreamDev &d, const double *freq
   return gwk::launch_acc_stream(d, !exact, c->stream);
 }
 
-// The same for a grid that is not uniform (phenom_acc.h, AccNodes; d.dfq its
-// scale): positive finite frequencies within the range of the bin tables, in
-// nodes_bytes of device memory at p.
+// The same for any other grid (phenom_acc.h, AccNodes; d.dfq its scale): positive
+// finite frequencies within the range of the bin tables, in nodes_bytes of device
+// memory at p.
 static size_t nodes_bytes(size_t row) { return 120 * row + sizeof(gwt::AccNodes); }
 static bool nodes_fit(const StreamDev &d, const double *freqs) {
   for (int k = 0; k < d.N; k++)
@@ -406,9 +406,12 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     if (std::fabs(freqs[k] - (freqs[0] + k * d.df)) > 1e-9 * d.df * (1 + k)) uniform = false;
   double n0f = freqs[0] / d.df;
   d.n0 = (int)std::llround(n0f);
-  d.dfq = (freqs[N - 1] - freqs[0]) / (N - 1);
   d.uniform_int = uniform && d.n0 >= 1 && std::fabs(n0f - d.n0) < 1e-6 && (d.n0 + (double)N) < 1.5e9;
-  if (!d.uniform_int) {
+  // the FP64 form's bins at n dfq where the frequencies are that to their rounding, else nodes
+  bool line = d.uniform_int;
+  if (line) d.dfq = gwt::acc_spacing(freqs[N - 1], d.n0 + N - 1);
+  for (int k = 0; k < N && line; k++) line = gwt::acc_on_line(freqs[k], d.n0 + k, d.dfq);
+  if (!line) {
     double fmax = 0;
     for (int k = 0; k < N; k++) fmax = std::fmax(fmax, freqs[k]);
     d.dfq = fmax > 0 && std::isfinite(fmax) ? std::ldexp(1.0, std::ilogb(fmax) - 19) : 1.0;
@@ -446,8 +449,8 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   const size_t row = ((size_t)N + 31) / 32 * 32, gat = row * (weights ? 60 : 52);
   const size_t nat = gat + 2 * sizeof(gwt::GridConst);
   // two-float arrays, by bin or by node, behind them
-  bool pairs = d.uniform_int && finite && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
-  bool nodes = !d.uniform_int && finite && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
+  bool pairs = line && finite && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
+  bool nodes = !line && finite && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
   const size_t more = pairs ? 28 * row : nodes ? nodes_bytes(row) : 0;
   char *mem;
   st = c->dalloc((void **)&mem, nat + more, "data stream");

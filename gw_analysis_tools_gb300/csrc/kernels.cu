@@ -354,7 +354,7 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
         for (int d = 0; d < ndet; d++)
           if (streams[__ldcg(handles + i * ndet + d)].N != s0.N) st = 1;
         sm.st[j] = st;
-        sm.uni[j] = s0.uniform_int ? 1 : ACC && s0.node ? 2 : 0;  // bins, nodes, neither
+        sm.uni[j] = ACC && s0.node ? 2 : s0.uniform_int ? 1 : 0;  // nodes, bins, neither
         sm.N[j] = s0.N;
         sm.n0[j] = s0.n0;
         head(i, sm.item0[j], sm.items[j]);

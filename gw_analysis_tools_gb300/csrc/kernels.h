@@ -36,14 +36,14 @@ struct StreamDev {
   unsigned long long wkey;
   // FP64 form on two-float bins (phenom_acc.h; null where the stream does not
   // qualify): W d / dscale and W / wscale as pairs, the bins' distances from
-  // (n0 + k) dfq (null: none), and the grid's spacing over its whole length
+  // (n0 + k) dfq (null: none), and the spacing that fits the whole grid
   // (df = f[1] - f[0] carries the rounding of f there)
   const gwt::ff4 *wd;
   const gwt::ff *wf;
   const float *dev;
   double dfq;
   const gwt::GridConst *grid;  // of df, of dfq
-  const gwt::AccNodes *node;   // grids that are not uniform: the same by node (dfq the nodes' scale), or null
+  const gwt::AccNodes *node;   // grids that are not n dfq: the same by node (dfq the nodes' scale), or null
 };
 
 struct Item {

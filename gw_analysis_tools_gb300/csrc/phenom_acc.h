@@ -29,7 +29,7 @@ struct AccTables {
   int nmax;            // valid for 1 <= n <= nmax
 };
 
-// A grid of any other spacing (quadrature nodes): bins at x = f / df, df the
+// A grid of any other spacing (quadrature nodes; acc_on_line): bins at x = f / df, df the
 // power of two that puts the highest frequency in [2^19, 2^20); the weights and
 // data products as on uniform grids, the tables by the bin's index.
 constexpr int kNodeBits = 42;
@@ -71,7 +71,7 @@ struct AccReq {
   ff us[4];                           // 1/s = us0 i + us1 t + us2 n + us3 (the Wigner angle)
   ff y2p, y1p, y0p, y2m, y1m;         // harmonics: sums and differences of Y_m and Y_-m
   ff c2z, s2z;                        // polarisation rotation
-  float tc;                           // model's t_c, for bins off the line n df (acc_dev_turns)
+  float tc;                           // model's t_c, for the rounding of a bin's frequency (acc_dev_turns)
   float bad;                          // NaN when a linear phase is (turns cannot hold it), else 0; joins the result
   // On nodes (acc_node_coeffs): slopes of the linear phases in turns per bin
   // 2^(node_shift + 64 - kNodeBits), region boundaries as the bits of the
@@ -407,10 +407,20 @@ GW_HD ff acc_amp(const AccReq &x, const B &b, ff t, ff m76, const AccLut &lut) {
   return ff_norm(ff_mul(ff_norm(a), m76));
 }
 
-// Phase of t_c at a bin whose frequency lies dev Hz off n df (a grid of 1 / T
-// with T no power of two is rounded bin by bin; |tc dev| is below 1e-9 turn).
+// The bins' rule: a uniform grid's bins are taken at n dfq, dfq = f_last / n_last,
+// where every frequency is n dfq to its own rounding, four units in its last
+// place (k (1 / T) and f0 + k df round to two).  What a bin's distance leaves
+// out is then below FP64's own rounding of the phase: 2 pi tau(f) 2^-50 f for the
+// series, whose time to coalescence tau falls from about T at the lowest
+// frequencies as f^(-8/3), and as little for an arrival time; t_c is as large
+// at every frequency and joins by acc_dev_turns.  Any other grid, 1e-9 of a bin
+// off or drifting by as much, takes the node arrays, which hold f itself.
+GW_HD double acc_spacing(double f_last, int n_last) { return f_last / n_last; }
+GW_HD bool acc_on_line(double f, int n, double dfq) { return fabs(fma(-(double)n, dfq, f)) <= 0x1p-50 * f; }
+// Phase of t_c at such a bin, whose frequency lies dev Hz off n dfq: |tc dev| is
+// 1e-11 turn on a segment of 32 s, 2e-3 for a t_c counted in GPS seconds.
 GW_HD uint64_t acc_dev_turns(const AccReq &x, float dev) {
-  return (uint64_t)(int64_t)f_to_int(f_mul(f_mul(-x.tc, dev), 36028797018963968.0f)) << 9;  // 2^-55 turns
+  return (uint64_t)f_to_int64(f_mul(f_mul(-x.tc, dev), 36028797018963968.0f)) << 9;  // 2^-55 turns
 }
 
 // IMRPhenomD bin: acc[2 d] weighted |h|^2 (detector 0 only when the detectors
