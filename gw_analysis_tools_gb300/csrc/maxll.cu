@@ -986,16 +986,18 @@ int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const floa
                  void **conv = nullptr) {
   void *kb, *kb32;
   const size_t b32 = up256(8 * ((size_t)M + N)), bconv = gwk::conv_table_bytes(M);
+  // a workspace that grows loses what it held, also when a later step fails
+  const bool have = c->chirp_n == N;
+  if (!have) c->chirp_n = 0;
   int st = c->workspace(gwgpu_context::kWsChirp, 16 * (size_t)M + 256, &kb);
   if (st) return st;
-  if (c->chirp_n != N) c->chirp_conv = bconv && c->workspace(gwgpu_context::kWsChirp32, b32 + bconv, &kb32) == GWGPU_OK;
+  if (!have) c->chirp_conv = bconv && c->workspace(gwgpu_context::kWsChirp32, b32 + bconv, &kb32) == GWGPU_OK;
   if ((st = c->workspace(gwgpu_context::kWsChirp32, b32 + (c->chirp_conv ? bconv : 0), &kb32))) return st;
   *B64 = (const double2 *)kb;
   *B32 = (const float2 *)kb32;
   *tab = *B32 + M;
   if (conv) *conv = c->chirp_conv ? (char *)kb32 + b32 : nullptr;
-  if (c->chirp_n == N) return GWGPU_OK;
-  c->chirp_n = 0;
+  if (have) return GWGPU_OK;
   int p1;
   if ((st = gwfft::plan(c, gwfft::kZ2Z, M, 1, &p1))) return st;
   const int gb = std::min((M + kBlock - 1) / kBlock, 1024);
@@ -1005,10 +1007,13 @@ int ensure_chirp(gwgpu_context *c, int N, int M, const double2 **B64, const floa
   k_absmax<<<1, kBlock, 0, c->stream>>>((const double2 *)kb, M, dmax);
   k_to_f32<<<gb, kBlock, 0, c->stream>>>((const double2 *)kb, (float2 *)kb32, M);
   k_chirp_tab<<<gb, kBlock, 0, c->stream>>>((float2 *)kb32 + M, N);
-  if (c->chirp_conv) gwk::launch_conv_tables((const float2 *)kb32, M, (char *)kb32 + b32, c->stream);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && c->chirp_conv)
+    e = gwk::launch_conv_tables((const float2 *)kb32, M, (char *)kb32 + b32, c->stream);
+  if (e != cudaSuccess) return c->fail(e, "Bluestein kernel");
   double bmax = 0;
   cudaMemcpyAsync(&bmax, dmax, 8, cudaMemcpyDeviceToHost, c->stream);
-  cudaError_t e = cudaStreamSynchronize(c->stream);
+  e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return c->fail(e, "Bluestein kernel");
   c->chirp_kscale = (double)M * bmax;
   c->chirp_n = N;
