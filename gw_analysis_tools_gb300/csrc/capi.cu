@@ -111,29 +111,34 @@ int gwgpu_context::pinned(int slot, size_t bytes, void **out) {
   return GWGPU_OK;
 }
 
+// n^(1/3), n^(-5/3), ln n, n^(3/4) for n < n1, one after the other (0 at n = 0).
+static std::vector<double> bin_powers(size_t n1) {
+  std::vector<double> v(4 * n1, 0.0);
+  for (size_t n = 1; n < n1; n++) {
+    const double x = (double)n;
+    v[n] = std::cbrt(x);
+    v[n1 + n] = std::pow(x, -5. / 3.);
+    v[2 * n1 + n] = std::log(x);
+    v[3 * n1 + n] = std::pow(x, 0.75);
+  }
+  return v;
+}
 // Per-bin tables n^(1/3), n^(-5/3), ln n, n^(3/4) (FP64) and n^(1/3), n^(-7/6) (FP32).
 int gwgpu_context::ensure_tables(int nmax) {
   if (nmax <= tables.nmax) return GWGPU_OK;
   int nm = std::max(nmax, 1 << 16);
   size_t n1 = (size_t)nm + 1;
-  std::vector<double> t13(n1), tm53(n1), tln(n1), t34(n1);
-  std::vector<float> t13f(n1), tm76f(n1);
+  const std::vector<double> v = bin_powers(n1);
+  std::vector<float> t13f(n1, 0.f), tm76f(n1, 0.f);
   for (size_t n = 1; n < n1; n++) {
-    double x = (double)n;
-    t13[n] = std::cbrt(x);
-    tm53[n] = std::pow(x, -5. / 3.);
-    tln[n] = std::log(x);
-    t34[n] = std::pow(x, 0.75);
-    t13f[n] = (float)std::cbrt(x);
-    tm76f[n] = (float)std::pow(x, -7. / 6.);
+    t13f[n] = (float)v[n];
+    tm76f[n] = (float)std::pow((double)n, -7. / 6.);
   }
-  t13[0] = tm53[0] = tln[0] = t34[0] = 0.0;
-  t13f[0] = tm76f[0] = 0.f;
   for (void *p : table_mem) dfree(p);
   table_mem.clear();
   void *p[6];
   size_t sz[6] = {8, 8, 8, 8, 4, 4};
-  const void *src[6] = {t13.data(), tm53.data(), tln.data(), t34.data(), t13f.data(), tm76f.data()};
+  const void *src[6] = {v.data(), v.data() + n1, v.data() + 2 * n1, v.data() + 3 * n1, t13f.data(), tm76f.data()};
   for (int i = 0; i < 6; i++) {
     int st = dalloc(&p[i], sz[i] * n1, "tables");
     if (st) return st;
@@ -188,7 +193,8 @@ int gwgpu_context::ensure_acc(int nmax) {
   if (!st) st = ensure_lut();
   if (st) return st;
   if (nmax <= acc.nmax) return GWGPU_OK;
-  const size_t n1 = (size_t)std::max(nmax, std::min(tables.nmax, std::max(2 * acc.nmax, 1 << 16))) + 1;
+  // twice the block before, which stays: all of them together less than twice the last
+  const size_t n1 = (size_t)std::max(nmax, std::min(std::max(2 * acc.nmax, 1 << 16), gwt::kAccMaxN)) + 1;
   void *p;
   if ((st = dalloc(&p, 80 * n1, "two-float tables"))) return st;
   gwt::AccTables t;
@@ -197,10 +203,16 @@ int gwgpu_context::ensure_acc(int nmax) {
   t.ph = q + n1;
   t.pv = q + 2 * n1;
   double *v = (double *)(q + 3 * n1);
-  const double *src[4] = {tables.t13, tables.tm53, tables.tln, tables.t34};
+  std::vector<double> powers;
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < 4 && e == cudaSuccess; i++)
-    e = cudaMemcpyAsync(v + i * n1, src[i], 8 * n1, cudaMemcpyDeviceToDevice, stream);
+  if (n1 <= (size_t)tables.nmax + 1) {
+    const double *src[4] = {tables.t13, tables.tm53, tables.tln, tables.t34};
+    for (int i = 0; i < 4 && e == cudaSuccess; i++)
+      e = cudaMemcpyAsync(v + i * n1, src[i], 8 * n1, cudaMemcpyDeviceToDevice, stream);
+  } else {
+    powers = bin_powers(n1);
+    e = cudaMemcpyAsync(v, powers.data(), 32 * n1, cudaMemcpyHostToDevice, stream);
+  }
   t.t13 = v;
   t.tm53 = v + n1;
   t.tln = v + 2 * n1;

@@ -42,7 +42,7 @@ struct gwgpu_context {
   std::vector<void *> table_mem;
   // FP64 form on two-float bins: tables by n and the sine/exp tables.  Grown
   // blocks stay allocated until the context goes (a launch captured by the
-  // caller may hold their addresses); each is at least twice the one before.
+  // caller may hold their addresses); each is twice the one before, up to kAccMaxN.
   gwt::AccTables acc{};
   gwt::AccLut *acc_lut = nullptr;
   double *tm76d = nullptr;  // FP64 n^(-7/6), built on first Fisher use
