@@ -134,20 +134,37 @@ int gwgpu_context::ensure_tables(int nmax) {
     t13f[n] = (float)v[n];
     tm76f[n] = (float)std::pow((double)n, -7. / 6.);
   }
-  for (void *p : table_mem) dfree(p);
-  table_mem.clear();
-  void *p[6];
-  size_t sz[6] = {8, 8, 8, 8, 4, 4};
+  // The old tables stay until the new ones are there (unless the budget holds one
+  // set only), and where they go, captured launches that hold them go too.
+  const size_t sz[6] = {8, 8, 8, 8, 4, 4};
   const void *src[6] = {v.data(), v.data() + n1, v.data() + 2 * n1, v.data() + 3 * n1, t13f.data(), tm76f.data()};
-  for (int i = 0; i < 6; i++) {
-    int st = dalloc(&p[i], sz[i] * n1, "tables");
-    if (st) return st;
-    table_mem.push_back(p[i]);
+  auto drop = [&] {
+    if (table_mem.empty()) return;
+    for (void *q : table_mem) dfree(q);
+    table_mem.clear();
+    tables = gwt::Tables{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+    tm76d_n = 0;
+    streams_epoch++;
+  };
+  size_t held = 0;
+  for (void *q : table_mem) held += sizes[q];
+  if (budget && in_use + 40 * n1 > budget && in_use - held + 40 * n1 <= budget) drop();
+  void *p[6] = {};
+  int st = GWGPU_OK;
+  for (int i = 0; i < 6 && !st; i++) {
+    st = dalloc(&p[i], sz[i] * n1, "tables");
+    if (st) break;
     cudaError_t e = cudaMemcpyAsync(p[i], src[i], sz[i] * n1, cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return fail(e, "tables upload");
+    if (e != cudaSuccess) st = fail(e, "tables upload");
   }
   cudaError_t e = cudaStreamSynchronize(stream);
-  if (e != cudaSuccess) return fail(e, "tables upload");
+  if (!st && e != cudaSuccess) st = fail(e, "tables upload");
+  if (st) {
+    for (void *q : p) dfree(q);
+    return st;
+  }
+  drop();
+  table_mem.assign(p, p + 6);
   tables.t13 = (const double *)p[0];
   tables.tm53 = (const double *)p[1];
   tables.tln = (const double *)p[2];

@@ -28,3 +28,40 @@ def test_tables_of_slowly_growing_grids(oracle):
         assert held[-1] <= 4 * held[0]
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("prec", [G.PREC_MIXED, G.PREC_FP64])
+def test_registration_that_fails(prec):
+    """A longer grid that gets its tables and not its own arrays, or neither: calls on the streams that
+    were there (replayed launches among them) go on as before."""
+    T, N, N2 = 8.0, 3000, 150000
+    f, g = 20.0 + np.arange(N) / T, 20.0 + np.arange(N2) / 64.0
+    psd, data = W.analytic_psd(f), W.noise(f, 3)
+    gpsd, gdata = W.analytic_psd(g), W.noise(g, 4)
+    p = G.params_array(W.prior_draws(6, 4))
+
+    def run(budget):
+        ctx = G.Context(0, hbm_budget=budget)
+        try:
+            h = ctx.register_data("Hanford", f, data, psd)
+            call = lambda: ctx.loglik_batch(p, 0, [h], T, prec)
+            out = [call()[0] for _ in range(3)]
+            held, failed = ctx.bytes_in_use(), 0
+            try:
+                ctx.register_data("Hanford", g, gdata, gpsd)
+            except Exception:
+                failed = 1
+            after = ctx.bytes_in_use()
+            for _ in range(2):
+                v, st = call()
+                assert np.all(st == 0)
+                out.append(v)
+            assert all(np.array_equal(v, out[0]) for v in out)
+            return held, after - held, failed
+        finally:
+            ctx.close()
+
+    held, need, failed = run(0)
+    assert not failed
+    parts = [run(held + int(need * x))[2] for x in np.linspace(0.0, 1.0, 9)]
+    assert parts[0] == 1 and parts[-1] == 0
