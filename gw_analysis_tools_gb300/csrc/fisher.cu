@@ -58,7 +58,7 @@ template <bool FF>
 __global__ void __launch_bounds__(32) k_fisher_setup(const GenParams *__restrict__ params, int method, int ndet,
                                                      double epsilon, int step_mode, int order,
                                                      const SlotOut *__restrict__ slots, FisherSrc *out, FfSrc *ffout,
-                                                     int *status) {
+                                                     int *status, int *beyond) {
   const int src = blockIdx.x, lane = threadIdx.x;
   const unsigned all = 0xffffffffu;
   const SlotOut *S = slots + (size_t)src * kSlots;
@@ -98,7 +98,10 @@ __global__ void __launch_bounds__(32) k_fisher_setup(const GenParams *__restrict
     bool ok = ff_pair(F, lane / 8, X.q[lane / 8], lane % 8, 8);
     if (lane == 1) ok = ff_centre(F, X) && ok;
     ok = __all_sync(all, ok);
-    if (lane == 0) X.ok = ok;
+    if (lane == 0) {
+      X.ok = ok;
+      if (!ok && !st && !F.needs_ref) *beyond = 1;
+    }
   }
 }
 
@@ -128,6 +131,7 @@ struct FisherArgs {
   unsigned *item_counter, *src_done;
   double *partials;  // items * kMaxDet * kSums
   double *fisher, *cov;
+  const int *beyond;        // set: a source that two floats cannot hold is among them
   int *status;
 };
 
@@ -288,6 +292,7 @@ __device__ __noinline__ double2 pair_fp64(const FisherSrc *F, int q, int n, doub
 // matrix's condition number.
 constexpr int kFfTile = 2048;
 __global__ void __launch_bounds__(kBlock, 4) k_fisher_ff(const __grid_constant__ FisherArgs a) {
+  if (*a.beyond) return;  // the chunk takes FP64 sums
   __shared__ int s_item, s_last;
   __shared__ FfSrc S;
   __shared__ gwt::AccLut lut;
@@ -619,7 +624,8 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   // their two-float weights.
   bool two_float = acc64 && !covariance;
   for (const auto *s : ws) two_float = two_float && s->dev.wf != nullptr;
-  const int N = s0->dev.N, tile = two_float ? kFfTile : 4096, ntiles = (N + tile - 1) / tile;
+  constexpr int kTile = 4096;  // of the FP64 and mixed sums: fewer tiles than kFfTile's
+  const int N = s0->dev.N, ntiles = (N + (two_float ? kFfTile : kTile) - 1) / (two_float ? kFfTile : kTile);
   const double df = s0->dev.df;
   // chunk sources to bound the scratch
   const int chunk = std::min(n, 2048);
@@ -673,8 +679,6 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   a.lut = c->acc_lut;
   a.n0 = s0->dev.n0;
   a.N = N;
-  a.tile = tile;
-  a.ntiles = ntiles;
   a.df = df;
   a.df_f = (float)df;
   a.fisher_df_ratio = (s0->host_freqs[1] - s0->host_freqs[0]) / s0->dev.simpson_df;
@@ -697,12 +701,13 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
     int tot = m * kSlots;
     k_fisher_slots<<<(tot + 63) / 64, 64, 0, c->stream>>>(dparams, m, method, ddets, ndet, df, epsilon, step_mode,
                                                           c->qnm_dev, slots);
+    cudaMemsetAsync(dstat + m, 0, sizeof(int), c->stream);
     if (two_float)
       k_fisher_setup<true><<<m, 32, 0, c->stream>>>(dparams, method, ndet, epsilon, step_mode, order, slots, srcs, ffs,
-                                                    dstat);
+                                                    dstat, dstat + m);
     else
       k_fisher_setup<false><<<m, 32, 0, c->stream>>>(dparams, method, ndet, epsilon, step_mode, order, slots, srcs,
-                                                     nullptr, dstat);
+                                                     nullptr, dstat, nullptr);
     a.src = srcs;
     a.nsrc = m;
     a.item_counter = cnt + m;
@@ -711,24 +716,28 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
     a.fisher = dfish;
     a.cov = covariance ? dcov : nullptr;
     a.status = dstat;
-    std::vector<int> hs(m);
+    a.beyond = dstat + m;
+    std::vector<int> hs(m + 1);  // and the flag
     cudaError_t e = cudaSuccess;
     for (bool again = two_float;; again = false) {
+      a.tile = again ? kFfTile : kTile;
+      a.ntiles = (N + a.tile - 1) / a.tile;
       cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (m + 8), c->stream);
-      int grid = std::min(m * ntiles * (again ? nw : 1), again ? grid_ff : grid_cache);
+      int grid = std::min(m * a.ntiles * (again ? nw : 1), again ? grid_ff : grid_cache);
       if (again) k_fisher_ff<<<grid, kBlock, 0, c->stream>>>(a);
       else if (acc64) launch_main<true>(a, nw, grid, c->stream);
       else launch_main<false>(a, nw, grid, c->stream);
       e = cudaGetLastError();
       if (e != cudaSuccess) return c->fail(e, "fisher batch launch");
-      cudaMemcpyAsync(hs.data(), dstat, sizeof(int) * m, cudaMemcpyDeviceToHost, c->stream);
+      cudaMemcpyAsync(hs.data(), dstat, sizeof(int) * (m + 1), cudaMemcpyDeviceToHost, c->stream);
       cudaMemcpyAsync(fisher + (size_t)s0i * kDim * kDim, dfish, sizeof(double) * m * kDim * kDim,
                       cudaMemcpyDeviceToHost, c->stream);
       if (!again) break;
       e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) return c->fail(e, "fisher batch");
-      // a source beyond what two floats hold: the chunk again with FP64 sums
-      if (std::find(hs.begin(), hs.end(), kStatusFp64) == hs.end()) break;
+      // a source beyond what two floats hold, by its coefficients (nothing has run
+      // then) or its sums: the chunk with FP64 sums
+      if (!hs[m] && std::find(hs.begin(), hs.end() - 1, kStatusFp64) == hs.end() - 1) break;
     }
     if (covariance)
       cudaMemcpyAsync(covariance + (size_t)s0i * kDim * kDim, dcov, sizeof(double) * m * kDim * kDim,
