@@ -596,10 +596,12 @@ __global__ void __launch_bounds__(kScreenBlock, 1) k_mx_screen(const gwt::ff4 *_
                                                       const gwt::AccReq *__restrict__ areq, int ndet, int N,
                                                       const StreamDev *__restrict__ streams,
                                                       const int *__restrict__ handles, const double *__restrict__ sums,
-                                                      int *__restrict__ cand, int *__restrict__ ncand) {
+                                                      const int *__restrict__ overflow, int *__restrict__ cand,
+                                                      int *__restrict__ ncand) {
   using namespace gwt;
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1;
   extern __shared__ float2 s_tw[];  // [kScreen][nj]
+  if (*overflow) return;  // the batch goes to the FP64 transforms
   __shared__ double s_part[kScreen * NP * 2][kScreenBlock / 32];
   __shared__ float s_lo[kCand], s_hi[kCand];
   __shared__ int s_k[kCand], s_keep;
@@ -715,11 +717,12 @@ __global__ void __launch_bounds__(kScreenBlock, 1) k_mx_screen(const gwt::ff4 *_
 // lambda (unaligned).  Persistent over the (pair, candidate) slots.
 template <bool UN>
 __global__ void k_mx_refine(const double2 *__restrict__ g64, int N, int pairs, const int *__restrict__ cand,
-                            const int *__restrict__ ncand, const double *__restrict__ sums,
-                            const StreamDev *__restrict__ streams, const int *__restrict__ handles,
-                            double *__restrict__ candval) {
+                            const int *__restrict__ ncand, const int *__restrict__ overflow,
+                            const double *__restrict__ sums, const StreamDev *__restrict__ streams,
+                            const int *__restrict__ handles, double *__restrict__ candval) {
   constexpr int NS = UN ? 5 : 2, NP = UN ? 2 : 1, NV = UN ? 4 : 2;
   extern __shared__ double2 s_wj[];
+  if (*overflow) return;
   __shared__ double s_red[NV][kWarps];
   const int nj = (N + kBlock - 1) / kBlock;
   // slot s = (candidate ci, pair q) with ci major, so that the first
@@ -812,6 +815,7 @@ __global__ void __launch_bounds__(kRefineBlock, 2) k_mx_refine_ff(const gwt::ff4
                                                          const gwt::AccReq *__restrict__ areq, int ndet,
                                                          const gwt::AccLut *__restrict__ glut, int N, int pairs,
                                                          const int *__restrict__ cand, const int *__restrict__ ncand,
+                                                         const int *__restrict__ overflow,
                                                          const double *__restrict__ sums,
                                                          const StreamDev *__restrict__ streams,
                                                          const int *__restrict__ handles, double *__restrict__ candval) {
@@ -821,6 +825,7 @@ __global__ void __launch_bounds__(kRefineBlock, 2) k_mx_refine_ff(const gwt::ff4
   ff4 *s_wf = (ff4 *)s_wj, *s_turn = s_wf + (N + kBlock - 1) / kBlock;
   __shared__ double s_red[NV][kRefineBlock / 32];
   constexpr int kLoads = UN ? 4 : 8;  // in flight per thread
+  if (*overflow) return;
   const int nj = (N + kBlock - 1) / kBlock, tid = threadIdx.x, bin = tid % kBlock;
   bool loaded = false;
   for (int sl = blockIdx.x; sl < pairs * kCand; sl += gridDim.x) {
@@ -1030,6 +1035,7 @@ struct MxIn {
   const int *req_status = nullptr;             // per request, or null
   int n = 0, ndet = 0, N = 0;
   bool un = false;
+  bool search = true;                          // false: a search has given up on these requests
   // the results and the search's overflow flag (*overflow, on the host at
   // *h_overflow once copied) go to the host in one copy
   void *results = nullptr, *h_results = nullptr;
@@ -1160,7 +1166,7 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
     auto screen = [&](auto kern) {
       if (tw > 48 * 1024) cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tw);
       kern<<<pairs, kScreenBlock, tw, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, in.N, in.streams, in.handles,
-                                              sums, cand, ncand);
+                                              sums, ovf, cand, ncand);
     };
     if (tw <= 200 * 1024) {  // longer rows keep every candidate
       if (in.un) screen(k_mx_screen<true>);
@@ -1170,14 +1176,14 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   auto refine = [&](auto kern) {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<gr, kBlock, smem, c->stream>>>(g64, in.N, pairs, cand, ncand, sums, in.streams, in.handles, cv);
+    kern<<<gr, kBlock, smem, c->stream>>>(g64, in.N, pairs, cand, ncand, ovf, sums, in.streams, in.handles, cv);
   };
   const size_t smem_ff = smem + sizeof(gwt::ff4) * gwt::kTurnTab;
   auto refine_ff = [&](auto kern) {
     if (smem_ff > 48 * 1024)
       cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ff);
     kern<<<gr, kRefineBlock, smem_ff, c->stream>>>((const gwt::ff4 *)g64, in.areq, in.ndet, c->acc_lut, in.N, pairs, cand,
-                                             ncand, sums, in.streams, in.handles, cv);
+                                             ncand, ovf, sums, in.streams, in.handles, cv);
   };
   if (two && in.un) refine_ff(k_mx_refine_ff<true>);
   else if (two) refine_ff(k_mx_refine_ff<false>);
@@ -1189,8 +1195,8 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
   else
     k_mx_final<false><<<(in.n + 127) / 128, 128, 0, c->stream>>>(cv, ncand, sums, in.n, in.ndet, in.streams,
                                                                   in.handles, in.req_status, out, status);
-  // the last candidates of a pair with too many of them were left out: its
-  // results, computed from the others, are not used
+  // with a pair of too many candidates the screen and the refinement do nothing,
+  // and the results are not used
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return c->fail(e, "maximised likelihood launch");
   cudaMemcpyAsync(in.h_results, in.results, in.result_bytes, cudaMemcpyDeviceToHost, c->stream);
@@ -1206,7 +1212,7 @@ bool search_fits(const gwgpu_context *c, int N) { return !c->maxll_fp64 && (N + 
 // transforms' inputs (in.req) will do.
 int maxll_run(gwgpu_context *c, const MxIn &in, double *out, int *status, bool *searched = nullptr) {
   if (searched) *searched = true;
-  if (search_fits(c, in.N)) {
+  if (in.search && search_fits(c, in.N)) {
     bool fb = false;
     int st = run_search(c, in, out, status, &fb);
     if (st || !fb) return st;
@@ -1347,7 +1353,7 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
   }
   int *dst = (int *)(b + o_st);
   cudaError_t e;
-  for (;;) {
+  for (bool search = true;; search = false) {
     e = gwk::launch_prologue((const gwt::GenParams *)(b + o_p), (const int *)(b + o_a), n, (const int *)(b + o_h),
                              ndet, 0.0, 0, c->streams_dev, c->qnm_dev, two ? nullptr : (Request *)(b + o_req), nullptr,
                              0, dst, c->stream, gwk::OrderArgs(), two ? (gwt::AccReq *)(b + o_req) : nullptr);
@@ -1362,6 +1368,7 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
     in.ndet = ndet;
     in.N = N;
     in.un = un;
+    in.search = search;
     in.results = b + o_out;
     in.h_results = h + o_req;
     in.result_bytes = total - o_out;
