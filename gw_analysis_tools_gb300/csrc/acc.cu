@@ -302,18 +302,23 @@ cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet
   }
   return cudaGetLastError();
 }
-cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev *streams, int ndet,
-                             const AccTables &tab, const AccLut *lut, double *partials, unsigned *counter, double *out, cudaStream_t s) {
+bool plain_two_float(const Request &r, const StreamDev *streams, int ndet, const AccTables &tab, const AccLut *lut) {
   bool acc = lut && !r.m.status && streams[0].n0 + streams[0].N - 1 <= tab.nmax;
+  for (int d = 0; d < ndet; d++) acc = acc && streams[d].wd;
+  return acc;
+}
+cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev *streams, int ndet,
+                             const AccTables &tab, const AccLut *lut, double *partials, unsigned *counter, double *out,
+                             cudaStream_t s, const PlainTab *fp64) {
+  if (!plain_two_float(r, streams, ndet, tab, lut))
+    return launch_plain(r, streams, ndet, partials, counter, out, nullptr, s, fp64);
   double ds[kMaxDet], ws[kMaxDet];
   unsigned long long wk[kMaxDet];
   for (int d = 0; d < ndet; d++) {
-    acc = acc && streams[d].wd;
     ds[d] = streams[d].dscale;
     ws[d] = streams[d].wscale;
     wk[d] = streams[d].wkey;
   }
-  if (!acc) return launch_plain(r, streams, ndet, partials, counter, out, nullptr, s);
   AccReq x;
   fast_acc(r, fx, grid_const(streams[0].dfq), x, ds, ws, wk);
   return launch_plain_acc(x, streams, ndet, tab, lut, partials, counter, out, s);

@@ -191,6 +191,12 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   const bool ordered = form != kFormFp64 && c->order_items && !c->prologue_serial && pl.nitems > grid;
   const int mixed = form == kFormMixed;
   gwk::OrderArgs ord;
+  // FP64 bins: the cooperative prologue writes each IMRPhenomD request's
+  // coefficients on the grid after the Request records, for the bin kernel's
+  // table form (with the FP64 n^(-7/6) table)
+  gwt::WaveF64 *w64 = nullptr;
+  if (form == kFormFp64 && !c->prologue_serial && c->tm76d && c->tm76d_n > 0)
+    w64 = (gwt::WaveF64 *)((char *)reqs + sizeof(gwt::Request) * (size_t)n);
   if (ordered) {
     ord.fill = (int *)(cnt + n + 32);
     ord.items = pl.order;
@@ -209,7 +215,7 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
     e = gwk::launch_prologue((const gwt::GenParams *)d_params, d_approx, n, pl.handles, ndet, T_segment, 1,
                              c->streams_dev, c->qnm_dev, form == kFormFp64 ? (gwt::Request *)reqs : nullptr,
                              mixed ? (gwt::MixedReq *)reqs : nullptr, mixed, d_status, L.stream, ord,
-                             two_float(form) ? (gwt::AccReq *)reqs : nullptr);
+                             two_float(form) ? (gwt::AccReq *)reqs : nullptr, w64);
   if (e != cudaSuccess) return c->fail(e, "prologue launch");
   if (timing) cudaEventRecord(c->t_ev[1], L.stream);
   gwk::BatchArgs a;
@@ -232,6 +238,9 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
   a.status = d_status;
   a.status_out = status_out ? status_out : d_status;
   a.tables = c->tables;
+  a.w64 = w64;
+  a.tm76d = w64 ? c->tm76d : nullptr;
+  a.tm76d_n = w64 ? c->tm76d_n : 0;
   a.areq = two_float(form) ? (const gwt::AccReq *)reqs : nullptr;
   a.acc = c->acc;
   a.lut = c->acc_lut;
@@ -286,6 +295,9 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
       tile = acc_tile(L.shape.bins, persistent_grid(c->device, form, ndet, 0));
   }
   const int occ = choose_occ(c, mixed, L.tk);
+  // FP64 bins: the n^(-7/6) table of the table form, built before any capture (a
+  // failure leaves the frequency form)
+  if (form == kFormFp64 && c->ensure_tm76d(c->tables.nmax) != GWGPU_OK) c->last_error.clear();
   bool replanned = false;
   if (!same || !L.plan.valid || L.plan.tile != tile) {
     int st = plan_batch(c, L, n, h_handles, ndet, tile);
@@ -296,7 +308,9 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
     L.plan.valid = true;
     replanned = true;
   }
-  size_t rq = mixed ? sizeof(gwt::MixedReq) : two_float(form) ? sizeof(gwt::AccReq) : sizeof(gwt::Request);
+  size_t rq = mixed ? sizeof(gwt::MixedReq)
+              : two_float(form) ? sizeof(gwt::AccReq)
+                                : sizeof(gwt::Request) + sizeof(gwt::WaveF64);
   size_t bytes = rq * n + 512 + sizeof(double) * (size_t)L.plan.nitems * gwk::kAcc + 256 +
                  sizeof(unsigned) * (size_t)(2 * (size_t)n + 32 + gwk::kOrderBuckets);
   void *old = L.work;
@@ -308,7 +322,7 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
   }
   char *p = (char *)L.work;
   void *reqs = p;
-  p = align256(p + rq * n);
+  p = align256(p + rq * n);  // FP64 bins: Request[n], then WaveF64[n]
   double *partials = (double *)p;
   p = align256(p + sizeof(double) * (size_t)L.plan.nitems * gwk::kAcc);
   unsigned *cnt = (unsigned *)p;

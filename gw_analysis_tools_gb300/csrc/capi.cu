@@ -440,6 +440,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   bool line = d.uniform_int;
   if (line) d.dfq = gwt::acc_spacing(freqs[N - 1], d.n0 + N - 1);
   for (int k = 0; k < N && line; k++) line = gwt::acc_on_line(freqs[k], d.n0 + k, d.dfq);
+  d.line = line;
   if (!line) {
     double fmax = 0;
     for (int k = 0; k < N; k++) fmax = std::fmax(fmax, freqs[k]);
@@ -713,7 +714,21 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   if (st) return st;
   cudaError_t e = cudaHostGetDevicePointer((void **)&hd, h, 0);
   if (e != cudaSuccess) return c->fail(e, "plain result mapping");
-  e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream);
+  // FP64 bins of IMRPhenomD on grids of n dfq: the waveform from the request's
+  // coefficients on the grid and the power tables
+  gwk::PlainTab pt;
+  const int nlast = sd[0].n0 + sd[0].N - 1;
+  if (!gwk::plain_two_float(r, sd, ndet, c->acc, c->acc_lut) && ap == gwt::kPhenomD && !r.m.status) {
+    bool line = true;
+    for (int d = 0; d < ndet; d++) line = line && sd[d].line;
+    if (line && nlast <= c->tables.nmax && c->ensure_tm76d(nlast) == GWGPU_OK && nlast <= c->tm76d_n) {
+      gwt::wave64_prologue(r, sd[0].dfq, pt.w);
+      pt.t = c->tables;
+      pt.tm76d = c->tm76d;
+      pt.use = 1;
+    }
+  }
+  e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream, &pt);
   if (e != cudaSuccess) return c->fail(e, "plain launch");
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return c->fail(e, "plain");

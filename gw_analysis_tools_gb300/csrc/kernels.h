@@ -42,6 +42,7 @@ struct StreamDev {
   const gwt::ff *wf;
   const float *dev;
   double dfq;
+  int line;                    // 1: f_k = (n0 + k) dfq to its rounding (acc_on_line)
   const gwt::GridConst *grid;  // of df, of dfq
   const gwt::AccNodes *node;   // grids that are not n dfq: the same by node (dfq the nodes' scale), or null
 };
@@ -67,18 +68,29 @@ cudaError_t launch_inner_product(const double *data, const double *psd, const do
 // The same with integration weights iw (4 w_i, times f_i ln 10 for log10F).
 cudaError_t launch_inner_product_weighted(const double *data, const double *psd, const double *resp, const double *iw,
                                           int N, double *partials, unsigned *counter, double *out, cudaStream_t s);
+// FP64 bins on grids of n dfq, IMRPhenomD: the waveform from the request's
+// coefficients on the grid (wave64_prologue) and the n-indexed power tables
+// instead of the powers, logarithm and cube root of each frequency.
+struct PlainTab {
+  gwt::WaveF64 w;
+  gwt::Tables t;
+  const double *tm76d = nullptr;  // n^(-7/6), FP64
+  int use = 0;                    // 1: the tables cover every bin of the call
+};
 // Plain form: one request, FP64, one launch.  out[0] = log L.
 cudaError_t launch_plain(const Request &r, const StreamDev *streams, int ndet, double *partials, unsigned *counter,
-                         double *out, int *status, cudaStream_t s);
+                         double *out, int *status, cudaStream_t s, const PlainTab *tab = nullptr);
 // The same on two-float bins (every stream has wd, wf; x from acc_prologue; one partial sum per block).
 cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
                              const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
                              cudaStream_t s);
 // One of the two: two-float bins when every stream has its pairs (and the
 // tables reach its grid), else FP64 bins.  partials: 2 kMaxDet per block.
+bool plain_two_float(const Request &r, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
+                     const gwt::AccLut *lut);
 cudaError_t launch_plain_any(const Request &r, const gwt::FastX &fx, const StreamDev *streams, int ndet,
                              const gwt::AccTables &tab, const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
-                             cudaStream_t s);
+                             cudaStream_t s, const PlainTab *fp64 = nullptr);
 int plain_blocks(int N);
 cudaError_t plain_acc_preload();
 cudaError_t plain_preload();  // loads the plain kernels' module (function-attribute query)
@@ -99,7 +111,8 @@ struct OrderArgs {
 cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
                             Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s,
-                            const OrderArgs &ord = OrderArgs(), AccReq *areq = nullptr);
+                            const OrderArgs &ord = OrderArgs(), AccReq *areq = nullptr,
+                            gwt::WaveF64 *w64 = nullptr);
 // One thread per request (the reference order of the prologue); kept to check
 // the cooperative kernel against.
 cudaError_t launch_prologue_serial(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
@@ -127,7 +140,13 @@ struct BatchArgs {
   int *status;      // per-request working status (device memory: the bounds flag is set atomically)
   int *status_out;  // where the finalize writes each request's status (status itself, or mapped host memory)
   gwt::Tables tables;
-  // FP64 form on two-float bins (null: every bin from its frequency, req)
+  // FP64 bins (req): IMRPhenomD's coefficients on grids of n dfq, written by the
+  // prologue (null: every bin from its frequency), and the FP64 n^(-7/6) table
+  // for n <= tm76d_n
+  const gwt::WaveF64 *w64 = nullptr;
+  const double *tm76d = nullptr;
+  int tm76d_n = 0;
+  // FP64 form on two-float bins (null: FP64 bins)
   const AccReq *areq = nullptr;
   gwt::AccTables acc{};
   const gwt::AccLut *lut = nullptr;
