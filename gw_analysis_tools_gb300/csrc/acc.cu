@@ -185,8 +185,9 @@ __global__ void __launch_bounds__(kAccBlock, 5) k_batch_acc(const BatchArgs a) {
 struct PlainAccStreams {
   StreamDev s[kMaxDet];
 };
-// One bin per thread; the last block adds the blocks' sums.
-template <int NDET>
+// One bin per thread; the last block adds the blocks' sums.  NODES: the grid's
+// node arrays instead of the bins (beyond the cut a node adds nothing).
+template <int NDET, bool NODES>
 __global__ void __launch_bounds__(kPlainBlock) k_plain_acc(const __grid_constant__ AccReq x,
                                                            const __grid_constant__ PlainAccStreams ps,
                                                            const __grid_constant__ AccTables tb,
@@ -194,12 +195,21 @@ __global__ void __launch_bounds__(kPlainBlock) k_plain_acc(const __grid_constant
                                                            unsigned *counter, double *out) {
   __shared__ AccLut lut;
   __shared__ double s_red[kPlainBlock / 32];
+  __shared__ StreamDev s_st[NODES ? NDET : 1];
+  __shared__ AccNodes s_nodes;
   const int tid = threadIdx.x, N = ps.s[0].N, k0 = blockIdx.x * kPlainBlock;
   double v = 0.0;
-  if (k0 < x.m.n_cut - ps.s[0].n0 + 1) {
+  if (NODES || k0 < x.m.n_cut - ps.s[0].n0 + 1) {
     copy_words(&lut, glut, sizeof(AccLut));
+    if (NODES && tid < NDET) {
+      StreamDev s = ps.s[tid];
+      s.wd = s.node->wd;
+      s.wf = s.node->wf;
+      if (tid == 0) s_nodes = *s.node;
+      s_st[tid] = s;
+    }
     __syncthreads();
-    v = acc_block<NDET>(x, ps.s, tb, lut, nullptr, k0, min(k0 + kPlainBlock, N), s_red);
+    v = acc_block<NDET>(x, NODES ? s_st : ps.s, tb, lut, NODES ? &s_nodes : nullptr, k0, min(k0 + kPlainBlock, N), s_red);
   }
   if (tid == 0) partials[blockIdx.x] = v;
   if (arrive_last(counter, gridDim.x)) {
@@ -288,24 +298,34 @@ cudaError_t launch_batch_acc(const BatchArgs &a, bool nodes, int grid, cudaStrea
   void *args[] = {(void *)&a};
   return launch_dependent(f, dim3(grid), dim3(kAccBlock), args, s, pdl);
 }
+template <int NDET>
+static void launch_plain_acc(const AccReq &x, const PlainAccStreams &ps, bool nodes, const AccTables &tab,
+                             const AccLut *lut, double *partials, unsigned *counter, double *out, cudaStream_t s) {
+  const int grid = plain_blocks(ps.s[0].N);
+  if (nodes) k_plain_acc<NDET, true><<<grid, kPlainBlock, 0, s>>>(x, ps, tab, lut, partials, counter, out);
+  else k_plain_acc<NDET, false><<<grid, kPlainBlock, 0, s>>>(x, ps, tab, lut, partials, counter, out);
+}
 cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet, const AccTables &tab,
                              const AccLut *lut, double *partials, unsigned *counter, double *out, cudaStream_t s) {
   PlainAccStreams ps;
   for (int d = 0; d < ndet; d++) ps.s[d] = streams[d];
-  const int grid = plain_blocks(streams[0].N);
+  const bool nodes = streams[0].node != nullptr;
   switch (ndet) {
-    case 1: k_plain_acc<1><<<grid, kPlainBlock, 0, s>>>(x, ps, tab, lut, partials, counter, out); break;
-    case 2: k_plain_acc<2><<<grid, kPlainBlock, 0, s>>>(x, ps, tab, lut, partials, counter, out); break;
-    case 3: k_plain_acc<3><<<grid, kPlainBlock, 0, s>>>(x, ps, tab, lut, partials, counter, out); break;
-    case 4: k_plain_acc<4><<<grid, kPlainBlock, 0, s>>>(x, ps, tab, lut, partials, counter, out); break;
+    case 1: launch_plain_acc<1>(x, ps, nodes, tab, lut, partials, counter, out, s); break;
+    case 2: launch_plain_acc<2>(x, ps, nodes, tab, lut, partials, counter, out, s); break;
+    case 3: launch_plain_acc<3>(x, ps, nodes, tab, lut, partials, counter, out, s); break;
+    case 4: launch_plain_acc<4>(x, ps, nodes, tab, lut, partials, counter, out, s); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
 }
 bool plain_two_float(const Request &r, const StreamDev *streams, int ndet, const AccTables &tab, const AccLut *lut) {
-  bool acc = lut && !r.m.status && streams[0].n0 + streams[0].N - 1 <= tab.nmax;
-  for (int d = 0; d < ndet; d++) acc = acc && streams[d].wd;
-  return acc;
+  bool bins = lut && !r.m.status && streams[0].n0 + streams[0].N - 1 <= tab.nmax, nodes = lut && !r.m.status;
+  for (int d = 0; d < ndet; d++) {
+    bins = bins && streams[d].wd;
+    nodes = nodes && streams[d].node;
+  }
+  return bins || nodes;
 }
 cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev *streams, int ndet,
                              const AccTables &tab, const AccLut *lut, double *partials, unsigned *counter, double *out,
@@ -321,14 +341,20 @@ cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev 
   }
   AccReq x;
   fast_acc(r, fx, grid_const(streams[0].dfq), x, ds, ws, wk);
+  if (streams[0].node) acc_node_coeffs(r, streams[0].dfq, x);
   return launch_plain_acc(x, streams, ndet, tab, lut, partials, counter, out, s);
 }
-cudaError_t plain_acc_preload() {
+template <int NDET>
+static cudaError_t plain_acc_preload_n() {
   cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, k_plain_acc<1>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_acc<2>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_acc<3>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_acc<4>);
+  const cudaError_t e = cudaFuncGetAttributes(&a, k_plain_acc<NDET, false>);
+  return e == cudaSuccess ? cudaFuncGetAttributes(&a, k_plain_acc<NDET, true>) : e;
+}
+cudaError_t plain_acc_preload() {
+  cudaError_t e = plain_acc_preload_n<1>();
+  if (e == cudaSuccess) e = plain_acc_preload_n<2>();
+  if (e == cudaSuccess) e = plain_acc_preload_n<3>();
+  if (e == cudaSuccess) e = plain_acc_preload_n<4>();
   return e;
 }
 cudaError_t launch_acc_tables(const AccTables &tab, cudaStream_t s) {

@@ -80,12 +80,15 @@ struct PlainTab {
 // Plain form: one request, FP64, one launch.  out[0] = log L.
 cudaError_t launch_plain(const Request &r, const StreamDev *streams, int ndet, double *partials, unsigned *counter,
                          double *out, int *status, cudaStream_t s, const PlainTab *tab = nullptr);
-// The same on two-float bins (every stream has wd, wf; x from acc_prologue; one partial sum per block).
+// The same on two-float bins (every stream has wd, wf, or every one node; x from
+// acc_prologue, and acc_node_coeffs for nodes; one partial sum per block).
 cudaError_t launch_plain_acc(const AccReq &x, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
                              const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
                              cudaStream_t s);
 // One of the two: two-float bins when every stream has its pairs (and the
-// tables reach its grid), else FP64 bins.  partials: 2 kMaxDet per block.
+// tables reach its grid) or its nodes, else FP64 bins.  partials: 2 kMaxDet per
+// block.  3 x 32,128 bins 1e-8 Hz off the line: IMRPhenomD 22 us, IMRPhenomPv2 27
+// (FP64 bins 48 and 67).
 bool plain_two_float(const Request &r, const StreamDev *streams, int ndet, const gwt::AccTables &tab,
                      const gwt::AccLut *lut);
 cudaError_t launch_plain_any(const Request &r, const gwt::FastX &fx, const StreamDev *streams, int ndet,
