@@ -367,7 +367,8 @@ __global__ void __launch_bounds__(kBlock, UN ? 2 : 4) k_mx_prep_ff(const gwt::Ac
   __shared__ __align__(16) unsigned char s_req[sizeof(AccReq)];
   __shared__ StreamDev s_st[kMaxDet];
   __shared__ ff s_sc[kMaxDet];
-  __shared__ double s_hs[kMaxDet], s_red[kMaxDet * NS][kWarps];
+  __shared__ float s_un[kMaxDet];  // about 1 / s_sc, a power of two: |g|^2 is summed without its scale's square
+  __shared__ double s_hs[kMaxDet], s_gs[kMaxDet], s_red[kMaxDet * NS][kWarps];
   const int r = blockIdx.y, tid = threadIdx.x;
   const AccReq &x = *(const AccReq *)s_req;
   const int k0 = blockIdx.x * kPrepTile, k1 = min(k0 + kPrepTile, pad);
@@ -384,6 +385,9 @@ __global__ void __launch_bounds__(kBlock, UN ? 2 : 4) k_mx_prep_ff(const gwt::Ac
     const StreamDev &st = s_st[tid];
     const double A = areq[r].m.A_scale;
     s_sc[tid] = ff_split(A * (3.0 * st.dscale / st.simpson_df));
+    const int e = min(126, max(-126, s_sc[tid].h != 0.0f ? ilogbf(s_sc[tid].h) : 0));
+    s_un[tid] = ldexpf(1.0f, -e);
+    s_gs[tid] = ldexp(1.0, 2 * e);
     s_hs[tid] = A * A * st.wscale * (3.0 / (4.0 * st.simpson_df));
   }
   __syncthreads();
@@ -415,11 +419,13 @@ __global__ void __launch_bounds__(kBlock, UN ? 2 : 4) k_mx_prep_ff(const gwt::Ac
       const float2 wv = __ldg((const float2 *)s_st[dd].wf + k);
       const ff wk{wv.x, wv.y}, sc{s_sc[dd].h * is, s_sc[dd].l * is};
       const ff dr = ff_norm(ff_mul(ff{w.ch, w.cl}, sc)), di = ff_norm(ff_mul(ff{w.sh, w.sl}, sc));
+      const float un = s_un[dd];
       auto product = [&](ff hr, ff hi, size_t row, ff &nn) {  // 4 conj(d) h / S
         const ff vr = ff_norm(ff_add(ff_mul(dr, hr), ff_mul(di, hi))), vi = ff_norm(ff_sub(ff_mul(dr, hi), ff_mul(di, hr)));
         g[row * N + k] = ff4{vr.h, vr.l, vi.h, vi.l};
         a32[row * ld + k] = make_float2(vr.h * ch.x - vi.h * ch.y, vr.h * ch.y + vi.h * ch.x);
-        nn.h = fmaf(vr.h, vr.h, fmaf(vi.h, vi.h, nn.h));  // |g|^2 for the search's error bound
+        const float ur = vr.h * un, ui = vi.h * un;
+        nn.h = fmaf(ur, ur, fmaf(ui, ui, nn.h));  // |g|^2 for the search's error bound
       };
       ff_acc(acc[dd * NS], ff_mul(wk, hh));
       if constexpr (UN) {
@@ -449,7 +455,7 @@ __global__ void __launch_bounds__(kBlock, UN ? 2 : 4) k_mx_prep_ff(const gwt::Ac
     double t = 0.0;
     for (int w = 0; w < kWarps; w++) t += s_red[tid][w];
     const int j = tid % NS;
-    part[((size_t)r * ndet * NS + tid) * gridDim.x + blockIdx.x] = j < (UN ? 3 : 1) ? t * s_hs[tid / NS] : t;
+    part[((size_t)r * ndet * NS + tid) * gridDim.x + blockIdx.x] = t * (j < (UN ? 3 : 1) ? s_hs : s_gs)[tid / NS];
   }
 }
 
