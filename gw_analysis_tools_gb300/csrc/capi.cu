@@ -411,6 +411,27 @@ static cudaError_t acc_nodes(gwgpu_context *c, StreamDev &d, size_t row, char *p
   return e;
 }
 
+// Whether FP32's exponents hold the pairs W / wscale and W d / dscale and what
+// the bins make of them to their 48 bits.  A term of the sums is the pair times
+// the amplitude's square, about x^(-7/3), or x^(-7/6), at bin x; its digits stay
+// normal numbers down to 2^-78, taken as 2^-72.  Every weight that is not zero
+// has to be within that of the largest: a PSD filled with 1e-100 beyond the band
+// would else push every live bin's weight to zero (a PSD of infinity does no
+// harm).  Data may fall to nothing where a signal does, but not in more than half of their bins.
+static bool pairs_hold(const StreamDev &d, const double *freqs, const double *data, const std::vector<double> &W) {
+  const double lim = 0x1p-72, x1 = *std::max_element(freqs, freqs + d.N) / d.dfq;
+  const double w1 = lim * std::pow(x1, 7. / 3.) * d.wscale, d1 = lim * std::pow(x1, 7. / 6.) * d.dscale;
+  int some = 0, small = 0;
+  for (int k = 0; k < d.N; k++) {
+    const double w = std::fabs(W[k]);
+    if (w > 0 && w < w1 && w < lim * std::pow(freqs[k] / d.dfq, 7. / 3.) * d.wscale) return false;
+    const double m = w * (std::fabs(data[2 * k]) + std::fabs(data[2 * k + 1]));
+    some += m > 0;
+    small += m > 0 && m < d1;
+  }
+  return 2 * small <= some;
+}
+
 // One detector stream; weights (GAUSSLEG) or null (Simpson's rule).
 static int register_stream(gwgpu_context *c, const char *detector, const double *freqs, int N, const double *data,
                            const double *psd, const double *weights, int log10F, int *handle) {
@@ -472,6 +493,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     dh[2 * k + 1] = (float)(W[k] * data[2 * k + 1] / d.dscale);
     wh[k] = (float)(W[k] / d.wscale);
   }
+  const bool two_float = finite && pairs_hold(d, freqs, data, W);
   int st;
   std::vector<double> ip(N);  // the reciprocal PSD: the FP64 kernels multiply instead of dividing
   for (int k = 0; k < N; k++) ip[k] = 1.0 / psd[k];
@@ -479,8 +501,8 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   const size_t row = ((size_t)N + 31) / 32 * 32, gat = row * (weights ? 60 : 52);
   const size_t nat = gat + 2 * sizeof(gwt::GridConst);
   // two-float arrays, by bin or by node, behind them
-  bool pairs = line && finite && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
-  bool nodes = !line && finite && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
+  bool pairs = line && two_float && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
+  bool nodes = !line && two_float && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
   const size_t more = pairs ? 28 * row : nodes ? nodes_bytes(row) : 0;
   char *mem;
   st = c->dalloc((void **)&mem, nat + more, "data stream");
