@@ -259,7 +259,8 @@ static int launch_sequence(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_
 int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, const int *d_approx, int n,
                   const int *h_handles, int ndet, double T_segment, int precision, double *d_out, int *d_status,
                   int tile, bool use_graph, const BatchCopies *io, int *status_out) {
-  const int mixed = precision == GWGPU_PREC_MIXED;
+  const int mixed = precision == GWGPU_PREC_MIXED, tile_arg = tile;
+  const bool off = c->two_float_off;
   const gwgpu_context::Stream *s0 = c->get_stream(h_handles[0]);
   if (!s0) return GWGPU_ENOTFOUND;
   // the batch shape (handles, sizes, registrations, precision) of the last
@@ -316,6 +317,9 @@ int enqueue_batch(gwgpu_context *c, Lane &L, const gwgpu_gen_params *d_params, c
   void *old = L.work;
   int st = lane_alloc(c, L, &L.work, &L.work_cap, bytes, "batch scratch");
   if (st) return st;
+  if (c->two_float_off != off)  // the two-float arrays gave way to the plan or the scratch
+    return enqueue_batch(c, L, d_params, d_approx, n, h_handles, ndet, T_segment, precision, d_out, d_status, tile_arg,
+                         use_graph, io, status_out);
   if (L.work != old || replanned) {  // captured graphs hold the old addresses
     for (auto &g : L.graphs) cudaGraphExecDestroy(g.second.exec);
     L.graphs.clear();
@@ -383,6 +387,8 @@ int gwgpu_loglik_batch_device(gwgpu_context *c, const gwgpu_gen_params *d_params
   cudaSetDevice(c->device);
   cudaStream_t user = (cudaStream_t)stream;
   gwb::Lane &L = c->lane0();
+  c->hold_if_capturing(user);
+  c->hold_if_capturing(L.stream);
   if (user && user != L.stream) {  // order after the caller's stream, then make it wait for us
     cudaEventRecord(c->ev_in, user);
     cudaStreamWaitEvent(L.stream, c->ev_in, 0);

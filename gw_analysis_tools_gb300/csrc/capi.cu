@@ -62,16 +62,59 @@ int gwgpu_context::fail(cudaError_t e, const char *where) {
   return GWGPU_ECUDA;
 }
 
-int gwgpu_context::dalloc(void **p, size_t bytes, const char *what) {
-  if (budget && in_use + bytes > budget) {
+// two_float: for two-float arrays, which do not displace others.
+int gwgpu_context::dalloc(void **p, size_t bytes, const char *what, bool two_float) {
+  if (two_float ? budget && in_use + bytes > budget : !room(bytes)) {
     last_error = std::string("HBM budget exceeded allocating ") + what;
     return GWGPU_ENOMEM;
   }
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !two_float && drop_two_float(0)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) return fail(e, what);
   sizes[*p] = bytes;
   in_use += bytes;
   return GWGPU_OK;
+}
+// Whether the budget holds so many bytes more, without the two-float arrays if need be.
+bool gwgpu_context::room(size_t bytes) { return !budget || in_use + bytes <= budget || drop_two_float(bytes); }
+// Frees every two-float array and table (see capi_internal.h); false where that
+// does not make room for bytes.
+bool gwgpu_context::drop_two_float(size_t bytes) {
+  size_t held = 0;
+  for (void *q : acc_mem) held += sizes[q];
+  for (const Stream &s : streams)
+    if (s.pairs) held += sizes[s.pairs];
+  if (!held || two_float_held || (budget && in_use - held + bytes > budget)) return false;
+  if (cudaDeviceSynchronize() != cudaSuccess) return false;  // launches in flight read them
+  for (Stream &s : streams) {
+    dfree(s.pairs);
+    s.pairs = nullptr;
+    s.dev.wd = nullptr;
+    s.dev.wf = nullptr;
+    s.dev.dev = nullptr;
+    s.dev.node = nullptr;
+  }
+  for (void *q : acc_mem) dfree(q);
+  acc_mem.clear();
+  acc = gwt::AccTables{};
+  two_float_off = true;
+  streams_epoch++;
+  if (streams_dev) {
+    std::vector<StreamDev> v;
+    for (const Stream &s : streams) v.push_back(s.dev);
+    cudaMemcpyAsync(streams_dev, v.data(), sizeof(StreamDev) * std::min(v.size(), streams_dev_cap), cudaMemcpyHostToDevice,
+                    stream);
+    cudaStreamSynchronize(stream);
+  }
+  return true;
+}
+void gwgpu_context::hold_if_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (s && !two_float_held && cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone)
+    two_float_held = true;
 }
 void gwgpu_context::dfree(void *p) {
   if (!p) return;
@@ -198,22 +241,22 @@ int gwgpu_context::ensure_lut() {
   std::vector<gwt::AccLut> h(1);
   gwt::ff_fill_tables(h[0].turn, h[0].ex);
   void *p;
-  int st = dalloc(&p, sizeof(gwt::AccLut), "sine table");
+  int st = dalloc(&p, sizeof(gwt::AccLut), "sine table", true);
   if (st) return st;
-  cudaError_t e = cudaMemcpy(p, h.data(), sizeof(gwt::AccLut), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpyAsync(p, h.data(), sizeof(gwt::AccLut), cudaMemcpyHostToDevice, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return fail(e, "sine table");
   acc_lut = (gwt::AccLut *)p;
   return GWGPU_OK;
 }
 int gwgpu_context::ensure_acc(int nmax) {
-  int st = ensure_tables(nmax);
-  if (!st) st = ensure_lut();
+  int st = ensure_lut();
   if (st) return st;
   if (nmax <= acc.nmax) return GWGPU_OK;
   // twice the block before, which stays: all of them together less than twice the last
   const size_t n1 = (size_t)std::max(nmax, std::min(std::max(2 * acc.nmax, 1 << 16), gwt::kAccMaxN)) + 1;
   void *p;
-  if ((st = dalloc(&p, 80 * n1, "two-float tables"))) return st;
+  if ((st = dalloc(&p, 80 * n1, "two-float tables", true))) return st;
   gwt::AccTables t;
   gwt::ff4 *q = (gwt::ff4 *)p;
   t.pw = q;
@@ -241,6 +284,7 @@ int gwgpu_context::ensure_acc(int nmax) {
     dfree(p);
     return fail(e, "two-float tables");
   }
+  acc_mem.push_back(p);
   acc = t;
   return GWGPU_OK;
 }
@@ -498,19 +542,30 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   std::vector<double> ip(N);  // the reciprocal PSD: the FP64 kernels multiply instead of dividing
   for (int k = 0; k < N; k++) ip[k] = 1.0 / psd[k];
   // one allocation for the stream's arrays, each on a 256-byte boundary
-  const size_t row = ((size_t)N + 31) / 32 * 32, gat = row * (weights ? 60 : 52);
-  const size_t nat = gat + 2 * sizeof(gwt::GridConst);
-  // two-float arrays, by bin or by node, behind them
-  bool pairs = line && two_float && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
-  bool nodes = !line && two_float && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
-  const size_t more = pairs ? 28 * row : nodes ? nodes_bytes(row) : 0;
-  char *mem;
-  st = c->dalloc((void **)&mem, nat + more, "data stream");
-  if (st && more) {  // without them the stream keeps the FP64 bins
-    pairs = nodes = false;
-    st = c->dalloc((void **)&mem, nat, "data stream");
+  const size_t row = ((size_t)N + 63) / 64 * 64, gat = row * (weights ? 60 : 52);
+  char *mem, *more = nullptr;
+  // with the bin tables at once, so that nothing is given up for a registration that fails
+  size_t tab = 0;
+  if (d.uniform_int && d.n0 + N > c->tables.nmax) {
+    tab = 40 * (size_t)(std::max(d.n0 + N, 1 << 16) + 1);
+    for (void *q : c->table_mem) tab -= c->sizes[q];
   }
-  if (st) return st;
+  if (!c->room(gat + 2 * sizeof(gwt::GridConst) + tab)) {
+    c->last_error = "HBM budget exceeded allocating data stream";
+    return GWGPU_ENOMEM;
+  }
+  if ((st = c->dalloc((void **)&mem, gat + 2 * sizeof(gwt::GridConst), "data stream"))) return st;
+  if (d.uniform_int && (st = c->ensure_tables(d.n0 + N))) {
+    c->dfree(mem);
+    return st;
+  }
+  // and one for the two-float arrays, by bin or by node; where there is no memory
+  // for them the stream keeps the FP64 bins
+  const bool fit = two_float && !c->two_float_off;
+  bool pairs = fit && line && (long long)d.n0 + N <= gwt::kAccMaxN && c->ensure_acc(d.n0 + N) == GWGPU_OK;
+  bool nodes = fit && !line && nodes_fit(d, freqs) && c->ensure_lut() == GWGPU_OK;
+  if ((pairs || nodes) && c->dalloc((void **)&more, pairs ? 28 * row : nodes_bytes(row), "two-float stream", true))
+    pairs = nodes = false;
   c->last_error.clear();
   const gwt::GridConst gc[2] = {gwt::grid_const(d.df), gwt::grid_const(d.dfq)};
   cudaMemcpyAsync(mem + gat, gc, sizeof(gc), cudaMemcpyHostToDevice, c->stream);
@@ -531,14 +586,16 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   d.dhat = (const float *)pdh;
   d.what = (const float *)pwh;
   d.iw = (const double *)piw;
-  cudaError_t e = pairs ? acc_stream(c, d, freqs, row, mem + nat) : nodes ? acc_nodes(c, d, row, mem + nat) : cudaSuccess;
+  cudaError_t e = pairs ? acc_stream(c, d, freqs, row, more) : nodes ? acc_nodes(c, d, row, more) : cudaSuccess;
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     c->dfree(mem);
+    c->dfree(more);
     return c->fail(e, "data upload");
   }
   s.live = true;
   s.mem = {mem};
+  s.pairs = more;
   s.host_freqs.assign(freqs, freqs + N);
   uint64_t hsh = 1469598103934665603ull;
   auto mix = [&](const double *v) {
@@ -558,10 +615,6 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
     const unsigned char *gb = (const unsigned char *)gv;
     for (size_t i = 0; i < sizeof(gv); i++) gk = (gk ^ gb[i]) * 1099511628211ull;
     s.dev.wkey = gk;
-  }
-  if (d.uniform_int && (st = c->ensure_tables(d.n0 + N))) {
-    c->dfree(mem);
-    return st;
   }
   c->streams.push_back(s);
   *handle = (int)c->streams.size() - 1;
@@ -586,6 +639,8 @@ int gwgpu_data_release(gwgpu_context *c, int handle) {
   if (handle < 0 || handle >= (int)c->streams.size() || !c->streams[handle].live) return GWGPU_ENOTFOUND;
   cudaStreamSynchronize(c->stream);
   for (void *p : c->streams[handle].mem) c->dfree(p);
+  c->dfree(c->streams[handle].pairs);
+  c->streams[handle].pairs = nullptr;
   c->streams[handle].live = false;
   c->streams[handle].dev.N = 0;
   return c->sync_streams_table();
@@ -736,6 +791,7 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   if (st) return st;
   cudaError_t e = cudaHostGetDevicePointer((void **)&hd, h, 0);
   if (e != cudaSuccess) return c->fail(e, "plain result mapping");
+  for (int d = 0; d < ndet; d++) sd[d] = c->get_stream(handles[d])->dev;  // an allocation may have changed them
   // FP64 bins of IMRPhenomD on grids of n dfq: the waveform from the request's
   // coefficients on the grid and the power tables
   gwk::PlainTab pt;

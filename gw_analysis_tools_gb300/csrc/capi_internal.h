@@ -22,6 +22,7 @@ struct gwgpu_context {
     gwk::StreamDev dev;
     bool live = false;
     std::vector<void *> mem;
+    void *pairs = nullptr;  // the two-float arrays that dev points to
     std::vector<double> host_freqs;
     uint64_t psd_hash = 0;  // FNV-1a of the PSD bytes: detectors with equal PSDs share weights
   };
@@ -45,6 +46,12 @@ struct gwgpu_context {
   // caller may hold their addresses); each is twice the one before, up to kAccMaxN.
   gwt::AccTables acc{};
   gwt::AccLut *acc_lut = nullptr;
+  std::vector<void *> acc_mem;
+  // Two-float arrays and tables give way where the memory for anything else does
+  // not suffice (dalloc), and the context keeps FP64 bins from then on: what it
+  // could do without them it can do.  Callers that decide by them look again
+  // after they have allocated.  They stay once a caller's captured launches may hold them.
+  bool two_float_off = false, two_float_held = false;
   double *tm76d = nullptr;  // FP64 n^(-7/6), built on first Fisher use
   int tm76d_n = 0;
   std::vector<Stream> streams;
@@ -77,7 +84,10 @@ struct gwgpu_context {
 
   ~gwgpu_context();
   int fail(cudaError_t e, const char *where);
-  int dalloc(void **p, size_t bytes, const char *what);
+  int dalloc(void **p, size_t bytes, const char *what, bool two_float = false);
+  bool room(size_t bytes);
+  bool drop_two_float(size_t bytes);
+  void hold_if_capturing(cudaStream_t s);  // a launch captured by the caller keeps the addresses it reads
   void dfree(void *p);
   int workspace(int slot, size_t bytes, void **out);
   int pinned(int slot, size_t bytes, void **out);

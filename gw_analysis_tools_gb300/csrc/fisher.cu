@@ -621,21 +621,28 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   int st = c->ensure_tm76d(s0->dev.n0 + s0->dev.N);
   if (st) return st;
   // Two-float sums for the FP64 calls without an inverse, on streams that have
-  // their two-float weights.
+  // their two-float weights and where there is memory for the sources' pairs.
   bool two_float = acc64 && !covariance;
   for (const auto *s : ws) two_float = two_float && s->dev.wf != nullptr;
   constexpr int kTile = 4096;  // of the FP64 and mixed sums: fewer tiles than kFfTile's
-  const int N = s0->dev.N, ntiles = (N + (two_float ? kFfTile : kTile) - 1) / (two_float ? kFfTile : kTile);
+  const int N = s0->dev.N;
   const double df = s0->dev.df;
   // chunk sources to bound the scratch
   const int chunk = std::min(n, 2048);
-  size_t bytes = sizeof(GenParams) * chunk + sizeof(SlotOut) * (size_t)chunk * kSlots + sizeof(FisherSrc) * chunk +
-                 sizeof(double) * (size_t)chunk * ntiles * kMaxDet * kSums + sizeof(double) * (size_t)chunk * 2 * kDim * kDim +
-                 sizeof(int) * (chunk + 8) + sizeof(unsigned) * (chunk + 8) + sizeof(FfSrc) * (two_float ? chunk : 0) +
-                 2048;
+  int ntiles;
   void *dev;
-  st = c->workspace(gwgpu_context::kWsFisher + 10, bytes, &dev);
-  if (st) return st;
+  for (;;) {
+    const int tile = two_float ? kFfTile : kTile;
+    ntiles = (N + tile - 1) / tile;
+    const size_t bytes = sizeof(GenParams) * chunk + sizeof(SlotOut) * (size_t)chunk * kSlots + sizeof(FisherSrc) * chunk +
+                         sizeof(double) * (size_t)chunk * ntiles * kMaxDet * kSums +
+                         sizeof(double) * (size_t)chunk * 2 * kDim * kDim + sizeof(int) * (chunk + 8) +
+                         sizeof(unsigned) * (chunk + 8) + sizeof(FfSrc) * (two_float ? chunk : 0) + 2048;
+    st = c->workspace(gwgpu_context::kWsFisher + 10, bytes, &dev);
+    if (!st) break;
+    if (!two_float) return st;
+    two_float = false;
+  }
   auto align = [](char *p) { return (char *)(((uintptr_t)p + 255) & ~(uintptr_t)255); };
   char *p = (char *)dev;
   GenParams *dparams = (GenParams *)p;
@@ -697,6 +704,7 @@ int gwf_moment_run(gwgpu_context *c, const gwgpu_gen_params *params, int n, int 
   }
   for (int s0i = 0; s0i < n; s0i += chunk) {
     int m = std::min(chunk, n - s0i);
+    two_float = two_float && !c->two_float_off;  // its arrays may have given way to an allocation
     cudaMemcpyAsync(dparams, params + s0i, sizeof(GenParams) * m, cudaMemcpyHostToDevice, c->stream);
     int tot = m * kSlots;
     k_fisher_slots<<<(tot + 63) / 64, 64, 0, c->stream>>>(dparams, m, method, ddets, ndet, df, epsilon, step_mode,

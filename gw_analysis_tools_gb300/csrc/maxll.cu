@@ -1097,7 +1097,8 @@ int run_fp64(gwgpu_context *c, const MxIn &in, double *out, int *status) {
 }
 
 // The FP32 search and its refinement; *fallback set when a pair had more
-// candidates than kCand (nothing written to out then).  128 IMRPhenomD requests
+// candidates than kCand, or the two-float arrays gave way to an allocation
+// (nothing written to out then).  128 IMRPhenomD requests
 // on 3 x 32,128 bins, device time by kernel: products 97, transforms and chirp
 // 209 (conv.cu; 434 with library transforms), candidates 55 (132 with its FP64 sums on every warp), screen 31 and
 // two-float refinement 46 (389 for FP64 sums of every candidate over the whole
@@ -1127,6 +1128,10 @@ int run_search(gwgpu_context *c, const MxIn &in, double *out, int *status, bool 
                total = o_v + up256(8 * (size_t)pairs * kCand);
   void *dev;
   if ((st = c->workspace(gwgpu_context::kWsMaxllRun, total, &dev))) return st;
+  if (two && c->two_float_off) {
+    *fallback = true;
+    return GWGPU_OK;
+  }
   char *b = (char *)dev;
   double2 *g64 = (double2 *)(b + o_g);
   float2 *a32 = (float2 *)(b + o_a);
@@ -1359,7 +1364,7 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
   }
   int *dst = (int *)(b + o_st);
   cudaError_t e;
-  for (bool search = true;; search = false) {
+  for (bool search = true;;) {
     e = gwk::launch_prologue((const gwt::GenParams *)(b + o_p), (const int *)(b + o_a), n, (const int *)(b + o_h),
                              ndet, 0.0, 0, c->streams_dev, c->qnm_dev, two ? nullptr : (Request *)(b + o_req), nullptr,
                              0, dst, c->stream, gwk::OrderArgs(), two ? (gwt::AccReq *)(b + o_req) : nullptr);
@@ -1383,6 +1388,7 @@ int gwgpu_maximized_loglik_batch(gwgpu_context *c, const gwgpu_gen_params *param
     bool searched = true;
     if ((st = maxll_run(c, in, (double *)(b + o_out), dst, &searched))) return st;
     if (searched) break;
+    search = search && c->two_float_off;  // no search yet where the two-float arrays gave way
     two = false;
   }
   drain.s = nullptr;

@@ -92,6 +92,7 @@ int gwgpu_mcmc_likelihood_extrinsic_noalloc(gwgpu_context *c, const gwgpu_gen_pa
   gwt::FastX fx;
   gwt::fast_request(r, fx, gp, ap, dets, ndet, c->qnm_host.data());
   if (r.m.status) return GWGPU_EDOMAIN;  // nothing is launched; d_loglik is left as it was
+  c->hold_if_capturing((cudaStream_t)stream);
   cudaError_t e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, scratch,
                                         (unsigned *)(scratch + kNoAllocPartials), d_loglik, (cudaStream_t)stream);
   return e == cudaSuccess ? GWGPU_OK : GWGPU_ECUDA;

@@ -56,7 +56,10 @@ def test_registration_that_fails(prec):
                 v, st = call()
                 assert np.all(st == 0)
                 out.append(v)
-            assert all(np.array_equal(v, out[0]) for v in out)
+            if failed or not budget:
+                assert all(np.array_equal(v, out[0]) for v in out)
+            else:  # the longer grid may have taken the place of the two-float arrays
+                assert all(np.all(np.abs(v - out[0]) <= 1e-9 * np.maximum(1.0, np.abs(out[0]))) for v in out)
             return held, after - held, failed
         finally:
             ctx.close()
