@@ -255,7 +255,12 @@ __global__ void k_maxll_reduce(const double2 *__restrict__ G, const double *__re
 
 // ======================================================= FP32 search path
 constexpr int kCand = 32;              // candidates per pair
-constexpr double kTau = 4e-5;          // FP32 transform error / (||a||_2 * kscale), with a 4x margin
+// FP32 transform error / (||a||_2 * kscale), for each entry and so for the norm.  The
+// library's transforms: with a 4x margin.  conv.cu, by its operations in units of
+// 2^-24: 7 for a butterfly of 16, 3 for a twiddle, so 21 for a length of 512; four
+// of those, the two steps between them and the spectrum 94 at the longest rows, the
+// chirp and its product 10: 6.3e-6, a margin of six.
+constexpr double kTau = 4e-5;
 constexpr int kMaxTwiddleRows = 12288; // shared twiddle table of the refinement: N <= 256 * this
 
 // e^{-i pi m^2 / N} in FP32 (phase reduced exactly in integers).
@@ -591,11 +596,14 @@ __global__ void __launch_bounds__(kCandBlock) k_mx_cand(const float2 *__restrict
 }
 
 // Fewer candidates for the refinement (two-float rows): the direct sum of each in
-// FP32, four at a time so that a row is read once for them.  Sums of 16 products
-// (FP32 twiddles, within 2^-22) join a two-float total, so each |G_k| is off by at
-// most 32 2^-24 ||g||_1 <= 32 2^-24 sqrt(N) ||g||_2 -- a few percent of the
-// transform's bound -- and the same interval test leaves those that may still be
-// the maximum.  One block per pair; pairs with one candidate have nothing to do.
+// FP32, four at a time so that a row is read once for them, groups of 16 products
+// joining a two-float total.  Bounds of a part's error in units of 2^-24 ||g||_1:
+// the 32 roundings of a group 32, its twiddles (within 2^-22 in each part) 4
+// sqrt(2) = 5.7, the rows' and the total's low words 1.4 each, the last product's
+// roundings 2 and twiddle 5.7: 48.2, and |G_k| is off by at most sqrt(2) times
+// that.  So 72 2^-24 sqrt(N) ||g||_2 holds every |G_k|'s error -- a tenth of the
+// transform's bound at most -- and the same interval test leaves those that may
+// still be the maximum.  One block per pair; pairs with one candidate have nothing to do.
 constexpr int kScreen = 4, kScreenBlock = 1024;
 template <bool UN>
 __global__ void __launch_bounds__(kScreenBlock, 1) k_mx_screen(const gwt::ff4 *__restrict__ rows,
@@ -623,7 +631,7 @@ __global__ void __launch_bounds__(kScreenBlock, 1) k_mx_screen(const gwt::ff4 *_
     return make_float2(c, -s);
   };
   const double *sm = sums + (size_t)q * NS;
-  const double unit = 32.0 / 16777216.0 * sqrt((double)N);
+  const double unit = 72.0 / 16777216.0 * sqrt((double)N);
   for (int c0 = 0; c0 < nc; c0 += kScreen) {
     const int mc = min(kScreen, nc - c0);
     __syncthreads();
