@@ -329,9 +329,8 @@ bool plain_two_float(const Request &r, const StreamDev *streams, int ndet, const
 }
 cudaError_t launch_plain_any(const Request &r, const FastX &fx, const StreamDev *streams, int ndet,
                              const AccTables &tab, const AccLut *lut, double *partials, unsigned *counter, double *out,
-                             cudaStream_t s, const PlainTab *fp64) {
-  if (!plain_two_float(r, streams, ndet, tab, lut))
-    return launch_plain(r, streams, ndet, partials, counter, out, nullptr, s, fp64);
+                             cudaStream_t s) {
+  if (!plain_two_float(r, streams, ndet, tab, lut)) return launch_plain(r, streams, ndet, partials, counter, out, nullptr, s);
   double ds[kMaxDet], ws[kMaxDet];
   unsigned long long wk[kMaxDet];
   for (int d = 0; d < ndet; d++) {

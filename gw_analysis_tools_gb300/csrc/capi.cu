@@ -413,13 +413,9 @@ size_t gwgpu_context_bytes_in_use(gwgpu_context *c) { return c ? c->in_use : 0; 
 // The two-float pairs of a registered stream with finite weights on a grid of n
 // dfq (FP64 form, phenom_acc.h), in 28 bytes per bin at p.  Without the memory
 // for them the stream keeps the FP64 bins.
-static cudaError_t acc_stream(gwgpu_context *c, StreamDev &d, const double *freqs, size_t row, char *p) {
-  // f_k = (n0 + k) dfq to the last bit when the product is exact (dfq with 24
-  // zero bits at its end) and equal; a grid that is not carries its distances
-  int ex;
-  const double mant = std::ldexp(std::frexp(d.dfq, &ex), 29);
-  bool exact = mant == std::floor(mant);
-  for (int k = 0; k < d.N && exact; k++) exact = (double)(d.n0 + k) * d.dfq == freqs[k];
+// exact: every f_k is (n0 + k) dfq to the last bit; a grid that is not carries its
+// distances.
+static cudaError_t acc_stream(gwgpu_context *c, StreamDev &d, bool exact, size_t row, char *p) {
   d.wd = (const gwt::ff4 *)p;
   d.wf = (const gwt::ff *)(d.wd + row);
   d.dev = exact ? nullptr : (const float *)(d.wf + row);
@@ -455,27 +451,6 @@ static cudaError_t acc_nodes(gwgpu_context *c, StreamDev &d, size_t row, char *p
   return e;
 }
 
-// Whether FP32's exponents hold the pairs W / wscale and W d / dscale and what
-// the bins make of them to their 48 bits.  A term of the sums is the pair times
-// the amplitude's square, about x^(-7/3), or x^(-7/6), at bin x; its digits stay
-// normal numbers down to 2^-78, taken as 2^-72.  Every weight that is not zero
-// has to be within that of the largest: a PSD filled with 1e-100 beyond the band
-// would else push every live bin's weight to zero (a PSD of infinity does no
-// harm).  Data may fall to nothing where a signal does, but not in more than half of their bins.
-static bool pairs_hold(const StreamDev &d, const double *freqs, const double *data, const std::vector<double> &W) {
-  const double lim = 0x1p-72, x1 = *std::max_element(freqs, freqs + d.N) / d.dfq;
-  const double w1 = lim * std::pow(x1, 7. / 3.) * d.wscale, d1 = lim * std::pow(x1, 7. / 6.) * d.dscale;
-  int some = 0, small = 0;
-  for (int k = 0; k < d.N; k++) {
-    const double w = std::fabs(W[k]);
-    if (w > 0 && w < w1 && w < lim * std::pow(freqs[k] / d.dfq, 7. / 3.) * d.wscale) return false;
-    const double m = w * (std::fabs(data[2 * k]) + std::fabs(data[2 * k + 1]));
-    some += m > 0;
-    small += m > 0 && m < d1;
-  }
-  return 2 * small <= some;
-}
-
 // One detector stream; weights (GAUSSLEG) or null (Simpson's rule).
 static int register_stream(gwgpu_context *c, const char *detector, const double *freqs, int N, const double *data,
                            const double *psd, const double *weights, int log10F, int *handle) {
@@ -502,12 +477,17 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   d.n0 = (int)std::llround(n0f);
   d.uniform_int = uniform && d.n0 >= 1 && std::fabs(n0f - d.n0) < 1e-6 && (d.n0 + (double)N) < 1.5e9;
   // the FP64 form's bins at n dfq where the frequencies are that to their rounding, else nodes
-  bool line = d.uniform_int;
+  bool line = d.uniform_int, exact = true;
   if (line) d.dfq = gwt::acc_spacing(freqs[N - 1], d.n0 + N - 1);
-  for (int k = 0; k < N && line; k++) line = gwt::acc_on_line(freqs[k], d.n0 + k, d.dfq);
-  d.line = line;
+  for (int k = 0; k < N && line; k++) {
+    const double off = gwt::acc_off_line(freqs[k], d.n0 + k, d.dfq);
+    exact = exact && off == 0;
+    line = gwt::acc_on_line(freqs[k], off);
+  }
+  if (d.uniform_int) d.uniform_int = line ? gwk::kOnLine : gwk::kUniform;
+  double fmax = freqs[N - 1];
   if (!line) {
-    double fmax = 0;
+    fmax = 0;
     for (int k = 0; k < N; k++) fmax = std::fmax(fmax, freqs[k]);
     d.dfq = fmax > 0 && std::isfinite(fmax) ? std::ldexp(1.0, std::ilogb(fmax) - 19) : 1.0;
   }
@@ -531,13 +511,31 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   }
   d.wscale = wmax > 0 ? wmax : 1.0;
   d.dscale = dmax > 0 ? dmax : 1.0;
+  // Whether FP32's exponents hold the pairs W / wscale and W d / dscale and what
+  // the two-float bins make of them to their 48 bits.  A term of the sums is the
+  // pair times the amplitude's square, about x^(-7/3), or x^(-7/6), at bin x; its
+  // digits stay normal numbers down to 2^-78, taken as 2^-72.  Every weight that is
+  // not zero has to be within that of the largest: a PSD filled with 1e-100 beyond
+  // the band would else push every live bin's weight to zero (a PSD of infinity
+  // does no harm).  Data may fall to nothing where a signal does, but not in more
+  // than half of their bins.
+  const double x1 = fmax / d.dfq, wlim = 0x1p-72 * std::pow(x1, 7. / 3.), dlim = 0x1p-72 * std::pow(x1, 7. / 6.);
+  int data_bins = 0, data_low = 0, weight_low = 0;
   std::vector<float> dh(2 * (size_t)N), wh(N);
   for (int k = 0; k < N; k++) {
-    dh[2 * k] = (float)(W[k] * data[2 * k] / d.dscale);
-    dh[2 * k + 1] = (float)(W[k] * data[2 * k + 1] / d.dscale);
-    wh[k] = (float)(W[k] / d.wscale);
+    const double re = W[k] * data[2 * k] / d.dscale, im = W[k] * data[2 * k + 1] / d.dscale, w = W[k] / d.wscale;
+    const double m = std::fabs(re) + std::fabs(im);
+    dh[2 * k] = (float)re;
+    dh[2 * k + 1] = (float)im;
+    wh[k] = (float)w;
+    data_bins += m > 0;
+    data_low += (m > 0) & (m < dlim);
+    weight_low += (w != 0) & (std::fabs(w) < wlim);
   }
-  const bool two_float = finite && pairs_hold(d, freqs, data, W);
+  bool hold = 2 * data_low <= data_bins;
+  for (int k = 0; k < N && hold && weight_low; k++)  // below the limit of the largest bin: by their own
+    hold = W[k] == 0 || std::fabs(W[k]) >= 0x1p-72 * std::pow(freqs[k] / d.dfq, 7. / 3.) * d.wscale;
+  const bool two_float = finite && hold;
   int st;
   std::vector<double> ip(N);  // the reciprocal PSD: the FP64 kernels multiply instead of dividing
   for (int k = 0; k < N; k++) ip[k] = 1.0 / psd[k];
@@ -586,7 +584,7 @@ static int register_stream(gwgpu_context *c, const char *detector, const double 
   d.dhat = (const float *)pdh;
   d.what = (const float *)pwh;
   d.iw = (const double *)piw;
-  cudaError_t e = pairs ? acc_stream(c, d, freqs, row, more) : nodes ? acc_nodes(c, d, row, more) : cudaSuccess;
+  cudaError_t e = pairs ? acc_stream(c, d, exact, row, more) : nodes ? acc_nodes(c, d, row, more) : cudaSuccess;
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     c->dfree(mem);
@@ -756,6 +754,23 @@ int gwgpu_log_likelihood_internal_weighted(gwgpu_context *c, const double *data,
   return GWGPU_OK;
 }
 
+// FP64 bins; of IMRPhenomD on grids of n dfq the waveform from the request's
+// coefficients on the grid and the power tables.
+static cudaError_t plain_fp64(gwgpu_context *c, const gwt::Request &r, const StreamDev *sd, int ndet, double *part,
+                              unsigned *cnt, double *out) {
+  gwk::PlainTab pt;
+  const int nlast = sd[0].n0 + sd[0].N - 1;
+  bool line = r.approximant == gwt::kPhenomD && !r.m.status;
+  for (int d = 0; d < ndet; d++) line = line && sd[d].uniform_int == gwk::kOnLine;
+  if (line && nlast <= c->tables.nmax && c->ensure_tm76d(nlast) == GWGPU_OK && nlast <= c->tm76d_n) {
+    gwt::wave64_prologue(r, sd[0].dfq, pt.w);
+    pt.t = c->tables;
+    pt.tm76d = c->tm76d;
+    pt.use = 1;
+  }
+  return gwk::launch_plain(r, sd, ndet, part, cnt, out, nullptr, c->stream, &pt);
+}
+
 int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p, const char *method,
                                     const int *handles, int ndet, double T_segment, double *loglik) {
   int ap = method_approx(method);
@@ -777,6 +792,7 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   gwt::Request r;
   gwt::FastX fx;
   gwt::fast_request(r, fx, gp, ap, dets, ndet, c->qnm_host.data());
+  const bool off = c->two_float_off;
   void *dev;
   int nblk = gwk::plain_blocks(sd[0].N);
   int st = c->workspace(gwgpu_context::kWsPlain, sizeof(double) * ((size_t)nblk * 2 * gwt::kMaxDet + 8), &dev);
@@ -791,22 +807,12 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *c, const gwgpu_gen_params *p,
   if (st) return st;
   cudaError_t e = cudaHostGetDevicePointer((void **)&hd, h, 0);
   if (e != cudaSuccess) return c->fail(e, "plain result mapping");
-  for (int d = 0; d < ndet; d++) sd[d] = c->get_stream(handles[d])->dev;  // an allocation may have changed them
-  // FP64 bins of IMRPhenomD on grids of n dfq: the waveform from the request's
-  // coefficients on the grid and the power tables
-  gwk::PlainTab pt;
-  const int nlast = sd[0].n0 + sd[0].N - 1;
-  if (!gwk::plain_two_float(r, sd, ndet, c->acc, c->acc_lut) && ap == gwt::kPhenomD && !r.m.status) {
-    bool line = true;
-    for (int d = 0; d < ndet; d++) line = line && sd[d].line;
-    if (line && nlast <= c->tables.nmax && c->ensure_tm76d(nlast) == GWGPU_OK && nlast <= c->tm76d_n) {
-      gwt::wave64_prologue(r, sd[0].dfq, pt.w);
-      pt.t = c->tables;
-      pt.tm76d = c->tm76d;
-      pt.use = 1;
-    }
-  }
-  e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream, &pt);
+  if (c->two_float_off != off)  // the two-float arrays gave way
+    for (int d = 0; d < ndet; d++) sd[d] = c->get_stream(handles[d])->dev;
+  if (gwk::plain_two_float(r, sd, ndet, c->acc, c->acc_lut))
+    e = gwk::launch_plain_any(r, fx, sd, ndet, c->acc, c->acc_lut, part, cnt, hd, c->stream);
+  else
+    e = plain_fp64(c, r, sd, ndet, part, cnt, hd);
   if (e != cudaSuccess) return c->fail(e, "plain launch");
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return c->fail(e, "plain");

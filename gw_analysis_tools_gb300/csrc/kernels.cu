@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(128) k_plain(const __grid_constant__ Request r
   for (int j = 0; j < 2 * NDET; j++) v[j] = 0.0;
   bool uniform = blockDim.x == 128 && (long long)gridDim.x * 128 >= N;  // one bin per thread
 #pragma unroll
-  for (int d = 0; d < NDET; d++) uniform = uniform && ps.s[d].line;
+  for (int d = 0; d < NDET; d++) uniform = uniform && ps.s[d].uniform_int == kOnLine;
   if (uniform) {
     const int k0 = blockIdx.x * 128;
     for (int e = threadIdx.x; e < NDET * kPlainRot; e += blockDim.x) {
@@ -647,7 +647,8 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
     if (coef) mx(i).status = st;
     status[i] = st;
     if (req) {
-      if (w64 && !pv2 && !st && streams[__ldcg(handles + i * ndet)].line) wave64_prologue(r, gc.df, w64[i]);
+      if (w64 && !pv2 && !st && streams[__ldcg(handles + i * ndet)].uniform_int == kOnLine)
+        wave64_prologue(r, gc.df, w64[i]);
       if (st) m.status = st;
       req[i] = r;
     }
@@ -670,7 +671,7 @@ __device__ __forceinline__ void prologue_coop_body(CoopSmem<REQ> &sm, int base, 
 // Bound by dependency waits and instruction fetch (2,450 instructions a warp, run
 // once; FP64 pipe 27 %): 512 IMRPhenomD requests 47 -> 27 us, 64 IMRPhenomPv2 100 ->
 // 43 us against stages of inlined FP64 code at 16 requests a block.
-template <int REQ, bool ACC>
+template <int REQ, bool ACC, bool W64>
 __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     const GenParams *__restrict__ params, const int *__restrict__ approx, int n, const int *__restrict__ handles,
     int ndet, double T_segment, int tc_from_segment, const StreamDev *__restrict__ streams,
@@ -691,8 +692,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32) k_prologue_coop(
     order_append(ord, kcut, live, first, slot, (kCoopWarps - 1) * (32 / REQ));
   };
   prologue_coop_body<REQ, ACC>(sm, base, threadIdx.x >> 5, threadIdx.x & 31, params, approx, n, handles,
-                               ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, w64, want_mixed, status,
-                               [] { __syncthreads(); }, head, tail);
+                               ndet, T_segment, tc_from_segment, streams, qnm, req, mreq, areq, W64 ? w64 : nullptr, want_mixed,
+                               status, [] { __syncthreads(); }, head, tail);
 }
 
 
@@ -702,12 +703,13 @@ static void launch_coop(const GenParams *params, const int *approx, int n, const
                         Request *req, MixedReq *mreq, AccReq *areq, gwt::WaveF64 *w64, int want_mixed, int *status,
                         cudaStream_t s, const OrderArgs &ord) {
   const int grid = (n + REQ - 1) / REQ, threads = kCoopWarps * 32;
-  if (areq)
-    k_prologue_coop<REQ, true><<<grid, threads, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment,
-                                                        streams, qnm, req, nullptr, areq, nullptr, 1, status, ord);
-  else
-    k_prologue_coop<REQ, false><<<grid, threads, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment,
-                                                         streams, qnm, req, mreq, nullptr, w64, want_mixed, status, ord);
+  auto run = [&](auto kern, int coef) {
+    kern<<<grid, threads, 0, s>>>(params, approx, n, handles, ndet, T_segment, tc_from_segment, streams, qnm, req, mreq,
+                                  areq, w64, coef, status, ord);
+  };
+  if (areq) run(k_prologue_coop<REQ, true, false>, 1);
+  else if (w64) run(k_prologue_coop<REQ, false, true>, want_mixed);
+  else run(k_prologue_coop<REQ, false, false>, want_mixed);
 }
 cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
@@ -926,14 +928,20 @@ __device__ __forceinline__ void mixed_item(const BatchArgs &a, const MixedReq &x
     for (int j = 0; j < kAccPerDet; j++) v[d * kAccPerDet + j] = j < NA ? acc[d * NA + j].s - acc[d * NA + j].c : 0.f;
 }
 
-// Shared buffers of one item of the fused bin kernel.
+// Shared buffers of one item of the fused bin kernel; those of the FP64 form apart.
 template <int NDET, int MIXED>
-struct BinSmem {
+struct Fp64Smem {};
+template <int NDET>
+struct Fp64Smem<NDET, 0> {
+  static constexpr int kRotPasses = kMaxTile / kBatchBlock;
+  double2 rot64[kRotPasses * NDET];  // grids of n dfq: each pass's arrival-time rotations
+  alignas(8) unsigned char w64[sizeof(gwt::WaveF64)];  // the table form's coefficients
+};
+template <int NDET, int MIXED>
+struct BinSmem : Fp64Smem<NDET, MIXED> {
   static constexpr int NV = MIXED ? NDET * kAccPerDet : 2 * NDET;
   // mixed form: segment node values and fitted phase / alpha polynomials
   static constexpr int kSegBuf = MIXED ? kMaxSegs : 1;
-  // FP64 form on grids of n dfq: each pass's arrival-time rotations
-  static constexpr int kRotPasses = MIXED ? 1 : kMaxTile / kBatchBlock;
   alignas(16) unsigned char req[MIXED ? sizeof(MixedReq) : sizeof(Request)];
   StreamDev st[NDET];
   double res[NV];
@@ -942,11 +950,9 @@ struct BinSmem {
   double node[kSegBuf * kSegEval], node_a[kSegBuf * kSegEval];
   SegPoly poly[kSegBuf], poly_a[kSegBuf];
   double coef[kSegBuf * 2 * kSegNodes];
-  double2 rot64[kRotPasses * NDET];
   // detector rotations: per segment pass (first bin) and per thread offset
   float2 rot_seg[kSegBuf * (MIXED ? NDET : 1)];
   float2 rot_off[(MIXED ? NDET : 1) * (MIXED ? kBatchBlock : 1)];
-  alignas(8) unsigned char w64[MIXED ? 8 : sizeof(gwt::WaveF64)];  // FP64 form: the table form's coefficients
 };
 
 // One item (iid, I) of a batch on the whole block: its partial sums into
@@ -958,7 +964,6 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
                                            Fin fin) {
   using BS = BinSmem<NDET, MIXED>;
   constexpr int NV = BS::NV;
-  constexpr int kRotPasses = BS::kRotPasses;
   unsigned char *s_req = sm.req;
   StreamDev *s_st = sm.st;
   double *s_res = sm.res;
@@ -967,7 +972,6 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
   double *s_node = sm.node, *s_node_a = sm.node_a;
   SegPoly *s_poly = sm.poly, *s_poly_a = sm.poly_a;
   double *s_coef = sm.coef;
-  double2 *s_rot64 = sm.rot64;
   float2 *s_rot_seg = sm.rot_seg, *s_rot_off = sm.rot_off;
   const int tid = threadIdx.x;
   // stage the request constants and its streams
@@ -1004,9 +1008,11 @@ __device__ __forceinline__ void batch_item(const BatchArgs &a, const int iid, co
     double v[NV];
 #pragma unroll
     for (int j = 0; j < NV; j++) v[j] = 0.0;
+    double2 *s_rot64 = sm.rot64;
+    constexpr int kRotPasses = BS::kRotPasses;
     bool uniform = true;
 #pragma unroll
-    for (int d = 0; d < NDET; d++) uniform = uniform && s_st[d].line;
+    for (int d = 0; d < NDET; d++) uniform = uniform && s_st[d].uniform_int == kOnLine;
     const int npass = (kend - I.k0 + kBatchBlock - 1) / kBatchBlock;
     if (uniform && npass <= kRotPasses) {  // 128 IMRPhenomD requests on 3 x 32,128 bins: 1,105 us, from frequencies 1,680
       // e^{i tau f_k} = e^{i tau f_(first bin of the pass)} e^{i tau (k - first) df}

@@ -17,11 +17,12 @@ using gwt::MixedReq;
 using gwt::Request;
 
 // One registered detector stream, as the kernels see it.
+constexpr int kUniform = 1, kOnLine = 2;  // StreamDev::uniform_int (0: neither)
 struct StreamDev {
   int det;            // detector index into the constant tables
   int N;              // bins
   int n0;             // f_k = (n0 + k) df when uniform_int
-  int uniform_int;    // 1 when the grid is uniform with f0 an integer multiple of df
+  int uniform_int;    // kUniform: the grid is uniform with f0 an integer multiple of df; kOnLine: and f_k = n dfq to its rounding
   double df;          // f[1] - f[0]
   double simpson_df;  // f[N/2] - f[N/2-1] (mcmc_gw.cpp:811)
   const double *freqs, *data, *psd;  // FP64 originals (data interleaved complex)
@@ -42,7 +43,6 @@ struct StreamDev {
   const gwt::ff *wf;
   const float *dev;
   double dfq;
-  int line;                    // 1: f_k = (n0 + k) dfq to its rounding (acc_on_line)
   const gwt::GridConst *grid;  // of df, of dfq
   const gwt::AccNodes *node;   // grids that are not n dfq: the same by node (dfq the nodes' scale), or null
 };
@@ -93,7 +93,7 @@ bool plain_two_float(const Request &r, const StreamDev *streams, int ndet, const
                      const gwt::AccLut *lut);
 cudaError_t launch_plain_any(const Request &r, const gwt::FastX &fx, const StreamDev *streams, int ndet,
                              const gwt::AccTables &tab, const gwt::AccLut *lut, double *partials, unsigned *counter, double *out,
-                             cudaStream_t s, const PlainTab *fp64 = nullptr);
+                             cudaStream_t s);
 int plain_blocks(int N);
 cudaError_t plain_acc_preload();
 cudaError_t plain_preload();  // loads the plain kernels' module (function-attribute query)
@@ -143,16 +143,16 @@ struct BatchArgs {
   int *status;      // per-request working status (device memory: the bounds flag is set atomically)
   int *status_out;  // where the finalize writes each request's status (status itself, or mapped host memory)
   gwt::Tables tables;
+  // FP64 form on two-float bins (null: FP64 bins)
+  const AccReq *areq = nullptr;
+  gwt::AccTables acc{};
+  const gwt::AccLut *lut = nullptr;
   // FP64 bins (req): IMRPhenomD's coefficients on grids of n dfq, written by the
   // prologue (null: every bin from its frequency), and the FP64 n^(-7/6) table
   // for n <= tm76d_n
   const gwt::WaveF64 *w64 = nullptr;
   const double *tm76d = nullptr;
   int tm76d_n = 0;
-  // FP64 form on two-float bins (null: FP64 bins)
-  const AccReq *areq = nullptr;
-  gwt::AccTables acc{};
-  const gwt::AccLut *lut = nullptr;
 };
 // occ: the launch shape's resident blocks per SM (mixed 3 or 4, FP64 2);
 // pdl: launched as a programmatic dependent of the kernel before it on s

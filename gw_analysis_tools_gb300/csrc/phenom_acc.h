@@ -416,7 +416,8 @@ GW_HD ff acc_amp(const AccReq &x, const B &b, ff t, ff m76, const AccLut &lut) {
 // at every frequency and joins by acc_dev_turns.  Any other grid, 1e-9 of a bin
 // off or drifting by as much, takes the node arrays, which hold f itself.
 GW_HD double acc_spacing(double f_last, int n_last) { return f_last / n_last; }
-GW_HD bool acc_on_line(double f, int n, double dfq) { return fabs(fma(-(double)n, dfq, f)) <= 0x1p-50 * f; }
+GW_HD double acc_off_line(double f, int n, double dfq) { return fma(-(double)n, dfq, f); }
+GW_HD bool acc_on_line(double f, double off) { return fabs(off) <= 0x1p-50 * f; }
 // Phase of t_c at such a bin, whose frequency lies dev Hz off n dfq: |tc dev| is
 // 1e-11 turn on a segment of 32 s, 2e-3 for a t_c counted in GPS seconds.
 GW_HD uint64_t acc_dev_turns(const AccReq &x, float dev) {

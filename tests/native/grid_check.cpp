@@ -12,7 +12,7 @@ extern "C" {
 int gwr_on_line(const double *f, int n0, int N) {
   const double dfq = acc_spacing(f[N - 1], n0 + N - 1);
   for (int k = 0; k < N; k++)
-    if (!acc_on_line(f[k], n0 + k, dfq)) return 0;
+    if (!acc_on_line(f[k], acc_off_line(f[k], n0 + k, dfq))) return 0;
   return 1;
 }
 // The rounding of a bin's frequency times t_c: error of its turns against long double.
