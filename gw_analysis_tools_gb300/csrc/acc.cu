@@ -9,8 +9,8 @@
 // IMRPhenomD requests on 3 x 32,128 bins 4,170 -> 256 us a call, 64
 // IMRPhenomPv2 requests on 2 x 32,448 bins 973 -> 103 us, the one-request call
 // on 3 x 32,128 bins 38.4 -> 22 us (Pv2, 3 x 16,224 bins: 48 -> 26 us), with
-// an error against 64-bit references of 7e-14 instead of 2e-13 (t_c's turns
-// leave no rounding behind).  512 requests on 3 x 3,000 quadrature nodes
+// an error against 80-bit references of 6e-13 instead of 9e-13 (Pv2 1e-13 instead
+// of 3e-13; rms over 6 x 48 draws: t_c's turns leave no rounding behind).  512 requests on 3 x 3,000 quadrature nodes
 // 745 -> 100 us (prologue 31): the powers of each node are tabulated
 // at registration, its linear phases 128-bit products.
 #include <cstdint>

@@ -32,7 +32,7 @@ struct Lane {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   Plan plan;
-  void *work = nullptr;  // Request/MixedReq[n], partials, counters
+  void *work = nullptr;  // AccReq, MixedReq or Request and WaveF64 [n], partials, counters
   size_t work_cap = 0;
   void *hio = nullptr, *dio = nullptr;  // staging for the host-array entry points
   size_t io_cap = 0;
@@ -51,9 +51,9 @@ struct Lane {
   struct Shape {
     std::vector<int> handles;
     int n = -1, ndet = -1, mixed = -1;
-    bool acc = false;
-  bool nodes = false;     // FP64 form: every stream has its two-float pairs
-    long long bins = 0;   // over all requests
+    bool acc = false;      // FP64 form: every stream has its two-float arrays
+    bool nodes = false;    // some of them nodes
+    long long bins = 0;    // over all requests
     uint64_t epoch = ~0ull;
   } shape;
   std::string tk;

@@ -110,7 +110,7 @@ struct OrderArgs {
   int *live = nullptr;          // per request: live items (the first ones)
   int nitems = 0, tile = 0;
 };
-// Batched: prologue (one thread per request) then the fused bin kernel.
+// Batched: the cooperative prologue (2 to 16 requests a block), then the fused bin kernel.
 cudaError_t launch_prologue(const GenParams *params, const int *approx, int n, const int *handles, int ndet,
                             double T_segment, int tc_from_segment, const StreamDev *streams, const double *qnm,
                             Request *req, MixedReq *mreq, int want_mixed, int *status, cudaStream_t s,

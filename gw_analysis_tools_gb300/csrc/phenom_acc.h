@@ -1,7 +1,7 @@
 // phenom_acc.h -- the FP64 form's bins in two-float arithmetic (host and device).
 //
-// The same quantity and grid rules as phenom_mixed.h (uniform grids, f_n = n df
-// with integer n), to FP64 accuracy: what is linear in n in the phase is exact
+// The same quantity as phenom_mixed.h, on grids of n dfq (acc_on_line) or of
+// nodes, to FP64 accuracy: what is linear in n in the phase is exact
 // 64-bit fixed-point turns, the inspiral and intermediate phase series (up to
 // 1e4 rad) stay FP64, and everything of order one -- amplitude, ringdown phase,
 // sine and cosine, projection, data products, sums -- is carried on pairs of

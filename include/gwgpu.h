@@ -35,7 +35,12 @@ extern "C" {
 /* ---- approximants and precision forms ---- */
 #define GWGPU_IMRPHENOMD 0
 #define GWGPU_IMRPHENOMPV2 1
-#define GWGPU_PREC_FP64 0   /* the reference arithmetic in FP64 on the device */
+/* GWGPU_PREC_FP64, also the plain forms: log L to 1e-9 of the reference's FP64
+ * arithmetic.  Constants, inspiral phases and final sums are FP64; amplitudes, the
+ * rest of the phase, products and short sums are pairs of FP32 numbers (48 bits,
+ * an error no larger than that of FP64 bins) on streams whose values lie within
+ * FP32's exponents, and FP64 on others. */
+#define GWGPU_PREC_FP64 0
 #define GWGPU_PREC_MIXED 1  /* FP32 amplitude/projection/products, FP64 phase, compensated sums */
 
 /* ---- Fisher parameterisations (unpack_parameters, fisher.cpp:1841-1961) ---- */
@@ -70,7 +75,10 @@ typedef struct {
 void gwgpu_default_params(gwgpu_gen_params *p);
 const char *gwgpu_status_string(int status);
 
-/* ---- context: one device, one HBM budget, device-resident data registry ---- */
+/* ---- context: one device, one HBM budget, device-resident data registry ----
+ * The budget (0: none) bounds every device allocation of the context.  A
+ * registered stream's 48-bit arrays and their tables are taken while there is room
+ * and given up, for FP64 arithmetic throughout, where another allocation needs it. */
 int gwgpu_context_create(int device, size_t hbm_budget_bytes, gwgpu_context **out);
 int gwgpu_context_destroy(gwgpu_context *ctx);
 const char *gwgpu_last_error_string(gwgpu_context *ctx);
@@ -116,7 +124,7 @@ int gwgpu_data_register_weighted(gwgpu_context *ctx, const char *detector, const
                                  int *handle);
 int gwgpu_data_release(gwgpu_context *ctx, int handle);
 
-/* ---- plain form: FP64, one request per launch (the drop-in) ---- */
+/* ---- plain form: one request per launch, precision of GWGPU_PREC_FP64 (the drop-in) ---- */
 /* Log_Likelihood_internal(std::complex<double>* data, double* psd, double* freqs,
  * double* weights, std::complex<double>* response, int length, bool log10F,
  * std::string "SIMPSONS")  (mcmc_gw.h:276, mcmc_gw.cpp:801-873). */
@@ -138,7 +146,7 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *ctx, const gwgpu_gen_params *
                                     const char *generation_method, const int *handles, int num_detectors,
                                     double T_segment, double *loglik);
 
-/* No counterpart in the reference.  The same plain FP64 likelihood for callers
+/* No counterpart in the reference.  The same plain likelihood for callers
  * that may not allocate memory while it runs (a fixed memory budget, or code
  * that must not call an allocator on this path): it allocates nothing, enqueues one launch on
  * `stream` (0: the legacy default stream) and writes log L to the device
@@ -151,7 +159,8 @@ int gwgpu_mcmc_likelihood_extrinsic(gwgpu_context *ctx, const gwgpu_gen_params *
  * that later calls belong to.  Calls share the array:
  * overlapping calls (several host threads, or work in flight on several
  * streams) race, so issue them in order on one stream.  A request outside the
- * model domain returns GWGPU_EDOMAIN without a launch. */
+ * model domain returns GWGPU_EDOMAIN without a launch.  A call captured into a
+ * graph keeps the arrays it reads allocated, under a budget too. */
 int gwgpu_mcmc_likelihood_extrinsic_noalloc(gwgpu_context *ctx, const gwgpu_gen_params *params,
                                             const char *generation_method, const int *handles,
                                             int num_detectors, double T_segment, double *d_loglik, void *stream);
@@ -179,6 +188,8 @@ int gwgpu_maximized_log_likelihood_unaligned_internal(gwgpu_context *ctx, const 
  * 10 for IMRPhenomD, 20 for IMRPhenomPv2), evaluated on the grid of the
  * request's first detector, and summed over its detectors: the aligned form
  * with r = h+ for GWGPU_IMRPHENOMD, the unaligned form for GWGPU_IMRPHENOMPV2.
+ * FP32 transforms find the lags that may hold the maximum; the values there have
+ * the precision of GWGPU_PREC_FP64.
  * One grid length for the whole batch (handles[i*num_detectors + d]).
  * status[i]: GWGPU_OK or GWGPU_EDOMAIN (loglik[i] NaN). */
 int gwgpu_maximized_loglik_batch(gwgpu_context *ctx, const gwgpu_gen_params *params, int n, int approximant,
@@ -301,9 +312,11 @@ int gwgpu_fisher_numerical(gwgpu_context *ctx, const double *frequencies, int le
 /* Batched network Fisher (MCMC_fisher_wrapper summing detectors,
  * mcmc_gw.cpp:2283-2317) for n sources over registered data: fisher[n][dim][dim]
  * and, if covariance != NULL, its FP64 inverse (gsl_cholesky_matrix_invert,
- * util.cpp:857-900).  Order 2, the moment form: FP64 waveform differences,
- * weights and Gram moment sums per bin (gwgpu_fisher_batch_ex with
- * GWGPU_FISHER_MOMENTS and GWGPU_PREC_FP64).  A source whose matrix that form
+ * util.cpp:857-900).  Order 2, the moment form: waveform differences, weights and
+ * Gram moment sums per bin (gwgpu_fisher_batch_ex with GWGPU_FISHER_MOMENTS and
+ * GWGPU_PREC_FP64), in FP64 with the inverse, which magnifies their rounding;
+ * without it in pairs of FP32 numbers (48 bits; elements within 1e-11 of
+ * sqrt(F_ii F_jj) of the FP64 sums), and FP64 for sources or streams beyond those.  A source whose matrix that form
  * cannot invert is recomputed with the FP64 reference algorithm.  status[i]:
  * GWGPU_OK, GWGPU_EDOMAIN, GWGPU_ESINGULAR (not invertible in FP64 either). */
 int gwgpu_fisher_batch(gwgpu_context *ctx, const gwgpu_gen_params *params, int n, int method, const int *handles,
@@ -342,8 +355,8 @@ int gwgpu_fisher_batch_ex(gwgpu_context *ctx, const gwgpu_gen_params *params, in
  * the given GMST), fisher_numerical("MCMC_IMRPhenomD", order 4 =
  * mcmc_deriv_order, mcmc_gw.h:45, epsilon 1e-8) summed over the detectors with
  * the first as reference, plus the prior diagonal of
- * MCMC_fisher_transformations, in the moment form with FP64 sums at order 4
- * (gwgpu_fisher_batch_ex, GWGPU_FISHER_MOMENTS).  fisher[n][11][11]; status
+ * MCMC_fisher_transformations, in the moment form at order 4 without an inverse
+ * (gwgpu_fisher_batch_ex, GWGPU_FISHER_MOMENTS and GWGPU_PREC_FP64).  fisher[n][11][11]; status
  * as above. */
 int gwgpu_mcmc_fisher_batch(gwgpu_context *ctx, const double *theta, int dim, int n, int approximant, double gmst,
                             const int *handles, int num_detectors, double *fisher, int *status);
