@@ -456,12 +456,20 @@ GW_HD void acc_twist(const AccReq &x, const B &b, const AccTables &tb, const Acc
   ff u = ff_add(ff_mul(x.us[0], ff{iw.ch, iw.cl}), ff_mul(x.us[1], t));
   u = ff_norm(ff_add(ff_add(u, acc_times(x.us[2], b, 0)), x.us[3]));
   ff cb, sb;
-  if (fabsf(u.h) < 1e9f) {
+  if (fabsf(u.h) < 1e6f) {
     sb = ff_rsqrt(ff_norm(ff_addf(ff_sqr(u), 1.0f)));
     cb = ff_norm(ff_mul(u.h < 0.0f ? ff_neg(u) : u, sb));
-  } else {  // beta below 1e-9; NaN stays NaN
-    sb = ff{f_rcp(fabsf(u.h)), 0.0f};
-    cb = ff{u.h == u.h ? 1.0f : u.h, 0.0f};
+  } else {
+    // beta below 1e-6: as the reference's half angles of cos beta = 1 / sqrt(1 + s^2)
+    // make it, whose distance from 1 is a whole number of 2^-52 there (1 + s^2
+    // rounds to 1 + j 2^-52, its root down to half of that); NaN stays NaN
+    const ff s = ff_div(ff{67108864.0f, 0.0f}, u), s2 = ff_norm(ff_sqr(s));  // 2^26 / u
+    int j = f_to_int(s2.h);
+    const float d = f_add(f_sub(s2.h, (float)j), s2.l);
+    j += d > 0.5f ? 1 : d < -0.5f ? -1 : 0;
+    const float r = (float)(j >> 1);
+    sb = ff{sqrtf(r) * 2.1073424255447017e-08f, 0.0f};  // 2 sqrt(r 2^-53)
+    cb = ff{u.h == u.h ? 1.0f : u.h, r * -2.2204460492503131e-16f};
   }
   ff ca, sa;
   ff_turns_sincos(al, lut.turn, ca, sa);

@@ -524,7 +524,21 @@ GW_HDNI void fast_pv2_frame(Source &s, ModelP &pm, const GenParams &in, const Fa
   }
   const double Jz = L0 + m1_2 * s.spin1z + m2_2 * s.spin2z;
   const double p2 = Jx * Jx + Jy * Jy, ip = p2 > 0 ? fast_rsqrt(p2) : 0.0, iJ = fast_rsqrt(p2 + Jz * Jz);
-  const double cA = p2 > 0 ? Jx * ip : 1.0, sA = -Jy * ip, cB = Jz * iJ, sB = -(p2 * ip) * iJ;
+  const double cA = p2 > 0 ? Jx * ip : 1.0, sA = -Jy * ip;
+  double cB = Jz * iJ, sB = -(p2 * ip) * iJ;
+  // Near the axis as the reference's theta_J = acos(J_z / J), which has few digits
+  // there, makes them (with J_z's bits, in its order): alpha_0 follows sB's sign
+  // alone, and J against the axis leaves theta_J = pi, whose sine is pi's rounding.
+  if (p2 == 0) {
+    cB = Jz < 0 ? -1.0 : 1.0;
+    sB = Jz < 0 ? -1.2246467991473532e-16 : 0.0;
+  } else if (p2 < 1e-10 * (Jz * Jz)) {
+    Pows pw, pp;
+    precalc_powers_PI(pp);
+    precalc_powers_ins(s.f_ref, s.M, pw);
+    const double Lr = s.M * s.M * L2PN(eta, pw.MF2third, pp.PI2third), z = Lr + m1_2 * s.spin1z + m2_2 * s.spin2z;
+    sincos(-acos(z / sqrt(p2 + z * z)), &sB, &cB);
+  }
   const double si = x.sn[3], ci = x.cn[3], sr = x.sn[4], cr = x.cn[4];
   // N = (si cos(pi/2 - phiRef), si sin(pi/2 - phiRef), ci) through A and B
   double tx = si * sr, ty = si * cr, t1 = tx * cA - ty * sA;
