@@ -62,6 +62,7 @@ __device__ __forceinline__ void acc_bins(const AccReq &x, const StreamDev *st, c
     if (nodes) {
       const int64_t f = __ldg((const long long *)st[0].freqs + k);
       if (f > x.fcut) continue;
+      acc[0].h += x.bad;  // a phase that is not a number, where a node is live
       const float2 v = __ldg((const float2 *)nodes->x + k);
       const AccNode b{k, f, __ldg((const long long *)nodes->X + k), ff{v.x, v.y}, 0};
       if constexpr (PV2) acc_bin_p<NDET>(x, b, nodes->tb, lut, wd, w, wsh, acc);
@@ -76,9 +77,9 @@ __device__ __forceinline__ void acc_bins(const AccReq &x, const StreamDev *st, c
 
 // The block's share of log L: its sums times the request's factors.  Warps
 // reduce in two floats, thread 0 adds the warps in FP64 in order.  s_red: one
-// double per warp.  Valid in thread 0.
+// double per warp.  bad: x.bad where the block has live bins.  Valid in thread 0.
 template <int NDET, bool PV2>
-__device__ __forceinline__ double acc_reduce(const AccReq &x, const ff *acc, double *s_red) {
+__device__ __forceinline__ double acc_reduce(const AccReq &x, const ff *acc, double bad, double *s_red) {
   constexpr int NA = PV2 ? kAccPerDet : 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double v = 0.0;
@@ -91,7 +92,7 @@ __device__ __forceinline__ double acc_reduce(const AccReq &x, const ff *acc, dou
     }
   if (lane == 0) s_red[warp] = v;
   __syncthreads();
-  double r = x.bad;
+  double r = bad;
   if (threadIdx.x == 0)
     for (int w = 0; w < nw; w++) r += s_red[w];
   return r;
@@ -103,18 +104,19 @@ __device__ __forceinline__ double acc_block(const AccReq &x, const StreamDev *st
                                             double *s_red) {
   // the model is zero beyond the cut
   const int kcut = nodes ? kend : min(kend, x.m.n_cut - st[0].n0 + 1);
+  const double bad = !nodes && kcut > k0 ? x.bad : 0.f;
   if (x.m.approximant == kPhenomPv2) {
     ff acc[NDET * kAccPerDet];
 #pragma unroll
     for (int j = 0; j < NDET * kAccPerDet; j++) acc[j] = ff{0.f, 0.f};
     acc_bins<NDET, true>(x, st, tb, lut, nodes, k0 + threadIdx.x, kcut, blockDim.x, acc);
-    return acc_reduce<NDET, true>(x, acc, s_red);
+    return acc_reduce<NDET, true>(x, acc, bad, s_red);
   }
   ff acc[NDET * 2];
 #pragma unroll
   for (int j = 0; j < NDET * 2; j++) acc[j] = ff{0.f, 0.f};
   acc_bins<NDET, false>(x, st, tb, lut, nodes, k0 + threadIdx.x, kcut, blockDim.x, acc);
-  return acc_reduce<NDET, false>(x, acc, s_red);
+  return acc_reduce<NDET, false>(x, acc, bad, s_red);
 }
 
 __device__ __forceinline__ void copy_words(void *dst, const void *src, int bytes) {
