@@ -419,9 +419,14 @@ GW_HD double acc_spacing(double f_last, int n_last) { return f_last / n_last; }
 GW_HD double acc_off_line(double f, int n, double dfq) { return fma(-(double)n, dfq, f); }
 GW_HD bool acc_on_line(double f, double off) { return fabs(off) <= 0x1p-50 * f; }
 // Phase of t_c at such a bin, whose frequency lies dev Hz off n dfq: |tc dev| is
-// 1e-11 turn on a segment of 32 s, 2e-3 for a t_c counted in GPS seconds.
+// 1e-11 turn on a segment of 32 s, 2e-3 for a t_c counted in GPS seconds.  In two
+// 32-bit conversions (2^-23 turn, the rest in 2^-55): one of 64 bits takes 1 % of
+// the FP64 IMRPhenomD batch.
 GW_HD uint64_t acc_dev_turns(const AccReq &x, float dev) {
-  return (uint64_t)f_to_int64(f_mul(f_mul(-x.tc, dev), 36028797018963968.0f)) << 9;  // 2^-55 turns
+  const float t = f_mul(-x.tc, dev);
+  const int hi = f_to_int(f_mul(t, 8388608.0f));
+  const int lo = f_to_int(f_mul(f_fma((float)hi, -1.0f / 8388608.0f, t), 36028797018963968.0f));
+  return ((uint64_t)(int64_t)hi << 41) + ((uint64_t)(int64_t)lo << 9);
 }
 
 // IMRPhenomD bin: acc[2 d] weighted |h|^2 (detector 0 only when the detectors

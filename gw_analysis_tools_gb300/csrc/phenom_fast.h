@@ -503,6 +503,16 @@ GW_HDNI void fast_pv2_spins(Source &s, const GenParams &in) {
   s.SP = s.chip * (m1_2 * iM2);
   s.SL = (c1 * m1_2 + c2 * m2_2) * iM2;
 }
+// The rotation by -theta_J near the axis, in the reference's order (a function of
+// its own: rarely taken, and the parts are short of instruction fetch).
+GW_HDNI void fast_pv2_near_axis(const Source &s, double p2, double &sB, double &cB) {
+  const double m1_2 = s.mass1 * s.mass1, m2_2 = s.mass2 * s.mass2;
+  Pows pw, pp;
+  precalc_powers_PI(pp);
+  precalc_powers_ins(s.f_ref, s.M, pw);
+  const double L0 = s.M * s.M * L2PN(s.eta, pw.MF2third, pp.PI2third), z = L0 + m1_2 * s.spin1z + m2_2 * s.spin2z;
+  sincos(-acos(z / sqrt(p2 + z * z)), &sB, &cB);
+}
 // The J frame (IMRPhenomP.cpp:1130-1210): rotations by -phi_J about z, -theta_J
 // about y and kappa about z, their sines and cosines from the components that
 // define the angles.  sn/cn: of the inclination [3] and phiRef [4].
@@ -533,11 +543,7 @@ GW_HDNI void fast_pv2_frame(Source &s, ModelP &pm, const GenParams &in, const Fa
     cB = Jz < 0 ? -1.0 : 1.0;
     sB = Jz < 0 ? -1.2246467991473532e-16 : 0.0;
   } else if (p2 < 1e-10 * (Jz * Jz)) {
-    Pows pw, pp;
-    precalc_powers_PI(pp);
-    precalc_powers_ins(s.f_ref, s.M, pw);
-    const double Lr = s.M * s.M * L2PN(eta, pw.MF2third, pp.PI2third), z = Lr + m1_2 * s.spin1z + m2_2 * s.spin2z;
-    sincos(-acos(z / sqrt(p2 + z * z)), &sB, &cB);
+    fast_pv2_near_axis(s, p2, sB, cB);
   }
   const double si = x.sn[3], ci = x.cn[3], sr = x.sn[4], cr = x.cn[4];
   // N = (si cos(pi/2 - phiRef), si sin(pi/2 - phiRef), ci) through A and B

@@ -45,7 +45,6 @@ TF_HD float f_rsqrt(float a) {
 TF_HD int f_bits(float a) { return __float_as_int(a); }
 TF_HD float f_from_bits(int a) { return __int_as_float(a); }
 TF_HD int f_to_int(float a) { return __float2int_rn(a); }
-TF_HD int64_t f_to_int64(float a) { return __float2ll_rn(a); }
 #else
 TF_HD float f_add(float a, float b) { return a + b; }
 TF_HD float f_sub(float a, float b) { return a - b; }
@@ -64,7 +63,6 @@ TF_HD float f_from_bits(int a) {
   return f;
 }
 TF_HD int f_to_int(float a) { return (int)std::lrintf(a); }
-TF_HD int64_t f_to_int64(float a) { return (int64_t)std::llrintf(a); }
 #endif
 
 TF_HD ff ff_split(double v) {
